@@ -47,7 +47,7 @@ class GemmParams(ctypes.Structure):
                 ("divisor", ctypes.c_float), ("alpha", ctypes.c_float), ("beta", ctypes.c_float),
                 ("act_param", ctypes.c_float * 3), ("split_k", ctypes.c_int32),
                 ("tile_n", ctypes.c_int32), ("b_constant", ctypes.c_int32), ("l2_prefetch", ctypes.c_void_p),
-                ("l2_prefetch_bytes", ctypes.c_uint64)]
+                ("l2_prefetch_bytes", ctypes.c_uint64), ("b_packed", ctypes.c_void_p), ("ctas_per_sm", ctypes.c_int32)]
 
 
 class ConvParams(ctypes.Structure):
@@ -278,7 +278,17 @@ def gemm_params(precision=GEMM_AUTO, act=ACT_NONE, divisor=1.0, alpha=1.0, beta=
 class GemmPlanInfo(ctypes.Structure):
     _fields_ = [("uses_tensor_cores", ctypes.c_int32), ("tile_n", ctypes.c_int32), ("split_k", ctypes.c_int32),
                 ("stages", ctypes.c_int32), ("b_mn_major", ctypes.c_int32), ("three_pass", ctypes.c_int32),
-                ("shared_memory_bytes", ctypes.c_uint64)]
+                ("shared_memory_bytes", ctypes.c_uint64), ("uses_packed", ctypes.c_int32)]
+
+
+def gemm_pack(b, stream=None) -> "DeviceBuffer":
+    """The packed copy of a constant right-hand side [K, N] for GemmParams.b_packed; keep it alive."""
+    L = lib()
+    L.fml_gemm_packed_bytes.restype = ctypes.c_size_t
+    n = L.fml_gemm_packed_bytes(ctypes.c_int64(b.shape[0]), ctypes.c_int64(b.shape[1]))
+    buf = DeviceBuffer(n)
+    check(L.fml_gemm_pack(_ref(b), ctypes.c_void_p(buf.ptr), ctypes.c_size_t(n), stream))
+    return buf
 
 
 def gemm_plan(a, b, c, params) -> GemmPlanInfo:

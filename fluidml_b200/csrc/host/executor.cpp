@@ -151,10 +151,10 @@ public:
 private:
   // One file per (model bytes, mode, options that shape the plan): text lines
   //   layout <tensor> <p0> <p1> ...      physical position of every logical dim
-  //   tiles <node> <tile_n> <split_k>    tuned GEMM tiles
+  //   tiles <node> <tile_n> <split_k> <CTAs per SM>    tuned GEMM tiles
   struct PlanCacheEntry {
     std::map<std::string, std::vector<size_t>> layouts;
-    std::map<std::string, std::pair<int, int>> tiles;
+    std::map<std::string, kernel::GemmTiles> tiles;
     bool Load(const std::string &path) {
       std::ifstream in(path);
       if (!in) return false;
@@ -172,9 +172,10 @@ private:
           while (ls >> v) l.push_back(v);
           layouts[name] = l;
         } else if (tag == "tiles") {
-          int tn = 0, sk = 0;
-          ls >> tn >> sk;
-          if (tn > 0 && sk > 0) tiles[name] = {tn, sk};
+          kernel::GemmTiles t;
+          ls >> t.tile_n >> t.split_k;
+          if (!(ls >> t.ctas_per_sm)) t.ctas_per_sm = 0;
+          if (t.tile_n > 0 && t.split_k > 0) tiles[name] = t;
         }
       }
       return complete;  // a truncated file (interrupted writer) is a miss
@@ -189,7 +190,7 @@ private:
           for (size_t v : kv.second) out << " " << v;
           out << "\n";
         }
-        for (const auto &kv : tiles) out << "tiles " << kv.first << " " << kv.second.first << " " << kv.second.second << "\n";
+        for (const auto &kv : tiles) out << "tiles " << kv.first << " " << kv.second.tile_n << " " << kv.second.split_k << " " << kv.second.ctas_per_sm << "\n";
         out << "end\n";
       }
       std::rename(tmp.c_str(), path.c_str());
@@ -251,7 +252,7 @@ private:
       }
       if (!cache_hit) cached = PlanCacheEntry();
     }
-    options_.gemm_tiles = std::make_shared<std::map<std::string, std::pair<int, int>>>();
+    options_.gemm_tiles = std::make_shared<std::map<std::string, kernel::GemmTiles>>();
     if (cache_hit) {
       for (const auto &r : sequence.regions) {
         auto it = cached.layouts.find(r->name);
@@ -343,6 +344,7 @@ private:
     stats_.Set("sequence", seq);
     if (program) {
       stats_.Set("weight_bytes", json::Value((double)program->weight_bytes));
+      stats_.Set("packed_weight_bytes", json::Value((double)program->packed_bytes));
       stats_.Set("interface_bytes", json::Value((double)program->io_bytes));
       stats_.Set("launches", json::Value((double)program->launches.size()));
       stats_.Set("resident_programs", json::Value((double)program->resident_programs.size()));

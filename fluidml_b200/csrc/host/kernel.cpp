@@ -553,25 +553,46 @@ public:
   std::string GetKernelName() const override { return c_.name; }
   bool StreamedConstant(const void **ptr, size_t *bytes) const override {
     if (!c_.has_const_b) return false;
+    if (c_.params.b_packed) {
+      *ptr = c_.params.b_packed;
+      *bytes = packed_bytes_;
+      return true;
+    }
     size_t n = 4;
     for (int i = 0; i < c_.const_b.rank; ++i) n *= (size_t)c_.const_b.shape[i];
     *ptr = c_.const_b.data;
     *bytes = n;
     return true;
   }
+  size_t PackedBytes(const std::vector<fml_tensor> &in, const fml_tensor &output, fml_tensor *source) const override {
+    if (!c_.has_const_b) return 0;
+    fml_tensor a, b, bias{}, res{};
+    Resolve(in, a, b, bias, res);
+    if (b.rank != 2) return 0;
+    fml_gemm_params p = c_.params;
+    p.b_packed = b.data;  // any aligned address: would the library take the packed path?
+    fml_gemm_plan_info info;
+    if (fml_gemm_plan(&a, &b, &output, &p, &info) != FML_OK || !info.uses_packed) return 0;
+    *source = b;
+    return fml_gemm_packed_bytes(b.shape[0], b.shape[1]);
+  }
+  void SetPacked(const void *packed, size_t bytes) override {
+    c_.params.b_packed = packed;
+    packed_bytes_ = bytes;
+  }
   void SetPrefetch(const void *ptr, size_t bytes) override {
     c_.params.l2_prefetch = ptr;
     c_.params.l2_prefetch_bytes = bytes;
   }
-  void PresetTiles(int tile_n, int split_k) override {
-    c_.params.tile_n = tile_n;
-    c_.params.split_k = split_k;
+  void PresetTiles(const GemmTiles &t) override {
+    c_.params.tile_n = t.tile_n;
+    c_.params.split_k = t.split_k;
+    c_.params.ctas_per_sm = t.ctas_per_sm;
     c_.autotune = false;
   }
-  bool TunedTiles(int *tile_n, int *split_k) const override {
-    if (tuned_tn_ <= 0) return false;
-    *tile_n = tuned_tn_;
-    *split_k = tuned_sk_;
+  bool TunedTiles(GemmTiles *t) const override {
+    if (tuned_.tile_n <= 0) return false;
+    *t = tuned_;
     return true;
   }
 
@@ -616,8 +637,7 @@ public:
                             &c.params, nullptr, &tuned) != FML_OK)
         throw Error(std::string(c.name) + ": " + fml_last_error());
       c.params = tuned;
-      tuned_tn_ = tuned.tile_n;
-      tuned_sk_ = tuned.split_k;
+      tuned_ = {tuned.tile_n, tuned.split_k, tuned.ctas_per_sm};
     }
     rec.Add(c.name, [=](void *s) {
       return fml_gemm(&a, &b, &output, c.has_bias ? &bias : nullptr, c.has_residual ? &res : nullptr, &c.params, s);
@@ -626,7 +646,8 @@ public:
 
 private:
   Config c_;
-  mutable int tuned_tn_ = 0, tuned_sk_ = 0;
+  size_t packed_bytes_ = 0;
+  mutable GemmTiles tuned_;
 };
 
 // conv.cpp:27-280

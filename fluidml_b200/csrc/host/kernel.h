@@ -39,6 +39,10 @@ struct Buffer {
   size_t bytes = 0;
 };
 
+struct GemmTiles {
+  int tile_n = 0, split_k = 0, ctas_per_sm = 0;
+};
+
 class Kernel {
 public:
   virtual ~Kernel() = default;
@@ -68,10 +72,18 @@ public:
     return false;
   }
   virtual void SetPrefetch(const void *ptr, size_t bytes) { (void)ptr; (void)bytes; }
-  // Tile choices that can be carried from one Compile to the next (GEMM tile_n / split_k): a
-  // preset replaces the on-device tuning; TunedTiles reports what Launch ended up using.
-  virtual void PresetTiles(int tile_n, int split_k) { (void)tile_n; (void)split_k; }
-  virtual bool TunedTiles(int *tile_n, int *split_k) const { (void)tile_n; (void)split_k; return false; }
+  // Device bytes of the packed form of its weights this kernel's launch would use (0 = none), and the
+  // call that makes it: the builder provides the memory, which lives as long as the program.
+  // `source` names the constant, so that kernels sharing one share its packed form.
+  virtual size_t PackedBytes(const std::vector<fml_tensor> &inputs, const fml_tensor &output, fml_tensor *source) const {
+    (void)inputs; (void)output; (void)source;
+    return 0;
+  }
+  virtual void SetPacked(const void *packed, size_t bytes) { (void)packed; (void)bytes; }
+  // Tile choices that can be carried from one Compile to the next (GEMM tile_n, split_k, CTAs per SM):
+  // a preset replaces the on-device tuning; TunedTiles reports what Launch ended up using.
+  virtual void PresetTiles(const GemmTiles &tiles) { (void)tiles; }
+  virtual bool TunedTiles(GemmTiles *tiles) const { (void)tiles; return false; }
   // Stage of a resident program (fml_resident_stage) that computes what this kernel's launch
   // computes on these operands, if the kernel has such a form: a constant-weight GEMM with its
   // epilogue, or the attention core.  `out_external` is left for the builder to decide.

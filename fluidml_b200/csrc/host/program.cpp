@@ -118,6 +118,7 @@ Program::~Program() {
   for (fml_resident *r : resident_programs) fml_resident_destroy(r);
   if (arena) fml_free(arena);
   if (weights) fml_free(weights);
+  if (packed) fml_free(packed);
   if (io) fml_free(io);
 }
 
@@ -202,6 +203,36 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
   for (const auto &node : sequence.nodes) {
     if (aliases.count(node->output.get())) { ++prog->aliased_nodes; continue; }
     kernels.emplace_back(node, kernel::SelectKernel(*node, resolve, ko));
+  }
+  // ---- packed weights: one blob for all kernels that have a packed form, made on the device
+  if (!options.resident) {
+    struct Packed { fml_tensor source; size_t offset, bytes; };
+    std::vector<Packed> blobs;
+    std::vector<std::pair<kernel::Kernel *, size_t>> users;
+    size_t total = 0;
+    for (const auto &kv : kernels) {
+      std::vector<fml_tensor> ins;
+      for (const auto &r : kv.first->inputs) ins.push_back(tensor_of(r));
+      fml_tensor source;
+      const size_t bytes = kv.second->PackedBytes(ins, tensor_of(kv.first->output), &source);
+      if (!bytes) continue;
+      size_t i = 0;
+      for (; i < blobs.size(); ++i)
+        if (memcmp(&blobs[i].source, &source, sizeof(source)) == 0) break;
+      if (i == blobs.size()) {
+        blobs.push_back({source, total, bytes});
+        total = AlignUp(total + bytes, 1024);
+      }
+      users.push_back({kv.second.get(), i});
+    }
+    if (total) {
+      Check(fml_malloc(&prog->packed, total), "allocating the packed weights");
+      for (const Packed &b : blobs)
+        Check(fml_gemm_pack(&b.source, (char *)prog->packed + b.offset, b.bytes, nullptr), "packing a weight");
+      Check(fml_stream_sync(nullptr), "packing the weights");
+      for (const auto &u : users) u.first->SetPacked((char *)prog->packed + blobs[u.second].offset, blobs[u.second].bytes);
+    }
+    prog->packed_bytes = total;
   }
   // Weight prefetch chain: every kernel that streams constant weights is told about the next
   // such kernel's bytes (circularly: the last one names the first, for the next pass), so
@@ -344,12 +375,12 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
     }
     if (options.gemm_tiles) {
       auto it = options.gemm_tiles->find(node->name);
-      if (it != options.gemm_tiles->end()) k->PresetTiles(it->second.first, it->second.second);
+      if (it != options.gemm_tiles->end()) k->PresetTiles(it->second);
     }
     rec.SetNode(node->name);
     k->Launch(rec, ins, out, buf);
-    int tn = 0, sk = 0;
-    if (options.gemm_tiles && k->TunedTiles(&tn, &sk)) (*options.gemm_tiles)[node->name] = {tn, sk};
+    kernel::GemmTiles tiles;
+    if (options.gemm_tiles && k->TunedTiles(&tiles)) (*options.gemm_tiles)[node->name] = tiles;
   }
   prog->launches = rec.Launches();
   for (const auto &l : prog->launches) ++prog->kernel_histogram[l.kernel];

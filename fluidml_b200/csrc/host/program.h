@@ -39,7 +39,7 @@ struct Options {
   // plan, so that compiling the same model again skips the layout search and the on-device tuning.
   std::string plan_cache;
   // node name -> (tile_n, split_k): read by the Builder as presets, filled with what it tuned
-  std::shared_ptr<std::map<std::string, std::pair<int, int>>> gemm_tiles;
+  std::shared_ptr<std::map<std::string, kernel::GemmTiles>> gemm_tiles;
 };
 
 // region -> the region whose memory it shares (itself when it owns memory).
@@ -68,8 +68,8 @@ struct IoBinding {
 struct Program {
   std::vector<kernel::Launch> launches;
   std::vector<IoBinding> inputs, outputs;
-  void *arena = nullptr, *weights = nullptr, *io = nullptr;
-  size_t arena_bytes = 0, weight_bytes = 0, io_bytes = 0;
+  void *arena = nullptr, *weights = nullptr, *packed = nullptr, *io = nullptr;  // packed: half-pair weights of the GEMMs
+  size_t arena_bytes = 0, weight_bytes = 0, packed_bytes = 0, io_bytes = 0;
   size_t aliased_nodes = 0;
   std::map<std::string, int> kernel_histogram;
   std::vector<fml_resident *> resident_programs;  // owned

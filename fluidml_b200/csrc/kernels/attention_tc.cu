@@ -75,7 +75,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   // tensor memory: scores [0, 128), P hi / lo per 32 keys [128, 384), O_blk [384, 384 + D_v)
   constexpr uint32_t kColS = 0, kColP = 128, kColO = 384;
 
-  pdl_launch_dependents();
   if (threadIdx.x == 0) {
     tma_prefetch_map(&map_q);
     tma_prefetch_map(&map_k);
@@ -94,6 +93,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Only now may the next kernel start: its CTAs must not take tensor memory that this one still has
+  // to allocate (they give theirs back after waiting for this grid, so that would never end).
+  pdl_launch_dependents();
   pdl_wait();
 
   if (warp == 0) {

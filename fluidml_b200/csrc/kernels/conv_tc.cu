@@ -172,7 +172,6 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   uint32_t tmem_cols = 32;
   while (tmem_cols < a_col0 + a_cols * (uint32_t)NS) tmem_cols <<= 1;
 
-  pdl_launch_dependents();
   if (threadIdx.x == 0) CTRACE(0);
   if (threadIdx.x == 32) {  // descriptors ready for the first loads after the dependency wait
     tma_prefetch_map(&map_x);
@@ -202,6 +201,9 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Only now may the next kernel start: its CTAs must not take tensor memory that this one still has
+  // to allocate (they give theirs back after waiting for this grid, so that would never end).
+  pdl_launch_dependents();
   pdl_wait();
   if (threadIdx.x == 0) CTRACE(1);
 

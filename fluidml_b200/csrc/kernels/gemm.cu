@@ -184,14 +184,25 @@ extern "C" void fml_gemm_default_params(fml_gemm_params *p) {
   p->act_param[2] = 0.5f;
 }
 
+namespace {
+enum class Path { kSimt, kTc, kPair };
+struct Choice {
+  Path path;
+  TcPlan tc;
+  PairPlan pair;
+};
+}  // namespace
+
 static int resolve(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
                    const fml_tensor *bias, const fml_tensor *res, const fml_gemm_params *gp,
-                   GemmProblem &p, TcPlan &plan, bool &use_tc) {
+                   GemmProblem &p, Choice &ch) {
   FML_REQUIRE(gp, FML_BAD_ARG, "fml_gemm: null params");
   int st = analyse_gemm(a, b, c, bias, res, p);
   if (st != FML_OK) return st;
-  use_tc = gp->precision != FML_GEMM_FP32 && plan_gemm_tc(p, *gp, plan);
-  FML_REQUIRE(use_tc || gp->precision == FML_GEMM_AUTO || gp->precision == FML_GEMM_FP32,
+  ch.path = Path::kSimt;
+  if (plan_gemm_pair(p, *gp, ch.pair)) ch.path = Path::kPair;
+  else if (gp->precision != FML_GEMM_FP32 && plan_gemm_tc(p, *gp, ch.tc)) ch.path = Path::kTc;
+  FML_REQUIRE(ch.path != Path::kSimt || gp->precision == FML_GEMM_AUTO || gp->precision == FML_GEMM_FP32,
               FML_MISALIGNED,
               "fml_gemm: a tensor-core precision was requested but the operands cannot be fed to "
               "TMA (need a unit-stride k or n dim, 16-byte aligned bases and row strides)");
@@ -202,13 +213,17 @@ extern "C" int fml_gemm_plan(const fml_tensor *a, const fml_tensor *b, const fml
                              const fml_gemm_params *gp, fml_gemm_plan_info *info) {
   FML_REQUIRE(info, FML_BAD_ARG, "fml_gemm_plan: null argument");
   GemmProblem p;
-  TcPlan plan;
-  bool use_tc = false;
-  int st = resolve(a, b, c, nullptr, nullptr, gp, p, plan, use_tc);
+  Choice ch;
+  int st = resolve(a, b, c, nullptr, nullptr, gp, p, ch);
   if (st != FML_OK) return st;
   memset(info, 0, sizeof(*info));
-  info->uses_tensor_cores = use_tc ? 1 : 0;
-  if (use_tc) {
+  info->uses_tensor_cores = ch.path != Path::kSimt ? 1 : 0;
+  if (ch.path == Path::kPair) {
+    info->tile_n = ch.pair.tile_n; info->split_k = ch.pair.split_k; info->stages = ch.pair.stages_b;
+    info->three_pass = 1; info->uses_packed = 1;
+    info->shared_memory_bytes = ch.pair.smem_bytes;
+  } else if (ch.path == Path::kTc) {
+    const TcPlan &plan = ch.tc;
     info->tile_n = plan.tile_n; info->split_k = plan.split_k; info->stages = plan.stages;
     info->b_mn_major = plan.b_mn_major; info->three_pass = plan.three_pass;
     info->shared_memory_bytes = plan.smem_bytes;
@@ -220,11 +235,10 @@ extern "C" int fml_gemm_uses_tensor_cores(const fml_tensor *a, const fml_tensor 
                                           const fml_tensor *c, const fml_gemm_params *gp, int *uses) {
   FML_REQUIRE(uses, FML_BAD_ARG, "fml_gemm_uses_tensor_cores: null argument");
   GemmProblem p;
-  TcPlan plan;
-  bool use_tc = false;
-  int st = resolve(a, b, c, nullptr, nullptr, gp, p, plan, use_tc);
+  Choice ch;
+  int st = resolve(a, b, c, nullptr, nullptr, gp, p, ch);
   if (st != FML_OK) return st;
-  *uses = use_tc ? 1 : 0;
+  *uses = ch.path != Path::kSimt ? 1 : 0;
   return FML_OK;
 }
 
@@ -232,9 +246,8 @@ extern "C" int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tens
                         const fml_tensor *bias, const fml_tensor *residual,
                         const fml_gemm_params *gp, void *stream) {
   GemmProblem p;
-  TcPlan plan;
-  bool use_tc = false;
-  int st = resolve(a, b, c, bias, residual, gp, p, plan, use_tc);
+  Choice ch;
+  int st = resolve(a, b, c, bias, residual, gp, p, ch);
   if (st != FML_OK) return st;
   if (p.M == 0 || p.N == 0 || p.nb0 * p.nb1 == 0) return FML_OK;
   GemmEpilogue e = make_epilogue(*gp, bias != nullptr, residual != nullptr);
@@ -245,7 +258,8 @@ extern "C" int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tens
     p.prefetch = static_cast<const char *>(gp->l2_prefetch);
     p.prefetch_bytes = gp->l2_prefetch_bytes;
   }
-  if (use_tc) return launch_gemm_tc(p, e, plan, as_stream(stream));
+  if (ch.path == Path::kPair) return launch_gemm_pair(p, e, ch.pair, gp->b_packed, as_stream(stream));
+  if (ch.path == Path::kTc) return launch_gemm_tc(p, e, ch.tc, as_stream(stream));
   if (skinny_eligible(p)) return launch_gemm_skinny(p, e, as_stream(stream));
   return launch_gemm_simt(p, e, as_stream(stream));
 }
@@ -260,21 +274,27 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
   FML_REQUIRE(gp && tuned, FML_BAD_ARG, "fml_gemm_autotune: null argument");
   *tuned = *gp;
   GemmProblem p;
-  TcPlan plan;
-  bool use_tc = false;
-  int st = resolve(a, b, c, bias, residual, gp, p, plan, use_tc);
+  Choice ch;
+  int st = resolve(a, b, c, bias, residual, gp, p, ch);
   if (st != FML_OK) return st;
-  if (!use_tc || gp->tile_n != 0 || gp->split_k != 0) return FML_OK;  // nothing to choose
+  if (ch.path == Path::kSimt || gp->tile_n != 0 || gp->split_k != 0) return FML_OK;  // nothing to choose
+  const bool pair = ch.path == Path::kPair;
   char key[256];
-  snprintf(key, sizeof(key), "%lld,%lld,%lld,%lld,%lld|%d%d|%d,%d,%d,%d|%lld,%lld", (long long)p.M, (long long)p.N,
-           (long long)p.K, (long long)p.nb0, (long long)p.nb1, plan.b_mn_major, plan.three_pass, gp->act,
-           bias != nullptr, residual != nullptr, gp->divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn);
-  static std::map<std::string, std::pair<int, int>> cache;
+  snprintf(key, sizeof(key), "%lld,%lld,%lld,%lld,%lld|%d%d%d|%d,%d,%d,%d|%lld,%lld", (long long)p.M, (long long)p.N,
+           (long long)p.K, (long long)p.nb0, (long long)p.nb1, pair, pair ? 0 : ch.tc.b_mn_major, pair ? 1 : ch.tc.three_pass,
+           gp->act, bias != nullptr, residual != nullptr, gp->divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn);
+  struct Tiles { int tile_n, split_k, ctas_per_sm; };
+  static std::map<std::string, Tiles> cache;
   static std::mutex mu;
+  auto take = [&](const Tiles &t) {
+    tuned->tile_n = t.tile_n;
+    tuned->split_k = t.split_k;
+    tuned->ctas_per_sm = t.ctas_per_sm;
+  };
   {
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
-    if (it != cache.end()) { tuned->tile_n = it->second.first; tuned->split_k = it->second.second; return FML_OK; }
+    if (it != cache.end()) { take(it->second); return FML_OK; }
   }
   cudaStream_t s = as_stream(stream);
   cudaEvent_t e0, e1;
@@ -284,36 +304,53 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
   const int tn_opts[] = {32, 48, 64, 96, 128, 192, 256};
   const int sk_opts[] = {1, 2, 4, 8};
   float best = 1e30f;
-  int best_tn = plan.tile_n, best_sk = plan.split_k;
-  std::vector<std::pair<int, int>> seen;
+  Tiles best_tiles = pair ? Tiles{ch.pair.tile_n, ch.pair.split_k, ch.pair.ctas_per_sm} : Tiles{ch.tc.tile_n, ch.tc.split_k, 0};
+  std::vector<Tiles> seen;
   for (int tn : tn_opts)
-    for (int sk : sk_opts) {
-      fml_gemm_params q = *gp;
-      q.tile_n = tn;
-      q.split_k = sk;
-      TcPlan cand;
-      if (!plan_gemm_tc(p, q, cand)) continue;
-      const std::pair<int, int> id(cand.tile_n, cand.split_k);
-      bool dup = false;
-      for (const auto &x : seen) dup = dup || x == id;
-      if (dup) continue;
-      seen.push_back(id);
-      const int reps = 6;
-      if (launch_gemm_tc(p, epi, cand, s) != FML_OK) { cudaGetLastError(); continue; }  // warm-up; skip what cannot launch
-      cudaEventRecord(e0, s);
-      bool ok = true;
-      for (int r = 0; r < reps && ok; ++r) ok = launch_gemm_tc(p, epi, cand, s) == FML_OK;
-      cudaEventRecord(e1, s);
-      if (cudaEventSynchronize(e1) != cudaSuccess || !ok) { cudaGetLastError(); continue; }
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (ms < best) { best = ms; best_tn = cand.tile_n; best_sk = cand.split_k; }
-    }
+    for (int sk : sk_opts)
+      for (int ctas = 1; ctas <= (pair ? 2 : 1); ++ctas) {
+        fml_gemm_params q = *gp;
+        q.tile_n = tn;
+        q.split_k = sk;
+        q.ctas_per_sm = ctas;
+        Choice cand;
+        if (pair ? !plan_gemm_pair(p, q, cand.pair) : !plan_gemm_tc(p, q, cand.tc)) continue;
+        const Tiles id = pair ? Tiles{cand.pair.tile_n, cand.pair.split_k, cand.pair.ctas_per_sm}
+                              : Tiles{cand.tc.tile_n, cand.tc.split_k, 0};
+        bool dup = false;
+        for (const auto &x : seen)
+          dup = dup || (x.tile_n == id.tile_n && x.split_k == id.split_k && x.ctas_per_sm == id.ctas_per_sm);
+        if (dup) continue;
+        seen.push_back(id);
+        auto launch = [&] {
+          return pair ? launch_gemm_pair(p, epi, cand.pair, gp->b_packed, s) : launch_gemm_tc(p, epi, cand.tc, s);
+        };
+        const int reps = 6;
+        if (launch() != FML_OK) { cudaGetLastError(); continue; }  // warm-up; skip what cannot launch
+        cudaEventRecord(e0, s);
+        bool ok = true;
+        for (int r = 0; r < reps && ok; ++r) ok = launch() == FML_OK;
+        cudaEventRecord(e1, s);
+        if (cudaEventSynchronize(e1) != cudaSuccess || !ok) { cudaGetLastError(); continue; }
+        float ms = 0;
+        cudaEventElapsedTime(&ms, e0, e1);
+        if (ms < best) { best = ms; best_tiles = id; }
+      }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  tuned->tile_n = best_tn;
-  tuned->split_k = best_sk;
+  take(best_tiles);
   std::lock_guard<std::mutex> lock(mu);
-  cache[key] = {best_tn, best_sk};
+  cache[key] = best_tiles;
   return FML_OK;
+}
+
+// Packed weights of the half-precision-pair kernel (gemm_pair.cu).
+extern "C" size_t fml_gemm_packed_bytes(int64_t k, int64_t n) { return k > 0 && n > 0 ? pair_packed_bytes(k, n) : 0; }
+
+extern "C" int fml_gemm_pack(const fml_tensor *b, void *packed, size_t bytes, void *stream) {
+  FML_REQUIRE(valid_tensor(b) && b->dtype == FML_F32 && b->rank == 2 && packed, FML_BAD_ARG, "fml_gemm_pack: bad argument");
+  const int64_t K = b->shape[0], N = b->shape[1];
+  FML_REQUIRE(K > 0 && N > 0 && bytes >= pair_packed_bytes(K, N), FML_BAD_ARG, "fml_gemm_pack: the destination is too small");
+  FML_REQUIRE(aligned16(packed), FML_MISALIGNED, "fml_gemm_pack: the destination must be 16-byte aligned");
+  return pair_pack((const float *)b->data, K, N, b->stride[0], b->stride[1], packed, as_stream(stream));
 }

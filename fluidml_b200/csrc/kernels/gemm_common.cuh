@@ -73,6 +73,16 @@ struct TcPlan {
 bool plan_gemm_tc(const GemmProblem &p, const fml_gemm_params &gp, TcPlan &plan);
 int launch_gemm_tc(const GemmProblem &p, const GemmEpilogue &e, const TcPlan &plan, cudaStream_t s);
 
+// half-precision-pair path with packed weights (gemm_pair.cu) ------------------------------
+struct PairPlan {
+  int tile_n, split_k, stages_a, stages_b, ctas_per_sm;
+  size_t smem_bytes;
+};
+size_t pair_packed_bytes(int64_t K, int64_t N);
+int pair_pack(const float *b, int64_t K, int64_t N, int64_t sk, int64_t sn, void *dst, cudaStream_t s);
+bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &plan);
+int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const PairPlan &plan, const void *packed, cudaStream_t s);
+
 // pipelined depthwise convolution over dense NCHW planes (conv_depthwise_tma.cu); false = not taken
 bool launch_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,
                           const fml_conv_params *p, cudaStream_t s, int *status);

@@ -1,0 +1,174 @@
+// Epilogue of the tcgen05 GEMM kernels: sums the split-K partial tiles of a cluster, applies scaling,
+// bias, activation and residual, and stores C.  Shared by gemm_tc.cu and gemm_pair.cu.
+#pragma once
+#include "gemm_common.cuh"
+#include "tc_common.cuh"
+
+namespace fml {
+
+// The activation is a template parameter of the kernel and bias / residual / scaling are
+// cheap uniform predicates inside one short loop: every CTA runs each phase of this kernel
+// once, so the cost of a phase is largely the instruction fetch of its (cold) code, and a
+// compact, straight-line epilogue matters more than a branch-free one.
+// erf by Abramowitz & Stegun 7.1.26 with the fast exponential and reciprocal: absolute error about
+// 6e-7 in fp32 arithmetic (the formula's 1.5e-7 plus the cancellation in 1 - p t exp(-x^2) near 0;
+// tests/test_erf_formula_cpu.py restates it on the host), below 1e-6 with ex2.approx's rounding,
+// i.e. a GELU value off by at most 5e-7 |v| -- far below the 3xTF32 product it is applied to.
+// The exact erff is ~45 dependent instructions per element; with one epilogue warp per scheduler
+// that was 35 us of a 134 us FFN launch at 2048 rows (4096 columns each).
+__device__ __forceinline__ float erf_fast(float x) {
+  const float ax = fabsf(x);
+  const float t = __fdividef(1.0f, fmaf(0.3275911f, ax, 1.0f));
+  float p = fmaf(1.061405429f, t, -1.453152027f);
+  p = fmaf(p, t, 1.421413741f);
+  p = fmaf(p, t, -0.284496736f);
+  p = fmaf(p, t, 0.254829592f);
+  return copysignf(fmaf(-p * t, __expf(-ax * ax), 1.0f), x);
+}
+
+template <int ACT>
+__device__ __forceinline__ float act_op(const GemmEpilogue &e, float v) {
+  if (ACT == FML_ACT_GELU_ERF) return v * (erf_fast(v * __frcp_rn(e.c0)) + e.c1) * e.c2;  // (the reciprocal is loop-invariant)
+  if (ACT == FML_ACT_RELU) return fmaxf(v, 0.0f);
+  if (ACT == FML_ACT_TANH) return tanhf(v);
+  if (ACT == FML_ACT_SIGMOID) return 1.0f / (1.0f + expf(-v));
+  if (ACT == FML_ACT_SILU) return v / (1.0f + expf(-v));
+  return v;
+}
+
+// Rows [split * 128 / S, (split + 1) * 128 / S) of the output tile: every rank of the cluster holds
+// its fp32 partial tile in `staging` (row pitch in floats), the sum runs over the ranks in rank order
+// (independent of timing), and consecutive threads take consecutive columns, so that the loads of bias
+// and residual and the stores of C are full lines.  `et` in [0, NT) numbers the calling threads.
+// COL_SCALE: column n of the accumulator is first multiplied by col_scale[n] (a power of two).
+template <int ACT, int NT, bool COL_SCALE>
+__device__ __forceinline__ void gemm_tile_epilogue(const GemmProblem &p, const GemmEpilogue &e, float *staging, int pitch,
+                                                   int BN, int tile_m, int tile_n, int split, int S, int z0, int z1, int et,
+                                                   const float *col_scale) {
+  const int rows_per = (kBM + S - 1) / S;
+  const int r0 = split * rows_per, r1 = min(kBM, r0 + rows_per);
+  const int64_t zc = (int64_t)z0 * p.c_b0 + (int64_t)z1 * p.c_b1;
+  const float *bias = p.bias ? p.bias + (int64_t)z0 * p.bias_b0 + (int64_t)z1 * p.bias_b1 : nullptr;
+  const float *res = p.res ? p.res + (int64_t)z0 * p.res_b0 + (int64_t)z1 * p.res_b1 : nullptr;
+  float *C = p.c + zc;
+  const int64_t n_base = (int64_t)tile_n * BN, m_base = (int64_t)tile_m * kBM;
+  // 16-byte path: unit column stride everywhere, every row start and the tile origin on a
+  // 16-byte boundary, no ragged column edge inside this tile
+  auto al4 = [](int64_t v) { return (v & 3) == 0; };
+  bool vec = p.c_sn == 1 && al4(p.c_sm) && al4(n_base) && n_base + BN <= p.N &&
+             ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
+  if (bias) vec = vec && (p.bias_sn == 1 || p.bias_sn == 0) && al4(p.bias_sm) &&
+                  ((reinterpret_cast<uintptr_t>(bias) & 15) == 0);
+  if (res) vec = vec && p.res_sn == 1 && al4(p.res_sm) && ((reinterpret_cast<uintptr_t>(res) & 15) == 0);
+  const bool scale = e.divisor != 1.0f || e.alpha != 1.0f || (bias && e.beta != 1.0f);
+  const float sc_div = e.divisor, sc_alpha = e.alpha, sc_beta = e.beta;
+  const uint32_t staging_addr = smem_u32(staging);
+  const int quads = BN >> 2;
+  // Thread -> (column quad, row within a pass); rows advance by a constant, so every pointer
+  // below is stepped with one add per iteration (no division, no 64-bit multiply in the loop:
+  // with one warp per scheduler every dependent instruction costs its full latency).
+  const int rows_pass = NT / quads;          // quads 4..64 -> 32..2 rows per pass
+  const int cq = et % quads, rsub = et / quads;
+  const int r_end = (int)min((int64_t)r1, p.M - m_base);  // rows that exist
+  if (vec) {
+    if (rsub < rows_pass) {
+      const int c = cq * 4;
+      const int64_t n = n_base + c;
+      int r = r0 + rsub;
+      const float *sp = staging + (size_t)r * pitch + c;
+      const int sp_step = rows_pass * pitch;
+      uint32_t rank_addr[8];
+      if (S > 1) {
+#pragma unroll
+        for (int rank = 0; rank < 8; ++rank)
+          rank_addr[rank] = rank < S ? cluster_smem_addr(staging_addr + (uint32_t)(r * pitch + c) * 4u, (uint32_t)rank) : 0u;
+      }
+      float *cp = C + (m_base + r) * p.c_sm + n;
+      const int64_t c_step = (int64_t)rows_pass * p.c_sm;
+      const float *rp = res ? res + (m_base + r) * p.res_sm + n : nullptr;
+      const int64_t r_step = (int64_t)rows_pass * p.res_sm;
+      const float *bp = bias ? bias + (m_base + r) * p.bias_sm + (p.bias_sn ? n : 0) : nullptr;
+      const int64_t b_step = (int64_t)rows_pass * p.bias_sm;
+      float4 bvec = make_float4(0.f, 0.f, 0.f, 0.f);
+      const bool bias_per_col = bias && p.bias_sm == 0 && p.bias_sn == 1;  // the usual [N] bias: load once
+      if (bias_per_col) bvec = *reinterpret_cast<const float4 *>(bp);
+      float4 cs = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (COL_SCALE) cs = *reinterpret_cast<const float4 *>(col_scale + n);
+      for (; r < r_end; r += rows_pass) {
+        float4 acc;
+        if (S == 1) {
+          acc = *reinterpret_cast<const float4 *>(sp);
+        } else {
+          float4 t[8];
+#pragma unroll
+          for (int rank = 0; rank < 8; ++rank)
+            if (rank < S)
+              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                           : "=f"(t[rank].x), "=f"(t[rank].y), "=f"(t[rank].z), "=f"(t[rank].w)
+                           : "r"(rank_addr[rank]) : "memory");
+          acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int rank = 0; rank < 8; ++rank)
+            if (rank < S) {
+              acc.x += t[rank].x; acc.y += t[rank].y; acc.z += t[rank].z; acc.w += t[rank].w;
+              rank_addr[rank] += (uint32_t)sp_step * 4u;
+            }
+        }
+        if (bias && !bias_per_col) {
+          if (p.bias_sn == 1) bvec = *reinterpret_cast<const float4 *>(bp);
+          else { const float t = *bp; bvec = make_float4(t, t, t, t); }
+        }
+        float4 rvec = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (res) rvec = *reinterpret_cast<const float4 *>(rp);
+        if (COL_SCALE) { acc.x *= cs.x; acc.y *= cs.y; acc.z *= cs.z; acc.w *= cs.w; }
+        float v[4] = {acc.x, acc.y, acc.z, acc.w};
+        const float bv[4] = {bvec.x, bvec.y, bvec.z, bvec.w}, rv[4] = {rvec.x, rvec.y, rvec.z, rvec.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float y = v[j];
+          if (scale) {
+            if (sc_div != 1.0f) y = y / sc_div;
+            y = bias ? sc_alpha * y + sc_beta * bv[j] : sc_alpha * y;
+          } else {
+            y += bv[j];
+          }
+          v[j] = act_op<ACT>(e, y) + rv[j];
+        }
+        *reinterpret_cast<float4 *>(cp) = make_float4(v[0], v[1], v[2], v[3]);
+        sp += sp_step; cp += c_step; rp += r_step; bp += b_step;
+      }
+    }
+  } else {
+    // ragged column edge or non-unit strides: one element at a time, indices recomputed
+    const int count = (r1 - r0) * quads;
+    for (int i = et; i < count; i += NT) {
+      const int rr = i / quads;
+      const int r = r0 + rr, c = (i - rr * quads) * 4;
+      const int64_t m = m_base + r;
+      if (m >= p.M) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t n = n_base + c + j;
+        if (n >= p.N) continue;
+        float acc = 0.0f;
+        const uint32_t off = staging_addr + (uint32_t)(r * pitch + c + j) * 4u;
+        if (S == 1) acc = staging[(size_t)r * pitch + c + j];
+        else
+          for (int rank = 0; rank < S; ++rank) acc += ld_cluster_f32(cluster_smem_addr(off, (uint32_t)rank));
+        if (COL_SCALE) acc *= col_scale[n];
+        const float bv = bias ? bias[m * p.bias_sm + n * p.bias_sn] : 0.0f;
+        const float rv = res ? res[m * p.res_sm + n * p.res_sn] : 0.0f;
+        float y = acc;
+        if (scale) {
+          if (sc_div != 1.0f) y = y / sc_div;
+          y = bias ? sc_alpha * y + sc_beta * bv : sc_alpha * y;
+        } else {
+          y += bv;
+        }
+        C[m * p.c_sm + n * p.c_sn] = act_op<ACT>(e, y) + rv;
+      }
+    }
+  }
+}
+
+}  // namespace fml

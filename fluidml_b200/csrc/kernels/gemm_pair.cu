@@ -1,0 +1,552 @@
+// tcgen05 GEMM for constant right-hand sides (weights) on pairs of half-precision numbers: every fp32
+// operand x is scaled by a power of two and split into hi = fp16(x), lo = fp16(x - hi), 22 significant
+// bits together, and lo*hi + hi*lo + hi*hi are accumulated in fp32 (kind::f16).  The same products as
+// the 3xTF32 kernel (gemm_tc.cu), whose truncated hi / lo carry 21 to 22 bits, but a kind::f16
+// instruction consumes 16 k values where kind::tf32 consumes 8 and both cost the same (47 clocks up to
+// N = 96, N / 2 beyond): half the tensor time.
+//
+// Range.  fp16 has 5 exponent bits, so both sides are scaled by powers of two (exact):
+//   B  per column, at packing time (fml_gemm_pack): the column's largest magnitude lands in
+//      [2^14, 2^15); elements 2^-28 below it still have all 22 bits.
+//   A  per row and k slice, on the fly: the first k block (64 values) of the row that is not all zero
+//      puts its largest magnitude into [2^3, 2^4).  Elements far below it keep an absolute error of
+//      2^-28 of that magnitude, below fp32's own rounding of the sum; 2^12 of headroom is left for
+//      larger values further along.  A row that outgrows even that overflows to infinity, which the
+//      finished accumulator shows in every column: the CTA then finds the exact row maxima and does
+//      its tile a second time with them.  Infinities and NaNs of the input come out as NaN, as in the
+//      3xTF32 kernel.
+// The powers of two are divided out again when the accumulator leaves tensor memory (rows) and in the
+// epilogue (columns).
+//
+// B is stored packed: per k block of 64, per 8 columns, the 1 KiB swizzled K-major atom of hi and the
+// one of lo side by side.  A tile's share of a k block is then one contiguous run, fetched by one
+// untiled bulk copy, and nothing of B is converted on chip.  (Bytes streamed: 4 per weight, as fp32.)
+//
+// Roles, 320 threads: warp 0 loads (A boxes of 32 floats x 128 rows by tensor map, B runs), warp 1
+// issues the MMAs, warps 2-9 convert: two sets of four warps (a warp may write the 32 TMEM lanes of its
+// index modulo 4), set h taking k values [32h, 32h + 32) of every block; thread = row.  A's fp32 stage
+// is free as soon as it is converted, the tensor-memory stage and B's stage when the MMAs are done, so
+// they form separate rings.  Epilogue, split-K over a cluster and bounded waits as in gemm_tc.cu.
+#include "gemm_epilogue.cuh"
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <algorithm>
+#include <cstdlib>
+
+namespace fml {
+namespace {
+
+constexpr int kPK = 64;                      // k values per block: 128 bytes of fp16
+constexpr int kPairA = 2 * kBM * 32 * 4;     // bytes of A per block: two boxes of 128 rows x 128 bytes
+constexpr int kPairThreads = 320;
+constexpr int kConvThreads = 256;
+
+struct PairArgs {
+  GemmProblem p;
+  GemmEpilogue e;
+  const char *packed;       // B atoms
+  const float *col_scale;   // 2^-s of each column
+  int n_pad;                // columns in the packed image (multiple of 16)
+  int tile_n, split_k, stages_a, stages_b;
+  int tiles_m, tiles_n, kb_total, kb_per_split;
+  int *status;
+};
+
+// The power of two that brings a largest magnitude m into [2^target, 2^(target + 1)), and its inverse;
+// the exponent is limited so that both are normal numbers.
+__device__ __forceinline__ void pow2_scale(float m, int target, float &s, float &inv) {
+  const int e = (int)(__float_as_uint(m) >> 23) - 127;
+  const int k = min(max(target - e, -126), 126);
+  s = __uint_as_float((uint32_t)(127 + k) << 23);
+  inv = __uint_as_float((uint32_t)(127 - k) << 23);
+}
+
+// Two fp32 values, already loaded -> (hi pair, lo pair) of x * s.
+__device__ __forceinline__ void split_pair(float x0, float x1, float s, uint32_t &hi, uint32_t &lo) {
+  const __half2 h = __floats2half2_rn(x0 * s, x1 * s);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(fmaf(x0, s, -f.x), fmaf(x1, s, -f.y));
+  hi = *reinterpret_cast<const uint32_t *>(&h);
+  lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(kPairThreads, 2)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const int BN = a.tile_n;
+  const int pitch = BN + 4;
+  const uint32_t b_bytes = (uint32_t)BN * 256u;  // hi and lo, 64 k values
+  const size_t ring_bytes = (size_t)a.stages_a * kPairA + (size_t)a.stages_b * b_bytes;
+  const size_t staging_bytes = ((size_t)kBM * pitch * 4 + 1023) / 1024 * 1024;
+  const size_t data_bytes = ring_bytes > staging_bytes ? ring_bytes : staging_bytes;
+  const uint32_t ring_a = smem_u32(smem), ring_b = ring_a + (uint32_t)a.stages_a * kPairA;
+  float *staging = reinterpret_cast<float *>(smem);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + data_bytes);
+  const uint32_t bar_full_a = smem_u32(bars), bar_empty_a = bar_full_a + 8u * a.stages_a;
+  const uint32_t bar_full_b = bar_empty_a + 8u * a.stages_a, bar_conv = bar_full_b + 8u * a.stages_b;
+  const uint32_t bar_empty_b = bar_conv + 8u * a.stages_b, bar_accum = bar_empty_b + 8u * a.stages_b;
+  const uint32_t bar_decide = bar_accum + 8u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * a.stages_a + 3 * a.stages_b + 2);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  volatile int *redo_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x, tile_m = tile % a.tiles_m, tile_n = tile / a.tiles_m;
+  const int split = blockIdx.y;
+  const int z = blockIdx.z, z0 = z % (int)a.p.nb0, z1 = z / (int)a.p.nb0;
+  const int kb0 = min(a.kb_total, split * a.kb_per_split);
+  const int kb1 = min(a.kb_total, kb0 + a.kb_per_split);
+  const int nkb = kb1 - kb0;
+  const uint32_t a_col0 = ((uint32_t)BN + 31u) & ~31u;
+  uint32_t tmem_cols = 32;
+  while (tmem_cols < a_col0 + 64u * (uint32_t)a.stages_b) tmem_cols <<= 1;
+  // the packed run of this tile in k block kb; the last tile of a ragged N stops at the image's edge
+  // (the columns it leaves unwritten in shared memory are never stored)
+  const int n_cols = min(BN, a.n_pad - tile_n * BN);
+  const uint32_t b_run = (uint32_t)n_cols * 256u;
+  const char *b_src = a.packed + ((size_t)kb0 * (a.n_pad / 8) + (size_t)tile_n * BN / 8) * 2048;
+  const size_t b_step = (size_t)(a.n_pad / 8) * 2048;
+  // Weights that one row of tiles reads cross L2 once per pass: evict-first (gemm_tc.cu).
+  const bool b_stream = a.tiles_m == 1;
+  const uint64_t b_policy = b_stream ? l2_policy_evict_first() : 0ull;
+  auto load_b = [&](int it, int s) {
+    const uint32_t dst = ring_b + (uint32_t)s * b_bytes, bar = bar_full_b + 8u * s;
+    mbar_expect_tx(bar, b_run);
+    if (b_stream) bulk_load_hint(dst, b_src + (size_t)it * b_step, b_run, bar, b_policy);
+    else bulk_load(dst, b_src + (size_t)it * b_step, b_run, bar);
+  };
+
+  if (threadIdx.x == 0) tma_prefetch_map(&map_a);
+  if (a.p.prefetch_bytes && threadIdx.x == 64) {  // the next launch's weights (gemm_tc.cu)
+    const uint64_t pf_policy = l2_policy_evict_first();
+    const unsigned long long ctas = (unsigned long long)gridDim.x * gridDim.y * gridDim.z;
+    const unsigned long long cta = blockIdx.x + (unsigned long long)gridDim.x * (blockIdx.y + (unsigned long long)gridDim.y * blockIdx.z);
+    const unsigned long long share = ((a.p.prefetch_bytes + ctas - 1) / ctas + 127ull) & ~127ull;
+    const unsigned long long lo = cta * share, hi = min(a.p.prefetch_bytes & ~15ull, lo + share);
+    for (unsigned long long off = lo; off < hi; off += 16384ull) {
+      const unsigned n = (unsigned)min(16384ull, hi - off);
+      asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;"
+                   ::"l"(a.p.prefetch + off), "r"(n), "l"(pf_policy) : "memory");
+    }
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.stages_a; ++s) {
+      mbar_init(bar_full_a + 8u * s, 1);
+      mbar_init(bar_empty_a + 8u * s, 8);  // one arrival per converter warp
+    }
+    for (int s = 0; s < a.stages_b; ++s) {
+      mbar_init(bar_full_b + 8u * s, 1);
+      mbar_init(bar_conv + 8u * s, 8);
+      mbar_init(bar_empty_b + 8u * s, 1);
+    }
+    mbar_init(bar_accum, 1);
+    mbar_init(bar_decide, 8);
+    *abort_flag = 0;
+    *redo_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), tmem_cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  // Only now may the next kernel start: its CTAs must not take tensor memory that this one still has
+  // to allocate (they give theirs back after waiting for this grid, so that would never end).
+  pdl_launch_dependents();
+  // Weights do not depend on the preceding kernel: the first stages are on their way while it drains.
+  const int pre_b = min(a.stages_b, nkb);
+  if (threadIdx.x == 0 && !g_drop_loads)
+    for (int it = 0; it < pre_b; ++it) load_b(it, it);
+  // vectors the epilogue will ask for, cold in HBM: into L2 now
+  if (warp == 2) {
+    const float *bp = a.p.bias && a.p.bias_sm == 0 && a.p.bias_sn == 1
+                          ? a.p.bias + (int64_t)z0 * a.p.bias_b0 + (int64_t)z1 * a.p.bias_b1 : nullptr;
+    for (int64_t n = (int64_t)tile_n * BN + lane * 8; n < min((int64_t)(tile_n + 1) * BN, a.p.N); n += 256) {
+      if (bp) asm volatile("prefetch.global.L2 [%0];" ::"l"(bp + n));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(a.col_scale + n));
+    }
+  }
+  pdl_wait();
+
+  float row_inv = 1.0f;  // converter threads: undoes the scale of this thread's row
+  if (warp == 0) {
+    // ------------------------------------------------------------ loads
+    if (lane == 0 && !g_drop_loads) {
+      const int ca2 = a.p.a_b0 ? z0 : 0, ca3 = a.p.a_b1 ? z1 : 0;
+      bool ok = true;
+      int issued_a = 0, issued_b = pre_b;  // counted over both attempts: ring positions go on
+      for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+        if (attempt) {
+          ok = mbar_wait(bar_decide, 0u, abort_flag);
+          if (!ok || !*redo_flag) break;
+        }
+        for (int it = 0; it < nkb && ok; ++it) {
+          const int at = attempt * nkb + it;
+          if (at >= issued_b) {
+            const int s = at % a.stages_b;
+            ok = mbar_wait(bar_empty_b + 8u * s, ((uint32_t)(at / a.stages_b) & 1u) ^ 1u, abort_flag);
+            if (!ok) break;
+            load_b(it, s);
+            issued_b = at + 1;
+          }
+          const int s = at % a.stages_a;
+          ok = mbar_wait(bar_empty_a + 8u * s, ((uint32_t)(at / a.stages_a) & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          const uint32_t dst = ring_a + (uint32_t)s * kPairA, bar = bar_full_a + 8u * s;
+          const int k = (kb0 + it) * kPK;
+          mbar_expect_tx(bar, kPairA);
+          tma_load_4d(dst, &map_a, bar, k, tile_m * kBM, ca2, ca3);
+          tma_load_4d(dst + kPairA / 2, &map_a, bar, k + 32, tile_m * kBM, ca2, ca3);
+          issued_a = at + 1;
+        }
+      }
+      if (!ok) {
+        atomicOr(a.status, kStatusTimeout);
+        *abort_flag = 1;
+        // bounded drain of the loads already in flight before the CTA may exit
+        volatile int never = 0;
+        for (int i = max(0, issued_a - a.stages_a); i < issued_a; ++i)
+          mbar_wait(bar_full_a + 8u * (i % a.stages_a), (uint32_t)(i / a.stages_a) & 1u, &never);
+        for (int i = max(0, issued_b - a.stages_b); i < issued_b; ++i)
+          mbar_wait(bar_full_b + 8u * (i % a.stages_b), (uint32_t)(i / a.stages_b) & 1u, &never);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      const uint32_t idesc = instr_desc_f16(BN);
+      const uint64_t desc_b = smem_desc(ring_b, 16u, 2048u);  // hi atoms; lo 1024 bytes further
+      bool ok = true;
+      for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+        if (attempt) {
+          ok = mbar_wait(bar_decide, 0u, abort_flag);
+          if (!ok || !*redo_flag) break;
+        }
+        for (int it = 0; it < nkb; ++it) {
+          const int at = attempt * nkb + it, s = at % a.stages_b;
+          const uint32_t ph = (uint32_t)(at / a.stages_b) & 1u;
+          ok = mbar_wait(bar_full_b + 8u * s, ph, abort_flag) && mbar_wait(bar_conv + 8u * s, ph, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t db0 = desc_b + (((uint32_t)s * b_bytes) >> 4);
+          const uint32_t ta = tmem_base + a_col0 + (uint32_t)s * 64u;
+#pragma unroll
+          for (int j = 0; j < kPK / 16; ++j) {
+            const uint32_t a_hi = ta + (uint32_t)j * 8u, a_lo = a_hi + 32u;
+            const uint64_t db = db0 + (uint32_t)j * 2u, dbl = db + (1024u >> 4);
+            umma_f16_ts(tmem_base, a_lo, db, idesc, (it == 0 && j == 0) ? 0u : 1u);
+            umma_f16_ts(tmem_base, a_hi, dbl, idesc, 1u);
+            umma_f16_ts(tmem_base, a_hi, db, idesc, 1u);
+          }
+          umma_commit(bar_empty_b + 8u * s);  // B stage and TMEM stage reusable
+        }
+        if (ok) umma_commit(bar_accum);  // with no MMA outstanding (nkb == 0) this arrives at once
+      }
+      if (!ok) {
+        atomicOr(a.status, kStatusTimeout);
+        *abort_flag = 1;
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ converter
+    const int q = warp & 3, row = q * 32 + lane, half = (warp - 2) >> 2, swz = row & 7;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    bool ok = true;
+    float s_mul = 1.0f;
+    for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+      bool scaled = false;
+      if (attempt) {
+        // exact maximum of this row over the CTA's k range, straight from global memory (rare)
+        float m = 0.0f;
+        const int64_t gm = (int64_t)tile_m * kBM + row;
+        if (gm < a.p.M) {
+          const float *src = a.p.a + (int64_t)z0 * a.p.a_b0 + (int64_t)z1 * a.p.a_b1 + gm * a.p.a_sm;
+          const int64_t k_end = min((int64_t)kb1 * kPK, a.p.K);
+          for (int64_t k = (int64_t)kb0 * kPK; k < k_end; ++k) m = fmaxf(m, fabsf(src[k]));
+        }
+        pow2_scale(m, 14, s_mul, row_inv);
+        scaled = true;
+      }
+      for (int it = 0; it < nkb && ok; ++it) {
+        const int at = attempt * nkb + it, sa = at % a.stages_a, sb = at % a.stages_b;
+        ok = mbar_wait(bar_full_a + 8u * sa, (uint32_t)(at / a.stages_a) & 1u, abort_flag);
+        if (!ok) break;
+        const uint8_t *st = smem + (size_t)sa * kPairA + row * 128;
+        const float4 *src = reinterpret_cast<const float4 *>(st + half * (kPairA / 2));
+        float4 x[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) x[c] = src[c ^ swz];
+        if (!scaled) {  // both sets look at the whole block, so they agree on the scale
+          const float4 *other = reinterpret_cast<const float4 *>(st + (half ^ 1) * (kPairA / 2));
+          float m = 0.0f;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const float4 y = other[c ^ swz];
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(x[c].x), fabsf(x[c].y)), fmaxf(fabsf(x[c].z), fabsf(x[c].w))));
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w))));
+          }
+          if (m > 0.0f) {
+            pow2_scale(m, 3, s_mul, row_inv);
+            scaled = true;
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_empty_a + 8u * sa);  // the values are in registers
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          split_pair(x[c].x, x[c].y, s_mul, hi[2 * c], lo[2 * c]);
+          split_pair(x[c].z, x[c].w, s_mul, hi[2 * c + 1], lo[2 * c + 1]);
+        }
+        // the MMAs that read this tensor-memory stage last are done
+        ok = mbar_wait(bar_empty_b + 8u * sb, ((uint32_t)(at / a.stages_b) & 1u) ^ 1u, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t t_hi = lane_addr + a_col0 + (uint32_t)sb * 64u + (uint32_t)half * 16u;
+        tmem_st16(t_hi, hi);
+        tmem_st16(t_hi + 32u, lo);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_conv + 8u * sb);
+      }
+      if (ok) ok = mbar_wait(bar_accum, (uint32_t)attempt, abort_flag);
+      if (!ok || attempt) break;
+      // A row whose hi overflowed shows it in every column of the accumulator.
+      tc_fence_after();
+      const float v0 = nkb > 0 ? tmem_ld1(lane_addr) : 0.0f;
+      tc_fence_before();
+      if (__any_sync(0xffffffffu, !(fabsf(v0) <= 3.4028235e38f)) && lane == 0) *redo_flag = 1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_decide);
+      ok = mbar_wait(bar_decide, 0u, abort_flag);
+      if (!ok || !*redo_flag) break;
+    }
+    if (!ok) {
+      atomicOr(a.status, kStatusTimeout);
+      *abort_flag = 1;
+    }
+    // Accumulator row -> staging row; the rings are free (every load has been consumed).  The two
+    // sets take alternate groups of 32 columns.
+    tc_fence_after();
+    float *dst = staging + (size_t)row * pitch;
+    for (int c0 = half * 32; c0 < BN; c0 += 64) {
+      float v[32];
+      if (ok && nkb > 0) {
+        tmem_ld32(lane_addr + (uint32_t)c0, v);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+      }
+#pragma unroll
+      for (int i = 0; i < 32; i += 4)
+        if (c0 + i < BN)
+          *reinterpret_cast<float4 *>(dst + c0 + i) =
+              make_float4(v[i] * row_inv, v[i + 1] * row_inv, v[i + 2] * row_inv, v[i + 3] * row_inv);
+    }
+  }
+
+  // ---------------------------------------------------------------- reduce + epilogue
+  tc_fence_before();
+  __syncthreads();
+  const int S = a.split_k;
+  if (S > 1) cluster_sync_all();
+  if (warp >= 2)
+    gemm_tile_epilogue<ACT, kConvThreads, true>(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1,
+                                                threadIdx.x - 64, a.col_scale);
+  if (S > 1) cluster_sync_all();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, tmem_cols);
+  }
+}
+
+// ---------------------------------------------------------------- packing
+// One block per 8 columns: the columns' largest magnitudes, then their k blocks.
+__global__ void __launch_bounds__(256) gemm_pack_kernel(const float *b, int64_t K, int64_t N, int64_t sk, int64_t sn,
+                                                        char *packed, float *col_scale, int n_pad, int kb_total) {
+  __shared__ unsigned m_bits[8];
+  const int n0 = blockIdx.x * 8;
+  if (threadIdx.x < 8) m_bits[threadIdx.x] = 0u;
+  __syncthreads();
+  const int r = threadIdx.x & 7;
+  float m = 0.0f;
+  if (n0 + r < N)
+    for (int64_t k = threadIdx.x >> 3; k < K; k += 32) m = fmaxf(m, fabsf(b[k * sk + (n0 + r) * sn]));
+  atomicMax(&m_bits[r], __float_as_uint(m));  // non-negative floats order as their bits
+  __syncthreads();
+  float s = 1.0f, inv = 1.0f;
+  if (m_bits[r]) pow2_scale(__uint_as_float(m_bits[r]), 14, s, inv);
+  if (threadIdx.x < 8) col_scale[n0 + r] = inv;
+  for (int64_t i = threadIdx.x >> 3; i < (int64_t)kb_total * 8; i += 32) {  // (k block, 16-byte chunk) of column r
+    const int64_t kb = i >> 3;
+    const int c = (int)(i & 7);
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int64_t k = kb * kPK + c * 8 + j * 2;
+      const float x0 = n0 + r < N && k < K ? b[k * sk + (n0 + r) * sn] : 0.0f;
+      const float x1 = n0 + r < N && k + 1 < K ? b[(k + 1) * sk + (n0 + r) * sn] : 0.0f;
+      split_pair(x0, x1, s, hi[j], lo[j]);
+    }
+    char *atom = packed + ((size_t)kb * (n_pad / 8) + blockIdx.x) * 2048 + r * 128 + ((c ^ r) * 16);
+    *reinterpret_cast<uint4 *>(atom) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4 *>(atom + 1024) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// ---------------------------------------------------------------- host side
+int n_padded(int64_t n) { return (int)((n + 15) / 16 * 16); }
+int k_blocks(int64_t k) { return (int)((k + kPK - 1) / kPK); }
+size_t atoms_bytes(int64_t k, int64_t n) { return (size_t)k_blocks(k) * n_padded(n) * 256; }
+
+size_t pair_smem(int tile_n, int stages_a, int stages_b) {
+  const size_t ring = (size_t)stages_a * kPairA + (size_t)stages_b * tile_n * 256;
+  const size_t staging = ((size_t)kBM * (tile_n + 4) * 4 + 1023) / 1024 * 1024;
+  return std::max(ring, staging) + (2 * stages_a + 3 * stages_b + 2) * 8 + 16 + 1024;
+}
+
+constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;
+constexpr size_t kSmemHalf = kSmemSm / 2 - 1024;  // what lets two CTAs share an SM
+
+// Ring depths for a tile width: the deepest that fits the budget and the 512 TMEM columns.
+bool pair_stages(int tile_n, int per, bool two_ctas, int *stages_a, int *stages_b, size_t *smem) {
+  const int acc = (tile_n + 31) / 32 * 32;
+  const size_t budget = two_ctas ? kSmemHalf : kSmemCta;
+  const int tmem = two_ctas ? 256 : 512;
+  int best_a = 0, best_b = 0;
+  double best = 0.0;
+  for (int sb = 1; sb <= 6 && acc + 64 * sb <= tmem; ++sb)
+    for (int sa = 1; sa <= 6; ++sa) {
+      if (pair_smem(tile_n, sa, sb) > budget) continue;
+      if (sa > per || sb > per) continue;  // no deeper than the k loop
+      // both rings count; the shallower one limits
+      const double score = std::min(sa, sb) * 8 + sa + sb;
+      if (score > best) { best = score; best_a = sa; best_b = sb; }
+    }
+  if (!best_a) return false;
+  if (two_ctas && per > 1 && std::min(best_a, best_b) < 2) return false;
+  *stages_a = best_a;
+  *stages_b = best_b;
+  size_t need = pair_smem(tile_n, best_a, best_b);
+  // no more CTAs on an SM than its 512 TMEM columns serve at once (gemm_tc.cu)
+  unsigned cols = 32;
+  while ((int)cols < acc + 64 * best_b) cols <<= 1;
+  need = std::max(need, kSmemSm / (512 / cols + 1) + 1024);
+  *smem = need;
+  return need <= kSmemCta;
+}
+
+}  // namespace
+
+size_t pair_packed_bytes(int64_t K, int64_t N) { return atoms_bytes(K, N) + (size_t)n_padded(N) * sizeof(float); }
+
+int pair_pack(const float *b, int64_t K, int64_t N, int64_t sk, int64_t sn, void *dst, cudaStream_t s) {
+  const int np = n_padded(N), kb = k_blocks(K);
+  char *packed = static_cast<char *>(dst);
+  gemm_pack_kernel<<<np / 8, 256, 0, s>>>(b, K, N, sk, sn, packed, reinterpret_cast<float *>(packed + atoms_bytes(K, N)), np, kb);
+  FML_CUDA(cudaGetLastError());
+  return FML_OK;
+}
+
+bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &plan) {
+  if (!gp.b_packed || gp.precision != FML_GEMM_AUTO) return false;
+  // A goes through a tensor map (K contiguous, 16-byte aligned rows); fewer than 32 rows stay on the
+  // weight-streaming fp32 kernel, as with the 3xTF32 kernel
+  if (p.M < 32 || p.N < 16 || p.K < 16 || p.a_sk != 1 || !aligned16(p.a) || p.a_sm <= 0 || p.a_sm % 4) return false;
+  auto stride_ok = [](int64_t s) { return s == 0 || (s > 0 && s % 4 == 0); };
+  if (!stride_ok(p.a_b0) || !stride_ok(p.a_b1) || p.b_b0 || p.b_b1) return false;
+  if (p.M > (1ll << 30) || p.N > (1ll << 24) || p.K > (1ll << 30) || p.nb0 * p.nb1 > 65535) return false;
+  if (!aligned16(gp.b_packed)) return false;
+  const int kb_total = k_blocks(p.K);
+  const int64_t tiles_m = (p.M + kBM - 1) / kBM, batch = p.nb0 * p.nb1;
+  // Default tile and split (the tuner measures the alternatives): time of a CTA = set-up and epilogue
+  // plus its k blocks at the slower of the MMAs (12 per block, 47 clocks each or N / 2) and one SM's
+  // fill path; waves of CTAs at one or two per SM.
+  const int tn_opts[] = {32, 64, 96, 128, 192, 256};
+  const int sk_opts[] = {1, 2, 4, 8};
+  double best = 1e30;
+  bool found = false;
+  for (int tn : tn_opts) {
+    if (gp.tile_n) tn = gp.tile_n;
+    tn = std::min(tn, n_padded(p.N));
+    tn = std::max(16, std::min(256, tn / 16 * 16));
+    for (int sk : sk_opts) {
+      if (gp.split_k) sk = gp.split_k;
+      if (sk > 8 || sk > kb_total) { if (gp.split_k) break; continue; }
+      const int per = (kb_total + sk - 1) / sk;
+      for (int two = 1; two >= 0; --two) {
+        if (gp.tile_n && gp.ctas_per_sm && gp.ctas_per_sm != two + 1) continue;
+        int sa, sb;
+        size_t smem;
+        if (!pair_stages(tn, per, two != 0, &sa, &sb, &smem)) continue;
+        const int64_t ctas = tiles_m * ((p.N + tn - 1) / tn) * batch * sk;
+        const int slots = (two ? 296 : 148) * (sk == 8 ? 0.87 : sk == 4 ? 0.97 : 1.0);
+        const double waves = (double)((ctas + slots - 1) / slots);
+        const double t_kb = std::max(12 * std::max(47.0, tn / 2.0) / 1.9e3, (kPairA + tn * 256.0) / 80e3);
+        const double t_fixed = 3.0 + (double)kBM * tn / sk * 4.0 / 20e3 + (sk > 1 ? 0.6 : 0.0);
+        const double t = waves * (t_fixed + per * t_kb * (two && ctas > 148 ? 2.0 : 1.0));
+        if (t < best) {
+          best = t;
+          found = true;
+          plan.tile_n = tn; plan.split_k = sk; plan.stages_a = sa; plan.stages_b = sb;
+          plan.smem_bytes = smem; plan.ctas_per_sm = two + 1;
+        }
+      }
+      if (gp.split_k) break;
+    }
+    if (gp.tile_n) break;
+  }
+  return found;
+}
+
+int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const PairPlan &plan, const void *packed, cudaStream_t s) {
+  PairArgs a;
+  a.p = p; a.e = e;
+  a.packed = static_cast<const char *>(packed);
+  a.col_scale = reinterpret_cast<const float *>(a.packed + atoms_bytes(p.K, p.N));
+  a.n_pad = n_padded(p.N);
+  a.tile_n = plan.tile_n; a.split_k = plan.split_k; a.stages_a = plan.stages_a; a.stages_b = plan.stages_b;
+  a.tiles_m = (int)((p.M + kBM - 1) / kBM);
+  a.tiles_n = (int)((p.N + plan.tile_n - 1) / plan.tile_n);
+  a.kb_total = k_blocks(p.K);
+  a.kb_per_split = (a.kb_total + plan.split_k - 1) / plan.split_k;
+  a.status = device_status_word();
+  FML_REQUIRE(a.status, FML_CUDA_ERROR, "fml_gemm: no device status word");
+  CUtensorMap map_a;
+  int st = make_gemm_map(&map_a, p.a, p.K, p.M, p.a_sm, p.nb0, p.a_b0, p.nb1, p.a_b1, 32, kBM, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (st != FML_OK) return st;
+  using KernelFn = void (*)(const CUtensorMap, const PairArgs);
+  static const KernelFn kernels[6] = {gemm_pair_kernel<FML_ACT_NONE>, gemm_pair_kernel<FML_ACT_GELU_ERF>, gemm_pair_kernel<FML_ACT_RELU>,
+                                      gemm_pair_kernel<FML_ACT_TANH>, gemm_pair_kernel<FML_ACT_SIGMOID>, gemm_pair_kernel<FML_ACT_SILU>};
+  FML_REQUIRE(e.act >= 0 && e.act <= FML_ACT_SILU, FML_BAD_ARG, "fml_gemm: unknown activation %d", e.act);
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  FML_CUDA(cudaGetDevice(&dev));
+  if (!attr_set[dev & 63]) {
+    for (KernelFn k : kernels) FML_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCta));
+    attr_set[dev & 63] = true;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(a.tiles_m * a.tiles_n), (unsigned)plan.split_k, (unsigned)(p.nb0 * p.nb1));
+  cfg.blockDim = dim3(kPairThreads);
+  cfg.dynamicSmemBytes = plan.smem_bytes;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = (unsigned)plan.split_k;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  FML_CUDA(cudaLaunchKernelEx(&cfg, kernels[e.act], map_a, a));
+  return FML_OK;
+}
+
+}  // namespace fml

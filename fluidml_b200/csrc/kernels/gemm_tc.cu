@@ -33,8 +33,7 @@
 //
 // Each CTA loads its own tiles with plain TMA loads; nothing here is shared between CTAs
 // at load time, and nothing reads another device's memory.
-#include "gemm_common.cuh"
-#include "tc_common.cuh"
+#include "gemm_epilogue.cuh"
 #include <cuda.h>
 #include <algorithm>
 #include <cstdlib>
@@ -73,37 +72,6 @@ __device__ __forceinline__ unsigned long long gtime() {
 #else
 #define TRACE(slot) do { } while (0)
 #endif
-
-// ---------------------------------------------------------------- epilogue helpers
-// The activation is a template parameter of the kernel and bias / residual / scaling are
-// cheap uniform predicates inside one short loop: every CTA runs each phase of this kernel
-// once, so the cost of a phase is largely the instruction fetch of its (cold) code, and a
-// compact, straight-line epilogue matters more than a branch-free one.
-// erf by Abramowitz & Stegun 7.1.26 with the fast exponential and reciprocal: absolute error about
-// 6e-7 in fp32 arithmetic (the formula's 1.5e-7 plus the cancellation in 1 - p t exp(-x^2) near 0;
-// tests/test_erf_formula_cpu.py restates it on the host), below 1e-6 with ex2.approx's rounding,
-// i.e. a GELU value off by at most 5e-7 |v| -- far below the 3xTF32 product it is applied to.
-// The exact erff is ~45 dependent instructions per element; with one epilogue warp per scheduler
-// that was 35 us of a 134 us FFN launch at 2048 rows (4096 columns each).
-__device__ __forceinline__ float erf_fast(float x) {
-  const float ax = fabsf(x);
-  const float t = __fdividef(1.0f, fmaf(0.3275911f, ax, 1.0f));
-  float p = fmaf(1.061405429f, t, -1.453152027f);
-  p = fmaf(p, t, 1.421413741f);
-  p = fmaf(p, t, -0.284496736f);
-  p = fmaf(p, t, 0.254829592f);
-  return copysignf(fmaf(-p * t, __expf(-ax * ax), 1.0f), x);
-}
-
-template <int ACT>
-__device__ __forceinline__ float act_op(const GemmEpilogue &e, float v) {
-  if (ACT == FML_ACT_GELU_ERF) return v * (erf_fast(v * __frcp_rn(e.c0)) + e.c1) * e.c2;  // (the reciprocal is loop-invariant)
-  if (ACT == FML_ACT_RELU) return fmaxf(v, 0.0f);
-  if (ACT == FML_ACT_TANH) return tanhf(v);
-  if (ACT == FML_ACT_SIGMOID) return 1.0f / (1.0f + expf(-v));
-  if (ACT == FML_ACT_SILU) return v / (1.0f + expf(-v));
-  return v;
-}
 
 // ---------------------------------------------------------------- kernel
 // THREE_PASS / B_MN are compile-time so that each variant carries only its own code: the kernel
@@ -163,7 +131,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint32_t tmem_cols = 32;
   while (tmem_cols < tmem_need) tmem_cols <<= 1;
 
-  pdl_launch_dependents();  // the next kernel may start its own set-up while this one runs
   if (threadIdx.x == 0) {  // the first A load comes right after the dependency wait: have its descriptor ready
     tma_prefetch_map(&map_a);
     tma_prefetch_map(&map_b);
@@ -199,6 +166,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Only now may the next kernel start: its CTAs must not take tensor memory that this one still has
+  // to allocate (they give theirs back after waiting for this grid, so that would never end).
+  pdl_launch_dependents();
   // Barriers, TMEM and descriptors are ready.  Weights do not depend on the preceding kernel:
   // with a constant B the producer fills the B half of the first stages right away, so that
   // HBM latency overlaps the tail of that kernel; the A halves follow after the wait.
@@ -432,126 +402,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (S > 1) cluster_sync_all();  // every rank's partial tile is in its shared memory
   if (warp >= 2) {
     const int et = threadIdx.x - 64;
-    const int rows_per = (kBM + S - 1) / S;
-    const int r0 = split * rows_per, r1 = min(kBM, r0 + rows_per);
-    const int64_t zc = (int64_t)z0 * a.p.c_b0 + (int64_t)z1 * a.p.c_b1;
-    const float *bias = a.p.bias ? a.p.bias + (int64_t)z0 * a.p.bias_b0 + (int64_t)z1 * a.p.bias_b1 : nullptr;
-    const float *res = a.p.res ? a.p.res + (int64_t)z0 * a.p.res_b0 + (int64_t)z1 * a.p.res_b1 : nullptr;
-    float *C = a.p.c + zc;
-    const int64_t n_base = (int64_t)tile_n * BN, m_base = (int64_t)tile_m * kBM;
-    // 16-byte path: unit column stride everywhere, every row start and the tile origin on a
-    // 16-byte boundary, no ragged column edge inside this tile
-    auto al4 = [](int64_t v) { return (v & 3) == 0; };
-    bool vec = a.p.c_sn == 1 && al4(a.p.c_sm) && al4(n_base) && n_base + BN <= a.p.N &&
-               ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
-    if (bias) vec = vec && (a.p.bias_sn == 1 || a.p.bias_sn == 0) && al4(a.p.bias_sm) &&
-                    ((reinterpret_cast<uintptr_t>(bias) & 15) == 0);
-    if (res) vec = vec && a.p.res_sn == 1 && al4(a.p.res_sm) && ((reinterpret_cast<uintptr_t>(res) & 15) == 0);
-    const bool scale = a.e.divisor != 1.0f || a.e.alpha != 1.0f || (bias && a.e.beta != 1.0f);
-    const float sc_div = a.e.divisor, sc_alpha = a.e.alpha, sc_beta = a.e.beta;
-    const uint32_t staging_addr = smem_u32(staging);
-    const int quads = BN >> 2;
-    // Thread -> (column quad, row within a pass); rows advance by a constant, so every pointer
-    // below is stepped with one add per iteration (no division, no 64-bit multiply in the loop:
-    // with one warp per scheduler every dependent instruction costs its full latency).
-    const int rows_pass = 128 / quads;          // quads 4..64 -> 32..2 rows per pass
-    const int cq = et % quads, rsub = et / quads;
-    const int r_end = (int)min((int64_t)r1, a.p.M - m_base);  // rows that exist
-    if (vec) {
-      if (rsub < rows_pass) {
-        const int c = cq * 4;
-        const int64_t n = n_base + c;
-        int r = r0 + rsub;
-        const float *sp = staging + (size_t)r * pitch + c;
-        const int sp_step = rows_pass * pitch;
-        uint32_t rank_addr[8];
-        if (S > 1) {
-#pragma unroll
-          for (int rank = 0; rank < 8; ++rank)
-            rank_addr[rank] = rank < S ? cluster_smem_addr(staging_addr + (uint32_t)(r * pitch + c) * 4u, (uint32_t)rank) : 0u;
-        }
-        float *cp = C + (m_base + r) * a.p.c_sm + n;
-        const int64_t c_step = (int64_t)rows_pass * a.p.c_sm;
-        const float *rp = res ? res + (m_base + r) * a.p.res_sm + n : nullptr;
-        const int64_t r_step = (int64_t)rows_pass * a.p.res_sm;
-        const float *bp = bias ? bias + (m_base + r) * a.p.bias_sm + (a.p.bias_sn ? n : 0) : nullptr;
-        const int64_t b_step = (int64_t)rows_pass * a.p.bias_sm;
-        float4 bvec = make_float4(0.f, 0.f, 0.f, 0.f);
-        const bool bias_per_col = bias && a.p.bias_sm == 0 && a.p.bias_sn == 1;  // the usual [N] bias: load once
-        if (bias_per_col) bvec = *reinterpret_cast<const float4 *>(bp);
-        for (; r < r_end; r += rows_pass) {
-          float4 acc;
-          if (S == 1) {
-            acc = *reinterpret_cast<const float4 *>(sp);
-          } else {
-            float4 t[8];
-#pragma unroll
-            for (int rank = 0; rank < 8; ++rank)
-              if (rank < S)
-                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                             : "=f"(t[rank].x), "=f"(t[rank].y), "=f"(t[rank].z), "=f"(t[rank].w)
-                             : "r"(rank_addr[rank]) : "memory");
-            acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int rank = 0; rank < 8; ++rank)
-              if (rank < S) {
-                acc.x += t[rank].x; acc.y += t[rank].y; acc.z += t[rank].z; acc.w += t[rank].w;
-                rank_addr[rank] += (uint32_t)sp_step * 4u;
-              }
-          }
-          if (bias && !bias_per_col) {
-            if (a.p.bias_sn == 1) bvec = *reinterpret_cast<const float4 *>(bp);
-            else { const float t = *bp; bvec = make_float4(t, t, t, t); }
-          }
-          float4 rvec = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (res) rvec = *reinterpret_cast<const float4 *>(rp);
-          float v[4] = {acc.x, acc.y, acc.z, acc.w};
-          const float bv[4] = {bvec.x, bvec.y, bvec.z, bvec.w}, rv[4] = {rvec.x, rvec.y, rvec.z, rvec.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float y = v[j];
-            if (scale) {
-              if (sc_div != 1.0f) y = y / sc_div;
-              y = bias ? sc_alpha * y + sc_beta * bv[j] : sc_alpha * y;
-            } else {
-              y += bv[j];
-            }
-            v[j] = act_op<ACT>(a.e, y) + rv[j];
-          }
-          *reinterpret_cast<float4 *>(cp) = make_float4(v[0], v[1], v[2], v[3]);
-          sp += sp_step; cp += c_step; rp += r_step; bp += b_step;
-        }
-      }
-    } else {
-      // ragged column edge or non-unit strides: one element at a time, indices recomputed
-      const int count = (r1 - r0) * quads;
-      for (int i = et; i < count; i += 128) {
-        const int rr = i / quads;
-        const int r = r0 + rr, c = (i - rr * quads) * 4;
-        const int64_t m = m_base + r;
-        if (m >= a.p.M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int64_t n = n_base + c + j;
-          if (n >= a.p.N) continue;
-          float acc = 0.0f;
-          const uint32_t off = staging_addr + (uint32_t)(r * pitch + c + j) * 4u;
-          if (S == 1) acc = staging[(size_t)r * pitch + c + j];
-          else
-            for (int rank = 0; rank < S; ++rank) acc += ld_cluster_f32(cluster_smem_addr(off, (uint32_t)rank));
-          const float bv = bias ? bias[m * a.p.bias_sm + n * a.p.bias_sn] : 0.0f;
-          const float rv = res ? res[m * a.p.res_sm + n * a.p.res_sn] : 0.0f;
-          float y = acc;
-          if (scale) {
-            if (sc_div != 1.0f) y = y / sc_div;
-            y = bias ? sc_alpha * y + sc_beta * bv : sc_alpha * y;
-          } else {
-            y += bv;
-          }
-          C[m * a.p.c_sm + n * a.p.c_sn] = act_op<ACT>(a.e, y) + rv;
-        }
-      }
-    }
+    gemm_tile_epilogue<ACT, 128, false>(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
     if (et == 0) TRACE(5);
   }
   if (S > 1) cluster_sync_all();  // nobody leaves while a peer may still read its tile
@@ -564,27 +415,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 }
 
 // ---------------------------------------------------------------- host side
-// 4-D map: (inner contiguous dim, row dim, batch0, batch1), fp32.
-int make_map(CUtensorMap *map, const float *base, int64_t inner, int64_t rows, int64_t row_stride,
-             int64_t nb0, int64_t b0_stride, int64_t nb1, int64_t b1_stride, int box_inner,
-             int box_rows, CUtensorMapSwizzle swizzle) {
-  EncodeTiledFn fn = encode_fn();
-  FML_REQUIRE(fn, FML_CUDA_ERROR, "fml_gemm: cuTensorMapEncodeTiled is not available");
-  // extent-1 dims take any valid stride
-  const int64_t dummy = row_stride * rows;
-  cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)(b0_stride ? nb0 : 1),
-                        (cuuint64_t)(b1_stride ? nb1 : 1)};
-  cuuint64_t strides[3] = {(cuuint64_t)row_stride * 4, (cuuint64_t)(b0_stride ? b0_stride : dummy) * 4,
-                           (cuuint64_t)(b1_stride ? b1_stride : dummy) * 4};
-  cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  FML_REQUIRE(r == CUDA_SUCCESS, FML_CUDA_ERROR, "fml_gemm: cuTensorMapEncodeTiled failed (%d)", (int)r);
-  return FML_OK;
-}
-
 bool stride_ok(int64_t s) { return s == 0 || (s > 0 && s % 4 == 0); }
 
 size_t stage_bytes_for(int tile_n, int three_pass, int a_tmem) {
@@ -610,6 +440,27 @@ unsigned long long *g_trace = nullptr;
 #endif
 
 }  // namespace
+
+// 4-D map: (inner contiguous dim, row dim, batch0, batch1), fp32.
+int make_gemm_map(CUtensorMap *map, const float *base, int64_t inner, int64_t rows, int64_t row_stride,
+             int64_t nb0, int64_t b0_stride, int64_t nb1, int64_t b1_stride, int box_inner,
+             int box_rows, CUtensorMapSwizzle swizzle) {
+  EncodeTiledFn fn = encode_fn();
+  FML_REQUIRE(fn, FML_CUDA_ERROR, "fml_gemm: cuTensorMapEncodeTiled is not available");
+  // extent-1 dims take any valid stride
+  const int64_t dummy = row_stride * rows;
+  cuuint64_t dims[4] = {(cuuint64_t)inner, (cuuint64_t)rows, (cuuint64_t)(b0_stride ? nb0 : 1),
+                        (cuuint64_t)(b1_stride ? nb1 : 1)};
+  cuuint64_t strides[3] = {(cuuint64_t)row_stride * 4, (cuuint64_t)(b0_stride ? b0_stride : dummy) * 4,
+                           (cuuint64_t)(b1_stride ? b1_stride : dummy) * 4};
+  cuuint32_t box[4] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides,
+                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  FML_REQUIRE(r == CUDA_SUCCESS, FML_CUDA_ERROR, "fml_gemm: cuTensorMapEncodeTiled failed (%d)", (int)r);
+  return FML_OK;
+}
 
 bool plan_gemm_tc(const GemmProblem &p, const fml_gemm_params &gp, TcPlan &plan) {
   // A must be K-major; B either K-major or MN-major; bases and row strides 16-byte aligned.
@@ -716,14 +567,14 @@ int launch_gemm_tc(const GemmProblem &p, const GemmEpilogue &e, const TcPlan &pl
 #endif
   FML_REQUIRE(a.status, FML_CUDA_ERROR, "fml_gemm: no device status word");
   CUtensorMap map_a, map_b;
-  int st = make_map(&map_a, p.a, p.K, p.M, p.a_sm, p.nb0, p.a_b0, p.nb1, p.a_b1, kBK, kBM,
+  int st = make_gemm_map(&map_a, p.a, p.K, p.M, p.a_sm, p.nb0, p.a_b0, p.nb1, p.a_b1, kBK, kBM,
                     CU_TENSOR_MAP_SWIZZLE_128B);
   if (st != FML_OK) return st;
   if (!plan.b_mn_major)
-    st = make_map(&map_b, p.b, p.K, p.N, p.b_sn, p.nb0, p.b_b0, p.nb1, p.b_b1, kBK, plan.tile_n,
+    st = make_gemm_map(&map_b, p.b, p.K, p.N, p.b_sn, p.nb0, p.b_b0, p.nb1, p.b_b1, kBK, plan.tile_n,
                   CU_TENSOR_MAP_SWIZZLE_128B);
   else
-    st = make_map(&map_b, p.b, p.N, p.K, p.b_sk, p.nb0, p.b_b0, p.nb1, p.b_b1, 32, kBK,
+    st = make_gemm_map(&map_b, p.b, p.N, p.K, p.b_sk, p.nb0, p.b_b0, p.nb1, p.b_b1, 32, kBK,
                   CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
   if (st != FML_OK) return st;
   using KernelFn = void (*)(const CUtensorMap, const CUtensorMap, const TcArgs);

@@ -28,6 +28,10 @@ static struct WaitTestRegistrar { WaitTestRegistrar() { register_wait_test_sette
 int make_f32_tensor_map(CUtensorMap *map, const float *base, int rank, const cuuint64_t *dims,
                         const cuuint64_t *strides_bytes, const cuuint32_t *box);
 
+// 4-D fp32 map of a GEMM operand: (inner contiguous dim, row dim, batch0, batch1) (gemm_tc.cu).
+int make_gemm_map(CUtensorMap *map, const float *base, int64_t inner, int64_t rows, int64_t row_stride, int64_t nb0,
+                  int64_t b0_stride, int64_t nb1, int64_t b1_stride, int box_inner, int box_rows, CUtensorMapSwizzle swizzle);
+
 // ---------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -118,6 +122,41 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, u
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// kind::f16 with fp16 operands and the fp32 accumulator; A from tensor memory (lane = row, two
+// consecutive k values per 32-bit column, the lower k in the lower half).  K = 16 per instruction.
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// 16 consecutive 32-bit columns of this thread's TMEM lane, written from registers.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// One fp32 column of this thread's TMEM lane.
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
+  uint32_t r;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  return __uint_as_float(r);
+}
+// Untiled bulk copy global -> shared, 16-byte aligned on both sides, with an L2 eviction policy.
+__device__ __forceinline__ void bulk_load_hint(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar, uint64_t policy) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
 // 32 consecutive 32-bit columns of this thread's TMEM lane, written from registers.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t *r) {
   asm volatile(
@@ -191,7 +230,10 @@ __host__ __device__ constexpr uint32_t instr_desc(int n, int b_mn_major) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)b_mn_major << 16) |
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
 }
-
+// Instruction descriptor for kind::f16 with fp16 A and B (both K-major): fp32 accumulate, M = 128, N = n.
+__host__ __device__ constexpr uint32_t instr_desc_f16(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
+}
 
 // ---------------------------------------------------------------- host: TMA descriptor encoder
 // (fetched from the driver through the runtime, so the library links no libcuda symbol)

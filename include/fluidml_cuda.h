@@ -305,7 +305,18 @@ typedef struct fml_gemm_params {
    * bytes must stay valid and unchanged; they are only read. */
   const void *l2_prefetch;
   uint64_t l2_prefetch_bytes;
+  /* Optional: B (rank 2, constant) as fml_gemm_pack laid it out, 16-byte aligned, for products of at
+   * least 32 rows with precision AUTO: the operands are then split into pairs of half-precision
+   * numbers (22 significant bits, scaled per row and column so that no range is lost) and multiplied
+   * on the 16-bit tensor-core path at half the cost of 3xTF32.  NULL = not packed. */
+  const void *b_packed;
+  int32_t ctas_per_sm; /* tuning choice that goes with tile_n (packed B only); 0 = library    */
 } fml_gemm_params;
+
+/* Packs a constant right-hand side [K, N] (any strides) for fml_gemm_params::b_packed: about 4 bytes
+ * per element.  The bytes are read by every fml_gemm that names them and must stay unchanged. */
+size_t fml_gemm_packed_bytes(int64_t k, int64_t n);
+int fml_gemm_pack(const fml_tensor *b, void *packed, size_t bytes, void *stream);
 
 void fml_gemm_default_params(fml_gemm_params *p);
 
@@ -322,6 +333,7 @@ int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
 typedef struct fml_gemm_plan_info {
   int32_t uses_tensor_cores, tile_n, split_k, stages, b_mn_major, three_pass;
   uint64_t shared_memory_bytes;
+  int32_t uses_packed; /* 1 = the packed-weight path (fml_gemm_params::b_packed) */
 } fml_gemm_plan_info;
 int fml_gemm_plan(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
                   const fml_gemm_params *p, fml_gemm_plan_info *info);
