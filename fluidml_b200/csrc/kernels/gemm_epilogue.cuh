@@ -41,40 +41,74 @@ __device__ __forceinline__ float act_op(const GemmEpilogue &e, float v) {
 // (independent of timing), and consecutive threads take consecutive columns, so that the loads of bias
 // and residual and the stores of C are full lines.  `et` in [0, NT) numbers the calling threads.
 // COL_SCALE: column n of the accumulator is first multiplied by col_scale[n] (a power of two).
-template <int ACT, int NT, bool COL_SCALE>
-__device__ __forceinline__ void gemm_tile_epilogue(const GemmProblem &p, const GemmEpilogue &e, float *staging, int pitch,
-                                                   int BN, int tile_m, int tile_n, int split, int S, int z0, int z1, int et,
-                                                   const float *col_scale) {
-  const int rows_per = (kBM + S - 1) / S;
-  const int r0 = split * rows_per, r1 = min(kBM, r0 + rows_per);
-  const int64_t zc = (int64_t)z0 * p.c_b0 + (int64_t)z1 * p.c_b1;
-  const float *bias = p.bias ? p.bias + (int64_t)z0 * p.bias_b0 + (int64_t)z1 * p.bias_b1 : nullptr;
-  const float *res = p.res ? p.res + (int64_t)z0 * p.res_b0 + (int64_t)z1 * p.res_b1 : nullptr;
-  float *C = p.c + zc;
-  const int64_t n_base = (int64_t)tile_n * BN, m_base = (int64_t)tile_m * kBM;
-  // 16-byte path: unit column stride everywhere, every row start and the tile origin on a
-  // 16-byte boundary, no ragged column edge inside this tile
-  auto al4 = [](int64_t v) { return (v & 3) == 0; };
-  bool vec = p.c_sn == 1 && al4(p.c_sm) && al4(n_base) && n_base + BN <= p.N &&
-             ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
-  if (bias) vec = vec && (p.bias_sn == 1 || p.bias_sn == 0) && al4(p.bias_sm) &&
-                  ((reinterpret_cast<uintptr_t>(bias) & 15) == 0);
-  if (res) vec = vec && p.res_sn == 1 && al4(p.res_sm) && ((reinterpret_cast<uintptr_t>(res) & 15) == 0);
-  const bool scale = e.divisor != 1.0f || e.alpha != 1.0f || (bias && e.beta != 1.0f);
-  const float sc_div = e.divisor, sc_alpha = e.alpha, sc_beta = e.beta;
-  const uint32_t staging_addr = smem_u32(staging);
-  const int quads = BN >> 2;
-  // Thread -> (column quad, row within a pass); rows advance by a constant, so every pointer
-  // below is stepped with one add per iteration (no division, no 64-bit multiply in the loop:
-  // with one warp per scheduler every dependent instruction costs its full latency).
-  const int rows_pass = NT / quads;          // quads 4..64 -> 32..2 rows per pass
-  const int cq = et % quads, rsub = et / quads;
-  const int r_end = (int)min((int64_t)r1, p.M - m_base);  // rows that exist
-  if (vec) {
-    if (rsub < rows_pass) {
-      const int c = cq * 4;
+//
+// preload() may run while the product is still being computed (after the dependency wait): it issues
+// the loads that do not depend on it -- bias, column scales, the first row's residual -- whose L2 round
+// trip is then off the critical path of a launch that does each phase once.  Only those values stay in
+// registers; finish() works the geometry out again (kept live across the accumulator reads it spilled).
+template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
+  float4 bvec, cs, rvec;
+
+  // Where this thread works.
+  struct Where {
+    const float *bias, *res;
+    float *C;
+    int64_t n_base, m_base;
+    int rows_pass, r0, r1, r_end, r, c;
+    bool vec, bias_per_col;
+    __device__ __forceinline__ Where(const GemmProblem &p, int BN, int tile_m, int tile_n, int split, int S, int z0, int z1, int et) {
+      const int rows_per = (kBM + S - 1) / S;
+      r0 = split * rows_per;
+      r1 = min(kBM, r0 + rows_per);
+      bias = p.bias ? p.bias + (int64_t)z0 * p.bias_b0 + (int64_t)z1 * p.bias_b1 : nullptr;
+      res = p.res ? p.res + (int64_t)z0 * p.res_b0 + (int64_t)z1 * p.res_b1 : nullptr;
+      C = p.c + (int64_t)z0 * p.c_b0 + (int64_t)z1 * p.c_b1;
+      n_base = (int64_t)tile_n * BN;
+      m_base = (int64_t)tile_m * kBM;
+      r_end = (int)min((int64_t)r1, p.M - m_base);  // rows that exist
+      // 16-byte path: unit column stride everywhere, every row start and the tile origin on a
+      // 16-byte boundary, no ragged column edge inside this tile
+      auto al4 = [](int64_t v) { return (v & 3) == 0; };
+      vec = p.c_sn == 1 && al4(p.c_sm) && al4(n_base) && n_base + BN <= p.N && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
+      if (bias) vec = vec && (p.bias_sn == 1 || p.bias_sn == 0) && al4(p.bias_sm) && ((reinterpret_cast<uintptr_t>(bias) & 15) == 0);
+      if (res) vec = vec && p.res_sn == 1 && al4(p.res_sm) && ((reinterpret_cast<uintptr_t>(res) & 15) == 0);
+      bias_per_col = bias && p.bias_sm == 0 && p.bias_sn == 1;  // the usual [N] bias: loaded once
+      // Thread -> (column quad, row within a pass); rows advance by a constant, so every pointer of the
+      // loop is stepped with one add per iteration.
+      const int quads = BN >> 2, rsub = et / quads;
+      rows_pass = NT / quads;
+      c = (et - rsub * quads) * 4;
+      r = vec && rsub < rows_pass ? r0 + rsub : kBM;  // threads beyond the last full row of quads stay out
+    }
+  };
+
+  __device__ __forceinline__ void preload(const GemmProblem &p, int BN, int tile_m, int tile_n, int split, int S, int z0, int z1,
+                                          int et, const float *col_scale) {
+    bvec = rvec = make_float4(0.f, 0.f, 0.f, 0.f);
+    cs = make_float4(1.f, 1.f, 1.f, 1.f);
+    const Where w(p, BN, tile_m, tile_n, split, S, z0, z1, et);
+    if (w.r >= w.r_end) return;
+    if (w.bias_per_col) bvec = *reinterpret_cast<const float4 *>(w.bias + w.n_base + w.c);
+    if (COL_SCALE) cs = *reinterpret_cast<const float4 *>(col_scale + w.n_base + w.c);
+    if (w.res) rvec = *reinterpret_cast<const float4 *>(w.res + (w.m_base + w.r) * p.res_sm + w.n_base + w.c);
+  }
+
+  __device__ __forceinline__ void finish(const GemmProblem &p, const GemmEpilogue &e, float *staging, int pitch, int BN, int tile_m,
+                                         int tile_n, int split, int S, int z0, int z1, int et, const float *col_scale) {
+    asm volatile("" : "+r"(tile_m), "+r"(tile_n), "+r"(et));  // recompute: nothing of preload()'s geometry is kept
+    const Where w(p, BN, tile_m, tile_n, split, S, z0, z1, et);
+    const float *bias = w.bias, *res = w.res;
+    float *C = w.C;
+    const int64_t n_base = w.n_base, m_base = w.m_base;
+    const int r0 = w.r0, r1 = w.r1, r_end = w.r_end, c = w.c;
+    const bool bias_per_col = w.bias_per_col;
+    const bool scale = e.divisor != 1.0f || e.alpha != 1.0f || (bias && e.beta != 1.0f);
+    const float sc_div = e.divisor, sc_alpha = e.alpha, sc_beta = e.beta;
+    const uint32_t staging_addr = smem_u32(staging);
+    if (w.vec) {
+      const int rows_pass = w.rows_pass;
+      int r = w.r;
       const int64_t n = n_base + c;
-      int r = r0 + rsub;
       const float *sp = staging + (size_t)r * pitch + c;
       const int sp_step = rows_pass * pitch;
       uint32_t rank_addr[8];
@@ -89,11 +123,40 @@ __device__ __forceinline__ void gemm_tile_epilogue(const GemmProblem &p, const G
       const int64_t r_step = (int64_t)rows_pass * p.res_sm;
       const float *bp = bias ? bias + (m_base + r) * p.bias_sm + (p.bias_sn ? n : 0) : nullptr;
       const int64_t b_step = (int64_t)rows_pass * p.bias_sm;
-      float4 bvec = make_float4(0.f, 0.f, 0.f, 0.f);
-      const bool bias_per_col = bias && p.bias_sm == 0 && p.bias_sn == 1;  // the usual [N] bias: load once
-      if (bias_per_col) bvec = *reinterpret_cast<const float4 *>(bp);
-      float4 cs = make_float4(1.f, 1.f, 1.f, 1.f);
-      if (COL_SCALE) cs = *reinterpret_cast<const float4 *>(col_scale + n);
+      auto one = [&](float4 acc, float4 bq, float4 rq) {
+        if (COL_SCALE) { acc.x *= cs.x; acc.y *= cs.y; acc.z *= cs.z; acc.w *= cs.w; }
+        float v[4] = {acc.x, acc.y, acc.z, acc.w};
+        const float bv[4] = {bq.x, bq.y, bq.z, bq.w}, rv[4] = {rq.x, rq.y, rq.z, rq.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float y = v[j];
+          if (scale) {
+            if (sc_div != 1.0f) y = y / sc_div;
+            y = bias ? sc_alpha * y + sc_beta * bv[j] : sc_alpha * y;
+          } else {
+            y += bv[j];
+          }
+          v[j] = act_op<ACT>(e, y) + rv[j];
+        }
+        return make_float4(v[0], v[1], v[2], v[3]);
+      };
+      if (S == 1 && (!bias || bias_per_col)) {
+        // Four rows at a time: their shared-memory and residual loads are all in flight before the first
+        // store (the compiler keeps a load behind an earlier store, so row by row every load's latency
+        // would be exposed: 32 rows per thread at tile 256).
+        while (r + 3 * rows_pass < r_end) {
+          float4 acc[4], rq[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            acc[u] = *reinterpret_cast<const float4 *>(sp + u * sp_step);
+            rq[u] = res ? *reinterpret_cast<const float4 *>(rp + u * r_step) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) *reinterpret_cast<float4 *>(cp + u * c_step) = one(acc[u], bvec, rq[u]);
+          r += 4 * rows_pass; sp += 4 * sp_step; cp += 4 * c_step; rp += 4 * r_step;
+        }
+        if (res && r < r_end) rvec = *reinterpret_cast<const float4 *>(rp);
+      }
       for (; r < r_end; r += rows_pass) {
         float4 acc;
         if (S == 1) {
@@ -118,57 +181,43 @@ __device__ __forceinline__ void gemm_tile_epilogue(const GemmProblem &p, const G
           if (p.bias_sn == 1) bvec = *reinterpret_cast<const float4 *>(bp);
           else { const float t = *bp; bvec = make_float4(t, t, t, t); }
         }
-        float4 rvec = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (res) rvec = *reinterpret_cast<const float4 *>(rp);
-        if (COL_SCALE) { acc.x *= cs.x; acc.y *= cs.y; acc.z *= cs.z; acc.w *= cs.w; }
-        float v[4] = {acc.x, acc.y, acc.z, acc.w};
-        const float bv[4] = {bvec.x, bvec.y, bvec.z, bvec.w}, rv[4] = {rvec.x, rvec.y, rvec.z, rvec.w};
+        const float4 rq = rvec;
+        rp += r_step;
+        if (res && r + rows_pass < r_end) rvec = *reinterpret_cast<const float4 *>(rp);  // the next row's, under this row's arithmetic
+        *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq);
+        sp += sp_step; cp += c_step; bp += b_step;
+      }
+    } else {
+      // ragged column edge or non-unit strides: one element at a time, indices recomputed
+      const int quads = BN >> 2, count = (r1 - r0) * quads;
+      for (int i = et; i < count; i += NT) {
+        const int rr = i / quads, row = r0 + rr, col = (i - rr * quads) * 4;
+        const int64_t m = m_base + row;
+        if (m >= p.M) continue;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          float y = v[j];
+          const int64_t n = n_base + col + j;
+          if (n >= p.N) continue;
+          float acc = 0.0f;
+          const uint32_t off = staging_addr + (uint32_t)(row * pitch + col + j) * 4u;
+          if (S == 1) acc = staging[(size_t)row * pitch + col + j];
+          else
+            for (int rank = 0; rank < S; ++rank) acc += ld_cluster_f32(cluster_smem_addr(off, (uint32_t)rank));
+          if (COL_SCALE) acc *= col_scale[n];
+          const float bv = bias ? bias[m * p.bias_sm + n * p.bias_sn] : 0.0f;
+          const float rv = res ? res[m * p.res_sm + n * p.res_sn] : 0.0f;
+          float y = acc;
           if (scale) {
             if (sc_div != 1.0f) y = y / sc_div;
-            y = bias ? sc_alpha * y + sc_beta * bv[j] : sc_alpha * y;
+            y = bias ? sc_alpha * y + sc_beta * bv : sc_alpha * y;
           } else {
-            y += bv[j];
+            y += bv;
           }
-          v[j] = act_op<ACT>(e, y) + rv[j];
+          C[m * p.c_sm + n * p.c_sn] = act_op<ACT>(e, y) + rv;
         }
-        *reinterpret_cast<float4 *>(cp) = make_float4(v[0], v[1], v[2], v[3]);
-        sp += sp_step; cp += c_step; rp += r_step; bp += b_step;
-      }
-    }
-  } else {
-    // ragged column edge or non-unit strides: one element at a time, indices recomputed
-    const int count = (r1 - r0) * quads;
-    for (int i = et; i < count; i += NT) {
-      const int rr = i / quads;
-      const int r = r0 + rr, c = (i - rr * quads) * 4;
-      const int64_t m = m_base + r;
-      if (m >= p.M) continue;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int64_t n = n_base + c + j;
-        if (n >= p.N) continue;
-        float acc = 0.0f;
-        const uint32_t off = staging_addr + (uint32_t)(r * pitch + c + j) * 4u;
-        if (S == 1) acc = staging[(size_t)r * pitch + c + j];
-        else
-          for (int rank = 0; rank < S; ++rank) acc += ld_cluster_f32(cluster_smem_addr(off, (uint32_t)rank));
-        if (COL_SCALE) acc *= col_scale[n];
-        const float bv = bias ? bias[m * p.bias_sm + n * p.bias_sn] : 0.0f;
-        const float rv = res ? res[m * p.res_sm + n * p.res_sn] : 0.0f;
-        float y = acc;
-        if (scale) {
-          if (sc_div != 1.0f) y = y / sc_div;
-          y = bias ? sc_alpha * y + sc_beta * bv : sc_alpha * y;
-        } else {
-          y += bv;
-        }
-        C[m * p.c_sm + n * p.c_sn] = act_op<ACT>(e, y) + rv;
       }
     }
   }
-}
+};
 
 }  // namespace fml

@@ -8,25 +8,29 @@
 // Range.  fp16 has 5 exponent bits, so both sides are scaled by powers of two (exact):
 //   B  per column, at packing time (fml_gemm_pack): the column's largest magnitude lands in
 //      [2^14, 2^15); elements 2^-28 below it still have all 22 bits.
-//   A  per row and k slice, on the fly: the first k block (64 values) of the row that is not all zero
-//      puts its largest magnitude into [2^3, 2^4).  Elements far below it keep an absolute error of
-//      2^-28 of that magnitude, below fp32's own rounding of the sum; 2^12 of headroom is left for
-//      larger values further along.  A row that outgrows even that overflows to infinity, which the
-//      finished accumulator shows in every column: the CTA then finds the exact row maxima and does
-//      its tile a second time with them.  Infinities and NaNs of the input come out as NaN, as in the
-//      3xTF32 kernel.
+//   A  per row and k slice, on the fly: the first k block (32 values) of the row puts its largest
+//      magnitude into [2^3, 2^4).  Elements far below it keep an absolute error of 2^-28 of that
+//      magnitude, below fp32's own rounding of the sum; 2^12 of headroom is left for larger values
+//      further along.  A row whose first block is all zero takes 2^8, right for magnitudes from 2^-12 to
+//      2^7.  A row that outgrows its scale overflows to infinity, which the finished accumulator shows
+//      in every column, and one whose magnitudes stay below the default scale's reach is noticed by
+//      their maximum: the CTA then finds the exact row maxima and does its tile a second time with
+//      them.  Infinities and NaNs of the input come out as NaN, as in the 3xTF32 kernel.
 // The powers of two are divided out again when the accumulator leaves tensor memory (rows) and in the
 // epilogue (columns).
 //
-// B is stored packed: per k block of 64, per 8 columns, the 1 KiB swizzled K-major atom of hi and the
-// one of lo side by side.  A tile's share of a k block is then one contiguous run, fetched by one
+// B is stored packed: per k block of 32, per 8 columns, the 512-byte K-major atom (64-byte swizzle) of hi
+// and the one of lo side by side.  A tile's share of a k block is then one contiguous run, fetched by one
 // untiled bulk copy, and nothing of B is converted on chip.  (Bytes streamed: 4 per weight, as fp32.)
+// Blocks of 32 rather than 64 k values: at tile 256 shared memory holds 128 KiB of B, and four blocks in
+// flight cover the ~1 us of an L2 round trip where two did not (each block is ~0.4 us of MMAs).
 //
-// Roles, 320 threads: warp 0 loads (A boxes of 32 floats x 128 rows by tensor map, B runs), warp 1
-// issues the MMAs, warps 2-9 convert: two sets of four warps (a warp may write the 32 TMEM lanes of its
-// index modulo 4), set h taking k values [32h, 32h + 32) of every block; thread = row.  A's fp32 stage
-// is free as soon as it is converted, the tensor-memory stage and B's stage when the MMAs are done, so
-// they form separate rings.  Epilogue, split-K over a cluster and bounded waits as in gemm_tc.cu.
+// Roles, 320 threads: warp 0 loads (A boxes of 32 floats x 128 rows by tensor map, B runs; the two rings
+// are filled independently, whichever has room), warp 1 issues the MMAs, warps 2-9 convert: two sets of
+// four warps (a warp may write the 32 TMEM lanes of its index modulo 4) that take alternate blocks;
+// thread = row.  A's fp32 stage is free as soon as it is converted, the
+// tensor-memory stage and B's stage when the MMAs are done.  Epilogue, split-K over a cluster and
+// bounded waits as in gemm_tc.cu.
 #include "gemm_epilogue.cuh"
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -36,8 +40,11 @@
 namespace fml {
 namespace {
 
-constexpr int kPK = 64;                      // k values per block: 128 bytes of fp16
-constexpr int kPairA = 2 * kBM * 32 * 4;     // bytes of A per block: two boxes of 128 rows x 128 bytes
+constexpr int kPK = 32;                      // k values per block: 128 bytes of fp32, 64 of fp16
+constexpr int kPairA = kBM * kPK * 4;        // bytes of A per block: a box of 128 rows x 128 bytes
+constexpr int kPairB = kPK * 4;              // bytes of B per block and column: hi and lo
+constexpr int kAtom = 8 * kPK * 2;           // bytes of an atom: 8 columns x 32 k values of fp16
+constexpr int kDefaultExponent = 8;          // scale 2^8 of a row whose first k block is all zero
 constexpr int kPairThreads = 320;
 constexpr int kConvThreads = 256;
 
@@ -52,13 +59,12 @@ struct PairArgs {
   int *status;
 };
 
-// The power of two that brings a largest magnitude m into [2^target, 2^(target + 1)), and its inverse;
-// the exponent is limited so that both are normal numbers.
-__device__ __forceinline__ void pow2_scale(float m, int target, float &s, float &inv) {
-  const int e = (int)(__float_as_uint(m) >> 23) - 127;
-  const int k = min(max(target - e, -126), 126);
-  s = __uint_as_float((uint32_t)(127 + k) << 23);
-  inv = __uint_as_float((uint32_t)(127 - k) << 23);
+// 2^k for -126 <= k <= 127.
+__device__ __forceinline__ float pow2(int k) { return __uint_as_float((uint32_t)(127 + k) << 23); }
+// The exponent that brings a largest magnitude m into [2^target, 2^(target + 1)), limited so that the
+// power and its inverse are normal numbers.
+__device__ __forceinline__ int scale_exponent(float m, int target) {
+  return min(max(target - ((int)(__float_as_uint(m) >> 23) - 127), -126), 126);
 }
 
 // Two fp32 values, already loaded -> (hi pair, lo pair) of x * s.
@@ -73,11 +79,11 @@ __device__ __forceinline__ void split_pair(float x0, float x1, float s, uint32_t
 template <int ACT>
 __global__ void __launch_bounds__(kPairThreads, 2)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  // (no static shared memory in this kernel: the dynamic part starts on a 1024-byte boundary)
+  extern __shared__ __align__(1024) uint8_t smem[];
   const int BN = a.tile_n;
   const int pitch = BN + 4;
-  const uint32_t b_bytes = (uint32_t)BN * 256u;  // hi and lo, 64 k values
+  const uint32_t b_bytes = (uint32_t)BN * kPairB;
   const size_t ring_bytes = (size_t)a.stages_a * kPairA + (size_t)a.stages_b * b_bytes;
   const size_t staging_bytes = ((size_t)kBM * pitch * 4 + 1023) / 1024 * 1024;
   const size_t data_bytes = ring_bytes > staging_bytes ? ring_bytes : staging_bytes;
@@ -91,8 +97,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * a.stages_a + 3 * a.stages_b + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   volatile int *redo_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
+  unsigned *row_seen = reinterpret_cast<unsigned *>(tmem_slot + 4);          // [128], rows on the default scale: largest scaled magnitude
+  signed char *row_exp = reinterpret_cast<signed char *>(row_seen + kBM);  // [128], scale exponent; -128: the default one
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const bool leader = elect_one();
   const int tile = blockIdx.x, tile_m = tile % a.tiles_m, tile_n = tile / a.tiles_m;
   const int split = blockIdx.y;
   const int z = blockIdx.z, z0 = z % (int)a.p.nb0, z1 = z / (int)a.p.nb0;
@@ -101,13 +110,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   const int nkb = kb1 - kb0;
   const uint32_t a_col0 = ((uint32_t)BN + 31u) & ~31u;
   uint32_t tmem_cols = 32;
-  while (tmem_cols < a_col0 + 64u * (uint32_t)a.stages_b) tmem_cols <<= 1;
+  while (tmem_cols < a_col0 + 32u * (uint32_t)a.stages_b) tmem_cols <<= 1;
   // the packed run of this tile in k block kb; the last tile of a ragged N stops at the image's edge
   // (the columns it leaves unwritten in shared memory are never stored)
   const int n_cols = min(BN, a.n_pad - tile_n * BN);
-  const uint32_t b_run = (uint32_t)n_cols * 256u;
-  const char *b_src = a.packed + ((size_t)kb0 * (a.n_pad / 8) + (size_t)tile_n * BN / 8) * 2048;
-  const size_t b_step = (size_t)(a.n_pad / 8) * 2048;
+  const uint32_t b_run = (uint32_t)n_cols * kPairB;
+  const char *b_src = a.packed + ((size_t)kb0 * a.n_pad + (size_t)tile_n * BN) * kPairB;
+  const size_t b_step = (size_t)a.n_pad * kPairB;
   // Weights that one row of tiles reads cross L2 once per pass: evict-first (gemm_tc.cu).
   const bool b_stream = a.tiles_m == 1;
   const uint64_t b_policy = b_stream ? l2_policy_evict_first() : 0ull;
@@ -134,11 +143,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages_a; ++s) {
       mbar_init(bar_full_a + 8u * s, 1);
-      mbar_init(bar_empty_a + 8u * s, 8);  // one arrival per converter warp
+      mbar_init(bar_empty_a + 8u * s, 4);  // one arrival per warp of the converter set
     }
     for (int s = 0; s < a.stages_b; ++s) {
       mbar_init(bar_full_b + 8u * s, 1);
-      mbar_init(bar_conv + 8u * s, 8);
+      mbar_init(bar_conv + 8u * s, 4);
       mbar_init(bar_empty_b + 8u * s, 1);
     }
     mbar_init(bar_accum, 1);
@@ -147,6 +156,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     *redo_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + kBM) row_seen[threadIdx.x - 64] = 0u;
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), tmem_cols);
   tc_fence_before();
   __syncthreads();
@@ -170,40 +180,45 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   }
   pdl_wait();
 
+  TileEpilogue<ACT, kConvThreads, true> epi;
   float row_inv = 1.0f;  // converter threads: undoes the scale of this thread's row
   if (warp == 0) {
     // ------------------------------------------------------------ loads
-    if (lane == 0 && !g_drop_loads) {
+    if (!g_drop_loads) {
       const int ca2 = a.p.a_b0 ? z0 : 0, ca3 = a.p.a_b1 ? z1 : 0;
       bool ok = true;
       int issued_a = 0, issued_b = pre_b;  // counted over both attempts: ring positions go on
+      RingPos ra, rb;
+      for (int it = 0; it < pre_b; ++it) rb.step(a.stages_b);
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
         if (attempt) {
           ok = mbar_wait(bar_decide, 0u, abort_flag);
           if (!ok || !*redo_flag) break;
         }
-        for (int it = 0; it < nkb && ok; ++it) {
-          const int at = attempt * nkb + it;
-          if (at >= issued_b) {
-            const int s = at % a.stages_b;
-            ok = mbar_wait(bar_empty_b + 8u * s, ((uint32_t)(at / a.stages_b) & 1u) ^ 1u, abort_flag);
-            if (!ok) break;
-            load_b(it, s);
-            issued_b = at + 1;
+        int ia = 0, ib = attempt ? 0 : pre_b;
+        uint32_t idle = 0;
+        while (ia < nkb || ib < nkb) {  // whichever ring has room
+          bool moved = false;
+          if (ia < nkb && mbar_test(bar_empty_a + 8u * ra.s, ra.ph ^ 1u)) {
+            const uint32_t bar = bar_full_a + 8u * ra.s;
+            if (leader) {
+              mbar_expect_tx(bar, kPairA);
+              tma_load_4d(ring_a + (uint32_t)ra.s * kPairA, &map_a, bar, (kb0 + ia) * kPK, tile_m * kBM, ca2, ca3);
+            }
+            ++ia; ++issued_a; moved = true;
+            ra.step(a.stages_a);
           }
-          const int s = at % a.stages_a;
-          ok = mbar_wait(bar_empty_a + 8u * s, ((uint32_t)(at / a.stages_a) & 1u) ^ 1u, abort_flag);
-          if (!ok) break;
-          const uint32_t dst = ring_a + (uint32_t)s * kPairA, bar = bar_full_a + 8u * s;
-          const int k = (kb0 + it) * kPK;
-          mbar_expect_tx(bar, kPairA);
-          tma_load_4d(dst, &map_a, bar, k, tile_m * kBM, ca2, ca3);
-          tma_load_4d(dst + kPairA / 2, &map_a, bar, k + 32, tile_m * kBM, ca2, ca3);
-          issued_a = at + 1;
+          if (ib < nkb && mbar_test(bar_empty_b + 8u * rb.s, rb.ph ^ 1u)) {
+            if (leader) load_b(ib, rb.s);
+            ++ib; ++issued_b; moved = true;
+            rb.step(a.stages_b);
+          }
+          if (moved) idle = 0;
+          else if ((++idle & 255u) == 0 && (*abort_flag || idle >= 64u * g_wait_limit)) { ok = false; break; }
         }
       }
       if (!ok) {
-        atomicOr(a.status, kStatusTimeout);
+        if (leader) atomicOr(a.status, kStatusTimeout);
         *abort_flag = 1;
         // bounded drain of the loads already in flight before the CTA may exit
         volatile int never = 0;
@@ -215,113 +230,154 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = instr_desc_f16(BN);
-      const uint64_t desc_b = smem_desc(ring_b, 16u, 2048u);  // hi atoms; lo 1024 bytes further
-      bool ok = true;
-      for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-        if (attempt) {
-          ok = mbar_wait(bar_decide, 0u, abort_flag);
-          if (!ok || !*redo_flag) break;
-        }
-        for (int it = 0; it < nkb; ++it) {
-          const int at = attempt * nkb + it, s = at % a.stages_b;
-          const uint32_t ph = (uint32_t)(at / a.stages_b) & 1u;
-          ok = mbar_wait(bar_full_b + 8u * s, ph, abort_flag) && mbar_wait(bar_conv + 8u * s, ph, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t db0 = desc_b + (((uint32_t)s * b_bytes) >> 4);
-          const uint32_t ta = tmem_base + a_col0 + (uint32_t)s * 64u;
+    const uint32_t idesc = instr_desc_f16(BN);
+    const uint64_t desc_b = smem_desc(ring_b, 16u, 2 * kAtom, 4u);  // hi atoms (64-byte swizzle); lo one atom further
+    RingPos rb;
+    bool ok = true;
+    for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+      if (attempt) {
+        ok = mbar_wait(bar_decide, 0u, abort_flag);
+        if (!ok || !*redo_flag) break;
+      }
+      for (int it = 0; it < nkb; ++it) {
+        ok = mbar_wait(bar_full_b + 8u * rb.s, rb.ph, abort_flag) && mbar_wait(bar_conv + 8u * rb.s, rb.ph, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        if (leader) {
+          const uint64_t db0 = desc_b + (((uint32_t)rb.s * b_bytes) >> 4);
+          const uint32_t ta = tmem_base + a_col0 + (uint32_t)rb.s * 32u;
 #pragma unroll
           for (int j = 0; j < kPK / 16; ++j) {
-            const uint32_t a_hi = ta + (uint32_t)j * 8u, a_lo = a_hi + 32u;
-            const uint64_t db = db0 + (uint32_t)j * 2u, dbl = db + (1024u >> 4);
+            const uint32_t a_hi = ta + (uint32_t)j * 8u, a_lo = a_hi + 16u;
+            const uint64_t db = db0 + (uint32_t)j * 2u, dbl = db + (kAtom >> 4);
             umma_f16_ts(tmem_base, a_lo, db, idesc, (it == 0 && j == 0) ? 0u : 1u);
             umma_f16_ts(tmem_base, a_hi, dbl, idesc, 1u);
             umma_f16_ts(tmem_base, a_hi, db, idesc, 1u);
           }
-          umma_commit(bar_empty_b + 8u * s);  // B stage and TMEM stage reusable
+          umma_commit(bar_empty_b + 8u * rb.s);  // B stage and TMEM stage reusable
         }
-        if (ok) umma_commit(bar_accum);  // with no MMA outstanding (nkb == 0) this arrives at once
+        __syncwarp();
+        rb.step(a.stages_b);
       }
-      if (!ok) {
-        atomicOr(a.status, kStatusTimeout);
-        *abort_flag = 1;
-      }
+      if (ok && leader) umma_commit(bar_accum);  // with no MMA outstanding (nkb == 0) this arrives at once
+      __syncwarp();
+    }
+    if (!ok) {
+      if (leader) atomicOr(a.status, kStatusTimeout);
+      *abort_flag = 1;
     }
   } else {
     // ------------------------------------------------------------ converter
-    const int q = warp & 3, row = q * 32 + lane, half = (warp - 2) >> 2, swz = row & 7;
+    const int q = warp & 3, row = q * 32 + lane, set = (warp - 2) >> 2, swz = row & 7;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    const bool real_row = (int64_t)tile_m * kBM + row < a.p.M;
     bool ok = true;
-    float s_mul = 1.0f;
+    int k_row = 0;       // the row is scaled by 2^k_row
+    auto load_row = [&](int slot, float4 *x) {  // 16-byte chunks swizzled by (row & 7)
+      const float4 *src = reinterpret_cast<const float4 *>(smem + (size_t)slot * kPairA + row * 128);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) x[c] = src[c ^ swz];
+    };
+    bool guess = false;  // this row's scale is the default one
+    float seen = 0.0f;   // largest scaled magnitude this thread converted (kept while a row of its warp has the default scale)
     for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-      bool scaled = false;
+      // positions of this set's block in the two rings (the second attempt's blocks follow the first's)
+      const int at = attempt * nkb + set;
+      RingPos ma{at % a.stages_a, (uint32_t)(at / a.stages_a) & 1u}, mb{at % a.stages_b, (uint32_t)(at / a.stages_b) & 1u};
+      float4 x[8];
+      bool have = false;
       if (attempt) {
         // exact maximum of this row over the CTA's k range, straight from global memory (rare)
         float m = 0.0f;
-        const int64_t gm = (int64_t)tile_m * kBM + row;
-        if (gm < a.p.M) {
-          const float *src = a.p.a + (int64_t)z0 * a.p.a_b0 + (int64_t)z1 * a.p.a_b1 + gm * a.p.a_sm;
+        if (real_row) {
+          const float *src = a.p.a + (int64_t)z0 * a.p.a_b0 + (int64_t)z1 * a.p.a_b1 + ((int64_t)tile_m * kBM + row) * a.p.a_sm;
           const int64_t k_end = min((int64_t)kb1 * kPK, a.p.K);
           for (int64_t k = (int64_t)kb0 * kPK; k < k_end; ++k) m = fmaxf(m, fabsf(src[k]));
         }
-        pow2_scale(m, 14, s_mul, row_inv);
-        scaled = true;
-      }
-      for (int it = 0; it < nkb && ok; ++it) {
-        const int at = attempt * nkb + it, sa = at % a.stages_a, sb = at % a.stages_b;
-        ok = mbar_wait(bar_full_a + 8u * sa, (uint32_t)(at / a.stages_a) & 1u, abort_flag);
-        if (!ok) break;
-        const uint8_t *st = smem + (size_t)sa * kPairA + row * 128;
-        const float4 *src = reinterpret_cast<const float4 *>(st + half * (kPairA / 2));
-        float4 x[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) x[c] = src[c ^ swz];
-        if (!scaled) {  // both sets look at the whole block, so they agree on the scale
-          const float4 *other = reinterpret_cast<const float4 *>(st + (half ^ 1) * (kPairA / 2));
+        k_row = scale_exponent(m, 14);
+      } else {
+        // set 0 finds the scale in block 0, set 1 takes it over
+        if (set == 0) {
           float m = 0.0f;
+          if (nkb > 0) {
+            ok = mbar_wait(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
+            if (ok) {
+              load_row(ma.s, x);
+              have = true;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const float4 y = other[c ^ swz];
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(x[c].x), fabsf(x[c].y)), fmaxf(fabsf(x[c].z), fabsf(x[c].w))));
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w))));
+              for (int c = 0; c < 8; ++c)
+                m = fmaxf(m, fmaxf(fmaxf(fabsf(x[c].x), fabsf(x[c].y)), fmaxf(fabsf(x[c].z), fabsf(x[c].w))));
+            }
           }
-          if (m > 0.0f) {
-            pow2_scale(m, 3, s_mul, row_inv);
-            scaled = true;
-          }
+          guess = !(m > 0.0f);
+          k_row = guess ? kDefaultExponent : scale_exponent(m, 3);
+          row_exp[row] = (signed char)(guess ? -128 : k_row);
+          asm volatile("bar.arrive 1, 256;" ::: "memory");  // also when the wait gave up: set 1 must not be left behind
+        } else {
+          asm volatile("bar.sync 1, 256;" ::: "memory");
+          k_row = row_exp[row];
+          guess = k_row == -128;
+          if (guess) k_row = kDefaultExponent;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_empty_a + 8u * sa);  // the values are in registers
+      }
+      const float s_mul = pow2(k_row);
+      row_inv = pow2(-k_row);
+      const bool watch = attempt == 0 && __any_sync(0xffffffffu, guess);
+      for (int it = set; it < nkb && ok; it += 2) {
+        if (!have) {
+          ok = mbar_wait(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
+          if (!ok) break;
+          load_row(ma.s, x);
+        }
+        if (watch) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            seen = fmaxf(seen, s_mul * fmaxf(fmaxf(fabsf(x[c].x), fabsf(x[c].y)), fmaxf(fabsf(x[c].z), fabsf(x[c].w))));
+        }
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           split_pair(x[c].x, x[c].y, s_mul, hi[2 * c], lo[2 * c]);
           split_pair(x[c].z, x[c].w, s_mul, hi[2 * c + 1], lo[2 * c + 1]);
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_empty_a + 8u * ma.s);  // the values are in registers
+        ma.step(a.stages_a); ma.step(a.stages_a);
         // the MMAs that read this tensor-memory stage last are done
-        ok = mbar_wait(bar_empty_b + 8u * sb, ((uint32_t)(at / a.stages_b) & 1u) ^ 1u, abort_flag);
+        ok = mbar_wait(bar_empty_b + 8u * mb.s, mb.ph ^ 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t t_hi = lane_addr + a_col0 + (uint32_t)sb * 64u + (uint32_t)half * 16u;
+        const uint32_t t_hi = lane_addr + a_col0 + (uint32_t)mb.s * 32u;
         tmem_st16(t_hi, hi);
-        tmem_st16(t_hi + 32u, lo);
+        tmem_st16(t_hi + 16u, lo);
+        // the next block of this set, if it is there: its shared-memory latency runs under these stores
+        have = it + 2 < nkb && __all_sync(0xffffffffu, mbar_test(bar_full_a + 8u * ma.s, ma.ph));
+        if (have) load_row(ma.s, x);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_conv + 8u * sb);
+        if (lane == 0) mbar_arrive(bar_conv + 8u * mb.s);
+        mb.step(a.stages_b); mb.step(a.stages_b);
       }
+      if (!attempt) epi.preload(a.p, BN, tile_m, tile_n, split, a.split_k, z0, z1, threadIdx.x - 64, a.col_scale);
       if (ok) ok = mbar_wait(bar_accum, (uint32_t)attempt, abort_flag);
-      if (!ok || attempt) break;
-      // A row whose hi overflowed shows it in every column of the accumulator.
+      if (attempt) break;
+      // A row whose hi overflowed shows it in every column of the accumulator; one on the default scale
+      // must have had a value that this scale resolves, unless it is all zero.
       tc_fence_after();
-      const float v0 = nkb > 0 ? tmem_ld1(lane_addr) : 0.0f;
+      const float v0 = ok && nkb > 0 ? tmem_ld1(lane_addr) : 0.0f;
       tc_fence_before();
-      if (__any_sync(0xffffffffu, !(fabsf(v0) <= 3.4028235e38f)) && lane == 0) *redo_flag = 1;
+      if (watch && guess && seen > 0.0f) atomicMax(&row_seen[row], __float_as_uint(seen));
+      asm volatile("bar.sync 2, 256;" ::: "memory");  // every converter warp comes here, whether its waits were met or not
+      bool bad = !(fabsf(v0) <= 3.4028235e38f);
+      if (watch && guess) {
+        const float m = __uint_as_float(row_seen[row]);
+        bad = bad || (m > 0.0f && m < 0.0625f);
+      }
+      if (__any_sync(0xffffffffu, bad) && lane == 0) *redo_flag = 1;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_decide);
-      ok = mbar_wait(bar_decide, 0u, abort_flag);
+      ok = ok && mbar_wait(bar_decide, 0u, abort_flag);
       if (!ok || !*redo_flag) break;
     }
     if (!ok) {
@@ -332,7 +388,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     // sets take alternate groups of 32 columns.
     tc_fence_after();
     float *dst = staging + (size_t)row * pitch;
-    for (int c0 = half * 32; c0 < BN; c0 += 64) {
+    for (int c0 = set * 32; c0 < BN; c0 += 64) {
       float v[32];
       if (ok && nkb > 0) {
         tmem_ld32(lane_addr + (uint32_t)c0, v);
@@ -354,8 +410,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   const int S = a.split_k;
   if (S > 1) cluster_sync_all();
   if (warp >= 2)
-    gemm_tile_epilogue<ACT, kConvThreads, true>(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1,
-                                                threadIdx.x - 64, a.col_scale);
+    epi.finish(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, threadIdx.x - 64, a.col_scale);
   if (S > 1) cluster_sync_all();
   __syncthreads();
   if (warp == 1) {
@@ -379,11 +434,15 @@ __global__ void __launch_bounds__(256) gemm_pack_kernel(const float *b, int64_t 
   atomicMax(&m_bits[r], __float_as_uint(m));  // non-negative floats order as their bits
   __syncthreads();
   float s = 1.0f, inv = 1.0f;
-  if (m_bits[r]) pow2_scale(__uint_as_float(m_bits[r]), 14, s, inv);
+  if (m_bits[r]) {
+    const int e = scale_exponent(__uint_as_float(m_bits[r]), 14);
+    s = pow2(e);
+    inv = pow2(-e);
+  }
   if (threadIdx.x < 8) col_scale[n0 + r] = inv;
-  for (int64_t i = threadIdx.x >> 3; i < (int64_t)kb_total * 8; i += 32) {  // (k block, 16-byte chunk) of column r
-    const int64_t kb = i >> 3;
-    const int c = (int)(i & 7);
+  for (int64_t i = threadIdx.x >> 3; i < (int64_t)kb_total * 4; i += 32) {  // (k block, 16-byte chunk) of column r
+    const int64_t kb = i >> 2;
+    const int c = (int)(i & 3);
     uint32_t hi[4], lo[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -392,21 +451,22 @@ __global__ void __launch_bounds__(256) gemm_pack_kernel(const float *b, int64_t 
       const float x1 = n0 + r < N && k + 1 < K ? b[(k + 1) * sk + (n0 + r) * sn] : 0.0f;
       split_pair(x0, x1, s, hi[j], lo[j]);
     }
-    char *atom = packed + ((size_t)kb * (n_pad / 8) + blockIdx.x) * 2048 + r * 128 + ((c ^ r) * 16);
+    // 64-byte swizzle: the chunk index is XORed with bits 7-8 of the address, i.e. (row / 2) mod 4
+    char *atom = packed + ((size_t)kb * n_pad + n0) * kPairB + r * (kPK * 2) + ((c ^ (r >> 1)) * 16);
     *reinterpret_cast<uint4 *>(atom) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    *reinterpret_cast<uint4 *>(atom + 1024) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    *reinterpret_cast<uint4 *>(atom + kAtom) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
 }
 
 // ---------------------------------------------------------------- host side
 int n_padded(int64_t n) { return (int)((n + 15) / 16 * 16); }
 int k_blocks(int64_t k) { return (int)((k + kPK - 1) / kPK); }
-size_t atoms_bytes(int64_t k, int64_t n) { return (size_t)k_blocks(k) * n_padded(n) * 256; }
+size_t atoms_bytes(int64_t k, int64_t n) { return (size_t)k_blocks(k) * n_padded(n) * kPairB; }
 
 size_t pair_smem(int tile_n, int stages_a, int stages_b) {
-  const size_t ring = (size_t)stages_a * kPairA + (size_t)stages_b * tile_n * 256;
+  const size_t ring = (size_t)stages_a * kPairA + (size_t)stages_b * tile_n * kPairB;
   const size_t staging = ((size_t)kBM * (tile_n + 4) * 4 + 1023) / 1024 * 1024;
-  return std::max(ring, staging) + (2 * stages_a + 3 * stages_b + 2) * 8 + 16 + 1024;
+  return std::max(ring, staging) + (2 * stages_a + 3 * stages_b + 2) * 8 + 16 + kBM * 5;
 }
 
 constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;
@@ -419,22 +479,22 @@ bool pair_stages(int tile_n, int per, bool two_ctas, int *stages_a, int *stages_
   const int tmem = two_ctas ? 256 : 512;
   int best_a = 0, best_b = 0;
   double best = 0.0;
-  for (int sb = 1; sb <= 6 && acc + 64 * sb <= tmem; ++sb)
-    for (int sa = 1; sa <= 6; ++sa) {
+  for (int sb = 1; sb <= 8 && acc + 32 * sb <= tmem; ++sb)
+    for (int sa = 1; sa <= 8; ++sa) {
       if (pair_smem(tile_n, sa, sb) > budget) continue;
-      if (sa > per || sb > per) continue;  // no deeper than the k loop
+      if (sa > per || sb > per) continue;   // no deeper than the k loop
       // both rings count; the shallower one limits
       const double score = std::min(sa, sb) * 8 + sa + sb;
       if (score > best) { best = score; best_a = sa; best_b = sb; }
     }
   if (!best_a) return false;
-  if (two_ctas && per > 1 && std::min(best_a, best_b) < 2) return false;
+  if (two_ctas && per > 1 && std::min(best_a, best_b) < std::min(per, 3)) return false;
   *stages_a = best_a;
   *stages_b = best_b;
   size_t need = pair_smem(tile_n, best_a, best_b);
   // no more CTAs on an SM than its 512 TMEM columns serve at once (gemm_tc.cu)
   unsigned cols = 32;
-  while ((int)cols < acc + 64 * best_b) cols <<= 1;
+  while ((int)cols < acc + 32 * best_b) cols <<= 1;
   need = std::max(need, kSmemSm / (512 / cols + 1) + 1024);
   *smem = need;
   return need <= kSmemCta;
@@ -464,7 +524,7 @@ bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &p
   const int kb_total = k_blocks(p.K);
   const int64_t tiles_m = (p.M + kBM - 1) / kBM, batch = p.nb0 * p.nb1;
   // Default tile and split (the tuner measures the alternatives): time of a CTA = set-up and epilogue
-  // plus its k blocks at the slower of the MMAs (12 per block, 47 clocks each or N / 2) and one SM's
+  // plus its k blocks at the slower of the MMAs (6 per block, 47 clocks each or N / 2) and one SM's
   // fill path; waves of CTAs at one or two per SM.
   const int tn_opts[] = {32, 64, 96, 128, 192, 256};
   const int sk_opts[] = {1, 2, 4, 8};
@@ -486,7 +546,7 @@ bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &p
         const int64_t ctas = tiles_m * ((p.N + tn - 1) / tn) * batch * sk;
         const int slots = (two ? 296 : 148) * (sk == 8 ? 0.87 : sk == 4 ? 0.97 : 1.0);
         const double waves = (double)((ctas + slots - 1) / slots);
-        const double t_kb = std::max(12 * std::max(47.0, tn / 2.0) / 1.9e3, (kPairA + tn * 256.0) / 80e3);
+        const double t_kb = std::max(6 * std::max(47.0, tn / 2.0) / 1.9e3, (double)(kPairA + tn * kPairB) / 80e3);
         const double t_fixed = 3.0 + (double)kBM * tn / sk * 4.0 / 20e3 + (sk > 1 ? 0.6 : 0.0);
         const double t = waves * (t_fixed + per * t_kb * (two && ctas > 148 ? 2.0 : 1.0));
         if (t < best) {

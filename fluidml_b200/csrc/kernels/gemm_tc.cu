@@ -207,9 +207,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const int cb2 = a.p.b_b0 ? z0 : 0, cb3 = a.p.b_b1 ? z1 : 0;
       int issued = 0;
       bool ok = true;
-      for (int it = 0; it < nkb && ok; ++it) {
-        const int s = it % a.stages;
-        const uint32_t ph = (uint32_t)(it / a.stages) & 1u;
+      RingPos ring;
+      for (int it = 0; it < nkb && ok; ++it, ring.step(a.stages)) {
+        const int s = ring.s;
+        const uint32_t ph = ring.ph;
         const uint32_t sa = tiles_base + (uint32_t)s * stage_bytes, sb = sa + kABytes;
         const int k = (kb0 + it) * kBK;
         if (it < pre_b) {  // B of this stage is already on its way, the byte count already posted
@@ -253,9 +254,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint64_t desc_al = smem_desc(tiles_base + kABytes + b_bytes, 16u, 1024u);
       const uint64_t desc_bl = smem_desc(tiles_base + (A_TMEM ? kABytes + b_bytes : 2 * kABytes + b_bytes), b_lbo, b_sbo, b_type);
       bool ok = true;
-      for (int it = 0; it < nkb; ++it) {
-        const int s = it % a.stages;
-        const uint32_t ph = (uint32_t)(it / a.stages) & 1u;
+      RingPos ring;
+      for (int it = 0; it < nkb; ++it, ring.step(a.stages)) {
+        const int s = ring.s;
+        const uint32_t ph = ring.ph;
         ok = mbar_wait(ready + 8u * s, ph, abort_flag);
         if (!ok) break;
         if (it == 0) TRACE(2);
@@ -303,9 +305,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool ok = true;
     if (THREE_PASS) {
       const int b_vec = (int)b_bytes / 16;  // 16-byte units in the B tile: 8 per row of tile_n
-      for (int it = 0; it < nkb && ok; ++it) {
-        const int s = it % a.stages;
-        const uint32_t ph = (uint32_t)(it / a.stages) & 1u;
+      RingPos ring;
+      for (int it = 0; it < nkb && ok; ++it, ring.step(a.stages)) {
+        const int s = ring.s;
+        const uint32_t ph = ring.ph;
         ok = mbar_wait(bar_full + 8u * s, ph, abort_flag);
         if (!ok) break;
         uint8_t *st = smem + (size_t)s * stage_bytes;
@@ -402,7 +405,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (S > 1) cluster_sync_all();  // every rank's partial tile is in its shared memory
   if (warp >= 2) {
     const int et = threadIdx.x - 64;
-    gemm_tile_epilogue<ACT, 128, false>(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
+    TileEpilogue<ACT, 128, false> epi;
+    epi.preload(a.p, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
+    epi.finish(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
     if (et == 0) TRACE(5);
   }
   if (S > 1) cluster_sync_all();  // nobody leaves while a peer may still read its tile

@@ -46,17 +46,60 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
-// Bounded wait: false when the limit ran out or another role raised `abort`.
+// One lane of the (converged) warp.  The single-thread roles run their loops with the whole warp and let
+// only the elected lane issue: in a branch taken by lane 0 alone the compiler cannot keep descriptors,
+// barriers and addresses in uniform registers, and moving them there for every instruction made a
+// tcgen05.mma cost 47 clocks to issue where its N = 32 / 64 / 128 tile needs 16 / 32 / 64, and a
+// barrier wait that is already over about 190.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(p));
+  return p != 0;
+}
+// The warp's index as a value the compiler knows to be the same in all lanes.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// Position in a ring of `n` stages: index and the parity of the current round.  Stepped, not computed:
+// a division by a run-time ring depth costs ~100 dependent clocks, per role and k block.
+struct RingPos {
+  int s = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void step(int n) {
+    if (++s == n) { s = 0; ph ^= 1u; }
+  }
+  __device__ __forceinline__ void back(int n) {
+    if (--s < 0) { s = n - 1; ph ^= 1u; }
+  }
+};
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// The same question without the suspended wait: is the phase over now?
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// Bounded wait: false when the limit ran out or another role raised `abort`.  The limit is a module
+// variable, i.e. a global load; a wait that is over at once or soon does not pay for it.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort) {
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
+#pragma unroll 1
+  for (int i = 0; i < 16; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
   const uint32_t limit = g_wait_limit;
+#pragma unroll 1
   for (uint32_t i = 0; i < limit; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
+    if (mbar_try_wait(bar, parity)) return true;
     if ((i & 255u) == 255u && *abort) return false;
   }
   return false;
@@ -140,6 +183,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r) {
       ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
         "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
+}
+// 8 consecutive 32-bit columns of this thread's TMEM lane, written from registers.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t *r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
 }
 // One fp32 column of this thread's TMEM lane.
 __device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
