@@ -490,7 +490,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     }
     if (threadIdx.x == 64) CTRACE(10);
-    cluster_sync_all();  // nobody leaves while a peer may still read its tile
+    cluster_sync_relaxed();  // nobody leaves while a peer may still read its tile
   }
   if (threadIdx.x == 64) CTRACE(4);
   tc_fence_before();

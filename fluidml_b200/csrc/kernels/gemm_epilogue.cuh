@@ -3,6 +3,7 @@
 #pragma once
 #include "gemm_common.cuh"
 #include "tc_common.cuh"
+#include <type_traits>
 
 namespace fml {
 
@@ -42,6 +43,17 @@ __device__ __forceinline__ float act_op(const GemmEpilogue &e, float v) {
 // and residual and the stores of C are full lines.  `et` in [0, NT) numbers the calling threads.
 // COL_SCALE: column n of the accumulator is first multiplied by col_scale[n] (a power of two).
 //
+// Epilogue thread -> (column quad, row within a pass), worked out on the host: a kernel that runs each
+// phase once feels an integer division (~100 dependent clocks).
+struct EpilogueShape {
+  int rows_pass;        // rows covered by one pass of the threads
+  uint32_t quad_magic;  // et / (tile_n / 4) == (et * quad_magic) >> 16 for et < 256
+};
+inline EpilogueShape epilogue_shape(int tile_n, int threads) {
+  const int quads = tile_n / 4;
+  return {threads / quads, (uint32_t)((65536 + quads - 1) / quads)};
+}
+
 // preload() may run while the product is still being computed (after the dependency wait): it issues
 // the loads that do not depend on it -- bias, column scales, the first row's residual -- whose L2 round
 // trip is then off the critical path of a launch that does each phase once.  Only those values stay in
@@ -56,8 +68,9 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
     int64_t n_base, m_base;
     int rows_pass, r0, r1, r_end, r, c;
     bool vec, bias_per_col;
-    __device__ __forceinline__ Where(const GemmProblem &p, int BN, int tile_m, int tile_n, int split, int S, int z0, int z1, int et) {
-      const int rows_per = (kBM + S - 1) / S;
+    __device__ __forceinline__ Where(const GemmProblem &p, const EpilogueShape &shape, int BN, int tile_m, int tile_n, int split, int S, int z0, int z1, int et) {
+      const bool pow2_ranks = (S & (S - 1)) == 0;
+      const int rows_per = pow2_ranks ? kBM >> (31 - __clz(S)) : (kBM + S - 1) / S;
       r0 = split * rows_per;
       r1 = min(kBM, r0 + rows_per);
       bias = p.bias ? p.bias + (int64_t)z0 * p.bias_b0 + (int64_t)z1 * p.bias_b1 : nullptr;
@@ -69,34 +82,34 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
       // 16-byte path: unit column stride everywhere, every row start and the tile origin on a
       // 16-byte boundary, no ragged column edge inside this tile
       auto al4 = [](int64_t v) { return (v & 3) == 0; };
-      vec = p.c_sn == 1 && al4(p.c_sm) && al4(n_base) && n_base + BN <= p.N && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
+      vec = pow2_ranks && p.c_sn == 1 && al4(p.c_sm) && al4(n_base) && n_base + BN <= p.N && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
       if (bias) vec = vec && (p.bias_sn == 1 || p.bias_sn == 0) && al4(p.bias_sm) && ((reinterpret_cast<uintptr_t>(bias) & 15) == 0);
       if (res) vec = vec && p.res_sn == 1 && al4(p.res_sm) && ((reinterpret_cast<uintptr_t>(res) & 15) == 0);
       bias_per_col = bias && p.bias_sm == 0 && p.bias_sn == 1;  // the usual [N] bias: loaded once
       // Thread -> (column quad, row within a pass); rows advance by a constant, so every pointer of the
       // loop is stepped with one add per iteration.
-      const int quads = BN >> 2, rsub = et / quads;
-      rows_pass = NT / quads;
+      const int quads = BN >> 2, rsub = (int)(((uint32_t)et * shape.quad_magic) >> 16);
+      rows_pass = shape.rows_pass;
       c = (et - rsub * quads) * 4;
       r = vec && rsub < rows_pass ? r0 + rsub : kBM;  // threads beyond the last full row of quads stay out
     }
   };
 
-  __device__ __forceinline__ void preload(const GemmProblem &p, int BN, int tile_m, int tile_n, int split, int S, int z0, int z1,
+  __device__ __forceinline__ void preload(const GemmProblem &p, const EpilogueShape &shape, int BN, int tile_m, int tile_n, int split, int S, int z0, int z1,
                                           int et, const float *col_scale) {
     bvec = rvec = make_float4(0.f, 0.f, 0.f, 0.f);
     cs = make_float4(1.f, 1.f, 1.f, 1.f);
-    const Where w(p, BN, tile_m, tile_n, split, S, z0, z1, et);
+    const Where w(p, shape, BN, tile_m, tile_n, split, S, z0, z1, et);
     if (w.r >= w.r_end) return;
     if (w.bias_per_col) bvec = *reinterpret_cast<const float4 *>(w.bias + w.n_base + w.c);
     if (COL_SCALE) cs = *reinterpret_cast<const float4 *>(col_scale + w.n_base + w.c);
     if (w.res) rvec = *reinterpret_cast<const float4 *>(w.res + (w.m_base + w.r) * p.res_sm + w.n_base + w.c);
   }
 
-  __device__ __forceinline__ void finish(const GemmProblem &p, const GemmEpilogue &e, float *staging, int pitch, int BN, int tile_m,
+  __device__ __forceinline__ void finish(const GemmProblem &p, const GemmEpilogue &e, const EpilogueShape &shape, float *staging, int pitch, int BN, int tile_m,
                                          int tile_n, int split, int S, int z0, int z1, int et, const float *col_scale) {
     asm volatile("" : "+r"(tile_m), "+r"(tile_n), "+r"(et));  // recompute: nothing of preload()'s geometry is kept
-    const Where w(p, BN, tile_m, tile_n, split, S, z0, z1, et);
+    const Where w(p, shape, BN, tile_m, tile_n, split, S, z0, z1, et);
     const float *bias = w.bias, *res = w.res;
     float *C = w.C;
     const int64_t n_base = w.n_base, m_base = w.m_base;
@@ -111,12 +124,6 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
       const int64_t n = n_base + c;
       const float *sp = staging + (size_t)r * pitch + c;
       const int sp_step = rows_pass * pitch;
-      uint32_t rank_addr[8];
-      if (S > 1) {
-#pragma unroll
-        for (int rank = 0; rank < 8; ++rank)
-          rank_addr[rank] = rank < S ? cluster_smem_addr(staging_addr + (uint32_t)(r * pitch + c) * 4u, (uint32_t)rank) : 0u;
-      }
       float *cp = C + (m_base + r) * p.c_sm + n;
       const int64_t c_step = (int64_t)rows_pass * p.c_sm;
       const float *rp = res ? res + (m_base + r) * p.res_sm + n : nullptr;
@@ -157,35 +164,63 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
         }
         if (res && r < r_end) rvec = *reinterpret_cast<const float4 *>(rp);
       }
-      for (; r < r_end; r += rows_pass) {
-        float4 acc;
-        if (S == 1) {
-          acc = *reinterpret_cast<const float4 *>(sp);
-        } else {
-          float4 t[8];
+      auto column_bias = [&]() {  // when it varies by row
+        if (p.bias_sn == 1) return *reinterpret_cast<const float4 *>(bp);
+        const float t = *bp;
+        return make_float4(t, t, t, t);
+      };
+      if (S == 1) {
+        for (; r < r_end; r += rows_pass) {
+          const float4 acc = *reinterpret_cast<const float4 *>(sp), rq = rvec;
+          if (bias && !bias_per_col) bvec = column_bias();
+          rp += r_step;
+          if (res && r + rows_pass < r_end) rvec = *reinterpret_cast<const float4 *>(rp);  // the next row's, under this row's arithmetic
+          *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq);
+          sp += sp_step; cp += c_step; bp += b_step;
+        }
+      } else {
+        // Partial sums of the ranks through distributed shared memory, eight 16-byte loads in flight:
+        // 8 / S rows of S ranks.
+        const uint32_t own = staging_addr + (uint32_t)(r * pitch + c) * 4u;
+        auto rows = [&](auto ranks) {
+          constexpr int kRanks = decltype(ranks)::value, kRows = 8 / kRanks;
+          uint32_t at[kRanks];
 #pragma unroll
-          for (int rank = 0; rank < 8; ++rank)
-            if (rank < S)
-              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                           : "=f"(t[rank].x), "=f"(t[rank].y), "=f"(t[rank].z), "=f"(t[rank].w)
-                           : "r"(rank_addr[rank]) : "memory");
-          acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int k = 0; k < kRanks; ++k) at[k] = cluster_smem_addr(own, (uint32_t)k);
+          while (r < r_end) {
+            float4 t[kRows][kRanks], rq[kRows];
+            rq[0] = rvec;
 #pragma unroll
-          for (int rank = 0; rank < 8; ++rank)
-            if (rank < S) {
-              acc.x += t[rank].x; acc.y += t[rank].y; acc.z += t[rank].z; acc.w += t[rank].w;
-              rank_addr[rank] += (uint32_t)sp_step * 4u;
+            for (int u = 0; u < kRows; ++u) {
+              const bool live = r + u * rows_pass < r_end;
+              if (u > 0) rq[u] = res && live ? *reinterpret_cast<const float4 *>(rp + u * r_step) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+              for (int k = 0; k < kRanks; ++k)
+                if (live)
+                  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                               : "=f"(t[u][k].x), "=f"(t[u][k].y), "=f"(t[u][k].z), "=f"(t[u][k].w)
+                               : "r"(at[k] + (uint32_t)(u * sp_step) * 4u) : "memory");
             }
-        }
-        if (bias && !bias_per_col) {
-          if (p.bias_sn == 1) bvec = *reinterpret_cast<const float4 *>(bp);
-          else { const float t = *bp; bvec = make_float4(t, t, t, t); }
-        }
-        const float4 rq = rvec;
-        rp += r_step;
-        if (res && r + rows_pass < r_end) rvec = *reinterpret_cast<const float4 *>(rp);  // the next row's, under this row's arithmetic
-        *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq);
-        sp += sp_step; cp += c_step; bp += b_step;
+#pragma unroll
+            for (int u = 0; u < kRows; ++u) {
+              if (r + u * rows_pass >= r_end) break;
+              float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+              for (int k = 0; k < kRanks; ++k) { acc.x += t[u][k].x; acc.y += t[u][k].y; acc.z += t[u][k].z; acc.w += t[u][k].w; }
+              if (bias && !bias_per_col) bvec = column_bias();
+              *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq[u]);
+              cp += c_step; bp += b_step;
+            }
+            r += kRows * rows_pass;
+            rp += kRows * r_step;
+            if (res && r < r_end) rvec = *reinterpret_cast<const float4 *>(rp);
+#pragma unroll
+            for (int k = 0; k < kRanks; ++k) at[k] += (uint32_t)(kRows * sp_step) * 4u;
+          }
+        };
+        if (S == 2) rows(std::integral_constant<int, 2>());
+        else if (S == 4) rows(std::integral_constant<int, 4>());
+        else rows(std::integral_constant<int, 8>());
       }
     } else {
       // ragged column edge or non-unit strides: one element at a time, indices recomputed

@@ -51,6 +51,7 @@ constexpr int kConvThreads = 256;
 struct PairArgs {
   GemmProblem p;
   GemmEpilogue e;
+  EpilogueShape shape;
   const char *packed;       // B atoms
   const float *col_scale;   // 2^-s of each column
   int n_pad;                // columns in the packed image (multiple of 16)
@@ -359,7 +360,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         if (lane == 0) mbar_arrive(bar_conv + 8u * mb.s);
         mb.step(a.stages_b); mb.step(a.stages_b);
       }
-      if (!attempt) epi.preload(a.p, BN, tile_m, tile_n, split, a.split_k, z0, z1, threadIdx.x - 64, a.col_scale);
+      if (!attempt) epi.preload(a.p, a.shape, BN, tile_m, tile_n, split, a.split_k, z0, z1, threadIdx.x - 64, a.col_scale);
       if (ok) ok = mbar_wait(bar_accum, (uint32_t)attempt, abort_flag);
       if (attempt) break;
       // A row whose hi overflowed shows it in every column of the accumulator; one on the default scale
@@ -410,8 +411,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   const int S = a.split_k;
   if (S > 1) cluster_sync_all();
   if (warp >= 2)
-    epi.finish(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, threadIdx.x - 64, a.col_scale);
-  if (S > 1) cluster_sync_all();
+    epi.finish(a.p, a.e, a.shape, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, threadIdx.x - 64, a.col_scale);
+  if (S > 1) cluster_sync_relaxed();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
@@ -566,6 +567,7 @@ bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &p
 int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const PairPlan &plan, const void *packed, cudaStream_t s) {
   PairArgs a;
   a.p = p; a.e = e;
+  a.shape = epilogue_shape(plan.tile_n, kConvThreads);
   a.packed = static_cast<const char *>(packed);
   a.col_scale = reinterpret_cast<const float *>(a.packed + atoms_bytes(p.K, p.N));
   a.n_pad = n_padded(p.N);

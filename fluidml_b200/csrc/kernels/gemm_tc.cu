@@ -49,6 +49,7 @@ constexpr size_t kSmemBudget = 200 * 1024;
 struct TcArgs {
   GemmProblem p;
   GemmEpilogue e;
+  EpilogueShape shape;
   int tile_n, split_k, stages, b_mn_major, three_pass, a_tmem;
   int tiles_m, tiles_n, kb_total, kb_per_split;
   int *status;
@@ -406,11 +407,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp >= 2) {
     const int et = threadIdx.x - 64;
     TileEpilogue<ACT, 128, false> epi;
-    epi.preload(a.p, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
-    epi.finish(a.p, a.e, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
+    epi.preload(a.p, a.shape, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
+    epi.finish(a.p, a.e, a.shape, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, et, nullptr);
     if (et == 0) TRACE(5);
   }
-  if (S > 1) cluster_sync_all();  // nobody leaves while a peer may still read its tile
+  if (S > 1) cluster_sync_relaxed();  // nobody leaves while a peer may still read its tile
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
@@ -560,6 +561,7 @@ bool plan_gemm_tc(const GemmProblem &p, const fml_gemm_params &gp, TcPlan &plan)
 int launch_gemm_tc(const GemmProblem &p, const GemmEpilogue &e, const TcPlan &plan, cudaStream_t s) {
   TcArgs a;
   a.p = p; a.e = e;
+  a.shape = epilogue_shape(plan.tile_n, 128);
   a.tile_n = plan.tile_n; a.split_k = plan.split_k; a.stages = plan.stages;
   a.b_mn_major = plan.b_mn_major; a.three_pass = plan.three_pass; a.a_tmem = plan.a_tmem;
   a.tiles_m = (int)((p.M + kBM - 1) / kBM);
