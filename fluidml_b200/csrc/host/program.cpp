@@ -1,4 +1,5 @@
 #include "program.h"
+#include "transfer.h"
 #include <algorithm>
 #include <unordered_set>
 #include <cstdio>
@@ -157,8 +158,15 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
   Check(fml_memset(prog->arena, 0, prog->arena_bytes, nullptr), "clearing the arena");
   std::unordered_map<const flow::Region *, size_t> io_offset;
   size_t io_bytes = 0;
+  for (const std::vector<std::string> *names : {&flow.inputs, &flow.outputs})  // side by side, in interface order
+    for (const std::string &name : *names) {
+      const flow::RegionPtr r = flow.Get(name);
+      if (io_offset.count(r.get())) continue;
+      io_offset[r.get()] = io_bytes;
+      io_bytes = AlignUp(io_bytes + r->meta.GetSize(), 256);
+    }
   for (const auto &r : flow.regions) {
-    if (r->kind != flow::Region::kInput && r->kind != flow::Region::kOutput) continue;
+    if ((r->kind != flow::Region::kInput && r->kind != flow::Region::kOutput) || io_offset.count(r.get())) continue;
     io_offset[r.get()] = io_bytes;
     io_bytes = AlignUp(io_bytes + r->meta.GetSize(), 256);
   }
@@ -389,7 +397,7 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
 
 // ------------------------------------------------------------------------------ Runner
 Runner::Runner(std::unique_ptr<Program> program, const Options &options)
-    : program_(std::move(program)), options_(options) {
+    : program_(std::move(program)), options_(options), transfer_(new Transfer(*program_)) {
   Check(fml_set_device(options_.device), "selecting the device");
   Check(fml_stream_create(&stream_), "creating the stream");
   Check(fml_event_create(&ev_start_), "creating an event");
@@ -442,17 +450,17 @@ size_t Runner::Run(const std::unordered_map<std::string, void *> &args, size_t e
   std::vector<void *> in_host, out_host;
   for (const auto &b : program_->inputs) in_host.push_back(args.at(b.name));
   for (const auto &b : program_->outputs) out_host.push_back(args.at(b.name));
-  for (size_t i = 0; i < in_host.size(); ++i) {
+  for (size_t i = 0; i < in_host.size(); ++i)
     if (!in_host[i]) throw Error("input '" + program_->inputs[i].name + "' is a null pointer");
-    Check(fml_memcpy_h2d(program_->inputs[i].device, in_host[i], program_->inputs[i].bytes, stream_), "copying an input");
-  }
+  for (size_t i = 0; i < out_host.size(); ++i)
+    if (!out_host[i]) throw Error("output '" + program_->outputs[i].name + "' is a null pointer");
+  transfer_->Begin(in_host, out_host);
+  transfer_->Upload(stream_);
   Check(fml_event_record(ev_start_, stream_), "recording an event");
   for (size_t e = 0; e < epoch; ++e) Replay();
   Check(fml_event_record(ev_stop_, stream_), "recording an event");
-  for (size_t i = 0; i < out_host.size(); ++i) {
-    if (!out_host[i]) throw Error("output '" + program_->outputs[i].name + "' is a null pointer");
-    Check(fml_memcpy_d2h(out_host[i], program_->outputs[i].device, program_->outputs[i].bytes, stream_), "copying an output");
-  }
+  transfer_->Download(stream_);
+  transfer_->Finish(stream_);
   const int status = fml_check_device(stream_);
   if (status == FML_DEVICE_TIMEOUT)  // a resident program's buffers hold mixed generations after an abandoned pass
     for (fml_resident *r : program_->resident_programs) fml_resident_reset(r, stream_);

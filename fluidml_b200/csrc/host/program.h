@@ -86,6 +86,8 @@ public:
                                       const Options &options);
 };
 
+class Transfer;
+
 class Runner {
 public:
   Runner(std::unique_ptr<Program> program, const Options &options);
@@ -111,6 +113,7 @@ private:
   void Replay();
   std::unique_ptr<Program> program_;
   Options options_;
+  std::unique_ptr<Transfer> transfer_;
   void *stream_ = nullptr;
   void *graph_exec_ = nullptr;
   void *ev_start_ = nullptr, *ev_stop_ = nullptr;

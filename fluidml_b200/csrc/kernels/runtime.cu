@@ -30,6 +30,8 @@ bool pdl_enabled() {
   return on;
 }
 
+// The status word of a device: page-locked host memory that its kernels write through the link (they
+// only do when something went wrong), so that a check after a synchronisation is a plain read.
 static int *g_status[64] = {nullptr};
 static std::mutex g_status_mu;
 
@@ -39,8 +41,8 @@ int *device_status_word() {
   std::lock_guard<std::mutex> lock(g_status_mu);
   if (!g_status[dev]) {
     int *p = nullptr;
-    if (cudaMalloc(&p, sizeof(int)) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, sizeof(int));
+    if (cudaHostAlloc(reinterpret_cast<void **>(&p), sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    *p = 0;
     g_status[dev] = p;
   }
   return g_status[dev];
@@ -50,6 +52,11 @@ int *device_status_word() {
 
 // Takes the device status word: *out = old value, word = 0.  `out` is pinned host memory.
 static __global__ void status_take_kernel(int *word, int *out) { *out = atomicExch(word, 0); }
+
+// Small blocks between page-locked host memory and the device (either direction).
+static __global__ void __launch_bounds__(256) copy_small_kernel(uint4 *dst, const uint4 *src, size_t n) {
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) dst[i] = src[i];
+}
 
 using namespace fml;
 
@@ -113,6 +120,18 @@ int fml_host_alloc_pinned(void **ptr, size_t bytes) {
 
 int fml_host_free_pinned(void *ptr) {
   FML_CUDA(cudaFreeHost(ptr));
+  return FML_OK;
+}
+
+int fml_copy_small(void *dst, const void *src, size_t bytes, void *stream) {
+  FML_REQUIRE(dst && src, FML_BAD_ARG, "fml_copy_small: null argument");
+  FML_REQUIRE(((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0, FML_MISALIGNED,
+              "fml_copy_small: both sides must be 16-byte aligned");
+  const size_t n = (bytes + 15) / 16;
+  if (!n) return FML_OK;
+  copy_small_kernel<<<(unsigned)((n + 255) / 256 < 64 ? (n + 255) / 256 : 64), 256, 0, as_stream(stream)>>>(
+      static_cast<uint4 *>(dst), static_cast<const uint4 *>(src), n);
+  FML_CUDA(cudaGetLastError());
   return FML_OK;
 }
 
@@ -207,10 +226,11 @@ int fml_warmup(void) {
 int fml_check_device(void *stream) {
   int *w = device_status_word();
   FML_REQUIRE(w, FML_CUDA_ERROR, "fml_check_device: no status word");
-  // One launch on the caller's stream takes the word (atomic exchange with 0, so a bit another
-  // stream's kernel sets at the same moment is either taken now or left for the next check, never
-  // lost) and writes it to a pinned host word; one synchronisation then serves both the caller's
-  // work and the check.  One pinned word per calling thread.
+  FML_CUDA(cudaStreamSynchronize(as_stream(stream)));
+  if (*static_cast<volatile int *>(w) == 0) return FML_OK;
+  // A bit is set: a launch on the caller's stream takes the word (device-side atomic exchange with 0,
+  // so a bit another stream's kernel sets at the same moment is either taken now or left for the next
+  // check, never lost) and writes it to a pinned host word.  One pinned word per calling thread.
   static thread_local int *pinned = nullptr;
   if (!pinned) FML_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&pinned), sizeof(int), cudaHostAllocDefault));
   status_take_kernel<<<1, 1, 0, as_stream(stream)>>>(w, pinned);

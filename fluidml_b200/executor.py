@@ -44,6 +44,8 @@ PLAIN_LINEAR, PLAIN_GREEDY, DP_GREEDY = 0, 1, 2
 class Executor:
     def __init__(self, name: str, mode: int, epoch: int = 1):
         self._h = ctypes.c_void_p()
+        self._names: dict = {}
+        self._invoke = lib().fml_executor_invoke
         st = lib().fml_executor_create(name.encode(), mode, ctypes.c_size_t(epoch), ctypes.byref(self._h))
         self._check(st)
 
@@ -97,17 +99,30 @@ class Executor:
         return self.stats()
 
     def invoke(self, args: Dict[str, np.ndarray]) -> int:
-        names, ptrs = [], []
+        # the binding itself is a visible part of a small model's pass: the name array of a set of
+        # arguments is kept, and addresses are taken through the buffer protocol (`ndarray.ctypes` builds
+        # an object per access, 2 us each)
+        keys = tuple(args)
+        entry = self._names.get(keys)
+        if entry is None:
+            n = len(keys)
+            entry = (n, (ctypes.c_char_p * n)(*[k.encode() for k in keys]), ctypes.c_void_p * n, ctypes.c_size_t(n))
+            if len(self._names) >= 16:
+                self._names.clear()
+            self._names[keys] = entry
+        n, c_names, ptr_array, count = entry
+        ptrs = ptr_array()
+        i = 0
         for k, a in args.items():
-            if not isinstance(a, np.ndarray) or not a.flags["C_CONTIGUOUS"]:
+            if not isinstance(a, np.ndarray) or not a.flags.c_contiguous:
                 raise TypeError(f"argument '{k}' must be a C-contiguous numpy array")
-            names.append(k.encode())
-            ptrs.append(a.ctypes.data)
-        n = len(names)
-        c_names = (ctypes.c_char_p * n)(*names)
-        c_ptrs = (ctypes.c_void_p * n)(*ptrs)
+            try:
+                ptrs[i] = ctypes.addressof(ctypes.c_char.from_buffer(a))
+            except (TypeError, ValueError, BufferError):  # read-only or empty
+                ptrs[i] = a.ctypes.data
+            i += 1
         ns = ctypes.c_size_t()
-        self._check(lib().fml_executor_invoke(self._h, c_names, c_ptrs, ctypes.c_size_t(n), ctypes.byref(ns)))
+        self._check(self._invoke(self._h, c_names, ptrs, count, ctypes.byref(ns)))
         return ns.value
 
     def profile(self, args: Dict[str, np.ndarray], passes: int = 1) -> dict:

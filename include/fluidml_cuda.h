@@ -70,6 +70,9 @@ int fml_memcpy_d2h(void *dst, const void *src, size_t bytes, void *stream);
 int fml_memcpy_d2d(void *dst, const void *src, size_t bytes, void *stream);
 int fml_host_alloc_pinned(void **ptr, size_t bytes);
 int fml_host_free_pinned(void *ptr);
+/* Copies a small block with a kernel, without the copy engine's latency: either side may be page-locked
+ * host memory.  Both addresses 16-byte aligned; up to 15 bytes beyond `bytes` are read and written. */
+int fml_copy_small(void *dst, const void *src, size_t bytes, void *stream);
 int fml_stream_create(void **stream);
 int fml_stream_destroy(void *stream);
 int fml_stream_sync(void *stream);
