@@ -296,8 +296,12 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
     auto it = cache.find(key);
     if (it != cache.end()) { take(it->second); return FML_OK; }
   }
-  cudaStream_t s = as_stream(stream);
+  // Candidates run as a captured graph of back-to-back launches, as the products of a model do: timed
+  // one by one from the host, launches of a few microseconds are paced by the host and the choice is noise.
+  FML_CUDA(cudaStreamSynchronize(as_stream(stream)));
+  cudaStream_t s;
   cudaEvent_t e0, e1;
+  FML_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   FML_CUDA(cudaEventCreate(&e0));
   FML_CUDA(cudaEventCreate(&e1));
   const GemmEpilogue epi = make_epilogue(*gp, bias != nullptr, residual != nullptr);
@@ -325,19 +329,31 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
         auto launch = [&] {
           return pair ? launch_gemm_pair(p, epi, cand.pair, gp->b_packed, s) : launch_gemm_tc(p, epi, cand.tc, s);
         };
-        const int reps = 6;
         if (launch() != FML_OK) { cudaGetLastError(); continue; }  // warm-up; skip what cannot launch
-        cudaEventRecord(e0, s);
-        bool ok = true;
+        const int reps = 8;
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         for (int r = 0; r < reps && ok; ++r) ok = launch() == FML_OK;
-        cudaEventRecord(e1, s);
-        if (cudaEventSynchronize(e1) != cudaSuccess || !ok) { cudaGetLastError(); continue; }
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
+        ok = cudaStreamEndCapture(s, &graph) == cudaSuccess && ok && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+        if (graph) cudaGraphDestroy(graph);
+        float ms = 1e30f;
+        for (int r = 0; r < 4 && ok; ++r) {  // the first replay warms up
+          cudaEventRecord(e0, s);
+          ok = cudaGraphLaunch(exec, s) == cudaSuccess;
+          cudaEventRecord(e1, s);
+          ok = cudaEventSynchronize(e1) == cudaSuccess && ok;
+          float t = 0;
+          cudaEventElapsedTime(&t, e0, e1);
+          if (r && t < ms) ms = t;
+        }
+        if (exec) cudaGraphExecDestroy(exec);
+        if (!ok) { cudaGetLastError(); continue; }
         if (ms < best) { best = ms; best_tiles = id; }
       }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  cudaStreamDestroy(s);
   take(best_tiles);
   std::lock_guard<std::mutex> lock(mu);
   cache[key] = best_tiles;
