@@ -53,7 +53,8 @@ class GemmParams(ctypes.Structure):
 class ConvParams(ctypes.Structure):
     _fields_ = [("pads_begin", ctypes.c_int64 * 2), ("strides", ctypes.c_int64 * 2),
                 ("dilations", ctypes.c_int64 * 2), ("group", ctypes.c_int64),
-                ("act", ctypes.c_int32), ("precision", ctypes.c_int32)]
+                ("act", ctypes.c_int32), ("precision", ctypes.c_int32), ("w_packed", ctypes.c_void_p),
+                ("tile_n", ctypes.c_int32), ("strips", ctypes.c_int32), ("split_k", ctypes.c_int32), ("ctas_per_sm", ctypes.c_int32)]
 
 
 _lib = None
@@ -326,8 +327,28 @@ def gemm_skinny_noalloc(a, b, c, bias=None, residual=None, params=None, stream=N
                                         ctypes.byref(params), stream))
 
 
-def conv(x, w, bias, y, pads_begin, strides, dilations, group=1, act=ACT_NONE, stream=None, precision=None):
+def conv_pack(w, stream=None) -> "DeviceBuffer":
+    """The packed copy of constant convolution weights for conv(..., packed=); keep it alive."""
+    L = lib()
+    L.fml_conv_packed_bytes.restype = ctypes.c_size_t
+    n = L.fml_conv_packed_bytes(_ref(w))
+    buf = DeviceBuffer(n)
+    check(L.fml_conv_pack(_ref(w), ctypes.c_void_p(buf.ptr), ctypes.c_size_t(n), stream))
+    return buf
+
+
+def conv_uses_packed(x, w, y, pads_begin, scaled=False) -> bool:
+    p, u = ConvParams(), ctypes.c_int()
+    for i in range(2):
+        p.pads_begin[i], p.strides[i], p.dilations[i] = pads_begin[i], 1, 1
+    p.group = 1
+    check(lib().fml_conv_uses_packed(_ref(x), _ref(w), _ref(y), ctypes.byref(p), int(scaled), ctypes.byref(u)))
+    return bool(u.value)
+
+
+def conv(x, w, bias, y, pads_begin, strides, dilations, group=1, act=ACT_NONE, stream=None, precision=None, packed=None):
     p = ConvParams()
+    p.w_packed = packed.ptr if packed is not None else None
     nd = len(pads_begin)
     for i in range(2):
         p.pads_begin[i] = pads_begin[i] if i < nd else 0
@@ -337,9 +358,10 @@ def conv(x, w, bias, y, pads_begin, strides, dilations, group=1, act=ACT_NONE, s
     check(lib().fml_conv(_ref(x), _ref(w), _ref(bias), _ref(y), ctypes.byref(p), stream))
 
 
-def conv_scaled(x, x_scale, w, bias, y, pads_begin, strides, dilations, act=ACT_NONE, stream=None, precision=None):
+def conv_scaled(x, x_scale, w, bias, y, pads_begin, strides, dilations, act=ACT_NONE, stream=None, precision=None, packed=None):
     """y = conv(x * x_scale, w) + bias with x_scale broadcastable to [N, IC, 1, 1] (group 1)."""
     p = ConvParams()
+    p.w_packed = packed.ptr if packed is not None else None
     nd = len(pads_begin)
     for i in range(2):
         p.pads_begin[i] = pads_begin[i] if i < nd else 0

@@ -151,7 +151,7 @@ public:
 private:
   // One file per (model bytes, mode, options that shape the plan): text lines
   //   layout <tensor> <p0> <p1> ...      physical position of every logical dim
-  //   tiles <node> <tile_n> <split_k> <CTAs per SM>    tuned GEMM tiles
+  //   tiles <node> <tile_n> <split_k> <CTAs per SM> <strips>    tuned GEMM / convolution tiles
   struct PlanCacheEntry {
     std::map<std::string, std::vector<size_t>> layouts;
     std::map<std::string, kernel::GemmTiles> tiles;
@@ -175,6 +175,7 @@ private:
           kernel::GemmTiles t;
           ls >> t.tile_n >> t.split_k;
           if (!(ls >> t.ctas_per_sm)) t.ctas_per_sm = 0;
+          if (!(ls >> t.strips)) t.strips = 0;
           if (t.tile_n > 0 && t.split_k > 0) tiles[name] = t;
         }
       }
@@ -190,7 +191,7 @@ private:
           for (size_t v : kv.second) out << " " << v;
           out << "\n";
         }
-        for (const auto &kv : tiles) out << "tiles " << kv.first << " " << kv.second.tile_n << " " << kv.second.split_k << " " << kv.second.ctas_per_sm << "\n";
+        for (const auto &kv : tiles) out << "tiles " << kv.first << " " << kv.second.tile_n << " " << kv.second.split_k << " " << kv.second.ctas_per_sm << " " << kv.second.strips << "\n";
         out << "end\n";
       }
       std::rename(tmp.c_str(), path.c_str());

@@ -576,6 +576,7 @@ public:
     *source = b;
     return fml_gemm_packed_bytes(b.shape[0], b.shape[1]);
   }
+  int Pack(const fml_tensor &source, void *packed, size_t bytes) const override { return fml_gemm_pack(&source, packed, bytes, nullptr); }
   void SetPacked(const void *packed, size_t bytes) override {
     c_.params.b_packed = packed;
     packed_bytes_ = bytes;
@@ -650,16 +651,44 @@ private:
   mutable GemmTiles tuned_;
 };
 
+// Tile choices of a convolution with packed weights: tuned on the device while the builder records
+// (device buffers are live), or taken over from an earlier Compile.
+fml_conv_params TuneConv(const char *name, const fml_tensor &x, const fml_tensor *scale, const fml_tensor &w, const fml_tensor *bias,
+                         const fml_tensor &y, const fml_conv_params &p, bool autotune) {
+  fml_conv_params tuned = p;
+  if (autotune && p.w_packed && fml_conv_autotune(&x, scale, &w, bias, &y, &p, nullptr, &tuned) != FML_OK)
+    throw Error(std::string(name) + ": " + fml_last_error());
+  return tuned;
+}
+void PresetConvTiles(const GemmTiles &t, fml_conv_params *p) {
+  p->tile_n = t.tile_n; p->split_k = t.split_k; p->ctas_per_sm = t.ctas_per_sm; p->strips = t.strips;
+}
+bool TunedConvTiles(const fml_conv_params &p, GemmTiles *t) {
+  if (p.tile_n <= 0) return false;
+  *t = {p.tile_n, p.split_k, p.ctas_per_sm, p.strips};
+  return true;
+}
+
 // conv.cpp:27-280
 class ConvKernel : public SingleInputWithoutBufferKernel {
 public:
-  ConvKernel(const char *name, fml_tensor w, bool has_bias, fml_tensor bias, fml_conv_params p)
-      : name_(name), w_(w), has_bias_(has_bias), bias_(bias), p_(p) {}
+  ConvKernel(const char *name, fml_tensor w, bool has_bias, fml_tensor bias, fml_conv_params p, bool autotune)
+      : name_(name), w_(w), has_bias_(has_bias), bias_(bias), p_(p), autotune_(autotune) {}
   std::string GetKernelName() const override { return name_; }
+  size_t PackedBytes(const std::vector<fml_tensor> &in, const fml_tensor &output, fml_tensor *source) const override {
+    int uses = 0;
+    if (fml_conv_uses_packed(&in.at(0), &w_, &output, &p_, 0, &uses) != FML_OK || !uses) return 0;
+    *source = w_;
+    return fml_conv_packed_bytes(&w_);
+  }
+  int Pack(const fml_tensor &source, void *packed, size_t bytes) const override { return fml_conv_pack(&source, packed, bytes, nullptr); }
+  void SetPacked(const void *packed, size_t) override { p_.w_packed = packed; }
+  void PresetTiles(const GemmTiles &t) override { PresetConvTiles(t, &p_); }
+  bool TunedTiles(GemmTiles *t) const override { return TunedConvTiles(tuned_, t); }
   void Run(LaunchRecorder &rec, const fml_tensor &input, const fml_tensor &output) const override {
     const fml_tensor w = w_, b = bias_;
     const bool hb = has_bias_;
-    const fml_conv_params p = p_;
+    const fml_conv_params p = tuned_ = TuneConv(name_, input, nullptr, w, hb ? &b : nullptr, output, p_, autotune_);
     rec.Add(name_, [=](void *s) { return fml_conv(&input, &w, hb ? &b : nullptr, &output, &p, s); });
   }
 
@@ -669,18 +698,30 @@ private:
   bool has_bias_;
   fml_tensor bias_;
   fml_conv_params p_;
+  bool autotune_;
+  mutable fml_conv_params tuned_{};
 };
 
 // mul.cpp + conv.cpp: the per-channel gate multiplies x inside the convolution's operand gather
 class ScaledConvKernel : public DoubleInputsWithoutBufferKernel {
 public:
-  ScaledConvKernel(const char *name, fml_tensor w, bool has_bias, fml_tensor bias, fml_conv_params p)
-      : name_(name), w_(w), has_bias_(has_bias), bias_(bias), p_(p) {}
+  ScaledConvKernel(const char *name, fml_tensor w, bool has_bias, fml_tensor bias, fml_conv_params p, bool autotune)
+      : name_(name), w_(w), has_bias_(has_bias), bias_(bias), p_(p), autotune_(autotune) {}
   std::string GetKernelName() const override { return name_; }
+  size_t PackedBytes(const std::vector<fml_tensor> &in, const fml_tensor &output, fml_tensor *source) const override {
+    int uses = 0;
+    if (fml_conv_uses_packed(&in.at(0), &w_, &output, &p_, 1, &uses) != FML_OK || !uses) return 0;
+    *source = w_;
+    return fml_conv_packed_bytes(&w_);
+  }
+  int Pack(const fml_tensor &source, void *packed, size_t bytes) const override { return fml_conv_pack(&source, packed, bytes, nullptr); }
+  void SetPacked(const void *packed, size_t) override { p_.w_packed = packed; }
+  void PresetTiles(const GemmTiles &t) override { PresetConvTiles(t, &p_); }
+  bool TunedTiles(GemmTiles *t) const override { return TunedConvTiles(tuned_, t); }
   void Run(LaunchRecorder &rec, const fml_tensor &x, const fml_tensor &scale, const fml_tensor &output) const override {
     const fml_tensor w = w_, b = bias_;
     const bool hb = has_bias_;
-    const fml_conv_params p = p_;
+    const fml_conv_params p = tuned_ = TuneConv(name_, x, &scale, w, hb ? &b : nullptr, output, p_, autotune_);
     rec.Add(name_, [=](void *s) { return fml_conv_scaled(&x, &scale, &w, hb ? &b : nullptr, &output, &p, s); });
   }
 
@@ -690,6 +731,8 @@ private:
   bool has_bias_;
   fml_tensor bias_;
   fml_conv_params p_;
+  bool autotune_;
+  mutable fml_conv_params tuned_{};
 };
 
 // maxpool.cpp:17-82, averagepool.cpp:19-87
@@ -847,8 +890,8 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
     p.act = n.act;
     p.precision = options.gemm_precision;
     const char *name = n.kind == Kind::ConvWithPadding ? "ConvWithPaddingKernel" : "ConvWithoutPaddingKernel";
-    if (n.has_in_scale) return std::make_unique<ScaledConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, p);
-    return std::make_unique<ConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, p);
+    if (n.has_in_scale) return std::make_unique<ScaledConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, p, options.autotune);
+    return std::make_unique<ConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, p, options.autotune);
   }
   case Kind::MaxPoolWithoutPadding:
     return std::make_unique<PoolKernel>("MaxPoolWithoutPaddingKernel", 0, n.kernel_shape, n.strides);

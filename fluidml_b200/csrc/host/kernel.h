@@ -40,7 +40,7 @@ struct Buffer {
 };
 
 struct GemmTiles {
-  int tile_n = 0, split_k = 0, ctas_per_sm = 0;
+  int tile_n = 0, split_k = 0, ctas_per_sm = 0, strips = 0;  // strips: convolutions
 };
 
 class Kernel {
@@ -72,12 +72,16 @@ public:
     return false;
   }
   virtual void SetPrefetch(const void *ptr, size_t bytes) { (void)ptr; (void)bytes; }
-  // Device bytes of the packed form of its weights this kernel's launch would use (0 = none), and the
-  // call that makes it: the builder provides the memory, which lives as long as the program.
+  // Device bytes of the packed form of its weights this kernel's launch would use (0 = none), the
+  // call that makes it, and the call that announces it: the builder provides the memory, which lives as long as the program.
   // `source` names the constant, so that kernels sharing one share its packed form.
   virtual size_t PackedBytes(const std::vector<fml_tensor> &inputs, const fml_tensor &output, fml_tensor *source) const {
     (void)inputs; (void)output; (void)source;
     return 0;
+  }
+  virtual int Pack(const fml_tensor &source, void *packed, size_t bytes) const {
+    (void)source; (void)packed; (void)bytes;
+    return FML_UNSUPPORTED;
   }
   virtual void SetPacked(const void *packed, size_t bytes) { (void)packed; (void)bytes; }
   // Tile choices that can be carried from one Compile to the next (GEMM tile_n, split_k, CTAs per SM):

@@ -214,7 +214,7 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
   }
   // ---- packed weights: one blob for all kernels that have a packed form, made on the device
   if (!options.resident) {
-    struct Packed { fml_tensor source; size_t offset, bytes; };
+    struct Packed { fml_tensor source; size_t offset, bytes; const kernel::Kernel *maker; };
     std::vector<Packed> blobs;
     std::vector<std::pair<kernel::Kernel *, size_t>> users;
     size_t total = 0;
@@ -228,7 +228,7 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
       for (; i < blobs.size(); ++i)
         if (memcmp(&blobs[i].source, &source, sizeof(source)) == 0) break;
       if (i == blobs.size()) {
-        blobs.push_back({source, total, bytes});
+        blobs.push_back({source, total, bytes, kv.second.get()});
         total = AlignUp(total + bytes, 1024);
       }
       users.push_back({kv.second.get(), i});
@@ -236,7 +236,7 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
     if (total) {
       Check(fml_malloc(&prog->packed, total), "allocating the packed weights");
       for (const Packed &b : blobs)
-        Check(fml_gemm_pack(&b.source, (char *)prog->packed + b.offset, b.bytes, nullptr), "packing a weight");
+        Check(b.maker->Pack(b.source, (char *)prog->packed + b.offset, b.bytes), "packing a weight");
       Check(fml_stream_sync(nullptr), "packing the weights");
       for (const auto &u : users) u.first->SetPacked((char *)prog->packed + blobs[u.second].offset, blobs[u.second].bytes);
     }
@@ -254,7 +254,8 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
       const void *own = nullptr;
       size_t own_bytes = 0;
       if (!kernels[i].second->StreamedConstant(&own, &own_bytes)) continue;
-      if (next_ptr && next_ptr != own) kernels[i].second->SetPrefetch(next_ptr, next_bytes);
+      // no more than L2 can hold beside the kernel's own data: the rest would only displace the start again
+      if (next_ptr && next_ptr != own) kernels[i].second->SetPrefetch(next_ptr, std::min<size_t>(next_bytes, 48u << 20));
       next_ptr = own;
       next_bytes = own_bytes;
     }

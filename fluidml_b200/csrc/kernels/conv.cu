@@ -637,6 +637,8 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
   if (a.scale) {
     // the tensor-core kernel applies the scale while it splits the operand; every other case
     // takes the general implicit GEMM (the specialised CUDA-core paths below read x unscaled)
+    if (nd == 2 && a.IC <= 4096 && p->w_packed && conv_pair_eligible(x, w, y, p, true))
+      return launch_conv_pair(x, w, bias, y, p, s, a.scale, a.scale_sn, a.scale_sc);
     if (nd == 2 && a.IC <= 4096 && conv_tc_eligible(x, w, y, p))
       return launch_conv_tc(x, w, bias, y, p, s, a.scale, a.scale_sn, a.scale_sc);
     FML_REQUIRE((M + CB - 1) / CB <= 65535, FML_UNSUPPORTED, "fml_conv_scaled: too many output pixels for one launch");
@@ -679,6 +681,7 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
     gp.act = a.act;
     return fml_gemm(&A, &B, &Cc, a.bias ? &bias_t : nullptr, nullptr, &gp, stream);
   }
+  if (group == 1 && nd == 2 && p->w_packed && conv_pair_eligible(x, w, y, p, false)) return launch_conv_pair(x, w, bias, y, p, s);
   if (group == 1 && nd == 2 && conv_tc_eligible(x, w, y, p)) return launch_conv_tc(x, w, bias, y, p, s);
   if (group == 1 && a.KH == 1 && a.KW == 1 && a.ph == 0 && a.pw == 0 && a.sh == 1 && a.sw == 1 && a.ws[1] == 1 &&
       a.xs[3] == 1 && (nd == 1 || a.xs[2] == a.IW) && a.ys[3] == 1 && (nd == 1 || a.ys[2] == a.OW) &&
@@ -786,6 +789,41 @@ extern "C" int fml_conv_uses_tensor_cores(const fml_tensor *x, const fml_tensor 
                   y->dtype == FML_F32 && p->group <= 1 && conv_tc_eligible(x, w, y, p)
               ? 1 : 0;
   return FML_OK;
+}
+
+extern "C" int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p,
+                                    int scaled, int *uses) {
+  FML_REQUIRE(valid_tensor(x) && valid_tensor(w) && valid_tensor(y) && p && uses, FML_BAD_ARG, "fml_conv_uses_packed: bad argument");
+  *uses = x->rank == 4 && w->rank == 4 && y->rank == 4 && x->dtype == FML_F32 && w->dtype == FML_F32 && y->dtype == FML_F32 &&
+                  p->group <= 1 && x->shape[2] * x->shape[3] > 1 && (!scaled || x->shape[1] <= 4096) &&
+                  conv_pair_eligible(x, w, y, p, scaled != 0)
+              ? 1 : 0;
+  return FML_OK;
+}
+
+extern "C" int fml_conv_autotune(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
+                                 const fml_tensor *y, const fml_conv_params *p, void *stream, fml_conv_params *tuned) {
+  FML_REQUIRE(p && tuned, FML_BAD_ARG, "fml_conv_autotune: null argument");
+  *tuned = *p;
+  int uses = 0;
+  const int st = fml_conv_uses_packed(x, w, y, p, x_scale != nullptr, &uses);
+  if (st != FML_OK) return st;
+  if (!p->w_packed || !uses || p->tile_n) return FML_OK;  // nothing to choose
+  FML_CUDA(cudaStreamSynchronize(as_stream(stream)));
+  return tune_conv_pair(x, w, bias, y, p, x_scale ? (const float *)x_scale->data : nullptr,
+                        x_scale && x_scale->shape[0] != 1 ? x_scale->stride[0] : 0, x_scale && x_scale->shape[1] != 1 ? x_scale->stride[1] : 0,
+                        tuned);
+}
+
+extern "C" size_t fml_conv_packed_bytes(const fml_tensor *w) {
+  return w && w->rank == 4 && numel(w) > 0 ? conv_packed_bytes(w) : 0;
+}
+
+extern "C" int fml_conv_pack(const fml_tensor *w, void *packed, size_t bytes, void *stream) {
+  FML_REQUIRE(valid_tensor(w) && w->dtype == FML_F32 && w->rank == 4 && numel(w) > 0 && packed, FML_BAD_ARG, "fml_conv_pack: bad argument");
+  FML_REQUIRE(bytes >= conv_packed_bytes(w), FML_BAD_ARG, "fml_conv_pack: the destination is too small");
+  FML_REQUIRE(aligned16(packed), FML_MISALIGNED, "fml_conv_pack: the destination must be 16-byte aligned");
+  return conv_pack(w, packed, as_stream(stream));
 }
 
 extern "C" int fml_pool2d(const fml_tensor *x, const fml_tensor *y, int mode, const int64_t *kernel,

@@ -1,0 +1,989 @@
+// Implicit-GEMM convolution with packed weights on pairs of half-precision numbers (the arithmetic of
+// gemm_pair.cu: x = hi + lo, 22 significant bits, lo*hi + hi*lo + hi*hi in fp32) for group-1 2-D
+// convolutions in NCHW.  M = output pixels, N = output channels, K = (channel block of 32, tap).
+//
+// What bounds these layers and what follows from it: cutting every tap's operand out of the patch with
+// threads (conv_tc.cu: gather, split, tensor-memory store, nine times per pixel for 3 x 3) is slower than
+// the MMAs it feeds, and a 128 x 128 tile re-reads its weights so often that the fill path of an SM (about
+// 45 bytes per clock) is the next limit.  So:
+//   * the patch is split ONCE per channel block, into chunks of 8 channels: [chunk][pixel][8 x fp16].  Eight
+//     consecutive pixels of a chunk are then a core matrix of the unswizzled K-major layout whatever pixel
+//     they start at (16-byte steps), so the MMA reads the tap-shifted operand straight from shared memory:
+//     tap (kh, kw) is a start address (kh * width + kw) * 16 bytes further.  M is 16 groups of 8 pixels, the
+//     rows of an 8-pixel-wide strip: one stride between groups.
+//   * a CTA takes two such strips (16 x 16 pixels, or 256 pixels of a plane when there are no taps): both
+//     use a weight tile once it is on chip.
+//
+// Where the raw patch comes from (mode):
+//   kBox     tensor-map box, rows / columns / channels outside the image arrive as zeros (the padding)
+//   kFlat    rows that are no multiple of 16 bytes (14 x 14 maps): whole rows as a run of the flattened
+//            plane, side padding masked when the patch is split
+//   kRun     pointwise: 128 or 256 consecutive pixels of the plane
+//   kImages  pointwise over planes that are no multiple of 16 bytes (7 x 7): whole planes of several images
+//   kIm2col  few input channels (IC * KH * KW <= 64, any stride up to 4): K = (channel, tap) flattened, the
+//            split gathers the taps itself, so that a 3 x 3 layer over 3 channels is one k block, not nine
+//
+// Range of fp16: one power of two per tile (all pixels of a patch feed all rows through the taps), from the
+// largest magnitude of the first channel block, which lands in [2^9, 2^10): values down to 2^-12 of it keep
+// all 22 bits, and 2^6 of headroom is left.  The largest magnitude of every block is tracked; a tile that
+// outgrows its scale, or started on an all-zero block and then stayed far below the default scale, is done
+// a second time with the exact maximum (gemm_pair.cu).
+//
+// Roles, 320 threads: warp 0 loads, warp 1 issues MMAs, warps 2-9 split the patches and do the epilogue.
+#include "gemm_common.cuh"
+#include "pair_common.cuh"
+#include <algorithm>
+#include <cmath>
+#include <map>
+#include <mutex>
+#include <string>
+#include <vector>
+
+namespace fml {
+namespace {
+
+enum { kBox = 0, kFlat = 1, kRun = 2, kImages = 3, kIm2col = 4 };
+enum { kPlain = 0, kGated = 1, kTaps = 2 };
+constexpr int kThreads = 320;
+constexpr int kTargetExp = 9;         // first block's largest magnitude lands in [2^9, 2^10)
+constexpr int kDefaultScaleExp = 4;   // of a tile whose first block is all zero
+constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;
+
+struct ConvPairArgs {
+  int mode, N, IC, OC, OH, OW, KH, KW, taps;
+  int strides[2], ph, pw;
+  int n_icb, kb_total, icb_per_split, split_k;  // split over the cluster (1, 1, split_k)
+  int mt, tile_n, stages_b, group;              // strips per CTA; k blocks per B stage
+  int tiles_w, tiles_h, tiles_img;              // pixel tiles (kRun: tiles_h = 1; kImages: tiles_img groups of images)
+  int TW, TH;                                   // output pixels of a tile (8 or 16) x 16; kRun / kImages: TW = 128 mt
+  int cw, px;                                   // split patch: width in pixels, pixels in all
+  int raw_w, raw_ch, xoff, raw_bufs;            // raw patch: row pitch, elements between channels, first column; buffers
+  int patch_bufs;                               // buffers of the split patch (1 or 2)
+  uint32_t raw_bytes, raw_pitch;
+  uint32_t cw_magic;                            // px / cw == (px * cw_magic) >> 16
+  int IH, IW, plane, imgs;                      // input plane; images per tile (kImages)
+  const float *x;
+  const char *packed;
+  const float *col_scale;
+  int n_pad;
+  float *y;
+  int64_t ys[4];
+  const float *bias;
+  int64_t bias_stride;
+  int act;
+  const float *scale;                           // optional gate of x per (image, channel)
+  int64_t scale_sn, scale_sc;
+  const float *res;                             // optional residual, laid out as y
+  int *status;
+};
+
+__device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+
+// exp2-based exponential and approximate reciprocal for the sigmoids (about 2 ulp each), as in conv_tc.cu
+template <int ACT> __device__ __forceinline__ float act_of(float v) {
+  if (ACT == FML_ACT_RELU) return fmaxf(v, 0.0f);
+  if (ACT == FML_ACT_TANH) return tanhf(v);
+  if (ACT == FML_ACT_SIGMOID) return __fdividef(1.0f, 1.0f + __expf(-v));
+  if (ACT == FML_ACT_SILU) return __fdividef(v, 1.0f + __expf(-v));
+  return v;
+}
+
+// 32 channels of one pixel: accumulator * column scale + bias, activation, residual, stores a plane apart.
+// The activation is dispatched outside the unrolled loop (each CTA fetches this code once, cold).
+template <int ACT>
+__device__ __forceinline__ void store_channels(const float *v, const float2 *cb, float inv, float *yp, const float *rp, int64_t step,
+                                               int left) {
+  if (rp) {
+    float r[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = i < left ? rp[i * step] : 0.0f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < left) yp[i * step] = act_of<ACT>(fmaf(v[i] * inv, cb[i].x, cb[i].y)) + r[i];
+    return;
+  }
+  if (left >= 32) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i, yp += step) *yp = act_of<ACT>(fmaf(v[i] * inv, cb[i].x, cb[i].y));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i, yp += step)
+      if (i < left) *yp = act_of<ACT>(fmaf(v[i] * inv, cb[i].x, cb[i].y));
+  }
+}
+
+// Offset of output row `row` (of 128 mt) of a tile in y; false when it lies outside the image.
+__device__ __forceinline__ bool pixel_offset(const ConvPairArgs &a, int row, int n0, int n_img, int oh0, int ow0, int64_t *off) {
+  int n = n0, oh, ow;
+  if (a.mode == kRun || a.mode == kImages) {
+    int p = ow0 + row;
+    if (a.mode == kImages) {
+      const int im = row / a.plane;
+      if (im >= n_img) return false;
+      n += im;
+      p = row - im * a.plane;
+    } else if (p >= a.plane) {
+      return false;
+    }
+    oh = p / a.OW;
+    ow = p - oh * a.OW;
+  } else {
+    oh = oh0 + ((row & 127) >> 3);
+    ow = ow0 + (row >> 7) * 8 + (row & 7);
+    if (oh >= a.OH || ow >= a.OW) return false;
+  }
+  *off = (int64_t)n * a.ys[0] + (int64_t)oh * a.ys[2] + (int64_t)ow * a.ys[3];
+  return true;
+}
+
+// Channels c0, c0 + step, ... of one pixel from its row of summed partial tiles.
+template <int ACT>
+__device__ __forceinline__ void store_sums(const ConvPairArgs &a, const float *src, const float2 *cb, int64_t off, int oc0, int c0, int step,
+                                           int c_end) {
+#pragma unroll 4
+  for (int c = c0; c < c_end; c += step) {
+    const int64_t at = off + (int64_t)(oc0 + c) * a.ys[1];
+    const float o = act_of<ACT>(fmaf(src[c], cb[c].x, cb[c].y));
+    a.y[at] = a.res ? o + a.res[at] : o;
+  }
+}
+
+// SOURCE: how the split of a patch finds its eight values -- kPlain: eight channels, kGated: eight channels
+// times the gate, kTaps: eight (channel, tap) pairs.  A template parameter, and the loads plain selects: with
+// uniform branches inside the inner loop the split of 128 pixels x 32 channels took 2000 clocks, 340 of them
+// work.
+template <int SOURCE>
+__global__ void __launch_bounds__(kThreads, 2)
+conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int BN = a.tile_n, NB = a.stages_b, RB = a.raw_bufs, MT = a.mt;
+  const uint32_t kb_bytes = (uint32_t)BN * kPairB, b_bytes = kb_bytes * (uint32_t)a.group;
+  const uint32_t chunk = (uint32_t)a.px * 16u, patch_bytes = 8u * chunk;  // 4 chunks of hi, 4 of lo
+  const uint32_t patch_pitch = (patch_bytes + 1023u) & ~1023u;
+  const int pitch = BN + 4;  // split-K: the partial tile is staged over the rings, [128 MT][BN + 4] floats
+  const uint32_t ring_b = smem_u32(smem), patch0 = ring_b + (uint32_t)NB * b_bytes, raw0 = patch0 + (uint32_t)a.patch_bufs * patch_pitch;
+  uint8_t *const patch_ptr = smem + (size_t)NB * b_bytes;
+  const float *const raw_ptr = reinterpret_cast<const float *>(patch_ptr + a.patch_bufs * (size_t)patch_pitch);
+  float *const staging = reinterpret_cast<float *>(smem);
+  size_t data = (size_t)NB * b_bytes + a.patch_bufs * (size_t)patch_pitch + (size_t)RB * a.raw_pitch;
+  if (a.split_k > 1) data = max(data, (((size_t)kBM * MT * pitch * 4) + 127) & ~(size_t)127);
+  uint64_t *const bars = reinterpret_cast<uint64_t *>(smem + data);
+  const uint32_t bar_bfull = smem_u32(bars), bar_bempty = bar_bfull + 8u * NB;
+  const uint32_t bar_rfull = bar_bempty + 8u * NB, bar_rempty = bar_rfull + 8u * RB;
+  const uint32_t bar_pfull = bar_rempty + 8u * RB, bar_pempty = bar_pfull + 16u;
+  const uint32_t bar_accum = bar_pempty + 16u, bar_decide = bar_accum + 8u;
+  uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NB + 2 * RB + 6);
+  volatile int *const abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  volatile int *const redo_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
+  unsigned *const first_max = tmem_slot + 3;                             // bits of the first block's largest magnitude
+  unsigned *const tile_max = tmem_slot + 4;                              // ... and of all blocks'
+  // (the barriers are an even number and start on 16 bytes, so this does too)
+  float2 *const cb_s = reinterpret_cast<float2 *>(tmem_slot + 8);        // [BN]: column scale, bias
+  int *const koff_s = reinterpret_cast<int *>(cb_s + BN);                // [64]: kTaps, raw offset of k; negative: none
+  float *const scale_s = reinterpret_cast<float *>(koff_s + 64);         // [imgs][channels of this split]: the gate
+
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const bool leader = elect_one();
+  int t = blockIdx.x;
+  const int tw = t % a.tiles_w; t /= a.tiles_w;
+  const int th = t % a.tiles_h; t /= a.tiles_h;
+  const int n0 = a.mode == kImages ? t * a.imgs : t;  // first image of the tile
+  const int n_img = a.mode == kImages ? min(a.imgs, a.N - n0) : 1;
+  const int oc0 = blockIdx.y * BN;
+  const int oh0 = th * a.TH, ow0 = tw * a.TW;  // kRun: ow0 = first pixel of the plane
+  const int split = (int)blockIdx.z;
+  const int icb_lo = min(a.n_icb, split * a.icb_per_split), icb_hi = min(a.n_icb, icb_lo + a.icb_per_split);
+  const int n_icb = icb_hi - icb_lo, nkb = n_icb * a.taps;
+  uint32_t tmem_cols = 32;
+  while (tmem_cols < (uint32_t)(BN * MT)) tmem_cols <<= 1;
+  const int n_cols = min(BN, a.n_pad - oc0);  // the last tile of a ragged OC stops at the packed image's edge
+  const uint32_t b_run = (uint32_t)n_cols * kPairB;
+  const char *const b_src = a.packed + ((size_t)icb_lo * a.taps * a.n_pad + oc0) * kPairB;
+  auto load_b = [&](int kb, int s) {  // k blocks [kb, kb + group) of this CTA
+    const int count = min(a.group, nkb - kb);
+    mbar_expect_tx(bar_bfull + 8u * s, b_run * (uint32_t)count);
+    for (int g = 0; g < count; ++g)
+      bulk_load(ring_b + (uint32_t)s * b_bytes + (uint32_t)g * kb_bytes, b_src + (size_t)(kb + g) * a.n_pad * kPairB, b_run, bar_bfull + 8u * s);
+  };
+
+  if (threadIdx.x == 0) {
+    if (a.mode != kImages) tma_prefetch_map(&map_x);
+    for (int s = 0; s < NB; ++s) { mbar_init(bar_bfull + 8u * s, 1); mbar_init(bar_bempty + 8u * s, 1); }
+    for (int s = 0; s < RB; ++s) { mbar_init(bar_rfull + 8u * s, 1); mbar_init(bar_rempty + 8u * s, 8); }
+    for (int s = 0; s < 2; ++s) { mbar_init(bar_pfull + 8u * s, 8); mbar_init(bar_pempty + 8u * s, 1); }
+    mbar_init(bar_accum, 1);
+    mbar_init(bar_decide, 8);
+    *abort_flag = 0;
+    *redo_flag = 0;
+    *first_max = 0u;
+    *tile_max = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc(smem_u32(tmem_slot), tmem_cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  // Only now may the next kernel start (tensor memory: see gemm_tc.cu).
+  pdl_launch_dependents();
+  // The packed weights do not depend on the preceding kernel: the first stages are on their way while it drains.
+  const int b_stages_total = (nkb + a.group - 1) / a.group, pre_b = min(NB, b_stages_total);
+  if (warp == 0 && leader && !g_drop_loads)
+    for (int j = 0; j < pre_b; ++j) load_b(j * a.group, j);
+  if (warp >= 2) {
+    const int i = threadIdx.x - 64;
+    if (i < BN) cb_s[i].x = oc0 + i < a.n_pad ? a.col_scale[oc0 + i] : 0.0f;
+    if (SOURCE == kTaps && i < 64) {
+      const int tp = a.KH * a.KW, c = i / tp, r = i - c * tp, kh = r / a.KW;
+      koff_s[i] = c < a.IC ? c * a.raw_ch + kh * a.raw_w + (r - kh * a.KW) : -(1 << 20);
+    }
+  }
+  pdl_wait();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ loads
+    if (!g_drop_loads) {
+      bool ok = true;
+      int issued_r = 0, issued_b = pre_b;
+      RingPos rr, rb;
+      for (int j = 0; j < pre_b; ++j) rb.step(NB);
+      for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+        if (attempt) {
+          ok = mbar_wait_warp(bar_decide, 0u, abort_flag);
+          if (!ok || !*redo_flag) break;
+        }
+        int ir = 0, jb = attempt ? 0 : pre_b;
+        uint32_t idle = 0;
+        while (ir < n_icb || jb < b_stages_total) {  // whichever ring has room
+          bool moved = false;
+          if (ir < n_icb && mbar_test_warp(bar_rempty + 8u * rr.s, rr.ph ^ 1u)) {
+            const uint32_t bar = bar_rfull + 8u * rr.s, dst = raw0 + (uint32_t)rr.s * a.raw_pitch;
+            const int c0 = (icb_lo + ir) * kPK;
+            if (leader) {
+              if (a.mode == kBox) {
+                mbar_expect_tx(bar, a.raw_bytes);
+                tma_load_4d(dst, &map_x, bar, ow0 - a.pw - a.xoff, oh0 - a.ph, c0, n0);
+              } else if (a.mode == kIm2col) {  // every k block cuts its k values from the same few channels
+                mbar_expect_tx(bar, a.raw_bytes);
+                tma_load_4d(dst, &map_x, bar, ow0 * a.strides[1] - a.pw - a.xoff, oh0 * a.strides[0] - a.ph, 0, n0);
+              } else if (a.mode == kFlat) {
+                mbar_expect_tx(bar, a.raw_bytes);
+                tma_3d(dst, &map_x, bar, (oh0 - a.ph) * a.IW + ow0 - a.pw - a.xoff, c0, n0);
+              } else if (a.mode == kRun) {
+                mbar_expect_tx(bar, a.raw_bytes);
+                tma_3d(dst, &map_x, bar, ow0, c0, n0);
+              } else {
+                const uint32_t bytes = (uint32_t)(kPK * a.plane) * 4u;
+                mbar_expect_tx(bar, bytes * (uint32_t)n_img);
+                for (int i = 0; i < n_img; ++i)
+                  bulk_load(dst + (uint32_t)(i * kPK * a.plane) * 4u, a.x + ((size_t)(n0 + i) * a.IC + c0) * a.plane, bytes, bar);
+              }
+            }
+            ++ir; ++issued_r; moved = true;
+            rr.step(RB);
+          }
+          if (jb < b_stages_total && mbar_test_warp(bar_bempty + 8u * rb.s, rb.ph ^ 1u)) {
+            if (leader) load_b(jb * a.group, rb.s);
+            ++jb; ++issued_b; moved = true;
+            rb.step(NB);
+          }
+          if (moved) idle = 0;
+          else if ((++idle & 255u) == 0 && (*abort_flag || idle >= 64u * g_wait_limit)) { ok = false; break; }
+        }
+      }
+      if (!ok) {
+        if (leader) atomicOr(a.status, kStatusTimeout);
+        *abort_flag = 1;
+        volatile int never = 0;  // bounded drain of the loads in flight
+        for (int i = max(0, issued_r - RB); i < issued_r; ++i) mbar_wait_warp(bar_rfull + 8u * (i % RB), (uint32_t)(i / RB) & 1u, &never);
+        for (int i = max(0, issued_b - NB); i < issued_b; ++i) mbar_wait_warp(bar_bfull + 8u * (i % NB), (uint32_t)(i / NB) & 1u, &never);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    const uint32_t idesc = instr_desc_f16(BN);
+    const uint64_t desc_b = smem_desc(ring_b, 16u, 2 * kAtom, 4u);
+    // A: unswizzled core matrices of 8 pixels x 8 channels; LBO to the next 8 channels, SBO to the next group
+    const uint32_t group_bytes = a.mode == kRun || a.mode == kImages ? 128u : 16u * a.cw;
+    const uint32_t strip_bytes = a.mode == kRun || a.mode == kImages ? 2048u : 128u;
+    const uint64_t desc_a = smem_desc(patch0, chunk, group_bytes, 0u);
+    RingPos rb, rp;
+    bool ok = true;
+    for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+      if (attempt) {
+        ok = mbar_wait_warp(bar_decide, 0u, abort_flag);
+        if (!ok || !*redo_flag) break;
+      }
+      int in_group = 0, kb = 0;
+      for (int icb = 0; icb < n_icb && ok; ++icb) {
+        ok = mbar_wait_warp(bar_pfull + 8u * rp.s, rp.ph, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        int kh = 0, kw = 0;
+        for (int tap = 0; tap < a.taps; ++tap, ++kb) {
+          if (in_group == 0) {
+            ok = mbar_wait_warp(bar_bfull + 8u * rb.s, rb.ph, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          const bool last_of_group = in_group + 1 == a.group || kb + 1 == nkb;
+          if (leader) {
+            const uint64_t db0 = desc_b + (((uint32_t)rb.s * b_bytes + (uint32_t)in_group * kb_bytes) >> 4);
+            uint64_t da0 = desc_a + (((uint32_t)rp.s * patch_pitch + (uint32_t)(kh * a.cw + kw) * 16u) >> 4);
+            for (int m = 0; m < MT; ++m, da0 += strip_bytes >> 4) {
+              const uint32_t d = tmem_base + (uint32_t)(m * BN);
+#pragma unroll
+              for (int j = 0; j < kPK / 16; ++j) {
+                const uint64_t dah = da0 + (uint64_t)((2u * j * chunk) >> 4), dal = dah + (uint64_t)((4u * chunk) >> 4);
+                const uint64_t db = db0 + (uint32_t)j * 2u, dbl = db + (kAtom >> 4);
+                umma_f16_ss(d, dal, db, idesc, (kb == 0 && j == 0) ? 0u : 1u);
+                umma_f16_ss(d, dah, dbl, idesc, 1u);
+                umma_f16_ss(d, dah, db, idesc, 1u);
+              }
+            }
+            if (last_of_group) umma_commit(bar_bempty + 8u * rb.s);
+            if (tap + 1 == a.taps) umma_commit(bar_pempty + 8u * rp.s);
+          }
+          __syncwarp();
+          if (last_of_group) { in_group = 0; rb.step(NB); } else ++in_group;
+          if (++kw == a.KW) { kw = 0; ++kh; }
+        }
+        rp.step(a.patch_bufs);
+      }
+      if (ok && leader) umma_commit(bar_accum);
+      __syncwarp();
+    }
+    if (!ok) {
+      if (leader) atomicOr(a.status, kStatusTimeout);
+      *abort_flag = 1;
+    }
+  } else {
+    // ------------------------------------------------------------ patch split
+    const int et = threadIdx.x - 64, set = et >> 7;
+    const int q = warp & 3, m = q * 32 + lane;  // epilogue: this thread's TMEM lane
+    bool ok = true;
+    if (et < BN) cb_s[et].y = a.bias && oc0 + et < a.OC ? a.bias[(int64_t)(oc0 + et) * a.bias_stride] : 0.0f;
+    if (SOURCE == kGated)
+      for (int i = et; i < n_img * n_icb * kPK; i += 256) {
+        const int im = i / (n_icb * kPK), c = icb_lo * kPK + i - im * (n_icb * kPK);
+        scale_s[i] = c < a.IC ? a.scale[(int64_t)(n0 + im) * a.scale_sn + (int64_t)c * a.scale_sc] : 0.0f;
+      }
+    // This thread's pixels of the split patch (at most two; small patches: the two halves of the threads
+    // take alternate chunks of the same pixels), each with its raw offset, or -1 where it is padding.
+    const bool few = a.px <= 128;
+    const int c8_0 = few ? set : 0, c8_step = few ? 2 : 1;
+    int roff[2], gate[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int p = few ? (u ? a.px : (et & 127)) : et + 256 * u;
+      roff[u] = -2;  // no such pixel
+      gate[u] = 0;
+      if (p >= a.px) continue;
+      if (a.mode == kRun) {
+        roff[u] = p;  // (pixels beyond the plane arrive as zeros)
+      } else if (a.mode == kImages) {
+        const int im = p / a.plane;
+        roff[u] = im < n_img ? im * kPK * a.plane + (p - im * a.plane) : -1;
+        gate[u] = im < n_img ? im * n_icb * kPK : 0;
+      } else {
+        const int pr = (int)(((uint32_t)p * a.cw_magic) >> 16), pc = p - pr * a.cw;
+        if (a.mode == kIm2col) roff[u] = pr * a.strides[0] * a.raw_w + pc * a.strides[1] + a.xoff;
+        else if (a.mode == kBox) roff[u] = pr * a.raw_w + pc + a.xoff;
+        else roff[u] = (unsigned)(ow0 + pc - a.pw) < (unsigned)a.IW ? pr * a.raw_w + pc + a.xoff : -1;
+      }
+    }
+    named_barrier_sync(1, 256);  // the gate, the column data
+    // eight k values of one pixel (channels beyond IC arrive as zeros)
+    auto load8 = [&](const float *raw, int icb, int c8, int u, float *v) {
+      const int c0 = icb * kPK + c8 * 8;  // first channel (kTaps: k value) within this CTA's split
+      if (SOURCE == kTaps) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int k = koff_s[icb_lo * kPK + c0 + i];
+          v[i] = raw[max(roff[u] + k, 0)];
+          v[i] = k >= 0 ? v[i] : 0.0f;
+        }
+      } else {
+        const bool pixel = roff[u] >= 0;
+        const float *src = raw + max(roff[u], 0) + c8 * 8 * a.raw_ch;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = src[i * a.raw_ch];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = pixel ? v[i] : 0.0f;
+        if (SOURCE == kGated) {
+          const float4 *g = reinterpret_cast<const float4 *>(scale_s + gate[u] + c0);
+          const float4 g0 = g[0], g1 = g[1];
+          const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = __fmul_rn(v[i], gv[i]);  // rounded as a separate Mul would
+        }
+      }
+    };
+    int k_tile = 0;  // the tile is scaled by 2^k_tile
+    RingPos rr, rp;
+    for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+      bool guess = false;
+      float seen = 0.0f;
+      if (attempt) {
+        k_tile = scale_exponent(__uint_as_float(*tile_max), 14);
+      } else {
+        // scale from the first channel block
+        float mx = 0.0f;
+        if (n_icb > 0) {
+          ok = mbar_wait_warp(bar_rfull, 0u, abort_flag);
+          if (ok)
+            for (int c8 = c8_0; c8 < 4; c8 += c8_step)
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                if (roff[u] == -2) continue;
+                float v[8];
+                load8(raw_ptr, 0, c8, u, v);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
+              }
+        }
+        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+        if (lane == 0 && wm) atomicMax(first_max, wm);
+        named_barrier_sync(1, 256);  // reached by every warp, whether its wait was met or not
+        mx = __uint_as_float(*first_max);
+        guess = !(mx > 0.0f);
+        k_tile = guess ? kDefaultScaleExp : scale_exponent(mx, kTargetExp);
+      }
+      const float s_mul = pow2(k_tile);
+      for (int icb = 0; icb < n_icb && ok; ++icb) {
+        ok = mbar_wait_warp(bar_rfull + 8u * rr.s, rr.ph, abort_flag) && mbar_wait_warp(bar_pempty + 8u * rp.s, rp.ph ^ 1u, abort_flag);
+        if (!ok) break;
+        const float *raw = raw_ptr + (size_t)rr.s * (a.raw_pitch / 4);
+        uint8_t *dst = patch_ptr + (size_t)rp.s * patch_pitch;
+        for (int c8 = c8_0; c8 < 4; c8 += c8_step)
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            if (roff[u] == -2) continue;
+            float v[8];
+            load8(raw, icb, c8, u, v);
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              seen = fmaxf(seen, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
+              split_pair(v[2 * i], v[2 * i + 1], s_mul, hi[i], lo[i]);
+            }
+            const int p = few ? (et & 127) : et + 256 * u;
+            uint4 *o = reinterpret_cast<uint4 *>(dst + (size_t)c8 * chunk) + p;
+            *o = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(o) + 4u * chunk) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+        fence_async_smem();  // visible to the tensor core
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(bar_pfull + 8u * rp.s); mbar_arrive(bar_rempty + 8u * rr.s); }
+        rr.step(RB);
+        rp.step(a.patch_bufs);
+      }
+      if (attempt) break;
+      // Was the scale right?  Known before the MMAs are done.
+      const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(seen));
+      if (lane == 0 && wm) atomicMax(tile_max, wm);
+      named_barrier_sync(1, 256);
+      const float all = __uint_as_float(*tile_max) * s_mul;
+      if (all > 65504.0f || (guess && all > 0.0f && all < 0.125f)) *redo_flag = 1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_decide);
+      ok = ok && mbar_wait_warp(bar_decide, 0u, abort_flag);
+      if (!ok || !*redo_flag) break;
+    }
+    if (ok) ok = mbar_wait_warp(bar_accum, 0u, abort_flag);
+    if (ok && *redo_flag) ok = mbar_wait_warp(bar_accum, 1u, abort_flag);
+    if (!ok) {
+      atomicOr(a.status, kStatusTimeout);
+      *abort_flag = 1;
+    }
+    tc_fence_after();
+    // ---- epilogue: thread = pixel; two strips: one per set of four warps, one strip: the sets take
+    // alternate groups of 32 channels
+    const float inv = pow2(-k_tile);
+    const int strip = MT == 2 ? set : 0;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(strip * BN);
+    const int g_first = MT == 2 ? 0 : set * 32, g_step = MT == 2 ? 32 : 64;
+    if (a.split_k > 1) {
+      float *dst = staging + (size_t)(strip * kBM + m) * pitch;
+      for (int c0 = g_first; c0 < BN; c0 += g_step) {
+        float v[32];
+        if (ok && nkb > 0) {
+          tmem_ld32(lane_addr + (uint32_t)c0, v);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i += 4)
+          *reinterpret_cast<float4 *>(dst + c0 + i) = make_float4(v[i] * inv, v[i + 1] * inv, v[i + 2] * inv, v[i + 3] * inv);
+      }
+    } else if (ok) {
+      int64_t off;
+      const bool inside = pixel_offset(a, strip * kBM + m, n0, n_img, oh0, ow0, &off);
+      for (int c0 = g_first; c0 < BN; c0 += g_step) {
+        float v[32];
+        tmem_ld32(lane_addr + (uint32_t)c0, v);
+        if (!inside || oc0 + c0 >= a.OC) continue;
+        const int64_t at = off + (int64_t)(oc0 + c0) * a.ys[1];
+        float *yp = a.y + at;
+        const float *rp_ = a.res ? a.res + at : nullptr;
+        const int left = a.OC - (oc0 + c0);
+        switch (a.act) {
+        case FML_ACT_RELU: store_channels<FML_ACT_RELU>(v, cb_s + c0, inv, yp, rp_, a.ys[1], left); break;
+        case FML_ACT_TANH: store_channels<FML_ACT_TANH>(v, cb_s + c0, inv, yp, rp_, a.ys[1], left); break;
+        case FML_ACT_SIGMOID: store_channels<FML_ACT_SIGMOID>(v, cb_s + c0, inv, yp, rp_, a.ys[1], left); break;
+        case FML_ACT_SILU: store_channels<FML_ACT_SILU>(v, cb_s + c0, inv, yp, rp_, a.ys[1], left); break;
+        default: store_channels<FML_ACT_NONE>(v, cb_s + c0, inv, yp, rp_, a.ys[1], left); break;
+        }
+      }
+    }
+  }
+  if (a.split_k > 1) {
+    // Rank r sums its share of the tile's pixels over the ranks in rank order, lanes along the channels
+    // (16-byte loads of contiguous remote shared memory, two times S in flight); the sums go back to its own
+    // staging rows, which nobody else reads, and leave with the lanes along the pixels: stored from the
+    // first arrangement they were 4-byte writes a plane apart (256 channels of 56 x 56: 9.5 us of a 27 us launch).
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp >= 2) {
+      const int S = a.split_k, rows_per = (kBM * MT) / S, quads = BN >> 2;
+      const int et = threadIdx.x - 64;
+      float *const own = staging + (size_t)split * rows_per * pitch;
+      const uint32_t base = smem_u32(own);
+      uint32_t rank_base[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) rank_base[r] = r < S ? cluster_smem_addr(base, (uint32_t)r) : 0u;
+      for (int i = et; i < rows_per * quads; i += 512) {
+        float4 part[2][8];
+        uint32_t at[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int j = i + 256 * u, row = j / quads;
+          at[u] = (uint32_t)(row * pitch + (j - row * quads) * 4) * 4u;
+#pragma unroll
+          for (int r = 0; r < 8; ++r)
+            if (r < S && j < rows_per * quads)
+              asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                           : "=f"(part[u][r].x), "=f"(part[u][r].y), "=f"(part[u][r].z), "=f"(part[u][r].w)
+                           : "r"(rank_base[r] + at[u]) : "memory");
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (i + 256 * u >= rows_per * quads) continue;
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int r = 0; r < 8; ++r)
+            if (r < S) { acc.x += part[u][r].x; acc.y += part[u][r].y; acc.z += part[u][r].z; acc.w += part[u][r].w; }
+          *reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(own) + at[u]) = acc;
+        }
+      }
+      named_barrier_sync(1, 256);
+      const int row = et & (rows_per - 1);  // rows_per is a power of two, at most 128
+      int64_t off;
+      if (pixel_offset(a, split * rows_per + row, n0, n_img, oh0, ow0, &off)) {
+        const float *src = own + (size_t)row * pitch;
+        const int c_step = 256 / rows_per, c_end = min(BN, a.OC - oc0);
+        switch (a.act) {
+        case FML_ACT_RELU: store_sums<FML_ACT_RELU>(a, src, cb_s, off, oc0, et / rows_per, c_step, c_end); break;
+        case FML_ACT_TANH: store_sums<FML_ACT_TANH>(a, src, cb_s, off, oc0, et / rows_per, c_step, c_end); break;
+        case FML_ACT_SIGMOID: store_sums<FML_ACT_SIGMOID>(a, src, cb_s, off, oc0, et / rows_per, c_step, c_end); break;
+        case FML_ACT_SILU: store_sums<FML_ACT_SILU>(a, src, cb_s, off, oc0, et / rows_per, c_step, c_end); break;
+        default: store_sums<FML_ACT_NONE>(a, src, cb_s, off, oc0, et / rows_per, c_step, c_end); break;
+        }
+      }
+    }
+    cluster_sync_relaxed();  // nobody leaves while a peer may still read its tile
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, tmem_cols);
+  }
+}
+
+// ---------------------------------------------------------------- packing
+// One block per 8 output channels; k block (channel block, tap) holds 32 channels of one tap (im2col: 32
+// consecutive values of the flattened (channel, tap)).
+__global__ void __launch_bounds__(256) conv_pack_kernel(const float *w, int IC, int OC, int KH, int KW, int64_t s_oc, int64_t s_ic,
+                                                        int64_t s_kh, int64_t s_kw, int im2col, int n_icb, char *packed,
+                                                        float *col_scale, int n_pad) {
+  __shared__ unsigned m_bits[8];
+  const int taps = KH * KW, n0 = blockIdx.x * 8, r = threadIdx.x & 7;
+  const bool real = n0 + r < OC;
+  if (threadIdx.x < 8) m_bits[threadIdx.x] = 0u;
+  __syncthreads();
+  auto value = [&](int c, int tap) {
+    return real && c < IC ? w[(int64_t)(n0 + r) * s_oc + (int64_t)c * s_ic + (int64_t)(tap / KW) * s_kh + (int64_t)(tap % KW) * s_kw] : 0.0f;
+  };
+  float m = 0.0f;
+  for (int i = threadIdx.x >> 3; i < IC * taps; i += 32) m = fmaxf(m, fabsf(value(i / taps, i % taps)));
+  atomicMax(&m_bits[r], __float_as_uint(m));
+  __syncthreads();
+  float s = 1.0f, inv = 1.0f;
+  if (m_bits[r]) {
+    const int e = scale_exponent(__uint_as_float(m_bits[r]), 14);
+    s = pow2(e);
+    inv = pow2(-e);
+  }
+  if (threadIdx.x < 8) col_scale[n0 + r] = inv;
+  const int blocks = im2col ? n_icb : n_icb * taps;
+  for (int i = threadIdx.x >> 3; i < blocks * 4; i += 32) {  // (k block, 16-byte chunk) of column r
+    const int kb = i >> 2, c = i & 3;
+    uint32_t hi[4], lo[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float x[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = c * 8 + j * 2 + h;
+        if (im2col) {
+          const int f = kb * kPK + k;
+          x[h] = value(f / taps, f % taps);
+        } else {
+          x[h] = value((kb / taps) * kPK + k, kb % taps);
+        }
+      }
+      split_pair(x[0], x[1], s, hi[j], lo[j]);
+    }
+    char *atom = packed + ((size_t)kb * n_pad + n0) * kPairB + r * (kPK * 2) + ((c ^ (r >> 1)) * 16);
+    *reinterpret_cast<uint4 *>(atom) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    *reinterpret_cast<uint4 *>(atom + kAtom) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
+}
+
+// ---------------------------------------------------------------- host side
+bool is_im2col(int64_t ic, int64_t taps) { return taps > 1 && ic * taps <= 64; }
+int conv_n_pad(int64_t oc) { return (int)((oc + 15) / 16 * 16); }
+int conv_k_blocks(int64_t ic, int64_t taps) {
+  return is_im2col(ic, taps) ? (int)((ic * taps + kPK - 1) / kPK) : (int)((ic + kPK - 1) / kPK * taps);
+}
+
+// Shared-memory bytes of a choice of tile; fills the derived fields.
+size_t finish_plan(ConvPairArgs &a, bool has_scale, size_t budget) {
+  const bool flat_m = a.mode == kRun || a.mode == kImages;
+  if (flat_m) {
+    a.TW = 128 * a.mt; a.TH = 1;
+    a.cw = a.TW; a.px = a.TW;
+  } else {
+    a.TW = 8 * a.mt; a.TH = 16;
+    a.cw = a.mode == kIm2col ? a.TW : a.TW + a.KW - 1;
+    a.px = a.mode == kIm2col ? a.TW * a.TH : a.cw * (a.TH + a.KH - 1);
+  }
+  a.cw_magic = (uint32_t)((65536 + a.cw - 1) / a.cw);
+  a.imgs = 1;
+  const int rows = (a.TH - 1) * a.strides[0] + a.KH;
+  a.xoff = 0;
+  switch (a.mode) {
+  case kRun: a.raw_w = a.TW; a.raw_ch = a.TW; break;
+  case kImages:
+    a.raw_w = a.IW; a.raw_ch = a.plane;
+    a.imgs = std::min(a.TW / a.plane, a.N);
+    if (has_scale) a.imgs = std::max(1, std::min(a.imgs, 6144 / (a.n_icb * kPK)));  // the gates of the images stay within 24 KiB
+    break;
+  case kFlat: {
+    const int start = -(a.ph * a.IW + a.pw);
+    a.xoff = ((start % 4) + 4) % 4;
+    a.raw_w = a.IW;
+    a.raw_ch = (rows * a.IW + a.pw + a.xoff + 3) / 4 * 4;
+    break;
+  }
+  default:
+    a.xoff = (4 - a.pw % 4) % 4;
+    a.raw_w = ((a.TW - 1) * a.strides[1] + a.KW + a.xoff + 3) / 4 * 4;
+    a.raw_ch = rows * a.raw_w;
+    break;
+  }
+  const int channels = a.mode == kIm2col ? a.IC : kPK;
+  a.raw_bytes = (uint32_t)(a.mode == kImages ? a.imgs * kPK * a.plane : channels * a.raw_ch) * 4u;
+  a.raw_pitch = (a.raw_bytes + 127u) & ~127u;
+  const size_t patch = (((size_t)a.px * 128) + 1023) / 1024 * 1024;
+  const size_t kb = (size_t)a.tile_n * kPairB;
+  const int nkb = a.icb_per_split * a.taps;
+  a.group = (int)std::max<size_t>(1, std::min<size_t>({(8 * 1024) / kb, (size_t)4, (size_t)nkb}));
+  const size_t fixed = (size_t)a.tile_n * 8 + 64 * 4 + (has_scale ? (size_t)a.imgs * a.icb_per_split * kPK * 4 : 0) + 32 + (2 * 8 + 2 * 4 + 6) * 8;
+  const size_t staging = a.split_k > 1 ? (size_t)kBM * a.mt * (a.tile_n + 4) * 4 + 128 : 0;
+  const int nstages = (nkb + a.group - 1) / a.group;
+  // Rings, no deeper than the work there is.  Without taps every k block waits for its own raw patch, which
+  // comes from HBM: patches in flight come first, then weight stages, then a second split patch.  With taps
+  // a patch lasts for many k blocks and the weight stages come first.
+  size_t best = 0;
+  int best_rb = 0, best_nb = 0, best_pb = 0;
+  double best_score = -1;
+  const int most_rb = std::min(a.taps == 1 ? 4 : 2, a.icb_per_split), most_nb = std::min(6, nstages), most_pb = std::min(2, a.icb_per_split);
+  for (int pb = 1; pb <= most_pb; ++pb)
+    for (int rb = 1; rb <= most_rb; ++rb)
+      for (int nb = 1; nb <= most_nb; ++nb) {
+        const size_t ring = nb * kb * a.group + pb * patch + (size_t)rb * a.raw_pitch;
+        const size_t total = std::max(ring, staging) + fixed;
+        if (total > budget) continue;
+        const double score = a.taps == 1 ? std::min(rb, 3) * 10 + std::min(nb, 2) * 8 + pb * 5 + nb + rb
+                                         : std::min(nb, 2) * 20 + pb * 15 + std::min(nb, 4) * 5 + rb * 4 + nb;
+        if (score > best_score) { best_score = score; best = total; best_rb = rb; best_nb = nb; best_pb = pb; }
+      }
+  a.patch_bufs = best_pb;
+  if (!best_rb) return 0;
+  a.raw_bufs = best_rb;
+  a.stages_b = best_nb;
+  return best;
+}
+
+struct Candidate {
+  double clocks;
+  size_t smem;
+  ConvPairArgs a;
+  int occ;
+};
+
+// Shape checks and the tiles a layer can take, in the order of the time model; empty when it is not taken.
+std::vector<Candidate> conv_pair_candidates(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p,
+                                            bool has_scale, bool only_named) {
+  std::vector<Candidate> found;
+  // what the 3xTF32 kernel takes (unit stride and dilation, dense NCHW, 16-byte aligned, AUTO precision)
+  if (p->precision != FML_GEMM_AUTO || !conv_tc_eligible(x, w, y, p)) return found;
+  ConvPairArgs a;
+  memset(&a, 0, sizeof(a));
+  a.N = (int)x->shape[0]; a.IC = (int)x->shape[1]; a.IH = (int)x->shape[2]; a.IW = (int)x->shape[3];
+  a.OC = (int)w->shape[0]; a.KH = (int)w->shape[2]; a.KW = (int)w->shape[3];
+  a.OH = (int)y->shape[2]; a.OW = (int)y->shape[3];
+  a.ph = (int)p->pads_begin[0]; a.pw = (int)p->pads_begin[1];
+  a.strides[0] = a.strides[1] = 1;
+  a.plane = a.IH * a.IW;
+  a.n_pad = conv_n_pad(a.OC);
+  const int taps = a.KH * a.KW;
+  const bool pointwise = taps == 1 && a.ph == 0 && a.pw == 0 && a.OH == a.IH && a.OW == a.IW;
+  if (pointwise && (a.plane & 3) == 0) a.mode = kRun;
+  else if (pointwise) a.mode = kImages;
+  else if (is_im2col(a.IC, taps)) a.mode = kIm2col;
+  else a.mode = (a.IW & 3) ? kFlat : kBox;
+  if (a.mode == kImages && ((a.IC & 31) || a.plane > 256)) return found;  // (whole channel blocks: nothing fills a tail with zeros)
+  if (a.mode == kFlat && (a.plane & 3)) return found;
+  if (a.mode == kIm2col && ((a.IW & 3) || has_scale)) return found;
+  a.taps = a.mode == kIm2col ? 1 : taps;
+  a.n_icb = a.mode == kIm2col ? conv_k_blocks(a.IC, taps) : (a.IC + kPK - 1) / kPK;
+  a.kb_total = a.n_icb * a.taps;
+  // Candidates scored in clocks of the busiest SM.  A CTA: set-up and pipeline fill, then per channel block
+  // the slowest of the MMAs (6 per k block and strip, 44 clocks or N / 2), the fill path (45 bytes per
+  // clock) and the split of the patch; then the stores (and the cluster's exchange with split-K).  Two CTAs
+  // on an SM overlap each other's fixed parts but share the rest.
+  for (int mt = 1; mt <= 2; ++mt) {
+    if (mt == 2 && a.mode != kRun && a.mode != kImages && a.OW <= 8) continue;
+    if (a.mode == kImages && a.plane > 128 * mt) continue;
+    for (int tn = 32; tn <= 256; tn += 32) {
+      if (tn > 32 && tn - 32 >= a.OC) break;
+      for (int sk = 1; sk <= 8; sk *= 2) {
+        if (sk > a.n_icb) break;
+        for (int occ = 2; occ >= 1; --occ) {
+          if (only_named && (tn != p->tile_n || mt != p->strips || sk != p->split_k || occ != p->ctas_per_sm)) continue;
+          ConvPairArgs c = a;
+          c.mt = mt; c.tile_n = tn; c.split_k = sk;
+          c.icb_per_split = (c.n_icb + sk - 1) / sk;
+          unsigned cols = 32;
+          while ((int)cols < tn * mt) cols <<= 1;
+          if (cols * occ > 512) continue;
+          size_t smem = finish_plan(c, has_scale, occ == 2 ? kSmemSm / 2 - 1024 : kSmemCta);
+          if (!smem) continue;
+          if (c.mode == kFlat && c.raw_ch > 256) continue;
+          if (c.mode == kImages) { c.tiles_w = c.tiles_h = 1; c.tiles_img = (c.N + c.imgs - 1) / c.imgs; }
+          else if (c.mode == kRun) { c.tiles_w = (c.plane + c.TW - 1) / c.TW; c.tiles_h = 1; c.tiles_img = c.N; }
+          else { c.tiles_w = (c.OW + c.TW - 1) / c.TW; c.tiles_h = (c.OH + c.TH - 1) / c.TH; c.tiles_img = c.N; }
+          const double ctas = (double)c.tiles_w * c.tiles_h * c.tiles_img * ((c.OC + tn - 1) / tn) * sk;
+          const double slots = 148.0 * occ * (sk == 8 ? 0.86 : sk == 4 ? 0.97 : 1.0);
+          double t_kb = std::max(mt * 6 * std::max(48.0, tn / 2.0) + 40.0, (tn * 128.0 + (double)c.raw_bytes / c.taps) / 45.0);
+          // a ring of one stage exposes the load latency, shared out over what the SM has in flight
+          t_kb = std::max(t_kb, 1800.0 / (c.stages_b * c.group));
+          if (c.taps == 1 && c.icb_per_split > 1) t_kb = std::max(t_kb, 2200.0 / c.raw_bufs);
+          const double t_split = ((c.px * 4 + 255) / 256) * 85.0 + 150.0;
+          const double shared = c.icb_per_split * std::max(c.taps * t_kb, t_split) + mt * 128.0 * tn * 4.0 / 40.0;
+          const double own = 4500.0 + t_split + (mt == 2 ? tn / 32 : (tn + 63) / 64) * 300.0 +
+                             (sk > 1 ? 2500.0 + mt * 128.0 * tn * 4.0 / 13.0 * (sk - 1) / sk : 0.0);
+          const double resident = std::min((double)occ, std::ceil(ctas / 148.0));
+          const double t = std::ceil(ctas / slots) * std::max(resident * shared, shared + own);
+          // no more CTAs on an SM than its 512 TMEM columns serve at once
+          smem = std::max(smem, kSmemSm / (512 / cols + 1) + 1024);
+          if (smem <= kSmemCta) found.push_back({t, smem, c, occ});
+        }
+      }
+    }
+  }
+  std::stable_sort(found.begin(), found.end(), [](const Candidate &l, const Candidate &r) { return l.clocks < r.clocks; });
+  return found;
+}
+
+// The candidate the caller's tuning choices name, else the best one.
+size_t plan_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool has_scale,
+                      ConvPairArgs &a) {
+  std::vector<Candidate> all = conv_pair_candidates(x, w, y, p, has_scale, p->tile_n != 0);
+  if (all.empty() && p->tile_n) all = conv_pair_candidates(x, w, y, p, has_scale, false);
+  if (all.empty()) return 0;
+  a = all[0].a;
+  return all[0].smem;
+}
+
+}  // namespace
+
+bool conv_pair_eligible(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool has_scale) {
+  ConvPairArgs a;
+  return plan_conv_pair(x, w, y, p, has_scale, a) != 0;
+}
+
+size_t conv_packed_bytes(const fml_tensor *w) {
+  const int64_t taps = w->shape[2] * w->shape[3];
+  return (size_t)conv_k_blocks(w->shape[1], taps) * conv_n_pad(w->shape[0]) * kPairB + (size_t)conv_n_pad(w->shape[0]) * sizeof(float);
+}
+
+int conv_pack(const fml_tensor *w, void *dst, cudaStream_t s) {
+  const int OC = (int)w->shape[0], IC = (int)w->shape[1], KH = (int)w->shape[2], KW = (int)w->shape[3];
+  const int np = conv_n_pad(OC), kb = conv_k_blocks(IC, KH * KW);
+  const bool im2col = is_im2col(IC, KH * KW);
+  char *packed = static_cast<char *>(dst);
+  conv_pack_kernel<<<np / 8, 256, 0, s>>>((const float *)w->data, IC, OC, KH, KW, w->stride[0], w->stride[1], w->stride[2], w->stride[3],
+                                          im2col, im2col ? kb : (IC + kPK - 1) / kPK, packed,
+                                          reinterpret_cast<float *>(packed + (size_t)kb * np * kPairB), np);
+  FML_CUDA(cudaGetLastError());
+  return FML_OK;
+}
+
+static int launch_planned(ConvPairArgs a, size_t smem, const fml_tensor *x, const fml_tensor *bias, const fml_tensor *y,
+                          const fml_conv_params *p, cudaStream_t s, const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc) {
+  a.x = (const float *)x->data;
+  a.packed = static_cast<const char *>(p->w_packed);
+  a.col_scale = reinterpret_cast<const float *>(a.packed + (size_t)conv_k_blocks(a.IC, a.KH * a.KW) * a.n_pad * kPairB);
+  a.y = (float *)y->data;
+  for (int i = 0; i < 4; ++i) a.ys[i] = y->stride[i];
+  if (bias) {
+    a.bias = (const float *)bias->data;
+    for (int i = 0; i < bias->rank; ++i) if (bias->shape[i] != 1) a.bias_stride = bias->stride[i];
+  }
+  a.act = p->act;
+  a.scale = x_scale; a.scale_sn = x_scale_sn; a.scale_sc = x_scale_sc;
+  a.res = nullptr;
+  a.status = device_status_word();
+  FML_REQUIRE(a.status, FML_CUDA_ERROR, "fml_conv: no device status word");
+  CUtensorMap map_x;
+  memset(&map_x, 0, sizeof(map_x));
+  if (a.mode == kBox || a.mode == kIm2col) {
+    const cuuint64_t dims[4] = {(cuuint64_t)a.IW, (cuuint64_t)a.IH, (cuuint64_t)a.IC, (cuuint64_t)a.N};
+    const cuuint64_t str[3] = {(cuuint64_t)a.IW * 4, (cuuint64_t)a.plane * 4, (cuuint64_t)a.IC * a.plane * 4};
+    const cuuint32_t box[4] = {(cuuint32_t)a.raw_w, (cuuint32_t)(a.raw_ch / a.raw_w), (cuuint32_t)(a.mode == kIm2col ? a.IC : kPK), 1};
+    const int st = make_f32_tensor_map(&map_x, a.x, 4, dims, str, box);
+    if (st != FML_OK) return st;
+  } else if (a.mode != kImages) {
+    const cuuint64_t dims[3] = {(cuuint64_t)a.plane, (cuuint64_t)a.IC, (cuuint64_t)a.N};
+    const cuuint64_t str[2] = {(cuuint64_t)a.plane * 4, (cuuint64_t)a.IC * a.plane * 4};
+    const cuuint32_t box[3] = {(cuuint32_t)a.raw_ch, (cuuint32_t)kPK, 1};
+    const int st = make_f32_tensor_map(&map_x, a.x, 3, dims, str, box);
+    if (st != FML_OK) return st;
+  }
+  using KernelFn = void (*)(const CUtensorMap, const ConvPairArgs);
+  static const KernelFn kernels[3] = {conv_pair_kernel<kPlain>, conv_pair_kernel<kGated>, conv_pair_kernel<kTaps>};
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  FML_CUDA(cudaGetDevice(&dev));
+  if (!attr_set[dev & 63]) {
+    for (KernelFn k : kernels) FML_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCta));
+    attr_set[dev & 63] = true;
+  }
+  const int64_t m_tiles = (int64_t)a.tiles_w * a.tiles_h * a.tiles_img;
+  FML_REQUIRE(m_tiles <= 0x7fffffff && (a.OC + a.tile_n - 1) / a.tile_n <= 65535, FML_UNSUPPORTED, "fml_conv: grid too large");
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)m_tiles, (unsigned)((a.OC + a.tile_n - 1) / a.tile_n), (unsigned)a.split_k);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;  // the split-K ranks of a tile share a cluster
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = (unsigned)a.split_k;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  FML_CUDA(cudaLaunchKernelEx(&cfg, kernels[a.mode == kIm2col ? kTaps : x_scale ? kGated : kPlain], map_x, a));
+  return FML_OK;
+}
+
+int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
+                     cudaStream_t s, const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc) {
+  ConvPairArgs a;
+  const size_t smem = plan_conv_pair(x, w, y, p, x_scale != nullptr, a);
+  FML_REQUIRE(smem, FML_UNSUPPORTED, "fml_conv: this layer has no packed form");
+  return launch_planned(a, smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc);
+}
+
+// Times the candidates the model ranks highest as captured graphs of back-to-back launches and keeps the
+// fastest, per problem signature (as fml_gemm_autotune).
+int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
+                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, fml_conv_params *tuned) {
+  char key[256];
+  snprintf(key, sizeof(key), "%lld,%lld,%lld,%lld|%lld,%lld,%lld|%lld,%lld|%d%d", (long long)x->shape[0], (long long)x->shape[1],
+           (long long)x->shape[2], (long long)x->shape[3], (long long)w->shape[0], (long long)w->shape[2], (long long)w->shape[3],
+           (long long)p->pads_begin[0], (long long)p->pads_begin[1], p->act, x_scale != nullptr);
+  struct Choice { int tile_n, strips, split_k, occ; };
+  static std::map<std::string, Choice> cache;
+  static std::mutex mu;
+  auto take = [&](const Choice &c) {
+    tuned->tile_n = c.tile_n; tuned->strips = c.strips; tuned->split_k = c.split_k; tuned->ctas_per_sm = c.occ;
+  };
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) { take(it->second); return FML_OK; }
+  }
+  const std::vector<Candidate> all = conv_pair_candidates(x, w, y, p, x_scale != nullptr, false);
+  FML_REQUIRE(!all.empty(), FML_UNSUPPORTED, "fml_conv_autotune: this layer has no packed form");
+  cudaStream_t s;
+  cudaEvent_t e0, e1;
+  FML_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  FML_CUDA(cudaEventCreate(&e0));
+  FML_CUDA(cudaEventCreate(&e1));
+  float best = 1e30f;
+  const Candidate *chosen = &all[0];
+  for (size_t i = 0; i < all.size() && i < 16; ++i) {
+    auto launch = [&] { return launch_planned(all[i].a, all[i].smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc); };
+    float one = 0;
+    bool ok = launch() == FML_OK;  // warm-up
+    cudaEventRecord(e0, s);
+    ok = ok && launch() == FML_OK;
+    cudaEventRecord(e1, s);
+    if (cudaEventSynchronize(e1) != cudaSuccess || !ok) { cudaGetLastError(); continue; }
+    cudaEventElapsedTime(&one, e0, e1);
+    if (one > 0.05f && one > 1.5f * best) continue;  // far behind
+    const int reps = one > 0.2f ? 2 : 8;
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    for (int r = 0; r < reps && ok; ++r) ok = launch() == FML_OK;
+    ok = cudaStreamEndCapture(s, &graph) == cudaSuccess && ok && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+    if (graph) cudaGraphDestroy(graph);
+    float ms = 1e30f;
+    for (int r = 0; r < 4 && ok; ++r) {
+      cudaEventRecord(e0, s);
+      ok = cudaGraphLaunch(exec, s) == cudaSuccess;
+      cudaEventRecord(e1, s);
+      ok = cudaEventSynchronize(e1) == cudaSuccess && ok;
+      float t = 0;
+      cudaEventElapsedTime(&t, e0, e1);
+      if (r && t / reps < ms) ms = t / reps;
+    }
+    if (exec) cudaGraphExecDestroy(exec);
+    if (!ok) { cudaGetLastError(); continue; }
+    if (ms < best) { best = ms; chosen = &all[i]; }
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  cudaStreamDestroy(s);
+  const Choice c{chosen->a.tile_n, chosen->a.mt, chosen->a.split_k, chosen->occ};
+  take(c);
+  std::lock_guard<std::mutex> lock(mu);
+  cache[key] = c;
+  return FML_OK;
+}
+
+}  // namespace fml

@@ -93,4 +93,13 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
                    const fml_conv_params *p, cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0,
                    int64_t x_scale_sc = 0);
 
+// half-precision-pair convolution with packed weights (conv_pair.cu)
+bool conv_pair_eligible(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool has_scale);
+size_t conv_packed_bytes(const fml_tensor *w);
+int conv_pack(const fml_tensor *w, void *dst, cudaStream_t s);
+int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
+                     cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0, int64_t x_scale_sc = 0);
+int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
+                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, fml_conv_params *tuned);
+
 }  // namespace fml

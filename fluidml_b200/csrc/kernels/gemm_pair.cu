@@ -32,18 +32,14 @@
 // tensor-memory stage and B's stage when the MMAs are done.  Epilogue, split-K over a cluster and
 // bounded waits as in gemm_tc.cu.
 #include "gemm_epilogue.cuh"
-#include <cuda.h>
-#include <cuda_fp16.h>
+#include "pair_common.cuh"
 #include <algorithm>
 #include <cstdlib>
 
 namespace fml {
 namespace {
 
-constexpr int kPK = 32;                      // k values per block: 128 bytes of fp32, 64 of fp16
 constexpr int kPairA = kBM * kPK * 4;        // bytes of A per block: a box of 128 rows x 128 bytes
-constexpr int kPairB = kPK * 4;              // bytes of B per block and column: hi and lo
-constexpr int kAtom = 8 * kPK * 2;           // bytes of an atom: 8 columns x 32 k values of fp16
 constexpr int kDefaultExponent = 8;          // scale 2^8 of a row whose first k block is all zero
 constexpr int kPairThreads = 320;
 constexpr int kConvThreads = 256;
@@ -59,23 +55,6 @@ struct PairArgs {
   int tiles_m, tiles_n, kb_total, kb_per_split;
   int *status;
 };
-
-// 2^k for -126 <= k <= 127.
-__device__ __forceinline__ float pow2(int k) { return __uint_as_float((uint32_t)(127 + k) << 23); }
-// The exponent that brings a largest magnitude m into [2^target, 2^(target + 1)), limited so that the
-// power and its inverse are normal numbers.
-__device__ __forceinline__ int scale_exponent(float m, int target) {
-  return min(max(target - ((int)(__float_as_uint(m) >> 23) - 127), -126), 126);
-}
-
-// Two fp32 values, already loaded -> (hi pair, lo pair) of x * s.
-__device__ __forceinline__ void split_pair(float x0, float x1, float s, uint32_t &hi, uint32_t &lo) {
-  const __half2 h = __floats2half2_rn(x0 * s, x1 * s);
-  const float2 f = __half22float2(h);
-  const __half2 l = __floats2half2_rn(fmaf(x0, s, -f.x), fmaf(x1, s, -f.y));
-  hi = *reinterpret_cast<const uint32_t *>(&h);
-  lo = *reinterpret_cast<const uint32_t *>(&l);
-}
 
 template <int ACT>
 __global__ void __launch_bounds__(kPairThreads, 2)
@@ -193,14 +172,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       for (int it = 0; it < pre_b; ++it) rb.step(a.stages_b);
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
         if (attempt) {
-          ok = mbar_wait(bar_decide, 0u, abort_flag);
+          ok = mbar_wait_warp(bar_decide, 0u, abort_flag);
           if (!ok || !*redo_flag) break;
         }
         int ia = 0, ib = attempt ? 0 : pre_b;
         uint32_t idle = 0;
         while (ia < nkb || ib < nkb) {  // whichever ring has room
           bool moved = false;
-          if (ia < nkb && mbar_test(bar_empty_a + 8u * ra.s, ra.ph ^ 1u)) {
+          if (ia < nkb && mbar_test_warp(bar_empty_a + 8u * ra.s, ra.ph ^ 1u)) {
             const uint32_t bar = bar_full_a + 8u * ra.s;
             if (leader) {
               mbar_expect_tx(bar, kPairA);
@@ -209,7 +188,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
             ++ia; ++issued_a; moved = true;
             ra.step(a.stages_a);
           }
-          if (ib < nkb && mbar_test(bar_empty_b + 8u * rb.s, rb.ph ^ 1u)) {
+          if (ib < nkb && mbar_test_warp(bar_empty_b + 8u * rb.s, rb.ph ^ 1u)) {
             if (leader) load_b(ib, rb.s);
             ++ib; ++issued_b; moved = true;
             rb.step(a.stages_b);
@@ -224,9 +203,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         // bounded drain of the loads already in flight before the CTA may exit
         volatile int never = 0;
         for (int i = max(0, issued_a - a.stages_a); i < issued_a; ++i)
-          mbar_wait(bar_full_a + 8u * (i % a.stages_a), (uint32_t)(i / a.stages_a) & 1u, &never);
+          mbar_wait_warp(bar_full_a + 8u * (i % a.stages_a), (uint32_t)(i / a.stages_a) & 1u, &never);
         for (int i = max(0, issued_b - a.stages_b); i < issued_b; ++i)
-          mbar_wait(bar_full_b + 8u * (i % a.stages_b), (uint32_t)(i / a.stages_b) & 1u, &never);
+          mbar_wait_warp(bar_full_b + 8u * (i % a.stages_b), (uint32_t)(i / a.stages_b) & 1u, &never);
       }
     }
   } else if (warp == 1) {
@@ -237,11 +216,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     bool ok = true;
     for (int attempt = 0; attempt < 2 && ok; ++attempt) {
       if (attempt) {
-        ok = mbar_wait(bar_decide, 0u, abort_flag);
+        ok = mbar_wait_warp(bar_decide, 0u, abort_flag);
         if (!ok || !*redo_flag) break;
       }
       for (int it = 0; it < nkb; ++it) {
-        ok = mbar_wait(bar_full_b + 8u * rb.s, rb.ph, abort_flag) && mbar_wait(bar_conv + 8u * rb.s, rb.ph, abort_flag);
+        ok = mbar_wait_warp(bar_full_b + 8u * rb.s, rb.ph, abort_flag) && mbar_wait_warp(bar_conv + 8u * rb.s, rb.ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (leader) {
@@ -301,7 +280,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         if (set == 0) {
           float m = 0.0f;
           if (nkb > 0) {
-            ok = mbar_wait(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
+            ok = mbar_wait_warp(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
             if (ok) {
               load_row(ma.s, x);
               have = true;
@@ -313,9 +292,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
           guess = !(m > 0.0f);
           k_row = guess ? kDefaultExponent : scale_exponent(m, 3);
           row_exp[row] = (signed char)(guess ? -128 : k_row);
-          asm volatile("bar.arrive 1, 256;" ::: "memory");  // also when the wait gave up: set 1 must not be left behind
+          named_barrier_arrive(1, 256);  // also when the wait gave up: set 1 must not be left behind
         } else {
-          asm volatile("bar.sync 1, 256;" ::: "memory");
+          named_barrier_sync(1, 256);
           k_row = row_exp[row];
           guess = k_row == -128;
           if (guess) k_row = kDefaultExponent;
@@ -326,7 +305,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       const bool watch = attempt == 0 && __any_sync(0xffffffffu, guess);
       for (int it = set; it < nkb && ok; it += 2) {
         if (!have) {
-          ok = mbar_wait(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
+          ok = mbar_wait_warp(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
           if (!ok) break;
           load_row(ma.s, x);
         }
@@ -345,7 +324,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         if (lane == 0) mbar_arrive(bar_empty_a + 8u * ma.s);  // the values are in registers
         ma.step(a.stages_a); ma.step(a.stages_a);
         // the MMAs that read this tensor-memory stage last are done
-        ok = mbar_wait(bar_empty_b + 8u * mb.s, mb.ph ^ 1u, abort_flag);
+        ok = mbar_wait_warp(bar_empty_b + 8u * mb.s, mb.ph ^ 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint32_t t_hi = lane_addr + a_col0 + (uint32_t)mb.s * 32u;
@@ -361,7 +340,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         mb.step(a.stages_b); mb.step(a.stages_b);
       }
       if (!attempt) epi.preload(a.p, a.shape, BN, tile_m, tile_n, split, a.split_k, z0, z1, threadIdx.x - 64, a.col_scale);
-      if (ok) ok = mbar_wait(bar_accum, (uint32_t)attempt, abort_flag);
+      if (ok) ok = mbar_wait_warp(bar_accum, (uint32_t)attempt, abort_flag);
       if (attempt) break;
       // A row whose hi overflowed shows it in every column of the accumulator; one on the default scale
       // must have had a value that this scale resolves, unless it is all zero.
@@ -369,7 +348,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       const float v0 = ok && nkb > 0 ? tmem_ld1(lane_addr) : 0.0f;
       tc_fence_before();
       if (watch && guess && seen > 0.0f) atomicMax(&row_seen[row], __float_as_uint(seen));
-      asm volatile("bar.sync 2, 256;" ::: "memory");  // every converter warp comes here, whether its waits were met or not
+      named_barrier_sync(2, 256);  // every converter warp comes here, whether its waits were met or not
       bool bad = !(fabsf(v0) <= 3.4028235e38f);
       if (watch && guess) {
         const float m = __uint_as_float(row_seen[row]);
@@ -378,7 +357,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       if (__any_sync(0xffffffffu, bad) && lane == 0) *redo_flag = 1;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_decide);
-      ok = ok && mbar_wait(bar_decide, 0u, abort_flag);
+      ok = ok && mbar_wait_warp(bar_decide, 0u, abort_flag);
       if (!ok || !*redo_flag) break;
     }
     if (!ok) {

@@ -89,6 +89,9 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "=r"(done) : "r"(bar), "r"(parity) : "memory");
   return done != 0;
 }
+__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) {  // one answer for the warp
+  return __all_sync(0xffffffffu, mbar_test(bar, parity));
+}
 // Bounded wait: false when the limit ran out or another role raised `abort`.  The limit is a module
 // variable, i.e. a global load; a wait that is over at once or soon does not pay for it.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort) {
@@ -103,6 +106,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if ((i & 255u) == 255u && *abort) return false;
   }
   return false;
+}
+// The same for a whole warp: the lanes come back together and with one answer, as the .aligned
+// tensor-memory and barrier instructions that follow need.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort));
+}
+// Named barrier of `threads` threads, whole warps.
+__device__ __forceinline__ void named_barrier_sync(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_barrier_arrive(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map, uint32_t bar,
                                             int c0, int c1, int c2, int c3) {
@@ -175,6 +192,14 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, ui
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// The same with both operands in shared memory.
+__device__ __forceinline__ void umma_f16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
 // 16 consecutive 32-bit columns of this thread's TMEM lane, written from registers.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *r) {
   asm volatile(
@@ -240,7 +265,10 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
+// (the barrier instructions are .aligned: the lanes of a warp must arrive together, also after code in
+// which they went different ways)
 __device__ __forceinline__ void cluster_sync_all() {  // every thread of every CTA in the cluster
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -248,6 +276,7 @@ __device__ __forceinline__ void cluster_sync_all() {  // every thread of every C
 // memory": the values read are in registers.  (A releasing arrive would first wait for the CTA's global
 // stores to be performed, ~1000 clocks at the end of every split-K launch.)
 __device__ __forceinline__ void cluster_sync_relaxed() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 }

@@ -1,0 +1,72 @@
+"""GPU parity of the half-precision-pair convolution (packed weights) against an fp64 convolution: every
+source of the raw patch (boxes, flattened rows, plane runs, whole small planes, flattened channel and
+tap), ragged tiles and channel tails, split-K, the input gate, and inputs whose first channel block
+misjudges the scale of the rest (the kernel then repeats the tile)."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from fluidml_b200 import cabi
+from fluidml_b200.cabi import DeviceTensor as DT
+
+
+def run(x, w, bias=None, pad=0, gate=None, act=cabi.ACT_NONE):
+    n, _, h, wd = x.shape
+    oc, _, k, _ = w.shape
+    dx, dw, y = DT.from_numpy(x), DT.from_numpy(w, [3, 2, 0, 1]), DT((n, oc, h + 2 * pad - k + 1, wd + 2 * pad - k + 1), np.float32)
+    assert cabi.conv_uses_packed(dx, dw, y, [pad, pad], scaled=gate is not None)
+    packed = cabi.conv_pack(dw)
+    db = None if bias is None else DT.from_numpy(bias)
+    if gate is None:
+        cabi.conv(dx, dw, db, y, [pad, pad], [1, 1], [1, 1], act=act, packed=packed)
+    else:
+        cabi.conv_scaled(dx, DT.from_numpy(gate), dw, db, y, [pad, pad], [1, 1], [1, 1], act=act, packed=packed)
+    cabi.check_device()
+    return y.numpy()
+
+
+def reference(x, w, bias=None, pad=0, gate=None):
+    t = lambda a: torch.from_numpy(a.astype(np.float64))
+    xs = x if gate is None else (x * gate).astype(np.float32)
+    return torch.nn.functional.conv2d(t(xs), t(w), None if bias is None else t(bias), padding=pad).numpy()
+
+
+@pytest.mark.parametrize("n,ic,oc,h,w,k,pad", [
+    (2, 32, 64, 24, 40, 3, 1), (1, 48, 36, 17, 20, 3, 1), (1, 64, 128, 16, 8, 3, 1), (1, 40, 32, 21, 12, 5, 2),  # boxes
+    (2, 64, 96, 14, 14, 3, 1), (1, 96, 512, 10, 10, 3, 1), (1, 512, 512, 14, 14, 3, 1),                          # flattened rows
+    (3, 16, 96, 20, 20, 1, 0), (1, 100, 24, 28, 28, 1, 0), (1, 320, 1280, 14, 14, 1, 0), (2, 24, 144, 56, 56, 1, 0),  # runs
+    (7, 192, 320, 7, 7, 1, 0), (2, 64, 40, 9, 9, 1, 0), (1, 1152, 192, 7, 7, 1, 0),                              # whole planes
+    (2, 3, 64, 32, 32, 3, 1), (1, 6, 32, 19, 36, 3, 1), (1, 2, 16, 33, 20, 5, 2),                                # channel x tap
+])
+def test_shapes(n, ic, oc, h, w, k, pad):
+    rng = np.random.default_rng(n * ic + oc + h)
+    x = rng.standard_normal((n, ic, h, w), np.float32)
+    wt = rng.standard_normal((oc, ic, k, k), np.float32) / np.float32(np.sqrt(ic * k * k))
+    b = rng.standard_normal(oc, np.float32)
+    ref = reference(x, wt, b, pad)
+    assert np.abs(run(x, wt, b, pad) - ref).max() <= 1e-5 * np.abs(ref).max()
+    assert np.abs(run(x, wt, b, pad, act=cabi.ACT_RELU) - np.maximum(ref, 0)).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n,ic,oc,hw", [(2, 96, 24, 28), (5, 480, 112, 7)])
+def test_gate(n, ic, oc, hw):
+    rng = np.random.default_rng(hw)
+    x, w = rng.standard_normal((n, ic, hw, hw), np.float32), rng.standard_normal((oc, ic, 1, 1), np.float32) * 0.1
+    g = rng.random((n, ic, 1, 1), np.float32)
+    ref = reference(x, w, gate=g)
+    assert np.abs(run(x, w, gate=g) - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("ic,hw,k", [(96, 16, 3), (128, 14, 1)])
+def test_scale_is_corrected(ic, hw, k):
+    rng = np.random.default_rng(ic)
+    w = rng.standard_normal((32, ic, k, k), np.float32)
+    base = rng.standard_normal((1, ic, hw, hw), np.float32)
+    for first, rest in ((1e-4, 1e3), (0.0, 1e-9), (0.0, 1e5), (1e20, 1e-3), (0.0, 0.0)):
+        x = base.copy()
+        x[:, :32] *= np.float32(first)
+        x[:, 32:] *= np.float32(rest)
+        ref, got = reference(x, w, pad=k // 2), run(x, w, pad=k // 2)
+        assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max() + 1e-37
