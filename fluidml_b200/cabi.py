@@ -234,8 +234,9 @@ def softmax(x, mask, divisor, out, axis, stream=None):
     check(lib().fml_softmax(_ref(x), _ref(mask), ctypes.c_float(divisor), _ref(out), int(axis), stream))
 
 
-def attention(q, kt, v, mask, divisor, out, stream=None):
-    check(lib().fml_attention(_ref(q), _ref(kt), _ref(v), _ref(mask), ctypes.c_float(divisor), _ref(out), stream))
+def attention(q, kt, v, mask, divisor, out, stream=None, causal=False):
+    f = lib().fml_attention_causal if causal else lib().fml_attention
+    check(f(_ref(q), _ref(kt), _ref(v), _ref(mask), ctypes.c_float(divisor), _ref(out), stream))
 
 
 def attention_uses_tensor_cores(q, kt, v) -> bool:

@@ -53,6 +53,7 @@ constexpr double kGemmStreamBytesPerNs = 3000.0; // operand streaming of one GEM
 constexpr double kFp32NsPerK = 90.0;             // CUDA-core GEMM: serial depth of the k loop
 constexpr double kAttentionFixedNs = 3000.0;     // staging K and V, softmax, exit
 constexpr double kAttentionFlopsPerNs = 9300.0;  // fp32 FMA attention, achieved
+constexpr double kAttentionPairFlopsPerNs = 140000.0;  // half-precision-pair attention, achieved
 constexpr double kStridedEfficiency = 0.125;     // 4 useful bytes per 32-byte sector
 constexpr double kStridedRowEfficiency = 0.035;  // row reductions walking a strided axis
 constexpr double kStridedRowNsPerElement = 20.0; // ... and their serial depth along the row
@@ -207,7 +208,9 @@ size_t CostModel::GetTimeCost(const flow::Node &n, const std::vector<Layout> &in
     const bool dflt = os[r - 1] == 1 && is[0][r - 1] == 1 && is[2][r - 1] == 1 && (is[1][r - 1] == 1 || is[1][r - 2] == 1);
     double bytes = obytes;
     for (const auto &r : n.inputs) bytes += (double)r->meta.GetSize();
-    cost = kLaunchNs + kAttentionFixedNs + std::max(flops / kAttentionFlopsPerNs, bytes / kHbmBytesPerNs) * (dflt ? 1.0 : 8.0);
+    // large blocks of head size 64: tensor cores, which want K along its head dimension
+    const bool pair = flops > 256e6 && is[1][r - 2] == 1 && fml_attention_any_size(n.inputs[0]->meta.GetShape().back(), o.meta.GetShape().back());
+    cost = kLaunchNs + kAttentionFixedNs + std::max(flops / (pair ? kAttentionPairFlopsPerNs : kAttentionFlopsPerNs), bytes / kHbmBytesPerNs) * (dflt ? 1.0 : 8.0);
     break;
   }
   case Kind::Softmax: case Kind::FusedSoftmax: case Kind::LayerNormalizationConstantScaleBias:

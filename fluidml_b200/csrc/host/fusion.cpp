@@ -230,6 +230,20 @@ bool FuseAddLayerNorm(Rewriter &rw, const NodePtr &add) {
   return true;
 }
 
+// A condition [1, .., S, S] that holds up to and including the diagonal and nowhere else.
+bool LowerTriangular(const flow::Region &cond) {
+  const auto &shape = cond.meta.GetShape();
+  const size_t rank = shape.size();
+  if (rank < 2 || shape[rank - 1] != shape[rank - 2]) return false;
+  for (size_t i = 0; i + 2 < rank; ++i)
+    if (shape[i] != 1) return false;
+  const int64_t n = shape[rank - 1];
+  for (int64_t r = 0; r < n; ++r)
+    for (int64_t c = 0; c < n; ++c)
+      if ((cond.constant->AsInt(r * n + c) != 0) != (c <= r)) return false;
+  return true;
+}
+
 // ---- x / c -> + mask -> Softmax  (attention scores); the mask may also be a constant-condition
 // Where that replaces masked scores by a scalar (a causal mask): Where(cond, s, y) feeds the
 // softmax the same values as s + m with m = cond ? 0 : y whenever y is so negative that
@@ -281,6 +295,7 @@ bool FuseScaledMaskedSoftmax(Rewriter &rw, const NodePtr &div) {
   } else if (where) {
     sm->inputs.push_back(mask);
     sm->has_mask = true;
+    sm->causal = LowerTriangular(*where->consts[0]) && where->value <= -1.0e30;
     rw.Kill(where);
   }
   rw.Kill(div);
@@ -308,21 +323,26 @@ bool FuseAttention(Rewriter &rw, const NodePtr &qk) {
   // launches it replaces are latency-bound; larger blocks are fused only when the tensor-core
   // attention kernel takes their head sizes (otherwise the score products are faster as GEMMs).
   double flops = 4.0 * (double)qs[rank - 2] * (double)ks[rank - 1] * (double)qs[rank - 1];
-  for (size_t i = 0; i + 2 < rank; ++i) flops *= (double)qs[i];
+  double heads = 1.0;
+  for (size_t i = 0; i + 2 < rank; ++i) heads *= (double)qs[i];
+  flops *= heads;
   {
     // FLUIDML_ATTENTION_FUSION_MFLOP moves the limit (for measurements); blocks the tensor-core
     // kernel takes are fused up to `tc_limit`: beyond a few key blocks its serial phases lose to
-    // the two batched tensor-core GEMMs around a softmax.
+    // the two batched tensor-core GEMMs around a softmax.  Head size 64 has a pipelined kernel and is
+    // fused whatever its size.
     static const double limit = [] { const char *e = getenv("FLUIDML_ATTENTION_FUSION_MFLOP"); return e ? atof(e) * 1e6 : 256e6; }();
     static const double tc_limit = [] { const char *e = getenv("FLUIDML_ATTENTION_TC_FUSION_MFLOP"); return e ? atof(e) * 1e6 : 256e6; }();
     const bool tc = fml_attention_on_tensor_cores(qs[rank - 2], ks[rank - 1], qs[rank - 1], vs[rank - 1]) != 0;
-    if (flops > (tc ? std::max(limit, tc_limit) : limit)) return false;
+    const bool any = tc && heads <= 65535.0 && fml_attention_any_size(qs[rank - 1], vs[rank - 1]) != 0;
+    if (!any && flops > (tc ? std::max(limit, tc_limit) : limit)) return false;
   }
   qk->kind = Kind::FusedAttention;
   qk->inputs = {q, kt, v};
   qk->divisor = sm->kind == Kind::FusedSoftmax ? sm->divisor : 1.0f;
   qk->has_mask = sm->kind == Kind::FusedSoftmax && sm->has_mask;
   if (qk->has_mask) qk->inputs.push_back(sm->inputs[1]);
+  qk->causal = qk->has_mask && sm->causal;
   qk->output = pv->output;
   rw.Kill(sm);
   rw.Kill(pv);

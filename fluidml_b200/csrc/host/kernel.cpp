@@ -457,13 +457,17 @@ private:
 // matmul.cpp:5-44 -> softmax.cpp:22-139 -> matmul.cpp:5-44 of one attention head group, fused
 class AttentionKernel : public Kernel {
 public:
-  AttentionKernel(float divisor, bool has_mask) : divisor_(divisor), has_mask_(has_mask) {}
+  AttentionKernel(float divisor, bool has_mask, bool causal) : divisor_(divisor), has_mask_(has_mask), causal_(causal) {}
   std::string GetKernelName() const override { return "FusedAttentionKernel"; }
   void Launch(LaunchRecorder &rec, const std::vector<fml_tensor> &in, const fml_tensor &output,
               const Buffer &) const override {
     const fml_tensor q = in.at(0), kt = in.at(1), v = in.at(2), mask = has_mask_ ? in.at(3) : fml_tensor{};
     const bool hm = has_mask_;
     const float d = divisor_;
+    if (causal_) {
+      rec.Add(GetKernelName(), [=](void *s) { return fml_attention_causal(&q, &kt, &v, &mask, d, &output, s); });
+      return;
+    }
     rec.Add(GetKernelName(), [=](void *s) { return fml_attention(&q, &kt, &v, hm ? &mask : nullptr, d, &output, s); });
   }
   bool DescribeResident(const std::vector<fml_tensor> &in, const fml_tensor &output, fml_resident_stage *st) const override {
@@ -478,7 +482,7 @@ public:
 
 private:
   float divisor_;
-  bool has_mask_;
+  bool has_mask_, causal_;
 };
 
 // layer_normalization.cpp:33-220 (+ the fused residual variant)
@@ -826,7 +830,7 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
     return std::make_unique<GatherConstantDataTensorAddTensorLhsAddTensorLhsKernel>(C(0), C(1), C(2));
   case Kind::Softmax: return std::make_unique<SoftmaxKernel>(n.axis, 1.0f, false);
   case Kind::FusedSoftmax: return std::make_unique<SoftmaxKernel>(n.axis, n.divisor, n.has_mask);
-  case Kind::FusedAttention: return std::make_unique<AttentionKernel>(n.divisor, n.has_mask);
+  case Kind::FusedAttention: return std::make_unique<AttentionKernel>(n.divisor, n.has_mask, n.causal);
   case Kind::LayerNormalizationConstantScaleBias:
     return std::make_unique<LayerNormalizationConstantScaleBiasKernel>(C(0), C(1), n.axis, n.epsilon, false);
   case Kind::FusedLayerNorm:

@@ -489,6 +489,11 @@ int launch_attention_tc(int64_t nb1, int64_t nb0, int64_t Sq, int64_t Sk, int64_
                         const int64_t *q_s, const float *k, const int64_t *k_s, const float *v, const int64_t *v_s,
                         const float *mask, const int64_t *m_s, float divisor, float *out, const int64_t *o_s,
                         cudaStream_t s);
+// attention_pair.cu
+bool attention_pair_shape_ok(int64_t d, int64_t d_v);
+int launch_attention_pair(int64_t nb1, int64_t nb0, int64_t Sq, int64_t Sk, const float *q, const int64_t *q_s, const float *k,
+                          const int64_t *k_s, const float *v, const int64_t *v_s, const float *mask, const int64_t *m_s, bool causal,
+                          float divisor, float *out, const int64_t *o_s, cudaStream_t s);
 }  // namespace fml
 
 // 1 when the tensor-core kernel (attention_tc.cu) takes blocks of these head sizes: such blocks are
@@ -504,8 +509,11 @@ extern "C" int fml_attention_supported(int64_t s_q, int64_t s_k, int64_t d, int6
              ? 1 : 0;
 }
 
-extern "C" int fml_attention(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v,
-                             const fml_tensor *mask, float divisor, const fml_tensor *out, void *stream) {
+// Blocks of any size are worth fusing when the half-precision-pair kernel takes their head size.
+extern "C" int fml_attention_any_size(int64_t d, int64_t d_v) { return attention_pair_shape_ok(d, d_v) ? 1 : 0; }
+
+static int attention_impl(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v, const fml_tensor *mask, bool causal,
+                          float divisor, const fml_tensor *out, void *stream) {
   FML_REQUIRE(q && kt && v && out, FML_BAD_ARG, "fml_attention: null tensor");
   FML_REQUIRE(q->dtype == FML_F32 && kt->dtype == FML_F32 && v->dtype == FML_F32 && out->dtype == FML_F32 &&
                   (!mask || mask->dtype == FML_F32), FML_UNSUPPORTED, "fml_attention: fp32 only");
@@ -538,9 +546,13 @@ extern "C" int fml_attention(const fml_tensor *q, const fml_tensor *kt, const fm
   a.mask = mask ? (const float *)mask->data : nullptr;
   a.out = (float *)out->data;
   a.divisor = divisor;
-  if (attention_tc_eligible(a.nb1, a.nb0, a.Sq, a.Sk, a.D, a.Dv, a.q_s, a.k_s, a.v_s, a.q, a.k, a.v))
+  if (attention_tc_eligible(a.nb1, a.nb0, a.Sq, a.Sk, a.D, a.Dv, a.q_s, a.k_s, a.v_s, a.q, a.k, a.v)) {
+    if (attention_pair_shape_ok(a.D, a.Dv))
+      return launch_attention_pair(a.nb1, a.nb0, a.Sq, a.Sk, a.q, a.q_s, a.k, a.k_s, a.v, a.v_s, a.mask, a.m_s, causal, divisor, a.out,
+                                   a.o_s, as_stream(stream));
     return launch_attention_tc(a.nb1, a.nb0, a.Sq, a.Sk, a.D, a.Dv, a.q, a.q_s, a.k, a.k_s, a.v, a.v_s, a.mask, a.m_s,
                                divisor, a.out, a.o_s, as_stream(stream));
+  }
   const bool whole = attn_smem_bytes(a.Sk, a.D, a.Dv) <= attn_flash_smem_bytes(a.D, a.Dv) ||
                      attn_flash_smem_bytes(a.D, a.Dv) > kSmemLimit;  // K and V of a head fit at once
   const size_t smem = whole ? attn_smem_bytes(a.Sk, a.D, a.Dv) : attn_flash_smem_bytes(a.D, a.Dv);
@@ -556,6 +568,17 @@ extern "C" int fml_attention(const fml_tensor *q, const fml_tensor *kt, const fm
   if (whole) FML_LAUNCH((attention_kernel), grid, kThreads, smem, as_stream(stream), a);
   else FML_LAUNCH((attention_flash_kernel), grid, kThreads, smem, as_stream(stream), a);
   return FML_OK;
+}
+
+extern "C" int fml_attention(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v,
+                             const fml_tensor *mask, float divisor, const fml_tensor *out, void *stream) {
+  return attention_impl(q, kt, v, mask, false, divisor, out, stream);
+}
+
+extern "C" int fml_attention_causal(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v, const fml_tensor *mask,
+                                    float divisor, const fml_tensor *out, void *stream) {
+  FML_REQUIRE(mask, FML_BAD_ARG, "fml_attention_causal: no mask");
+  return attention_impl(q, kt, v, mask, true, divisor, out, stream);
 }
 
 // Whether fml_attention would run these operands on the tensor cores (tests and planners).

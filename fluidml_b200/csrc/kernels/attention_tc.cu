@@ -386,8 +386,10 @@ bool attention_tc_eligible(int64_t nb1, int64_t nb0, int64_t Sq, int64_t Sk, int
   if (mode == 1) return true;
   // below ~200 Mflop, or with fewer tiles than two thirds of the SMs, the CUDA-core kernel's many
   // small CTAs finish sooner than a few large tiles (8 x 6 heads x 128 rows: 25 us against 30)
-  return 4.0 * (double)nb0 * (double)nb1 * (double)Sq * (double)Sk * (double)D >= 200e6 &&
-         nb0 * nb1 * ((Sq + kBM - 1) / kBM) >= 96;
+  const double flops = 4.0 * (double)nb0 * (double)nb1 * (double)Sq * (double)Sk * (double)D;
+  // (blocks beyond 256 Mflop that the pair kernel takes come here from the fusion pass whatever their tile count)
+  if (D == 64 && Dv == 64 && flops > 256e6) return true;
+  return flops >= 200e6 && nb0 * nb1 * ((Sq + kBM - 1) / kBM) >= 96;
 }
 
 int launch_attention_tc(int64_t nb1, int64_t nb0, int64_t Sq, int64_t Sk, int64_t D, int64_t Dv, const float *q,

@@ -247,8 +247,14 @@ int fml_attention_supported(int64_t s_q, int64_t s_k, int64_t d, int64_t d_v);
 int fml_attention_on_tensor_cores(int64_t s_q, int64_t s_k, int64_t d, int64_t d_v);
 /* The same question for concrete operands (shapes, strides, alignment, size). */
 int fml_attention_uses_tensor_cores(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v, int *uses);
+/* 1 when blocks of these head sizes stay fused whatever their size (the half-precision-pair kernel). */
+int fml_attention_any_size(int64_t d, int64_t d_v);
 int fml_attention(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v,
                   const fml_tensor *mask, float divisor, const fml_tensor *out, void *stream);
+/* The same when `mask` is known to be causal: 0 for keys up to the query's own position and so low beyond
+ * that the score plus it rounds to it (kernels may then skip the keys beyond instead of reading it). */
+int fml_attention_causal(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v, const fml_tensor *mask, float divisor,
+                         const fml_tensor *out, void *stream);
 
 /* LayerNormalizationConstantScaleBiasKernel (layer_normalization.cpp:33-220) in one pass:
  * mean, biased variance about the mean, y = (x-mean) * (1/sqrtf(var+eps)) * scale + bias.
