@@ -11,7 +11,9 @@
 //   A  per row and k slice, on the fly: the first k block (32 values) of the row puts its largest
 //      magnitude into [2^3, 2^4).  Elements far below it keep an absolute error of 2^-28 of that
 //      magnitude, below fp32's own rounding of the sum; 2^12 of headroom is left for larger values
-//      further along.  A row whose first block is all zero takes 2^8, right for magnitudes from 2^-12 to
+//      further along, and a CTA with a long k range looks at 64 values spread over it as well: what comes
+//      out of a convolution and a ReLU has stretches of zeros and of small values (VGG-16's first dense layer
+//      took 351 us instead of 64 when two of 32 rows needed a second attempt).  A row whose first block is all zero takes 2^8, right for magnitudes from 2^-12 to
 //      2^7.  A row that outgrows its scale overflows to infinity, which the finished accumulator shows
 //      in every column, and one whose magnitudes stay below the default scale's reach is noticed by
 //      their maximum: the CTA then finds the exact row maxima and does its tile a second time with
@@ -41,6 +43,7 @@ namespace {
 
 constexpr int kPairA = kBM * kPK * 4;        // bytes of A per block: a box of 128 rows x 128 bytes
 constexpr int kDefaultExponent = 8;          // scale 2^8 of a row whose first k block is all zero
+constexpr int kSampleBlocks = 48;            // from this many k blocks on, a row's scale is chosen with samples of all of them
 constexpr int kPairThreads = 320;
 constexpr int kConvThreads = 256;
 
@@ -260,6 +263,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     };
     bool guess = false;  // this row's scale is the default one
     float seen = 0.0f;   // largest scaled magnitude this thread converted (kept while a row of its warp has the default scale)
+    bool bad = false;    // this row needs a second attempt
+    const float *const a_row = a.p.a + (int64_t)z0 * a.p.a_b0 + (int64_t)z1 * a.p.a_b1 + ((int64_t)tile_m * kBM + row) * a.p.a_sm;
+    float sampled = 0.0f;
+    if (nkb >= kSampleBlocks && set == 0 && real_row) {
+      float4 y[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) y[i] = *reinterpret_cast<const float4 *>(a_row + (kb0 + (int64_t)i * (nkb - 1) / 16) * kPK);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sampled = fmaxf(sampled, fmaxf(fmaxf(fabsf(y[i].x), fabsf(y[i].y)), fmaxf(fabsf(y[i].z), fabsf(y[i].w))));
+    }
+    __syncwarp();
     for (int attempt = 0; attempt < 2 && ok; ++attempt) {
       // positions of this set's block in the two rings (the second attempt's blocks follow the first's)
       const int at = attempt * nkb + set;
@@ -267,18 +281,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       float4 x[8];
       bool have = false;
       if (attempt) {
-        // exact maximum of this row over the CTA's k range, straight from global memory (rare)
-        float m = 0.0f;
-        if (real_row) {
-          const float *src = a.p.a + (int64_t)z0 * a.p.a_b0 + (int64_t)z1 * a.p.a_b1 + ((int64_t)tile_m * kBM + row) * a.p.a_sm;
-          const int64_t k_end = min((int64_t)kb1 * kPK, a.p.K);
-          for (int64_t k = (int64_t)kb0 * kPK; k < k_end; ++k) m = fmaxf(m, fabsf(src[k]));
+        // exact maxima of those rows over the CTA's k range, straight from global memory (rare)
+        for (uint32_t left = __ballot_sync(0xffffffffu, bad); left; left &= left - 1) {
+          const int r = __ffs((int)left) - 1;
+          const float *src = a_row + (int64_t)(r - lane) * a.p.a_sm;
+          const float m = warp_row_max(src, (int64_t)kb0 * kPK, min((int64_t)kb1 * kPK, a.p.K), lane);
+          if (lane == r) k_row = scale_exponent(m, 14);
         }
-        k_row = scale_exponent(m, 14);
       } else {
         // set 0 finds the scale in block 0, set 1 takes it over
         if (set == 0) {
-          float m = 0.0f;
+          float m = sampled;
           if (nkb > 0) {
             ok = mbar_wait_warp(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
             if (ok) {
@@ -349,7 +362,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       tc_fence_before();
       if (watch && guess && seen > 0.0f) atomicMax(&row_seen[row], __float_as_uint(seen));
       named_barrier_sync(2, 256);  // every converter warp comes here, whether its waits were met or not
-      bool bad = !(fabsf(v0) <= 3.4028235e38f);
+      bad = !(fabsf(v0) <= 3.4028235e38f);
       if (watch && guess) {
         const float m = __uint_as_float(row_seen[row]);
         bad = bad || (m > 0.0f && m < 0.0625f);

@@ -27,4 +27,17 @@ __device__ __forceinline__ void split_pair(float x0, float x1, float s, uint32_t
   lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+// Largest magnitude of src[k0, k1) (16-byte aligned at k0, a multiple of 4), by the whole warp.
+__device__ __forceinline__ float warp_row_max(const float *src, int64_t k0, int64_t k1, int lane) {
+  float m = 0.0f;
+  const int64_t whole = k0 + ((k1 - k0) & ~3ll);
+#pragma unroll 4
+  for (int64_t k = k0 + lane * 4; k < whole; k += 128) {
+    const float4 x = *reinterpret_cast<const float4 *>(src + k);
+    m = fmaxf(m, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+  }
+  if (whole + lane < k1) m = fmaxf(m, fabsf(src[whole + lane]));
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));  // non-negative floats order as their bits
+}
+
 }  // namespace fml

@@ -76,3 +76,17 @@ def test_activations_match_the_unpacked_kernel(act):
     cabi.gemm(DT.from_numpy(a), DT.from_numpy(b), c, bias=DT.from_numpy(bias), params=cabi.gemm_params(act=act))
     ref = c.numpy()
     assert np.abs(got - ref).max() <= 2e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("split_k", [1, 2])
+def test_long_rows_with_stretches_of_zeros_and_small_values(split_k):
+    """Long k ranges: scales chosen with samples of the whole row; one row that the samples miss."""
+    rng = np.random.default_rng(11)
+    a, b = rng.standard_normal((70, 4100), np.float32), rng.standard_normal((4100, 64), np.float32) * 0.02
+    a *= np.repeat(rng.random((70, 82)) < 0.3, 50, axis=1)
+    a[:, :32] *= np.float32(1e-4)
+    a[5], a[6] = 0.0, 0.0
+    a[5, 4093], a[6, 1] = 3e5, 1e-5
+    got = run(a, b, tile_n=64, split_k=split_k)
+    scale = np.abs(a.astype(np.float64)) @ np.abs(b.astype(np.float64))
+    assert (np.abs(got - a.astype(np.float64) @ b.astype(np.float64)) <= 4e-6 * scale + 1e-37).all()
