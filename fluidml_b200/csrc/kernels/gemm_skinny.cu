@@ -5,9 +5,9 @@
 //   K-major B (b_sk == 1, e.g. Gemm with transB: weights stored [N, K]):
 //       one warp per output column walks its K slice with 16-byte loads (lane-contiguous in
 //       k), keeps M partial sums per lane and reduces them with shuffles;
-//   N-major B (b_sn == 1, e.g. MatMul with weights stored [K, N]):
-//       one thread per output column (lane-contiguous in n), A values broadcast from shared
-//       memory.
+//   N-major B (b_sn == 1, e.g. MatMul with weights stored [K, N]) and any other strides:
+//       one thread per output column (lane-contiguous in n) and k phase, A values broadcast from
+//       shared memory (gemm_skinny_rows_kernel).
 //
 // K is split over gridDim.y so that the grid covers the machine.  Each split writes its
 // partial [M, tile] block to scratch memory; the split that arrives last on the tile's
@@ -36,17 +36,30 @@ struct SkinnyArgs {
   float *partials;     // [batch * tiles_n][splits][M][kColsPerCta]
 };
 
-// FEW: the instantiation for at most four rows over 16-byte-aligned K-major operands (classifier
-// heads and poolers at batch 1 to 4).  It holds only that path's registers (the general path's 32
-// accumulators per lane made the shared kernel 176 registers = one CTA per SM = 12 % occupancy, and
-// a 411 MB weight matrix streamed at 48 % of DRAM's cycles), so three CTAs share an SM.
-template <bool KMAJOR, bool FEW>
-__global__ void __launch_bounds__(kThreads, FEW ? 3 : 1) gemm_skinny_kernel(SkinnyArgs a) {
+// Arrival of one split's partial sums at a tile; true in the CTA that is to finish the tile.
+__device__ __forceinline__ bool last_split(const SkinnyArgs &a, int64_t tile_id, int *flag) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) *flag = atomicAdd(a.counters + tile_id, 1u) == (unsigned)a.splits - 1u;
+  __syncthreads();
+  if (!*flag) return false;
+  __threadfence();
+  return true;
+}
+
+// K-major B.  ROWS 4 and 8: 16-byte-aligned operands, rows in groups of that many (4: at most four rows in
+// all, classifier heads and poolers at batch 1 to 4).  These hold only their own path's registers (the
+// general path's 32 accumulators per lane made a shared kernel 176 registers = one CTA per SM = 12 %
+// occupancy, and a 411 MB weight matrix streamed at 48 % of DRAM's cycles), so two or three CTAs share
+// an SM.  ROWS 0: anything else.
+template <int ROWS>
+__global__ void __launch_bounds__(kThreads, ROWS == 4 ? 3 : ROWS == 8 ? 2 : 1) gemm_skinny_kernel(SkinnyArgs a) {
+  constexpr bool FEW = ROWS != 0;
+  constexpr int R = FEW ? ROWS : 1;
   pdl_launch_dependents();
   // B is what this kernel streams; while the preceding kernel drains, start it towards L2
   l2_prefetch_span(a.p.b, ((a.p.K - 1) * a.p.b_sk + (a.p.N - 1) * a.p.b_sn + 1) * (int64_t)sizeof(float), 4 << 20);
   pdl_wait();
-  __shared__ float a_sh[KMAJOR ? 1 : kMaxM * 128];
   __shared__ float red[kMaxM][kColsPerCta];
   __shared__ int last_flag;
   const int M = (int)a.p.M;
@@ -58,39 +71,42 @@ __global__ void __launch_bounds__(kThreads, FEW ? 3 : 1) gemm_skinny_kernel(Skin
   const int64_t k0 = (int64_t)split * a.k_per_split, k1 = min(a.p.K, k0 + a.k_per_split);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-  if (KMAJOR) {
+  {
     // warp w owns columns n0 + w, n0 + w + 8, ... ; lanes stride over k in float4 steps
     const bool vec = a.p.a_sk == 1 && (a.p.a_sm & 3) == 0 && (a.p.b_sn & 3) == 0 && (k0 & 3) == 0 &&
                      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) == 0;
-    // At most four rows (batch-1 classifier heads, the pooler): the warp takes its four columns
-    // at once, so that eight weight loads are in flight per lane, the row chunks are loaded once
-    // for all four columns, and the shuffle reductions are amortised.  Same per-lane summation
-    // order as the general loop below.
-    if (FEW) {  // the launcher checks `vec && M <= 4` before it picks this instantiation
+    // The warp takes its four columns at once, so that eight weight loads are in flight per lane, the
+    // row chunks are loaded once for all four columns, and the shuffle reductions are amortised.  Same
+    // per-lane summation order as the general loop below.  (Row groups after the first find the
+    // columns in L1 or L2: 5 x 1280 x 1000 took 44 us with a column and 32 predicated rows at a time.)
+    for (int g = 0; FEW && g < (ROWS == 4 ? 1 : M); g += R) {  // the launcher checks `vec` before it picks these instantiations
+      const int rows = ROWS == 4 ? M : min(R, M - g);
+      const float *Ag = A + (int64_t)g * a.p.a_sm;
       const int64_t kv = k0 + ((k1 - k0) & ~(int64_t)3);
-      float acc4[4][4];
+      float acc4[4][R];
 #pragma unroll
       for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int m = 0; m < 4; ++m) acc4[j][m] = 0.0f;
+        for (int m = 0; m < R; ++m) acc4[j][m] = 0.0f;
       // columns past the edge of a ragged tile read the last column again (their sums are dropped below)
       const float *bcol[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) bcol[j] = B + min(n0 + warp * 4 + j, a.p.N - 1) * a.p.b_sn;
       auto dot4 = [](float4 x, float4 y, float t) { return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, t)))); };
+      auto weights4 = [](const float *x) { return R == 4 ? __ldcs(reinterpret_cast<const float4 *>(x)) : *reinterpret_cast<const float4 *>(x); };
       int64_t k = k0 + lane * 4;
       for (; k + 128 < kv; k += 256) {
         float4 bw[4][2];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          bw[j][0] = __ldcs(reinterpret_cast<const float4 *>(bcol[j] + k));
-          bw[j][1] = __ldcs(reinterpret_cast<const float4 *>(bcol[j] + k + 128));
+          bw[j][0] = weights4(bcol[j] + k);
+          bw[j][1] = weights4(bcol[j] + k + 128);
         }
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
-          if (m < M) {
-            const float4 a0 = *reinterpret_cast<const float4 *>(A + m * a.p.a_sm + k);
-            const float4 a1 = *reinterpret_cast<const float4 *>(A + m * a.p.a_sm + k + 128);
+        for (int m = 0; m < R; ++m)
+          if (m < rows) {
+            const float4 a0 = *reinterpret_cast<const float4 *>(Ag + m * a.p.a_sm + k);
+            const float4 a1 = *reinterpret_cast<const float4 *>(Ag + m * a.p.a_sm + k + 128);
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc4[j][m] = dot4(a1, bw[j][1], dot4(a0, bw[j][0], acc4[j][m]));
           }
@@ -98,10 +114,10 @@ __global__ void __launch_bounds__(kThreads, FEW ? 3 : 1) gemm_skinny_kernel(Skin
       for (; k < kv; k += 128) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float4 bv = __ldcs(reinterpret_cast<const float4 *>(bcol[j] + k));
+          const float4 bv = weights4(bcol[j] + k);
 #pragma unroll
-          for (int m = 0; m < 4; ++m)
-            if (m < M) acc4[j][m] = dot4(*reinterpret_cast<const float4 *>(A + m * a.p.a_sm + k), bv, acc4[j][m]);
+          for (int m = 0; m < R; ++m)
+            if (m < rows) acc4[j][m] = dot4(*reinterpret_cast<const float4 *>(Ag + m * a.p.a_sm + k), bv, acc4[j][m]);
         }
       }
       for (int64_t kt = kv + lane; kt < k1; kt += 32)
@@ -109,18 +125,18 @@ __global__ void __launch_bounds__(kThreads, FEW ? 3 : 1) gemm_skinny_kernel(Skin
         for (int j = 0; j < 4; ++j) {
           const float bv = bcol[j][kt];
 #pragma unroll
-          for (int m = 0; m < 4; ++m)
-            if (m < M) acc4[j][m] = fmaf(A[m * a.p.a_sm + kt], bv, acc4[j][m]);
+          for (int m = 0; m < R; ++m)
+            if (m < rows) acc4[j][m] = fmaf(Ag[m * a.p.a_sm + kt], bv, acc4[j][m]);
         }
 #pragma unroll
       for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
-          if (m < M) {
+        for (int m = 0; m < R; ++m)
+          if (m < rows) {
             float v = acc4[j][m];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) red[m][warp * 4 + j] = v;
+            if (lane == 0) red[g + m][warp * 4 + j] = v;
           }
     }
     for (int c = FEW ? kColsPerCta : warp; c < kColsPerCta; c += kThreads / 32) {
@@ -186,39 +202,6 @@ __global__ void __launch_bounds__(kThreads, FEW ? 3 : 1) gemm_skinny_kernel(Skin
           if (lane == 0) red[m][c] = v;
         }
     }
-  } else {
-    // thread (c, kq): column n0 + c, every 8th k of the slice; A staged in shared memory in
-    // chunks of 128 k values
-    const int c = threadIdx.x & 31, kq = threadIdx.x >> 5;
-    const int64_t n = n0 + c;
-    float acc[kMaxM];
-#pragma unroll
-    for (int m = 0; m < kMaxM; ++m) acc[m] = 0.0f;
-    for (int64_t kc = k0; kc < k1; kc += 128) {
-      const int len = (int)min((int64_t)128, k1 - kc);
-      __syncthreads();
-      for (int i = threadIdx.x; i < M * 128; i += kThreads) {
-        const int m = i >> 7, kk = i & 127;
-        a_sh[i] = kk < len ? A[m * a.p.a_sm + (kc + kk) * a.p.a_sk] : 0.0f;
-      }
-      __syncthreads();
-      if (n < a.p.N)
-#pragma unroll 4
-        for (int kk = kq; kk < len; kk += kThreads / 32) {
-          const float bv = __ldcs(B + (kc + kk) * a.p.b_sk + n * a.p.b_sn);
-#pragma unroll
-          for (int m = 0; m < kMaxM; ++m)
-            if (m < M) acc[m] = fmaf(a_sh[m * 128 + kk], bv, acc[m]);
-        }
-    }
-    // reduce the 8 k-phases of each column through shared memory, in phase order
-    for (int ph = 0; ph < kThreads / 32; ++ph) {
-      __syncthreads();
-      if (kq == ph)
-#pragma unroll
-        for (int m = 0; m < kMaxM; ++m)
-          if (m < M) red[m][c] = (ph == 0 ? 0.0f : red[m][c]) + acc[m];
-    }
   }
   __syncthreads();
 
@@ -230,12 +213,7 @@ __global__ void __launch_bounds__(kThreads, FEW ? 3 : 1) gemm_skinny_kernel(Skin
   if (a.splits > 1) {
     float *part = a.partials + ((tile_id * a.splits + split) * M) * kColsPerCta;
     for (int i = threadIdx.x; i < M * kColsPerCta; i += kThreads) part[i] = red[i / kColsPerCta][i % kColsPerCta];
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last_flag = atomicAdd(a.counters + tile_id, 1u) == (unsigned)a.splits - 1u;
-    __syncthreads();
-    if (!last_flag) return;
-    __threadfence();
+    if (!last_split(a, tile_id, &last_flag)) return;
   }
   for (int i = threadIdx.x; i < M * kColsPerCta; i += kThreads) {
     const int m = i / kColsPerCta, c = i % kColsPerCta;
@@ -252,6 +230,118 @@ __global__ void __launch_bounds__(kThreads, FEW ? 3 : 1) gemm_skinny_kernel(Skin
     const float bv = bias ? bias[m * a.p.bias_sm + n * a.p.bias_sn] : 0.0f;
     const float rv = res ? res[m * a.p.res_sm + n * a.p.res_sn] : 0.0f;
     C[m * a.p.c_sm + n * a.p.c_sn] = gemm_epilogue(a.e, acc, bv, rv);
+  }
+  if (a.splits > 1 && threadIdx.x == 0) a.counters[tile_id] = 0u;  // ready for the next launch
+}
+
+// N-major B: thread (c, kq) takes column n0 + c and every 8th k of the slice, for MR rows (M rounded up), in
+// chunks of 128 k.  What bounds the small ones (16 rows, K and N of a few hundred) is the chain of latencies
+// after the preceding kernel, so constant weights of the first chunk are in registers before the wait for
+// it, each later chunk's are loaded under the products of the one before, bias and residual are fetched
+// ahead, A is stored [k][row] (one 16-byte broadcast per four products), and the eight k phases are added
+// up behind one barrier.
+template <int MR>
+__global__ void __launch_bounds__(kThreads, MR == 32 ? 1 : 2) gemm_skinny_rows_kernel(SkinnyArgs a) {
+  constexpr int kChunk = 128, kPhases = kThreads / 32, kLoads = kChunk / kPhases, kPitch = MR + 4;
+  constexpr int kItems = (MR * kColsPerCta + kThreads - 1) / kThreads;  // outputs per thread
+  __shared__ __align__(16) float sh[kPhases * MR * kColsPerCta];         // A chunk, later the phases' sums
+  __shared__ int last_flag;
+  pdl_launch_dependents();
+  const int M = (int)a.p.M;
+  const int tile = blockIdx.x, split = blockIdx.y, z = blockIdx.z;
+  const int64_t z0 = z % a.p.nb0, z1 = z / a.p.nb0;
+  const float *A = a.p.a + z0 * a.p.a_b0 + z1 * a.p.a_b1;
+  const int64_t n0 = (int64_t)tile * kColsPerCta;
+  const int64_t k0 = (int64_t)split * a.k_per_split, k1 = min(a.p.K, k0 + a.k_per_split);
+  const int c = threadIdx.x & 31, kq = threadIdx.x >> 5;
+  const bool col = n0 + c < a.p.N;
+  const float *B = a.p.b + z0 * a.p.b_b0 + z1 * a.p.b_b1 + (n0 + c) * a.p.b_sn;
+  float w[kLoads];
+  auto load = [&](int64_t kc) {
+#pragma unroll
+    for (int i = 0; i < kLoads; ++i) {
+      const int64_t k = kc + kq + i * kPhases;
+      w[i] = col && k < k1 ? __ldcs(B + k * a.p.b_sk) : 0.0f;
+    }
+  };
+  if (a.p.b_constant) load(k0);
+  l2_prefetch_span(a.p.b, ((a.p.K - 1) * a.p.b_sk + (a.p.N - 1) * a.p.b_sn + 1) * (int64_t)sizeof(float), 4 << 20);
+  pdl_wait();
+  if (!a.p.b_constant) load(k0);
+  const float *bias = a.p.bias ? a.p.bias + z0 * a.p.bias_b0 + z1 * a.p.bias_b1 : nullptr;
+  const float *res = a.p.res ? a.p.res + z0 * a.p.res_b0 + z1 * a.p.res_b1 : nullptr;
+  float bv[kItems], rv[kItems];
+#pragma unroll
+  for (int j = 0; j < kItems; ++j) {
+    const int m = kq + j * kPhases;  // (output items: row m, column c)
+    const bool in = col && m < M;
+    bv[j] = bias && in ? bias[m * a.p.bias_sm + (n0 + c) * a.p.bias_sn] : 0.0f;
+    rv[j] = res && in ? res[m * a.p.res_sm + (n0 + c) * a.p.res_sn] : 0.0f;
+  }
+  float acc[MR];
+#pragma unroll
+  for (int m = 0; m < MR; ++m) acc[m] = 0.0f;
+  for (int64_t kc = k0; kc < k1; kc += kChunk) {
+    float x[MR * kChunk / kThreads];
+    const int kk = threadIdx.x & (kChunk - 1), m_first = threadIdx.x / kChunk;
+#pragma unroll
+    for (int i = 0; i < MR * kChunk / kThreads; ++i) {
+      const int m = m_first + i * (kThreads / kChunk);
+      x[i] = m < M && kc + kk < k1 ? A[m * a.p.a_sm + (kc + kk) * a.p.a_sk] : 0.0f;
+    }
+    if (kc > k0) __syncthreads();  // the chunk before has been read
+#pragma unroll
+    for (int i = 0; i < MR * kChunk / kThreads; ++i) sh[kk * kPitch + m_first + i * (kThreads / kChunk)] = x[i];
+    __syncthreads();
+    float u[kLoads];
+#pragma unroll
+    for (int i = 0; i < kLoads; ++i) u[i] = w[i];
+    if (kc + kChunk < k1) load(kc + kChunk);
+#pragma unroll
+    for (int i = 0; i < kLoads; ++i)
+#pragma unroll
+      for (int m = 0; m < MR; m += 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(sh + (kq + i * kPhases) * kPitch + m);
+        acc[m] = fmaf(v.x, u[i], acc[m]);
+        acc[m + 1] = fmaf(v.y, u[i], acc[m + 1]);
+        acc[m + 2] = fmaf(v.z, u[i], acc[m + 2]);
+        acc[m + 3] = fmaf(v.w, u[i], acc[m + 3]);
+      }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < MR; ++m) sh[(kq * MR + m) * kColsPerCta + c] = acc[m];
+  __syncthreads();
+  float v[kItems];
+#pragma unroll
+  for (int j = 0; j < kItems; ++j) {
+    const int m = kq + j * kPhases;
+    v[j] = 0.0f;
+    if (m < MR)
+#pragma unroll
+      for (int ph = 0; ph < kPhases; ++ph) v[j] += sh[(ph * MR + m) * kColsPerCta + c];
+  }
+  const int64_t tile_id = (int64_t)z * a.tiles_n + tile;
+  if (a.splits > 1) {
+    float *part = a.partials + (tile_id * a.splits * M) * kColsPerCta;
+#pragma unroll
+    for (int j = 0; j < kItems; ++j)
+      if (kq + j * kPhases < M) part[((int64_t)split * M + kq + j * kPhases) * kColsPerCta + c] = v[j];
+    if (!last_split(a, tile_id, &last_flag)) return;
+#pragma unroll
+    for (int j = 0; j < kItems; ++j) {
+      const int m = kq + j * kPhases;
+      v[j] = 0.0f;
+      if (m < M)
+#pragma unroll 8
+        for (int sp = 0; sp < a.splits; ++sp) v[j] += __ldcg(part + ((int64_t)sp * M + m) * kColsPerCta + c);
+    }
+  }
+  float *C = a.p.c + z0 * a.p.c_b0 + z1 * a.p.c_b1;
+#pragma unroll
+  for (int j = 0; j < kItems; ++j) {
+    const int m = kq + j * kPhases;
+    if (col && m < M) C[m * a.p.c_sm + (n0 + c) * a.p.c_sn] = gemm_epilogue(a.e, v[j], bv[j], rv[j]);
   }
   if (a.splits > 1 && threadIdx.x == 0) a.counters[tile_id] = 0u;  // ready for the next launch
 }
@@ -294,12 +384,19 @@ int launch_skinny(const GemmProblem &p, const GemmEpilogue &e, const SkinnyPlan 
   const dim3 grid((unsigned)pl.tiles_n, (unsigned)pl.splits, (unsigned)(p.nb0 * p.nb1));
   if (p.b_sk == 1 && p.b_sn != 1) {
     // (k slices start at multiples of 128, so every slice keeps the 16-byte alignment of its row)
-    const bool few = p.M <= 4 && p.a_sk == 1 && (p.a_sm & 3) == 0 && (p.b_sn & 3) == 0 && aligned16(p.a) && aligned16(p.b) &&
+    const bool vec = p.a_sk == 1 && (p.a_sm & 3) == 0 && (p.b_sn & 3) == 0 && aligned16(p.a) && aligned16(p.b) &&
                      (p.a_b0 & 3) == 0 && (p.a_b1 & 3) == 0 && (p.b_b0 & 3) == 0 && (p.b_b1 & 3) == 0;
-    if (few) FML_LAUNCH((gemm_skinny_kernel<true, true>), grid, kThreads, 0, s, a);
-    else FML_LAUNCH((gemm_skinny_kernel<true, false>), grid, kThreads, 0, s, a);
+    if (vec && p.M <= 4) FML_LAUNCH((gemm_skinny_kernel<4>), grid, kThreads, 0, s, a);
+    else if (vec) FML_LAUNCH((gemm_skinny_kernel<8>), grid, kThreads, 0, s, a);
+    else FML_LAUNCH((gemm_skinny_kernel<0>), grid, kThreads, 0, s, a);
+  } else if (p.M <= 4) {
+    FML_LAUNCH((gemm_skinny_rows_kernel<4>), grid, kThreads, 0, s, a);
+  } else if (p.M <= 8) {
+    FML_LAUNCH((gemm_skinny_rows_kernel<8>), grid, kThreads, 0, s, a);
+  } else if (p.M <= 16) {
+    FML_LAUNCH((gemm_skinny_rows_kernel<16>), grid, kThreads, 0, s, a);
   } else {
-    FML_LAUNCH((gemm_skinny_kernel<false, false>), grid, kThreads, 0, s, a);
+    FML_LAUNCH((gemm_skinny_rows_kernel<32>), grid, kThreads, 0, s, a);
   }
   return FML_OK;
 }
