@@ -458,21 +458,26 @@ struct PadArgs {
 };
 // One pass over the output: an element inside the window of the input copies it, the rest is
 // zero.  (A fill followed by a copy of the interior would be two launches and write the interior
-// twice.)
-__global__ void pad_kernel(PadArgs a, float *out, const float *in) {
+// twice.)  The dims come in the order of the output's memory, so that its writes are coalesced whatever
+// its layout; V = 4 when the innermost of them is contiguous on both sides and not padded; I as in
+// ew_f32_generic.  8 x 128 x 384 to 136 rows: 6.2 -> 3.6 us.
+template <typename I, int V> __global__ void pad_kernel(PadArgs a, float *out, const float *in) {
   pdl_prologue();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.total; i += (int64_t)gridDim.x * blockDim.x) {
-    int64_t lin = i, oo = 0, io = 0;
+  const I total = (I)a.total;
+  for (I i = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x; i < total; i += (I)gridDim.x * (I)blockDim.x) {
+    I lin = i, oo = 0, io = 0;
     bool inside = true;
     for (int d = a.rank - 1; d >= 0; --d) {
-      const int64_t q = lin / a.oshape[d], c = lin - q * a.oshape[d];
-      lin = q;
-      oo += c * a.ostride[d];
-      const int64_t ci = c - a.begin[d];
-      inside = inside && ci >= 0 && ci < a.ishape[d];
-      io += ci * a.istride[d];
+      I c = lin;
+      if (d > 0) { const I q = lin / (I)a.oshape[d]; c = lin - q * (I)a.oshape[d]; lin = q; }
+      if (V == 4 && d == a.rank - 1) c *= 4;
+      oo += c * (I)a.ostride[d];
+      const I ci = c - (I)a.begin[d];
+      inside = inside && ci >= 0 && ci < (I)a.ishape[d];
+      io += ci * (I)a.istride[d];
     }
-    out[oo] = inside ? in[io] : 0.0f;
+    if (V == 4) *reinterpret_cast<float4 *>(out + oo) = inside ? *reinterpret_cast<const float4 *>(in + io) : make_float4(0.f, 0.f, 0.f, 0.f);
+    else out[oo] = inside ? in[io] : 0.0f;
   }
 }
 }  // namespace
@@ -495,8 +500,33 @@ extern "C" int fml_pad(const fml_tensor *in, const fml_tensor *out, const int64_
     a.total *= out->shape[i];
   }
   if (a.total == 0) return FML_OK;
-  FML_LAUNCH((fml::pad_kernel), fml::grid_for(a.total, 256), 256, 0, fml::as_stream(stream), a, (float *)out->data,
-             (const float *)in->data);
+  for (int i = 1; i < a.rank; ++i)  // into the order of the output's memory
+    for (int j = i; j > 0 && a.ostride[j] > a.ostride[j - 1]; --j) {
+      std::swap(a.oshape[j], a.oshape[j - 1]); std::swap(a.ostride[j], a.ostride[j - 1]);
+      std::swap(a.ishape[j], a.ishape[j - 1]); std::swap(a.istride[j], a.istride[j - 1]);
+      std::swap(a.begin[j], a.begin[j - 1]);
+    }
+  int64_t o_top = 0, i_top = 0;
+  const int l = a.rank - 1;
+  bool narrow = a.total < (1ll << 30);
+  bool vec = a.rank > 0 && a.ostride[l] == 1 && a.istride[l] == 1 && a.begin[l] == 0 && a.ishape[l] == a.oshape[l] && a.oshape[l] % 4 == 0 &&
+             fml::aligned16(in->data) && fml::aligned16(out->data);
+  for (int i = 0; i < a.rank; ++i) {
+    narrow = narrow && a.ostride[i] >= 0 && a.istride[i] >= 0;
+    o_top += a.ostride[i] * (a.oshape[i] - 1);
+    i_top += a.istride[i] * (a.oshape[i] - 1);
+    if (i < l) vec = vec && a.ostride[i] % 4 == 0 && a.istride[i] % 4 == 0;
+  }
+  narrow = narrow && o_top < (1ll << 30) && i_top < (1ll << 30);
+  if (vec) { a.oshape[l] /= 4; a.total /= 4; }
+  const int grid = fml::grid_for(a.total, 256);
+  cudaStream_t s = fml::as_stream(stream);
+  float *dst = (float *)out->data;
+  const float *src = (const float *)in->data;
+  if (narrow && vec) FML_LAUNCH((fml::pad_kernel<int32_t, 4>), grid, 256, 0, s, a, dst, src);
+  else if (narrow) FML_LAUNCH((fml::pad_kernel<int32_t, 1>), grid, 256, 0, s, a, dst, src);
+  else if (vec) FML_LAUNCH((fml::pad_kernel<int64_t, 4>), grid, 256, 0, s, a, dst, src);
+  else FML_LAUNCH((fml::pad_kernel<int64_t, 1>), grid, 256, 0, s, a, dst, src);
   return FML_OK;
 }
 
