@@ -577,6 +577,34 @@ __global__ void __launch_bounds__(256) pool2x2_kernel(const float *__restrict__ 
 
 using namespace fml;
 
+// A 1-D pointwise convolution as the 2-D one over planes of one row, for the packed-weight kernel: ConvBERT's
+// 768 -> 384 over 8 x 128 took 25 us as a 3xTF32 product per image, now 13.5.  Only those whose product ran on tensor cores
+// (channel-contiguous weights, whole 16-byte groups of pixels); false for the others.
+struct Planes { fml_tensor x, w, y; };
+static fml_tensor with_rows(const fml_tensor *t) {  // [.., .., L] -> [.., .., 1, L]; rank 4 as it is
+  fml_tensor r = *t;
+  if (t->rank != 3) return r;
+  r.rank = 4;
+  r.shape[3] = t->shape[2]; r.stride[3] = t->stride[2];
+  r.shape[2] = 1; r.stride[2] = t->shape[2] * t->stride[2];
+  return r;
+}
+static bool as_planes(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, Planes *o) {
+  if (x->rank != 3 || w->rank != 3 || y->rank != 3 || p->group > 1 || w->shape[2] != 1 || w->stride[1] != 1) return false;
+  if (p->pads_begin[0] != 0 || p->strides[0] != 1 || p->dilations[0] != 1 || x->shape[2] != y->shape[2] || x->shape[2] % 4) return false;
+  if (x->stride[2] != 1 || y->stride[2] != 1 || x->stride[0] % 4 || x->stride[1] % 4 || !aligned16(x->data) || !aligned16(w->data)) return false;
+  if (w->shape[0] < 64 || w->shape[1] < 32 || x->shape[2] < 32 || w->stride[0] % 4) return false;
+  *o = {with_rows(x), with_rows(w), with_rows(y)};
+  // (only the packed copy of the weights is read: the layout the 2-D kernels want of the others)
+  o->w.stride[0] = 1; o->w.stride[1] = w->shape[0]; o->w.stride[2] = o->w.stride[3] = w->shape[0] * w->shape[1];
+  return true;
+}
+static fml_conv_params plane_params(const fml_conv_params *p) {
+  fml_conv_params r = *p;
+  for (int i = 0; i < 2; ++i) { r.pads_begin[i] = 0; r.strides[i] = r.dilations[i] = 1; }
+  return r;
+}
+
 // x_scale: nullptr, or a tensor broadcastable to [N, IC, 1, 1] that multiplies x (fml_conv_scaled)
 static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
                      const fml_tensor *y, const fml_conv_params *p, void *stream) {
@@ -682,6 +710,10 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
     return fml_gemm(&A, &B, &Cc, a.bias ? &bias_t : nullptr, nullptr, &gp, stream);
   }
   if (group == 1 && nd == 2 && p->w_packed && conv_pair_eligible(x, w, y, p, false)) return launch_conv_pair(x, w, bias, y, p, s);
+  if (Planes pl; nd == 1 && group == 1 && p->w_packed && as_planes(x, w, y, p, &pl)) {
+    const fml_conv_params q = plane_params(p);
+    if (conv_pair_eligible(&pl.x, &pl.w, &pl.y, &q, false)) return launch_conv_pair(&pl.x, &pl.w, bias, &pl.y, &q, s);
+  }
   if (group == 1 && nd == 2 && conv_tc_eligible(x, w, y, p)) return launch_conv_tc(x, w, bias, y, p, s);
   if (group == 1 && a.KH == 1 && a.KW == 1 && a.ph == 0 && a.pw == 0 && a.sh == 1 && a.sw == 1 && a.ws[1] == 1 &&
       a.xs[3] == 1 && (nd == 1 || a.xs[2] == a.IW) && a.ys[3] == 1 && (nd == 1 || a.ys[2] == a.OW) &&
@@ -794,6 +826,11 @@ extern "C" int fml_conv_uses_tensor_cores(const fml_tensor *x, const fml_tensor 
 extern "C" int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p,
                                     int scaled, int *uses) {
   FML_REQUIRE(valid_tensor(x) && valid_tensor(w) && valid_tensor(y) && p && uses, FML_BAD_ARG, "fml_conv_uses_packed: bad argument");
+  if (Planes pl; !scaled && as_planes(x, w, y, p, &pl)) {
+    const fml_conv_params q = plane_params(p);
+    *uses = x->dtype == FML_F32 && w->dtype == FML_F32 && y->dtype == FML_F32 && conv_pair_eligible(&pl.x, &pl.w, &pl.y, &q, false) ? 1 : 0;
+    return FML_OK;
+  }
   *uses = x->rank == 4 && w->rank == 4 && y->rank == 4 && x->dtype == FML_F32 && w->dtype == FML_F32 && y->dtype == FML_F32 &&
                   p->group <= 1 && x->shape[2] * x->shape[3] > 1 && (!scaled || x->shape[1] <= 4096) &&
                   conv_pair_eligible(x, w, y, p, scaled != 0)
@@ -810,20 +847,30 @@ extern "C" int fml_conv_autotune(const fml_tensor *x, const fml_tensor *x_scale,
   if (st != FML_OK) return st;
   if (!p->w_packed || !uses || p->tile_n) return FML_OK;  // nothing to choose
   FML_CUDA(cudaStreamSynchronize(as_stream(stream)));
+  if (Planes pl; !x_scale && as_planes(x, w, y, p, &pl)) {
+    const fml_conv_params q = plane_params(p);
+    fml_conv_params t = q;
+    const int ts = tune_conv_pair(&pl.x, &pl.w, bias, &pl.y, &q, nullptr, 0, 0, &t);
+    tuned->tile_n = t.tile_n; tuned->strips = t.strips; tuned->split_k = t.split_k; tuned->ctas_per_sm = t.ctas_per_sm;
+    return ts;
+  }
   return tune_conv_pair(x, w, bias, y, p, x_scale ? (const float *)x_scale->data : nullptr,
                         x_scale && x_scale->shape[0] != 1 ? x_scale->stride[0] : 0, x_scale && x_scale->shape[1] != 1 ? x_scale->stride[1] : 0,
                         tuned);
 }
 
 extern "C" size_t fml_conv_packed_bytes(const fml_tensor *w) {
-  return w && w->rank == 4 && numel(w) > 0 ? conv_packed_bytes(w) : 0;
+  if (!w || (w->rank != 3 && w->rank != 4) || numel(w) <= 0) return 0;
+  const fml_tensor v = with_rows(w);
+  return conv_packed_bytes(&v);
 }
 
 extern "C" int fml_conv_pack(const fml_tensor *w, void *packed, size_t bytes, void *stream) {
-  FML_REQUIRE(valid_tensor(w) && w->dtype == FML_F32 && w->rank == 4 && numel(w) > 0 && packed, FML_BAD_ARG, "fml_conv_pack: bad argument");
-  FML_REQUIRE(bytes >= conv_packed_bytes(w), FML_BAD_ARG, "fml_conv_pack: the destination is too small");
+  FML_REQUIRE(valid_tensor(w) && w->dtype == FML_F32 && (w->rank == 3 || w->rank == 4) && numel(w) > 0 && packed, FML_BAD_ARG, "fml_conv_pack: bad argument");
+  const fml_tensor v = with_rows(w);
+  FML_REQUIRE(bytes >= conv_packed_bytes(&v), FML_BAD_ARG, "fml_conv_pack: the destination is too small");
   FML_REQUIRE(aligned16(packed), FML_MISALIGNED, "fml_conv_pack: the destination must be 16-byte aligned");
-  return conv_pack(w, packed, as_stream(stream));
+  return conv_pack(&v, packed, as_stream(stream));
 }
 
 extern "C" int fml_pool2d(const fml_tensor *x, const fml_tensor *y, int mode, const int64_t *kernel,

@@ -70,3 +70,15 @@ def test_scale_is_corrected(ic, hw, k):
         x[:, 32:] *= np.float32(rest)
         ref, got = reference(x, w, pad=k // 2), run(x, w, pad=k // 2)
         assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max() + 1e-37
+
+
+@pytest.mark.parametrize("n,ic,oc,length", [(8, 768, 384, 128), (3, 40, 100, 36), (1, 32, 64, 1000)])
+def test_one_dimensional_pointwise(n, ic, oc, length):
+    rng = np.random.default_rng(length)
+    x, w, b = rng.standard_normal((n, ic, length), np.float32), rng.standard_normal((oc, ic, 1), np.float32) * 0.1, rng.standard_normal(oc, np.float32)
+    dx, dw, y = DT.from_numpy(x), DT.from_numpy(w), DT((n, oc, length), np.float32)
+    assert cabi.conv_uses_packed(dx, dw, y, [0, 0])
+    cabi.conv(dx, dw, DT.from_numpy(b), y, [0], [1], [1], packed=cabi.conv_pack(dw))
+    cabi.check_device()
+    ref = np.einsum("oi,nil->nol", w[..., 0].astype(np.float64), x.astype(np.float64)) + b[:, None]
+    assert np.abs(y.numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
