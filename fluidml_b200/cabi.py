@@ -359,6 +359,16 @@ def conv(x, w, bias, y, pads_begin, strides, dilations, group=1, act=ACT_NONE, s
     check(lib().fml_conv(_ref(x), _ref(w), _ref(bias), _ref(y), ctypes.byref(p), stream))
 
 
+def conv_residual(x, x_scale, w, bias, residual, y, pads_begin, act=ACT_NONE, stream=None, packed=None):
+    """fml_conv / fml_conv_scaled (unit strides) plus a residual of y's shape, added after the activation."""
+    p = ConvParams()
+    p.w_packed = packed.ptr if packed is not None else None
+    for i in range(2):
+        p.pads_begin[i], p.strides[i], p.dilations[i] = pads_begin[i], 1, 1
+    p.group, p.act, p.precision = 1, act, GEMM_AUTO
+    check(lib().fml_conv_residual(_ref(x), _ref(x_scale), _ref(w), _ref(bias), _ref(residual), _ref(y), ctypes.byref(p), stream))
+
+
 def conv_scaled(x, x_scale, w, bias, y, pads_begin, strides, dilations, act=ACT_NONE, stream=None, precision=None, packed=None):
     """y = conv(x * x_scale, w) + bias with x_scale broadcastable to [N, IC, 1, 1] (group 1)."""
     p = ConvParams()

@@ -227,14 +227,15 @@ size_t CostModel::GetTimeCost(const flow::Node &n, const std::vector<Layout> &in
   case Kind::ConvWithPadding: case Kind::ConvWithoutPadding: case Kind::MaxPoolWithoutPadding:
   case Kind::AveragePoolWithoutPadding: {
     // NCHW kernels: anything but the default layout on either side strides every access
-    const bool dflt = IsRowMajor(n.inputs[0]->meta.GetShape(), is[0]) && IsRowMajor(o.meta.GetShape(), os);
+    bool dflt = IsRowMajor(n.inputs[0]->meta.GetShape(), is[0]) && IsRowMajor(o.meta.GetShape(), os);
+    if (n.has_residual) dflt = dflt && IsRowMajor(o.meta.GetShape(), is[n.inputs.size() - 1]);
     double flops = 0;
     if (!n.consts.empty()) {
       double w = 1;
       for (size_t i = 1; i < n.consts[0]->meta.GetRank(); ++i) w *= (double)n.consts[0]->meta.GetShape()[i];
       flops = 2.0 * (double)o.meta.GetElementsNum() * w;
     }
-    const double bytes = obytes + (double)n.inputs[0]->meta.GetSize();
+    const double bytes = obytes * (n.has_residual ? 2.0 : 1.0) + (double)n.inputs[0]->meta.GetSize();
     cost = kLaunchNs + std::max(flops / kFp32FlopsPerNs, bytes / kHbmBytesPerNs) * (dflt ? 1.0 : 8.0);
     break;
   }

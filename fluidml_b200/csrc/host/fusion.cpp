@@ -471,6 +471,23 @@ bool FuseGateIntoConv(Rewriter &rw, const NodePtr &mul) {
   return true;
 }
 
+// ---- Conv + x -> the convolution's epilogue (the residual of an inverted bottleneck).  Group 1 and 2-D: what the
+// packed-weight kernel may take; where another kernel runs, the sum is a launch of its own as before.
+bool FuseResidualIntoConv(Rewriter &rw, const NodePtr &cv) {
+  if ((cv->kind != Kind::ConvWithPadding && cv->kind != Kind::ConvWithoutPadding) || cv->group != 1 || cv->act != 0 || cv->has_residual) return false;
+  NodePtr add = rw.SoleOfKind(cv->output, Kind::AddCommon);
+  if (!add) return false;
+  RegionPtr x = Other(add, cv->output);
+  if (IsConst(x) || x == cv->output || x->meta != cv->output->meta || add->output->meta != cv->output->meta) return false;
+  const auto &os = x->meta.GetShape();
+  if (os.size() != 4 || os[2] * os[3] < 32 || x->meta.GetType() != Type::kFloat32) return false;
+  cv->inputs.push_back(x);
+  cv->has_residual = true;
+  cv->output = add->output;
+  rw.Kill(add);
+  return true;
+}
+
 // ---- MulCommon -> FusedMulAdd -> FusedMulAdd ...: a sum of products (ConvBERT's span convolution
 // adds nine windows times nine softmax columns) becomes one pass.  Matched at the last node of the
 // chain and walked back to the plain product it starts from; every intermediate sum must have the
@@ -699,7 +716,7 @@ size_t FusionPasses::Run(flow::Flow &flow) {
   using Pass = bool (*)(Rewriter &, const NodePtr &);
   // order matters: bias before GELU / activation before residual, residual before Add+LN
   const Pass passes[] = {FuseEmbedding, FuseMask, FuseBias, FuseGeluIntoGemm, FuseBiasGelu, FuseActivation,
-                         FuseResidual, FuseSecondResidual, FuseAddLayerNorm, FuseScaledMaskedSoftmax, FuseAttention, FuseSilu, FuseSiluIntoConv, FuseSqueezeExcite, FuseGateIntoConv, FuseMulAdd, FuseRotary, FuseMulAddChain};
+                         FuseResidual, FuseSecondResidual, FuseAddLayerNorm, FuseScaledMaskedSoftmax, FuseAttention, FuseSilu, FuseSiluIntoConv, FuseSqueezeExcite, FuseGateIntoConv, FuseResidualIntoConv, FuseMulAdd, FuseRotary, FuseMulAddChain};
   for (Pass pass : passes) {
     bool again = true;
     while (again) {

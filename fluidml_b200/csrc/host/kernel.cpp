@@ -673,15 +673,16 @@ bool TunedConvTiles(const fml_conv_params &p, GemmTiles *t) {
   return true;
 }
 
-// conv.cpp:27-280
-class ConvKernel : public SingleInputWithoutBufferKernel {
+// conv.cpp:27-280; with a scale (mul.cpp + conv.cpp: the per-channel gate multiplies x inside the convolution's
+// operand gather) and a residual (conv.cpp + add.cpp: added in the epilogue) when the node has them
+class ConvKernel : public Kernel {
 public:
-  ConvKernel(const char *name, fml_tensor w, bool has_bias, fml_tensor bias, fml_conv_params p, bool autotune)
-      : name_(name), w_(w), has_bias_(has_bias), bias_(bias), p_(p), autotune_(autotune) {}
+  ConvKernel(const char *name, fml_tensor w, bool has_bias, fml_tensor bias, bool has_scale, bool has_residual, fml_conv_params p, bool autotune)
+      : name_(name), w_(w), has_bias_(has_bias), bias_(bias), has_scale_(has_scale), has_residual_(has_residual), p_(p), autotune_(autotune) {}
   std::string GetKernelName() const override { return name_; }
   size_t PackedBytes(const std::vector<fml_tensor> &in, const fml_tensor &output, fml_tensor *source) const override {
     int uses = 0;
-    if (fml_conv_uses_packed(&in.at(0), &w_, &output, &p_, 0, &uses) != FML_OK || !uses) return 0;
+    if (fml_conv_uses_packed(&in.at(0), &w_, &output, &p_, has_scale_, &uses) != FML_OK || !uses) return 0;
     *source = w_;
     return fml_conv_packed_bytes(&w_);
   }
@@ -689,11 +690,16 @@ public:
   void SetPacked(const void *packed, size_t) override { p_.w_packed = packed; }
   void PresetTiles(const GemmTiles &t) override { PresetConvTiles(t, &p_); }
   bool TunedTiles(GemmTiles *t) const override { return TunedConvTiles(tuned_, t); }
-  void Run(LaunchRecorder &rec, const fml_tensor &input, const fml_tensor &output) const override {
-    const fml_tensor w = w_, b = bias_;
-    const bool hb = has_bias_;
-    const fml_conv_params p = tuned_ = TuneConv(name_, input, nullptr, w, hb ? &b : nullptr, output, p_, autotune_);
-    rec.Add(name_, [=](void *s) { return fml_conv(&input, &w, hb ? &b : nullptr, &output, &p, s); });
+  void Launch(LaunchRecorder &rec, const std::vector<fml_tensor> &in, const fml_tensor &output, const Buffer &) const override {
+    const fml_tensor x = in.at(0), w = w_, b = bias_;
+    const fml_tensor scale = has_scale_ ? in.at(1) : fml_tensor{}, res = has_residual_ ? in.back() : fml_tensor{};
+    const bool hb = has_bias_, hs = has_scale_, hr = has_residual_;
+    const fml_conv_params p = tuned_ = TuneConv(name_, x, hs ? &scale : nullptr, w, hb ? &b : nullptr, output, p_, autotune_);
+    rec.Add(name_, [=](void *s) {
+      const fml_tensor *bias = hb ? &b : nullptr;
+      if (hr) return fml_conv_residual(&x, hs ? &scale : nullptr, &w, bias, &res, &output, &p, s);
+      return hs ? fml_conv_scaled(&x, &scale, &w, bias, &output, &p, s) : fml_conv(&x, &w, bias, &output, &p, s);
+    });
   }
 
 private:
@@ -701,39 +707,7 @@ private:
   fml_tensor w_;
   bool has_bias_;
   fml_tensor bias_;
-  fml_conv_params p_;
-  bool autotune_;
-  mutable fml_conv_params tuned_{};
-};
-
-// mul.cpp + conv.cpp: the per-channel gate multiplies x inside the convolution's operand gather
-class ScaledConvKernel : public DoubleInputsWithoutBufferKernel {
-public:
-  ScaledConvKernel(const char *name, fml_tensor w, bool has_bias, fml_tensor bias, fml_conv_params p, bool autotune)
-      : name_(name), w_(w), has_bias_(has_bias), bias_(bias), p_(p), autotune_(autotune) {}
-  std::string GetKernelName() const override { return name_; }
-  size_t PackedBytes(const std::vector<fml_tensor> &in, const fml_tensor &output, fml_tensor *source) const override {
-    int uses = 0;
-    if (fml_conv_uses_packed(&in.at(0), &w_, &output, &p_, 1, &uses) != FML_OK || !uses) return 0;
-    *source = w_;
-    return fml_conv_packed_bytes(&w_);
-  }
-  int Pack(const fml_tensor &source, void *packed, size_t bytes) const override { return fml_conv_pack(&source, packed, bytes, nullptr); }
-  void SetPacked(const void *packed, size_t) override { p_.w_packed = packed; }
-  void PresetTiles(const GemmTiles &t) override { PresetConvTiles(t, &p_); }
-  bool TunedTiles(GemmTiles *t) const override { return TunedConvTiles(tuned_, t); }
-  void Run(LaunchRecorder &rec, const fml_tensor &x, const fml_tensor &scale, const fml_tensor &output) const override {
-    const fml_tensor w = w_, b = bias_;
-    const bool hb = has_bias_;
-    const fml_conv_params p = tuned_ = TuneConv(name_, x, &scale, w, hb ? &b : nullptr, output, p_, autotune_);
-    rec.Add(name_, [=](void *s) { return fml_conv_scaled(&x, &scale, &w, hb ? &b : nullptr, &output, &p, s); });
-  }
-
-private:
-  const char *name_;
-  fml_tensor w_;
-  bool has_bias_;
-  fml_tensor bias_;
+  bool has_scale_, has_residual_;
   fml_conv_params p_;
   bool autotune_;
   mutable fml_conv_params tuned_{};
@@ -894,8 +868,7 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
     p.act = n.act;
     p.precision = options.gemm_precision;
     const char *name = n.kind == Kind::ConvWithPadding ? "ConvWithPaddingKernel" : "ConvWithoutPaddingKernel";
-    if (n.has_in_scale) return std::make_unique<ScaledConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, p, options.autotune);
-    return std::make_unique<ConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, p, options.autotune);
+    return std::make_unique<ConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, n.has_in_scale, n.has_residual, p, options.autotune);
   }
   case Kind::MaxPoolWithoutPadding:
     return std::make_unique<PoolKernel>("MaxPoolWithoutPaddingKernel", 0, n.kernel_shape, n.strides);

@@ -607,7 +607,7 @@ static fml_conv_params plane_params(const fml_conv_params *p) {
 
 // x_scale: nullptr, or a tensor broadcastable to [N, IC, 1, 1] that multiplies x (fml_conv_scaled)
 static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
-                     const fml_tensor *y, const fml_conv_params *p, void *stream) {
+                     const fml_tensor *y, const fml_conv_params *p, void *stream, const float *residual = nullptr) {
   FML_REQUIRE(valid_tensor(x) && valid_tensor(w) && valid_tensor(y) && p, FML_BAD_ARG, "fml_conv: bad argument");
   FML_REQUIRE(x->dtype == FML_F32 && w->dtype == FML_F32 && y->dtype == FML_F32, FML_UNSUPPORTED, "fml_conv: fp32 only");
   FML_REQUIRE((x->rank == 3 || x->rank == 4) && w->rank == x->rank && y->rank == x->rank, FML_BAD_ARG,
@@ -666,7 +666,7 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
     // the tensor-core kernel applies the scale while it splits the operand; every other case
     // takes the general implicit GEMM (the specialised CUDA-core paths below read x unscaled)
     if (nd == 2 && a.IC <= 4096 && p->w_packed && conv_pair_eligible(x, w, y, p, true))
-      return launch_conv_pair(x, w, bias, y, p, s, a.scale, a.scale_sn, a.scale_sc);
+      return launch_conv_pair(x, w, bias, y, p, s, a.scale, a.scale_sn, a.scale_sc, residual);
     if (nd == 2 && a.IC <= 4096 && conv_tc_eligible(x, w, y, p))
       return launch_conv_tc(x, w, bias, y, p, s, a.scale, a.scale_sn, a.scale_sc);
     FML_REQUIRE((M + CB - 1) / CB <= 65535, FML_UNSUPPORTED, "fml_conv_scaled: too many output pixels for one launch");
@@ -709,7 +709,8 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
     gp.act = a.act;
     return fml_gemm(&A, &B, &Cc, a.bias ? &bias_t : nullptr, nullptr, &gp, stream);
   }
-  if (group == 1 && nd == 2 && p->w_packed && conv_pair_eligible(x, w, y, p, false)) return launch_conv_pair(x, w, bias, y, p, s);
+  if (group == 1 && nd == 2 && p->w_packed && conv_pair_eligible(x, w, y, p, false))
+    return launch_conv_pair(x, w, bias, y, p, s, nullptr, 0, 0, residual);
   if (Planes pl; nd == 1 && group == 1 && p->w_packed && as_planes(x, w, y, p, &pl)) {
     const fml_conv_params q = plane_params(p);
     if (conv_pair_eligible(&pl.x, &pl.w, &pl.y, &q, false)) return launch_conv_pair(&pl.x, &pl.w, bias, &pl.y, &q, s);
@@ -811,6 +812,25 @@ extern "C" int fml_conv_scaled(const fml_tensor *x, const fml_tensor *x_scale, c
                                const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p, void *stream) {
   FML_REQUIRE(x_scale, FML_BAD_ARG, "fml_conv_scaled: no scale");
   return conv_impl(x, x_scale, w, bias, y, p, stream);
+}
+
+extern "C" int fml_conv_residual(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
+                                 const fml_tensor *residual, const fml_tensor *y, const fml_conv_params *p, void *stream) {
+  FML_REQUIRE(valid_tensor(residual) && valid_tensor(y) && p && residual->dtype == FML_F32 && residual->rank == y->rank, FML_BAD_ARG,
+              "fml_conv_residual: bad argument");
+  bool same = true;  // laid out as y: the packed-weight kernel adds it in its epilogue
+  for (int i = 0; i < y->rank; ++i) {
+    FML_REQUIRE(residual->shape[i] == y->shape[i], FML_BAD_ARG, "fml_conv_residual: the residual's shape is y's");
+    same = same && (y->shape[i] == 1 || residual->stride[i] == y->stride[i]);
+  }
+  int uses = 0;
+  if (same && y->rank == 4 && p->w_packed) {
+    const int st = fml_conv_uses_packed(x, w, y, p, x_scale != nullptr, &uses);
+    if (st != FML_OK) return st;
+  }
+  if (uses) return conv_impl(x, x_scale, w, bias, y, p, stream, (const float *)residual->data);
+  const int st = conv_impl(x, x_scale, w, bias, y, p, stream);
+  return st != FML_OK ? st : fml_elementwise(FML_ADD, y, residual, y, 0.0, 0.0, stream);
 }
 
 extern "C" int fml_conv_uses_tensor_cores(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y,

@@ -849,7 +849,8 @@ int conv_pack(const fml_tensor *w, void *dst, cudaStream_t s) {
 }
 
 static int launch_planned(ConvPairArgs a, size_t smem, const fml_tensor *x, const fml_tensor *bias, const fml_tensor *y,
-                          const fml_conv_params *p, cudaStream_t s, const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc) {
+                          const fml_conv_params *p, cudaStream_t s, const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc,
+                          const float *residual = nullptr) {
   a.x = (const float *)x->data;
   a.packed = static_cast<const char *>(p->w_packed);
   a.col_scale = reinterpret_cast<const float *>(a.packed + (size_t)conv_k_blocks(a.IC, a.KH * a.KW) * a.n_pad * kPairB);
@@ -861,7 +862,7 @@ static int launch_planned(ConvPairArgs a, size_t smem, const fml_tensor *x, cons
   }
   a.act = p->act;
   a.scale = x_scale; a.scale_sn = x_scale_sn; a.scale_sc = x_scale_sc;
-  a.res = nullptr;
+  a.res = residual;
   a.status = device_status_word();
   FML_REQUIRE(a.status, FML_CUDA_ERROR, "fml_conv: no device status word");
   CUtensorMap map_x;
@@ -910,11 +911,11 @@ static int launch_planned(ConvPairArgs a, size_t smem, const fml_tensor *x, cons
 }
 
 int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
-                     cudaStream_t s, const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc) {
+                     cudaStream_t s, const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual) {
   ConvPairArgs a;
   const size_t smem = plan_conv_pair(x, w, y, p, x_scale != nullptr, a);
   FML_REQUIRE(smem, FML_UNSUPPORTED, "fml_conv: this layer has no packed form");
-  return launch_planned(a, smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc);
+  return launch_planned(a, smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc, residual);
 }
 
 // Times the candidates the model ranks highest as captured graphs of back-to-back launches and keeps the

@@ -97,8 +97,10 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
 bool conv_pair_eligible(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool has_scale);
 size_t conv_packed_bytes(const fml_tensor *w);
 int conv_pack(const fml_tensor *w, void *dst, cudaStream_t s);
+// (residual: added after the activation, laid out as y)
 int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
-                     cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0, int64_t x_scale_sc = 0);
+                     cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0, int64_t x_scale_sc = 0,
+                     const float *residual = nullptr);
 int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
                    const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, fml_conv_params *tuned);
 

@@ -412,6 +412,10 @@ int fml_conv(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias,
  * the tensor-core kernel when it is eligible, else the general implicit GEMM. */
 int fml_conv_scaled(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w,
                     const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p, void *stream);
+/* Either of them (x_scale may be NULL) plus a residual of y's shape, added after the activation: in the
+ * convolution's epilogue where the packed-weight kernel runs and both have one layout, else by a kernel of its own. */
+int fml_conv_residual(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
+                      const fml_tensor *residual, const fml_tensor *y, const fml_conv_params *p, void *stream);
 
 /* Reports which path fml_conv takes: 1 = the tcgen05 implicit GEMM (2-D, group 1, unit stride
  * and dilation, dense NCHW input whose row length is a multiple of 4, weights stored

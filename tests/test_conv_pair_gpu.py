@@ -82,3 +82,19 @@ def test_one_dimensional_pointwise(n, ic, oc, length):
     cabi.check_device()
     ref = np.einsum("oi,nil->nol", w[..., 0].astype(np.float64), x.astype(np.float64)) + b[:, None]
     assert np.abs(y.numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n,ic,oc,hw,k,gated,layout", [
+    (2, 96, 24, 28, 1, True, None), (3, 240, 40, 14, 1, True, None), (5, 1152, 192, 7, 1, True, None), (1, 64, 64, 24, 3, False, None),
+    (1, 512, 512, 14, 3, False, None), (2, 96, 24, 28, 1, True, [0, 2, 3, 1])])  # the last: a residual laid out otherwise
+def test_residual(n, ic, oc, hw, k, gated, layout):
+    rng = np.random.default_rng(hw + oc)
+    x, w = rng.standard_normal((n, ic, hw, hw), np.float32), rng.standard_normal((oc, ic, k, k), np.float32) * np.float32(0.05)
+    res, b = rng.standard_normal((n, oc, hw, hw), np.float32), rng.standard_normal(oc, np.float32)
+    g = rng.random((n, ic, 1, 1), np.float32) if gated else None
+    dx, dw, y = DT.from_numpy(x), DT.from_numpy(w, [3, 2, 0, 1]), DT((n, oc, hw, hw), np.float32)
+    cabi.conv_residual(dx, None if g is None else DT.from_numpy(g), dw, DT.from_numpy(b), DT.from_numpy(res, layout), y, [k // 2, k // 2],
+                       act=cabi.ACT_RELU, packed=cabi.conv_pack(dw))
+    cabi.check_device()
+    ref = np.maximum(reference(x, w, b, k // 2, g), 0) + res
+    assert np.abs(y.numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
