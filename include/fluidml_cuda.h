@@ -395,11 +395,11 @@ typedef struct fml_conv_params {
 /* Packs constant weights [OC, IC, KH, KW] (any strides) for fml_conv_params::w_packed. */
 size_t fml_conv_packed_bytes(const fml_tensor *w);
 int fml_conv_pack(const fml_tensor *w, void *packed, size_t bytes, void *stream);
-/* Whether fml_conv (scaled: fml_conv_scaled) would use packed weights for these operands. */
 /* On-device choice of the tile for a layer with packed weights (x_scale: NULL, or the gate of
  * fml_conv_scaled), as fml_gemm_autotune: y is overwritten, the call synchronises. */
 int fml_conv_autotune(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,
                       const fml_conv_params *p, void *stream, fml_conv_params *tuned);
+/* Whether fml_conv (scaled: fml_conv_scaled) would use packed weights for these operands. */
 int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int scaled, int *uses);
 
 int fml_conv(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias,
