@@ -340,6 +340,7 @@ private:
       for (const auto &r : n->inputs) ins.Push(json::Value(r->name));
       e.Set("inputs", ins);
       e.Set("scratch", json::Value((double)n->buffer_size));
+      if (n->causal) e.Set("causal", json::Value(true));
       seq.Push(e);
     }
     stats_.Set("sequence", seq);

@@ -253,11 +253,14 @@ bool FuseAddLayerNorm(Rewriter &rw, const NodePtr &add) {
   return true;
 }
 
-// A condition [1, .., S, S] that holds up to and including the diagonal and nowhere else.
-bool LowerTriangular(const flow::Region &cond) {
-  const auto &shape = cond.meta.GetShape();
+// A condition [1, .., S, S] over scores [.., S, S] that holds up to and including the diagonal and nowhere
+// else.  It has to span both of the scores' own last dims: one true value broadcast over them is a
+// "lower-triangular" 1 x 1 matrix, but hides nothing.
+bool LowerTriangular(const flow::Region &cond, const Meta &scores) {
+  const auto &shape = cond.meta.GetShape(), &over = scores.GetShape();
   const size_t rank = shape.size();
-  if (rank < 2 || shape[rank - 1] != shape[rank - 2]) return false;
+  if (rank < 2 || over.size() < rank || shape[rank - 1] != shape[rank - 2]) return false;
+  if (shape[rank - 1] != over[over.size() - 1] || shape[rank - 2] != over[over.size() - 2]) return false;
   for (size_t i = 0; i + 2 < rank; ++i)
     if (shape[i] != 1) return false;
   const int64_t n = shape[rank - 1];
@@ -318,7 +321,7 @@ bool FuseScaledMaskedSoftmax(Rewriter &rw, const NodePtr &div) {
   } else if (where) {
     sm->inputs.push_back(mask);
     sm->has_mask = true;
-    sm->causal = LowerTriangular(*where->consts[0]) && where->value <= -1.0e30;
+    sm->causal = LowerTriangular(*where->consts[0], where->output->meta) && where->value <= -1.0e30;
     rw.Kill(where);
   }
   rw.Kill(div);
