@@ -492,9 +492,11 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
       if (lane == 0) mbar_arrive(bar_decide);
       ok = ok && mbar_wait_warp(bar_decide, 0u, abort_flag);
       if (!ok || !*redo_flag) break;
+      // The first attempt's phase is waited for before the second begins: once both are over, the parity of
+      // the first would look like a phase still to come.
+      ok = mbar_wait_warp(bar_accum, 0u, abort_flag);
     }
-    if (ok) ok = mbar_wait_warp(bar_accum, 0u, abort_flag);
-    if (ok && *redo_flag) ok = mbar_wait_warp(bar_accum, 1u, abort_flag);
+    if (ok) ok = mbar_wait_warp(bar_accum, *redo_flag ? 1u : 0u, abort_flag);
     if (!ok) {
       atomicOr(a.status, kStatusTimeout);
       *abort_flag = 1;

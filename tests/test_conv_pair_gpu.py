@@ -72,6 +72,19 @@ def test_scale_is_corrected(ic, hw, k):
         assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max() + 1e-37
 
 
+@pytest.mark.parametrize("ic,oc,h,w,k", [(64, 32, 128, 256, 1), (64, 512, 64, 64, 1), (96, 64, 128, 128, 3)])
+def test_every_tile_is_repeated(ic, oc, h, w, k):
+    """Hundreds of CTAs whose second attempt ends right after their last block is split: both attempts'
+    accumulator phases are waited for in order."""
+    rng = np.random.default_rng(oc)
+    x, wt = rng.standard_normal((2, ic, h, w), np.float32), rng.standard_normal((oc, ic, k, k), np.float32)
+    x[:, :32] = 0.0
+    x[:, 32:] *= np.float32(1e6)
+    ref = reference(x, wt, pad=k // 2)
+    for _ in range(4):
+        assert np.abs(run(x, wt, pad=k // 2) - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("n,ic,oc,length", [(8, 768, 384, 128), (3, 40, 100, 36), (1, 32, 64, 1000)])
 def test_one_dimensional_pointwise(n, ic, oc, length):
     rng = np.random.default_rng(length)
