@@ -23,11 +23,20 @@
 //   kIm2col  few input channels (IC * KH * KW <= 64, any stride up to 4): K = (channel, tap) flattened, the
 //            split gathers the taps itself, so that a 3 x 3 layer over 3 channels is one k block, not nine
 //
-// Range of fp16: one power of two per tile (all pixels of a patch feed all rows through the taps), from the
-// largest magnitude of the first channel block, which lands in [2^9, 2^10): values down to 2^-12 of it keep
-// all 22 bits, and 2^6 of headroom is left.  The largest magnitude of every block is tracked; a tile that
-// outgrows its scale, or started on an all-zero block and then stayed far below the default scale, is done
-// a second time with the exact maximum (gemm_pair.cu).
+// Range of fp16.  A product's row must not lose bits to a large value that it does not contain: pixels of one
+// tile may belong to different requests (kImages), and an infinity or a stray huge value stays with the pixels
+// that touch it.
+//   One k block per channel block (taps == 1): a pixel is a row and has its own power of two, chosen and
+//   corrected as in gemm_pair.cu -- the row's first block lands in [2^3, 2^4), a row that outgrows it (or
+//   began with zeros and stayed far below the default) is done a second time with its exact maximum.
+//   With taps a pixel of the patch feeds several rows, so the tile starts on one common power of two that puts
+//   the first block's largest finite magnitude into [2^9, 2^10), and the largest magnitude of every pixel is
+//   tracked.  When nothing overflowed and every row's window holds a pixel of at least 2^0 (or only zeros),
+//   that was precise: what a pair leaves out is 2^-25 of 2^0.  Otherwise the tile is done again in bands of
+//   2^14, the smallest first: a pass takes the pixels whose largest magnitude lies in its band (infinities ride
+//   in the last one), at the scale that puts them into [2^1, 2^15), and a row's accumulator is rescaled when
+//   the row's window has pixels in the band at hand.  One band is the usual case (a tile that outgrew its
+//   scale); a range beyond 2^14 within a tile costs one pass for every 2^14 in use.
 //
 // Roles, 320 threads: warp 0 loads, warp 1 issues MMAs, warps 2-9 split the patches and do the epilogue.
 #include "gemm_common.cuh"
@@ -45,8 +54,13 @@ namespace {
 enum { kBox = 0, kFlat = 1, kRun = 2, kImages = 3, kIm2col = 4 };
 enum { kPlain = 0, kGated = 1, kTaps = 2 };
 constexpr int kThreads = 320;
-constexpr int kTargetExp = 9;         // first block's largest magnitude lands in [2^9, 2^10)
+constexpr int kTargetExp = 9;         // tile scale: the first block's largest magnitude lands in [2^9, 2^10)
 constexpr int kDefaultScaleExp = 4;   // of a tile whose first block is all zero
+constexpr int kRowTargetExp = 3;      // scale of a row of its own: [2^3, 2^4) (gemm_pair.cu)
+constexpr int kRowDefaultExp = 8;     // of a row whose first block is all zero
+constexpr int kBandBits = 14;         // magnitudes of a band of the second attempt span 2^14
+constexpr float kMaxFinite = 3.4028235e38f;
+constexpr int kRowWords = 3 * kBM;    // row_max and row_inv
 constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;
 
 struct ConvPairArgs {
@@ -154,8 +168,8 @@ __device__ __forceinline__ void store_sums(const ConvPairArgs &a, const float *s
 // SOURCE: how the split of a patch finds its eight values -- kPlain: eight channels, kGated: eight channels
 // times the gate, kTaps: eight (channel, tap) pairs.  A template parameter, and the loads plain selects: with
 // uniform branches inside the inner loop the split of 128 pixels x 32 channels took 2000 clocks, 340 of them
-// work.
-template <int SOURCE>
+// work.  ROWS: a scale per pixel (one k block per channel block; then a thread has one pixel at most), not per tile.
+template <int SOURCE, bool ROWS>
 __global__ void __launch_bounds__(kThreads, 2)
 conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -178,12 +192,16 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
   uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NB + 2 * RB + 6);
   volatile int *const abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   volatile int *const redo_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
-  unsigned *const first_max = tmem_slot + 3;                             // bits of the first block's largest magnitude
+  unsigned *const first_max = tmem_slot + 3;                             // bits of the first block's largest finite magnitude
   unsigned *const tile_max = tmem_slot + 4;                              // ... and of all blocks'
+  volatile int *const suspect_flag = reinterpret_cast<volatile int *>(tmem_slot + 5);
+  unsigned *const band_mask = tmem_slot + 6;                             // bands that hold a pixel; bit 31: passes are needed
   // (the barriers are an even number and start on 16 bytes, so this does too)
   float2 *const cb_s = reinterpret_cast<float2 *>(tmem_slot + 8);        // [BN]: column scale, bias
   int *const koff_s = reinterpret_cast<int *>(cb_s + BN);                // [64]: kTaps, raw offset of k; negative: none
-  float *const scale_s = reinterpret_cast<float *>(koff_s + 64);         // [imgs][channels of this split]: the gate
+  unsigned *const row_max = reinterpret_cast<unsigned *>(koff_s + 64);   // [128]: largest magnitude of a row that two threads share
+  float *const row_inv = reinterpret_cast<float *>(row_max + kBM);       // [128 MT]: undoes the scale of a row (taps == 1)
+  float *const scale_s = reinterpret_cast<float *>(koff_s + 64) + (ROWS ? kRowWords : 0);  // [imgs][channels of this split]: the gate
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const bool leader = elect_one();
@@ -220,8 +238,11 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
     *redo_flag = 0;
     *first_max = 0u;
     *tile_max = 0u;
+    *suspect_flag = 0;
+    *band_mask = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (ROWS && threadIdx.x >= 64 && threadIdx.x < 64 + kBM) row_max[threadIdx.x - 64] = 0u;
   if (warp == 1) tmem_alloc(smem_u32(tmem_slot), tmem_cols);
   tc_fence_before();
   __syncthreads();
@@ -250,10 +271,13 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
       int issued_r = 0, issued_b = pre_b;
       RingPos rr, rb;
       for (int j = 0; j < pre_b; ++j) rb.step(NB);
-      for (int attempt = 0; attempt < 2 && ok; ++attempt) {
+      unsigned passes = 1u;  // one bit per pass to come
+      for (int attempt = 0; passes && ok; ++attempt) {
         if (attempt) {
-          ok = mbar_wait_warp(bar_decide, 0u, abort_flag);
-          if (!ok || !*redo_flag) break;
+          ok = mbar_wait_warp(bar_decide, (uint32_t)(attempt - 1) & 1u, abort_flag);
+          if (attempt == 1) passes = (unsigned)*redo_flag;
+          if (!ok || !passes) break;
+          passes &= passes - 1u;
         }
         int ir = 0, jb = attempt ? 0 : pre_b;
         uint32_t idle = 0;
@@ -312,11 +336,16 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
     const uint64_t desc_a = smem_desc(patch0, chunk, group_bytes, 0u);
     RingPos rb, rp;
     bool ok = true;
-    for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-      if (attempt) {
-        ok = mbar_wait_warp(bar_decide, 0u, abort_flag);
-        if (!ok || !*redo_flag) break;
+    unsigned passes = 1u;  // one bit per pass to come
+    for (int attempt = 0; passes && ok; ++attempt) {
+      if (attempt) {  // (the first of them starts the accumulators anew, the others add to them)
+        ok = mbar_wait_warp(bar_decide, (uint32_t)(attempt - 1) & 1u, abort_flag);
+        if (attempt == 1) passes = (unsigned)*redo_flag;
+        if (!ok || !passes) break;
+        passes &= passes - 1u;
+        tc_fence_after();
       }
+      const uint32_t first = attempt > 1 ? 1u : 0u;
       int in_group = 0, kb = 0;
       for (int icb = 0; icb < n_icb && ok; ++icb) {
         ok = mbar_wait_warp(bar_pfull + 8u * rp.s, rp.ph, abort_flag);
@@ -339,7 +368,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
               for (int j = 0; j < kPK / 16; ++j) {
                 const uint64_t dah = da0 + (uint64_t)((2u * j * chunk) >> 4), dal = dah + (uint64_t)((4u * chunk) >> 4);
                 const uint64_t db = db0 + (uint32_t)j * 2u, dbl = db + (kAtom >> 4);
-                umma_f16_ss(d, dal, db, idesc, (kb == 0 && j == 0) ? 0u : 1u);
+                umma_f16_ss(d, dal, db, idesc, (kb == 0 && j == 0) ? first : 1u);
                 umma_f16_ss(d, dah, dbl, idesc, 1u);
                 umma_f16_ss(d, dah, db, idesc, 1u);
               }
@@ -371,17 +400,18 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
         const int im = i / (n_icb * kPK), c = icb_lo * kPK + i - im * (n_icb * kPK);
         scale_s[i] = c < a.IC ? a.scale[(int64_t)(n0 + im) * a.scale_sn + (int64_t)c * a.scale_sc] : 0.0f;
       }
-    // This thread's pixels of the split patch (at most two; small patches: the two halves of the threads
+    // This thread's pixels of the split patch (at most kPixels; small patches: the two halves of the threads
     // take alternate chunks of the same pixels), each with its raw offset, or -1 where it is padding.
-    const bool few = a.px <= 128;
+    constexpr int kPixels = ROWS ? 1 : 2;
+    const bool few = ROWS && a.px <= 128;  // (with taps a patch has at least 8 x 17 pixels)
     const int c8_0 = few ? set : 0, c8_step = few ? 2 : 1;
     int roff[2], gate[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const int p = few ? (u ? a.px : (et & 127)) : et + 256 * u;
+      const int p = few ? (et & 127) : et + 256 * u;
       roff[u] = -2;  // no such pixel
       gate[u] = 0;
-      if (p >= a.px) continue;
+      if (u >= kPixels || p >= a.px) continue;
       if (a.mode == kRun) {
         roff[u] = p;  // (pixels beyond the plane arrive as zeros)
       } else if (a.mode == kImages) {
@@ -395,26 +425,31 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
         else roff[u] = (unsigned)(ow0 + pc - a.pw) < (unsigned)a.IW ? pr * a.raw_w + pc + a.xoff : -1;
       }
     }
+    int row = few ? (et & 127) : et;  // ROWS: this thread's pixel as a row of the product
+    if (ROWS && a.mode != kRun && a.mode != kImages) {
+      const int pr = (int)(((uint32_t)row * a.cw_magic) >> 16), pc = row - pr * a.cw;
+      row = (pc >> 3) * kBM + pr * 8 + (pc & 7);
+    }
     named_barrier_sync(1, 256);  // the gate, the column data
     // eight k values of one pixel (channels beyond IC arrive as zeros)
-    auto load8 = [&](const float *raw, int icb, int c8, int u, float *v) {
+    auto load8 = [&](const float *raw, int icb, int c8, int at, int gate_at, float *v) {
       const int c0 = icb * kPK + c8 * 8;  // first channel (kTaps: k value) within this CTA's split
       if (SOURCE == kTaps) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int k = koff_s[icb_lo * kPK + c0 + i];
-          v[i] = raw[max(roff[u] + k, 0)];
+          v[i] = raw[max(at + k, 0)];
           v[i] = k >= 0 ? v[i] : 0.0f;
         }
       } else {
-        const bool pixel = roff[u] >= 0;
-        const float *src = raw + max(roff[u], 0) + c8 * 8 * a.raw_ch;
+        const bool pixel = at >= 0;
+        const float *src = raw + max(at, 0) + c8 * 8 * a.raw_ch;
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = src[i * a.raw_ch];
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = pixel ? v[i] : 0.0f;
         if (SOURCE == kGated) {
-          const float4 *g = reinterpret_cast<const float4 *>(scale_s + gate[u] + c0);
+          const float4 *g = reinterpret_cast<const float4 *>(scale_s + gate_at + c0);
           const float4 g0 = g[0], g1 = g[1];
           const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
@@ -422,37 +457,67 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
         }
       }
     };
-    int k_tile = 0;  // the tile is scaled by 2^k_tile
+    const int strip = MT == 2 ? set : 0;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(strip * BN);
+    const int g_first = MT == 2 ? 0 : set * 32, g_step = MT == 2 ? 32 : 64;
+    int k_scale = 0;           // first attempt: exponent of the tile's (or this thread's row's) scale
+    int k_acc = 0;             // tile: exponent of the scale of the accumulator row of this thread
+    int k_top = 0;             // ... of the band of the largest magnitudes
+    unsigned row_bands = 0;    // bands that the window of this thread's row touches
+    int band[2] = {0, 0};      // bands of this thread's pixels
+    bool guess = false;
+    float seen[2] = {0.0f, 0.0f};  // largest magnitude of each of this thread's pixels (an infinity included, NaNs not)
+    unsigned passes = 1u;
     RingPos rr, rp;
-    for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-      bool guess = false;
-      float seen = 0.0f;
+    int attempt = 0;
+    for (; ok; ++attempt) {
+      int at[2] = {roff[0], roff[1]};
       if (attempt) {
-        k_tile = scale_exponent(__uint_as_float(*tile_max), 14);
+        if (!ROWS) {
+          const int now = 31 - __clz((int)passes);  // the smallest magnitudes first
+          passes &= ~(1u << now);
+          k_scale = k_top + kBandBits * now;
+#pragma unroll
+          for (int u = 0; u < kPixels; ++u)
+            if (band[u] != now) at[u] = min(at[u], -1);
+          if (attempt == 1) k_acc = k_scale;
+        }
       } else {
         // scale from the first channel block
-        float mx = 0.0f;
+        float mx[2] = {0.0f, 0.0f};
         if (n_icb > 0) {
           ok = mbar_wait_warp(bar_rfull, 0u, abort_flag);
           if (ok)
             for (int c8 = c8_0; c8 < 4; c8 += c8_step)
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                if (roff[u] == -2) continue;
+              for (int u = 0; u < kPixels; ++u) {
+                if (at[u] == -2) continue;
                 float v[8];
-                load8(raw_ptr, 0, c8, u, v);
+                load8(raw_ptr, 0, c8, at[u], gate[u], v);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(v[i]));
+                for (int i = 0; i < 8; ++i) mx[u] = fmaxf(mx[u], fabsf(v[i]));
               }
         }
-        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
-        if (lane == 0 && wm) atomicMax(first_max, wm);
-        named_barrier_sync(1, 256);  // reached by every warp, whether its wait was met or not
-        mx = __uint_as_float(*first_max);
-        guess = !(mx > 0.0f);
-        k_tile = guess ? kDefaultScaleExp : scale_exponent(mx, kTargetExp);
+        float m;
+        if (ROWS) {
+          m = mx[0];
+          if (few) {
+            if (m > 0.0f) atomicMax(row_max + row, __float_as_uint(m));
+            named_barrier_sync(1, 256);  // reached by every warp, whether its wait was met or not
+            m = __uint_as_float(row_max[row]);
+          }
+        } else {
+          m = fmaxf(mx[0] <= kMaxFinite ? mx[0] : 0.0f, mx[1] <= kMaxFinite ? mx[1] : 0.0f);
+          const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+          if (lane == 0 && wm) atomicMax(first_max, wm);
+          named_barrier_sync(1, 256);
+          m = __uint_as_float(*first_max);
+        }
+        guess = !(m > 0.0f);
+        k_scale = ROWS ? (guess ? kRowDefaultExp : scale_exponent(m, kRowTargetExp)) : guess ? kDefaultScaleExp : scale_exponent(m, kTargetExp);
+        k_acc = k_scale;
       }
-      const float s_mul = pow2(k_tile);
+      const float s_mul = pow2(k_scale);
       for (int icb = 0; icb < n_icb && ok; ++icb) {
         ok = mbar_wait_warp(bar_rfull + 8u * rr.s, rr.ph, abort_flag) && mbar_wait_warp(bar_pempty + 8u * rp.s, rp.ph ^ 1u, abort_flag);
         if (!ok) break;
@@ -460,14 +525,14 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
         uint8_t *dst = patch_ptr + (size_t)rp.s * patch_pitch;
         for (int c8 = c8_0; c8 < 4; c8 += c8_step)
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            if (roff[u] == -2) continue;
+          for (int u = 0; u < kPixels; ++u) {
+            if (at[u] == -2) continue;
             float v[8];
-            load8(raw, icb, c8, u, v);
+            load8(raw, icb, c8, at[u], gate[u], v);
             uint32_t hi[4], lo[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              seen = fmaxf(seen, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
+              seen[u] = fmaxf(seen[u], fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
               split_pair(v[2 * i], v[2 * i + 1], s_mul, hi[i], lo[i]);
             }
             const int p = few ? (et & 127) : et + 256 * u;
@@ -481,22 +546,100 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
         rr.step(RB);
         rp.step(a.patch_bufs);
       }
-      if (attempt) break;
-      // Was the scale right?  Known before the MMAs are done.
-      const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(seen));
-      if (lane == 0 && wm) atomicMax(tile_max, wm);
-      named_barrier_sync(1, 256);
-      const float all = __uint_as_float(*tile_max) * s_mul;
-      if (all > 65504.0f || (guess && all > 0.0f && all < 0.125f)) *redo_flag = 1;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_decide);
-      ok = ok && mbar_wait_warp(bar_decide, 0u, abort_flag);
-      if (!ok || !*redo_flag) break;
-      // The first attempt's phase is waited for before the second begins: once both are over, the parity of
-      // the first would look like a phase still to come.
-      ok = mbar_wait_warp(bar_accum, 0u, abort_flag);
+      if (attempt == 0) {
+        // Was the scale right?  Known before the MMAs are done.
+        if (ROWS) {
+          float m = seen[0];
+          if (few) {
+            if (m > 0.0f) atomicMax(row_max + row, __float_as_uint(m));
+            named_barrier_sync(1, 256);
+            m = __uint_as_float(row_max[row]);
+          }
+          // (a row that holds an infinity comes out as no number at any scale)
+          const bool bad = m <= kMaxFinite && (m * s_mul > 65504.0f || (guess && m > 0.0f && m * s_mul < 0.125f));
+          if (bad) k_scale = scale_exponent(m, 14);
+          row_inv[row] = pow2(-k_scale);  // (as many pixels as rows: every one has its thread)
+          if (__any_sync(0xffffffffu, bad) && lane == 0) *redo_flag = 1;
+        } else {
+          bool suspect = false;
+#pragma unroll
+          for (int u = 0; u < kPixels; ++u) {
+            if (!(seen[u] <= kMaxFinite)) seen[u] = 0.0f;
+            suspect = suspect || (seen[u] > 0.0f && !(seen[u] * s_mul >= 1.0f && seen[u] * s_mul <= 65504.0f));
+          }
+          if (__any_sync(0xffffffffu, suspect) && lane == 0) *suspect_flag = 1;
+          named_barrier_sync(1, 256);  // reached by every warp, whether its waits were met or not
+          if (*suspect_flag) {
+            // Pixel by pixel, in the raw patch's first buffer: nothing is in flight to it before the decision.
+            float *const pm = const_cast<float *>(raw_ptr);
+#pragma unroll
+            for (int u = 0; u < kPixels; ++u)
+              if (roff[u] != -2) pm[et + 256 * u] = seen[u];
+            const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(seen[0], seen[1])));
+            if (lane == 0 && wm) atomicMax(tile_max, wm);
+            named_barrier_sync(1, 256);
+            const float top = __uint_as_float(*tile_max);
+            k_top = scale_exponent(top, 14);
+            // the window of the row whose accumulator this thread reads
+            const float *win = pm + (m >> 3) * a.cw + strip * 8 + (m & 7);
+            float wmax = 0.0f;
+            for (int kh = 0; kh < a.KH; ++kh, win += a.cw)
+              for (int kw = 0; kw < a.KW; ++kw) {
+                const float x = win[kw];
+                if (x > 0.0f) row_bands |= 1u << ((scale_exponent(x, 14) - k_top) / kBandBits);
+                wmax = fmaxf(wmax, x);
+              }
+            unsigned bits = top * s_mul > 65504.0f || (wmax > 0.0f && wmax * s_mul < 1.0f) ? 1u << 31 : 0u;
+#pragma unroll
+            for (int u = 0; u < kPixels; ++u)
+              if (seen[u] > 0.0f) {
+                band[u] = (scale_exponent(seen[u], 14) - k_top) / kBandBits;
+                bits |= 1u << band[u];
+              }
+            bits = __reduce_or_sync(0xffffffffu, bits);
+            if (lane == 0) atomicOr(band_mask, bits);
+            named_barrier_sync(1, 256);
+            if (et == 0 && *band_mask >> 31) *redo_flag = (int)(*band_mask & 0x7fffffffu);
+            fence_async_smem();  // before the loads that may follow into that buffer
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_decide);
+        ok = ok && mbar_wait_warp(bar_decide, 0u, abort_flag);
+        if (!ok) break;
+        passes = (unsigned)*redo_flag;
+        if (!passes) break;
+        // The first attempt's phase is waited for before the second begins: once both are over, the parity of
+        // the first would look like a phase still to come.
+        ok = mbar_wait_warp(bar_accum, 0u, abort_flag);
+      } else {
+        if (ROWS || !passes || !ok) break;
+        // the next band's scale, for the rows that it touches
+        ok = mbar_wait_warp(bar_accum, (uint32_t)attempt & 1u, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const int next = k_top + kBandBits * (31 - __clz((int)passes));
+        float f0 = 1.0f, f1 = 1.0f;  // (the step may exceed a float's exponents)
+        if (row_bands >> (31 - __clz((int)passes)) & 1u) {
+          f0 = pow2(max(next - k_acc, -126));
+          f1 = pow2(min(next - k_acc + 126, 0));
+          k_acc = next;
+        }
+        for (int c0 = g_first; c0 < BN; c0 += g_step) {
+          float v[32];
+          uint32_t r[32];
+          tmem_ld32(lane_addr + (uint32_t)c0, v);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(v[i] * f0 * f1);
+          tmem_st32(lane_addr + (uint32_t)c0, r);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_decide);
+      }
     }
-    if (ok) ok = mbar_wait_warp(bar_accum, *redo_flag ? 1u : 0u, abort_flag);
+    if (ok) ok = mbar_wait_warp(bar_accum, (uint32_t)attempt & 1u, abort_flag);
     if (!ok) {
       atomicOr(a.status, kStatusTimeout);
       *abort_flag = 1;
@@ -504,10 +647,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
     tc_fence_after();
     // ---- epilogue: thread = pixel; two strips: one per set of four warps, one strip: the sets take
     // alternate groups of 32 channels
-    const float inv = pow2(-k_tile);
-    const int strip = MT == 2 ? set : 0;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(strip * BN);
-    const int g_first = MT == 2 ? 0 : set * 32, g_step = MT == 2 ? 32 : 64;
+    const float inv = ROWS ? row_inv[strip * kBM + m] : pow2(-k_acc);
     if (a.split_k > 1) {
       float *dst = staging + (size_t)(strip * kBM + m) * pitch;
       for (int c0 = g_first; c0 < BN; c0 += g_step) {
@@ -707,7 +847,7 @@ size_t finish_plan(ConvPairArgs &a, bool has_scale, size_t budget) {
   const size_t kb = (size_t)a.tile_n * kPairB;
   const int nkb = a.icb_per_split * a.taps;
   a.group = (int)std::max<size_t>(1, std::min<size_t>({(8 * 1024) / kb, (size_t)4, (size_t)nkb}));
-  const size_t fixed = (size_t)a.tile_n * 8 + 64 * 4 + (has_scale ? (size_t)a.imgs * a.icb_per_split * kPK * 4 : 0) + 32 + (2 * 8 + 2 * 4 + 6) * 8;
+  const size_t fixed = (size_t)a.tile_n * 8 + 64 * 4 + (a.taps == 1 ? kRowWords * 4 : 0) + (has_scale ? (size_t)a.imgs * a.icb_per_split * kPK * 4 : 0) + 32 + (2 * 8 + 2 * 4 + 6) * 8;
   const size_t staging = a.split_k > 1 ? (size_t)kBM * a.mt * (a.tile_n + 4) * 4 + 128 : 0;
   const int nstages = (nkb + a.group - 1) / a.group;
   // Rings, no deeper than the work there is.  Without taps every k block waits for its own raw patch, which
@@ -883,7 +1023,8 @@ static int launch_planned(ConvPairArgs a, size_t smem, const fml_tensor *x, cons
     if (st != FML_OK) return st;
   }
   using KernelFn = void (*)(const CUtensorMap, const ConvPairArgs);
-  static const KernelFn kernels[3] = {conv_pair_kernel<kPlain>, conv_pair_kernel<kGated>, conv_pair_kernel<kTaps>};
+  static const KernelFn kernels[5] = {conv_pair_kernel<kPlain, true>, conv_pair_kernel<kPlain, false>, conv_pair_kernel<kGated, true>,
+                                      conv_pair_kernel<kGated, false>, conv_pair_kernel<kTaps, true>};
   static bool attr_set[64] = {false};
   int dev = 0;
   FML_CUDA(cudaGetDevice(&dev));
@@ -908,7 +1049,7 @@ static int launch_planned(ConvPairArgs a, size_t smem, const fml_tensor *x, cons
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  FML_CUDA(cudaLaunchKernelEx(&cfg, kernels[a.mode == kIm2col ? kTaps : x_scale ? kGated : kPlain], map_x, a));
+  FML_CUDA(cudaLaunchKernelEx(&cfg, kernels[a.mode == kIm2col ? 4 : (x_scale ? 2 : 0) + (a.taps > 1)], map_x, a));
   return FML_OK;
 }
 
