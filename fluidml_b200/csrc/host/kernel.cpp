@@ -658,9 +658,9 @@ private:
 // Tile choices of a convolution with packed weights: tuned on the device while the builder records
 // (device buffers are live), or taken over from an earlier Compile.
 fml_conv_params TuneConv(const char *name, const fml_tensor &x, const fml_tensor *scale, const fml_tensor &w, const fml_tensor *bias,
-                         const fml_tensor &y, const fml_conv_params &p, bool autotune) {
+                         const fml_tensor *res, const fml_tensor &y, const fml_conv_params &p, bool autotune) {
   fml_conv_params tuned = p;
-  if (autotune && p.w_packed && fml_conv_autotune(&x, scale, &w, bias, &y, &p, nullptr, &tuned) != FML_OK)
+  if (autotune && p.w_packed && fml_conv_autotune_residual(&x, scale, &w, bias, res, &y, &p, nullptr, &tuned) != FML_OK)
     throw Error(std::string(name) + ": " + fml_last_error());
   return tuned;
 }
@@ -694,7 +694,7 @@ public:
     const fml_tensor x = in.at(0), w = w_, b = bias_;
     const fml_tensor scale = has_scale_ ? in.at(1) : fml_tensor{}, res = has_residual_ ? in.back() : fml_tensor{};
     const bool hb = has_bias_, hs = has_scale_, hr = has_residual_;
-    const fml_conv_params p = tuned_ = TuneConv(name_, x, hs ? &scale : nullptr, w, hb ? &b : nullptr, output, p_, autotune_);
+    const fml_conv_params p = tuned_ = TuneConv(name_, x, hs ? &scale : nullptr, w, hb ? &b : nullptr, hr ? &res : nullptr, output, p_, autotune_);
     rec.Add(name_, [=](void *s) {
       const fml_tensor *bias = hb ? &b : nullptr;
       if (hr) return fml_conv_residual(&x, hs ? &scale : nullptr, &w, bias, &res, &output, &p, s);

@@ -814,15 +814,23 @@ extern "C" int fml_conv_scaled(const fml_tensor *x, const fml_tensor *x_scale, c
   return conv_impl(x, x_scale, w, bias, y, p, stream);
 }
 
-extern "C" int fml_conv_residual(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
-                                 const fml_tensor *residual, const fml_tensor *y, const fml_conv_params *p, void *stream) {
-  FML_REQUIRE(valid_tensor(residual) && valid_tensor(y) && p && residual->dtype == FML_F32 && residual->rank == y->rank, FML_BAD_ARG,
+// A residual of y's shape; `same`: laid out as y.
+static int residual_laid_out_as(const fml_tensor *residual, const fml_tensor *y, bool *same) {
+  FML_REQUIRE(valid_tensor(residual) && valid_tensor(y) && residual->dtype == FML_F32 && residual->rank == y->rank, FML_BAD_ARG,
               "fml_conv_residual: bad argument");
-  bool same = true;  // laid out as y: the packed-weight kernel adds it in its epilogue
+  *same = true;
   for (int i = 0; i < y->rank; ++i) {
     FML_REQUIRE(residual->shape[i] == y->shape[i], FML_BAD_ARG, "fml_conv_residual: the residual's shape is y's");
-    same = same && (y->shape[i] == 1 || residual->stride[i] == y->stride[i]);
+    *same = *same && (y->shape[i] == 1 || residual->stride[i] == y->stride[i]);
   }
+  return FML_OK;
+}
+
+extern "C" int fml_conv_residual(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
+                                 const fml_tensor *residual, const fml_tensor *y, const fml_conv_params *p, void *stream) {
+  FML_REQUIRE(p, FML_BAD_ARG, "fml_conv_residual: bad argument");
+  bool same = false;  // then the packed-weight kernel adds it in its epilogue
+  if (const int rs = residual_laid_out_as(residual, y, &same); rs != FML_OK) return rs;
   int uses = 0;
   if (same && y->rank == 4 && p->w_packed) {
     const int st = fml_conv_uses_packed(x, w, y, p, x_scale != nullptr, &uses);
@@ -858,25 +866,47 @@ extern "C" int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, co
   return FML_OK;
 }
 
-extern "C" int fml_conv_autotune(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
-                                 const fml_tensor *y, const fml_conv_params *p, void *stream, fml_conv_params *tuned) {
+extern "C" int fml_conv_autotune_residual(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
+                                          const fml_tensor *residual, const fml_tensor *y, const fml_conv_params *p, void *stream,
+                                          fml_conv_params *tuned) {
   FML_REQUIRE(p && tuned, FML_BAD_ARG, "fml_conv_autotune: null argument");
   *tuned = *p;
   int uses = 0;
-  const int st = fml_conv_uses_packed(x, w, y, p, x_scale != nullptr, &uses);
+  bool same = false;
+  int st = fml_conv_uses_packed(x, w, y, p, x_scale != nullptr, &uses);
+  if (st == FML_OK && residual) st = residual_laid_out_as(residual, y, &same);
   if (st != FML_OK) return st;
   if (!p->w_packed || !uses || p->tile_n) return FML_OK;  // nothing to choose
   FML_CUDA(cudaStreamSynchronize(as_stream(stream)));
   if (Planes pl; !x_scale && as_planes(x, w, y, p, &pl)) {
     const fml_conv_params q = plane_params(p);
     fml_conv_params t = q;
-    const int ts = tune_conv_pair(&pl.x, &pl.w, bias, &pl.y, &q, nullptr, 0, 0, &t);
+    const int ts = tune_conv_pair(&pl.x, &pl.w, bias, &pl.y, &q, nullptr, 0, 0, nullptr, &t);
     tuned->tile_n = t.tile_n; tuned->strips = t.strips; tuned->split_k = t.split_k; tuned->ctas_per_sm = t.ctas_per_sm;
     return ts;
   }
   return tune_conv_pair(x, w, bias, y, p, x_scale ? (const float *)x_scale->data : nullptr,
                         x_scale && x_scale->shape[0] != 1 ? x_scale->stride[0] : 0, x_scale && x_scale->shape[1] != 1 ? x_scale->stride[1] : 0,
-                        tuned);
+                        same ? (const float *)residual->data : nullptr, tuned);
+}
+
+extern "C" int fml_conv_autotune(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
+                                 const fml_tensor *y, const fml_conv_params *p, void *stream, fml_conv_params *tuned) {
+  return fml_conv_autotune_residual(x, x_scale, w, bias, nullptr, y, p, stream, tuned);
+}
+
+extern "C" int fml_conv_tuning_key(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int scaled,
+                                   int residual, int device, char *key, size_t bytes) {
+  FML_REQUIRE(key && bytes, FML_BAD_ARG, "fml_conv_tuning_key: null argument");
+  int uses = 0;
+  const int st = fml_conv_uses_packed(x, w, y, p, scaled, &uses);
+  if (st != FML_OK) return st;
+  Planes pl;
+  const bool planes = !scaled && as_planes(x, w, y, p, &pl);
+  const fml_conv_params q = planes ? plane_params(p) : *p;
+  snprintf(key, bytes, "%s", !uses ? "" : planes ? conv_tuning_key(device, &pl.x, &pl.w, &pl.y, &q, false, false).c_str()
+                                                 : conv_tuning_key(device, x, w, y, &q, scaled != 0, residual != 0).c_str());
+  return FML_OK;
 }
 
 extern "C" size_t fml_conv_packed_bytes(const fml_tensor *w) {

@@ -992,7 +992,7 @@ int conv_pack(const fml_tensor *w, void *dst, cudaStream_t s) {
 
 static int launch_planned(ConvPairArgs a, size_t smem, const fml_tensor *x, const fml_tensor *bias, const fml_tensor *y,
                           const fml_conv_params *p, cudaStream_t s, const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc,
-                          const float *residual = nullptr) {
+                          const float *residual) {
   a.x = (const float *)x->data;
   a.packed = static_cast<const char *>(p->w_packed);
   a.col_scale = reinterpret_cast<const float *>(a.packed + (size_t)conv_k_blocks(a.IC, a.KH * a.KW) * a.n_pad * kPairB);
@@ -1061,14 +1061,24 @@ int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor 
   return launch_planned(a, smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc, residual);
 }
 
+// What a remembered choice of tiles belongs to: the device, the layer, the layout it writes and its epilogue.
+std::string conv_tuning_key(int device, const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled,
+                            bool residual) {
+  char key[320];
+  snprintf(key, sizeof(key), "%d|%lld,%lld,%lld,%lld|%lld,%lld,%lld|%lld,%lld|%lld,%lld,%lld,%lld|%d,%d,%d", device, (long long)x->shape[0],
+           (long long)x->shape[1], (long long)x->shape[2], (long long)x->shape[3], (long long)w->shape[0], (long long)w->shape[2],
+           (long long)w->shape[3], (long long)p->pads_begin[0], (long long)p->pads_begin[1], (long long)y->stride[0], (long long)y->stride[1],
+           (long long)y->stride[2], (long long)y->stride[3], p->act, scaled, residual);
+  return key;
+}
+
 // Times the candidates the model ranks highest as captured graphs of back-to-back launches and keeps the
-// fastest, per problem signature (as fml_gemm_autotune).
+// fastest, per device and problem signature (as fml_gemm_autotune).
 int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
-                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, fml_conv_params *tuned) {
-  char key[256];
-  snprintf(key, sizeof(key), "%lld,%lld,%lld,%lld|%lld,%lld,%lld|%lld,%lld|%d%d", (long long)x->shape[0], (long long)x->shape[1],
-           (long long)x->shape[2], (long long)x->shape[3], (long long)w->shape[0], (long long)w->shape[2], (long long)w->shape[3],
-           (long long)p->pads_begin[0], (long long)p->pads_begin[1], p->act, x_scale != nullptr);
+                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, fml_conv_params *tuned) {
+  int device = 0;
+  FML_CUDA(cudaGetDevice(&device));
+  const std::string key = conv_tuning_key(device, x, w, y, p, x_scale != nullptr, residual != nullptr);
   struct Choice { int tile_n, strips, split_k, occ; };
   static std::map<std::string, Choice> cache;
   static std::mutex mu;
@@ -1090,7 +1100,7 @@ int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
   float best = 1e30f;
   const Candidate *chosen = &all[0];
   for (size_t i = 0; i < all.size() && i < 16; ++i) {
-    auto launch = [&] { return launch_planned(all[i].a, all[i].smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc); };
+    auto launch = [&] { return launch_planned(all[i].a, all[i].smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc, residual); };
     float one = 0;
     bool ok = launch() == FML_OK;  // warm-up
     cudaEventRecord(e0, s);

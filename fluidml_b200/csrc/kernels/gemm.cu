@@ -264,7 +264,28 @@ extern "C" int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tens
   return launch_gemm_simt(p, e, as_stream(stream));
 }
 
-// One-off on-device tuning of (tile_n, split_k) for one GEMM, cached per problem signature.
+// What a remembered choice of tiles belongs to: the device, the problem and its epilogue.
+static std::string tuning_key(int device, const GemmProblem &p, const Choice &ch, const fml_gemm_params &gp, bool bias, bool residual) {
+  const bool pair = ch.path == Path::kPair;
+  char key[256];
+  snprintf(key, sizeof(key), "%d|%lld,%lld,%lld,%lld,%lld|%d%d%d|%d,%d,%d,%d|%lld,%lld", device, (long long)p.M, (long long)p.N, (long long)p.K,
+           (long long)p.nb0, (long long)p.nb1, pair, pair ? 0 : ch.tc.b_mn_major, pair ? 1 : ch.tc.three_pass, gp.act, bias, residual,
+           gp.divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn);
+  return key;
+}
+
+extern "C" int fml_gemm_tuning_key(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c, const fml_tensor *bias,
+                                   const fml_tensor *residual, const fml_gemm_params *gp, int device, char *key, size_t bytes) {
+  FML_REQUIRE(gp && key && bytes, FML_BAD_ARG, "fml_gemm_tuning_key: null argument");
+  GemmProblem p;
+  Choice ch;
+  const int st = resolve(a, b, c, bias, residual, gp, p, ch);
+  if (st != FML_OK) return st;
+  snprintf(key, bytes, "%s", ch.path == Path::kSimt ? "" : tuning_key(device, p, ch, *gp, bias != nullptr, residual != nullptr).c_str());
+  return FML_OK;
+}
+
+// One-off on-device tuning of (tile_n, split_k) for one GEMM, cached per device and problem signature.
 // The reference tunes its MatMul / Gemm kernels the same way -- by running the candidates
 // (there: six loop orders on the CPU, src/structure/kernel/generator/matmul.cpp:100-123) and
 // keeping the fastest per layout triple.
@@ -279,10 +300,9 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
   if (st != FML_OK) return st;
   if (ch.path == Path::kSimt || gp->tile_n != 0 || gp->split_k != 0) return FML_OK;  // nothing to choose
   const bool pair = ch.path == Path::kPair;
-  char key[256];
-  snprintf(key, sizeof(key), "%lld,%lld,%lld,%lld,%lld|%d%d%d|%d,%d,%d,%d|%lld,%lld", (long long)p.M, (long long)p.N,
-           (long long)p.K, (long long)p.nb0, (long long)p.nb1, pair, pair ? 0 : ch.tc.b_mn_major, pair ? 1 : ch.tc.three_pass,
-           gp->act, bias != nullptr, residual != nullptr, gp->divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn);
+  int device = 0;
+  FML_CUDA(cudaGetDevice(&device));
+  const std::string key = tuning_key(device, p, ch, *gp, bias != nullptr, residual != nullptr);
   struct Tiles { int tile_n, split_k, ctas_per_sm; };
   static std::map<std::string, Tiles> cache;
   static std::mutex mu;

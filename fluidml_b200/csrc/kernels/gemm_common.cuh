@@ -1,6 +1,7 @@
 // Shape analysis and epilogue shared by the two GEMM kernels (fp32 FMA and tcgen05).
 #pragma once
 #include "common.cuh"
+#include <string>
 
 namespace fml {
 
@@ -102,6 +103,8 @@ int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor 
                      cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0, int64_t x_scale_sc = 0,
                      const float *residual = nullptr);
 int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
-                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, fml_conv_params *tuned);
+                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, fml_conv_params *tuned);
+std::string conv_tuning_key(int device, const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled,
+                            bool residual);
 
 }  // namespace fml

@@ -349,7 +349,7 @@ int fml_gemm_plan(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
 
 /* On-device choice of tile_n and split_k for these operands: runs the candidate
  * configurations a few times each on `stream` (overwriting C with valid results), keeps the
- * fastest and remembers it per problem signature.  Synchronises; must not be stream-captured.
+ * fastest and remembers it per device and problem signature.  Synchronises; must not be stream-captured.
  * `tuned` receives a copy of `p` with tile_n / split_k filled in (unchanged when the fp32 FMA
  * kernel is used or the caller already fixed them).  The counterpart of the reference's
  * loop-order autotuning (src/structure/kernel/generator/matmul.cpp:88-131, gemm.cpp:107-151). */
@@ -396,9 +396,19 @@ typedef struct fml_conv_params {
 size_t fml_conv_packed_bytes(const fml_tensor *w);
 int fml_conv_pack(const fml_tensor *w, void *packed, size_t bytes, void *stream);
 /* On-device choice of the tile for a layer with packed weights (x_scale: NULL, or the gate of
- * fml_conv_scaled), as fml_gemm_autotune: y is overwritten, the call synchronises. */
+ * fml_conv_scaled), as fml_gemm_autotune: y is overwritten, the call synchronises.  The second form is for
+ * fml_conv_residual: the candidates are timed with the residual where they would add it themselves. */
 int fml_conv_autotune(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,
                       const fml_conv_params *p, void *stream, fml_conv_params *tuned);
+int fml_conv_autotune_residual(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
+                               const fml_tensor *residual, const fml_tensor *y, const fml_conv_params *p, void *stream,
+                               fml_conv_params *tuned);
+/* The signature under which fml_gemm_autotune / fml_conv_autotune remember a choice made on `device`; empty
+ * when there is nothing to choose.  Pure host computation. */
+int fml_gemm_tuning_key(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c, const fml_tensor *bias,
+                        const fml_tensor *residual, const fml_gemm_params *p, int device, char *key, size_t bytes);
+int fml_conv_tuning_key(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int scaled, int residual,
+                        int device, char *key, size_t bytes);
 /* Whether fml_conv (scaled: fml_conv_scaled) would use packed weights for these operands. */
 int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int scaled, int *uses);
 
