@@ -280,7 +280,7 @@ def gemm_params(precision=GEMM_AUTO, act=ACT_NONE, divisor=1.0, alpha=1.0, beta=
 class GemmPlanInfo(ctypes.Structure):
     _fields_ = [("uses_tensor_cores", ctypes.c_int32), ("tile_n", ctypes.c_int32), ("split_k", ctypes.c_int32),
                 ("stages", ctypes.c_int32), ("b_mn_major", ctypes.c_int32), ("three_pass", ctypes.c_int32),
-                ("shared_memory_bytes", ctypes.c_uint64), ("uses_packed", ctypes.c_int32)]
+                ("shared_memory_bytes", ctypes.c_uint64), ("uses_packed", ctypes.c_int32), ("stages_a", ctypes.c_int32)]
 
 
 def gemm_pack(b, stream=None) -> "DeviceBuffer":

@@ -220,7 +220,7 @@ extern "C" int fml_gemm_plan(const fml_tensor *a, const fml_tensor *b, const fml
   info->uses_tensor_cores = ch.path != Path::kSimt ? 1 : 0;
   if (ch.path == Path::kPair) {
     info->tile_n = ch.pair.tile_n; info->split_k = ch.pair.split_k; info->stages = ch.pair.stages_b;
-    info->three_pass = 1; info->uses_packed = 1;
+    info->three_pass = 1; info->uses_packed = 1; info->stages_a = ch.pair.stages_a;
     info->shared_memory_bytes = ch.pair.smem_bytes;
   } else if (ch.path == Path::kTc) {
     const TcPlan &plan = ch.tc;

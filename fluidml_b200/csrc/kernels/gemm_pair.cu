@@ -466,6 +466,11 @@ constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;
 constexpr size_t kSmemHalf = kSmemSm / 2 - 1024;  // what lets two CTAs share an SM
 
 // Ring depths for a tile width: the deepest that fits the budget and the 512 TMEM columns.
+// A's ring is even, or holds every block: the converter sets take alternate blocks, so with an odd ring a set
+// sees every other phase of a slot.  Loads land out of order, and while the other set's block is still on its
+// way the parity of the phase before it reads as this set's own: the set would convert what the slot held
+// before and give the slot back a second time.  (B's barriers need no such rule from two stages on: MMAs end in
+// order, and a set's previous wait covers the phase before.)
 bool pair_stages(int tile_n, int per, bool two_ctas, int *stages_a, int *stages_b, size_t *smem) {
   const int acc = (tile_n + 31) / 32 * 32;
   const size_t budget = two_ctas ? kSmemHalf : kSmemCta;
@@ -476,6 +481,7 @@ bool pair_stages(int tile_n, int per, bool two_ctas, int *stages_a, int *stages_
     for (int sa = 1; sa <= 8; ++sa) {
       if (pair_smem(tile_n, sa, sb) > budget) continue;
       if (sa > per || sb > per) continue;   // no deeper than the k loop
+      if ((sa & 1 && sa < per) || (sb == 1 && per > 1)) continue;
       // both rings count; the shallower one limits
       const double score = std::min(sa, sb) * 8 + sa + sb;
       if (score > best) { best = score; best_a = sa; best_b = sb; }

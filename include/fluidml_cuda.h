@@ -343,6 +343,7 @@ typedef struct fml_gemm_plan_info {
   int32_t uses_tensor_cores, tile_n, split_k, stages, b_mn_major, three_pass;
   uint64_t shared_memory_bytes;
   int32_t uses_packed; /* 1 = the packed-weight path (fml_gemm_params::b_packed) */
+  int32_t stages_a;    /* packed-weight path: depth of A's ring (`stages` is B's) */
 } fml_gemm_plan_info;
 int fml_gemm_plan(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
                   const fml_gemm_params *p, fml_gemm_plan_info *info);

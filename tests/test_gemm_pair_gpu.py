@@ -90,3 +90,14 @@ def test_long_rows_with_stretches_of_zeros_and_small_values(split_k):
     got = run(a, b, tile_n=64, split_k=split_k)
     scale = np.abs(a.astype(np.float64)) @ np.abs(b.astype(np.float64))
     assert (np.abs(got - a.astype(np.float64) @ b.astype(np.float64)) <= 4e-6 * scale + 1e-37).all()
+
+
+@pytest.mark.parametrize("tile_n,split_k,ctas", [(32, 1, 2), (32, 4, 2), (48, 1, 2), (64, 2, 2), (96, 1, 1), (128, 1, 1), (256, 1, 1)])
+def test_left_operand_larger_than_l2(tile_n, split_k, ctas):
+    """134 MB of A: loads miss L2 and land out of order, over every depth of A's ring that the planner takes."""
+    import torch
+    rng = np.random.default_rng(5)
+    a, b = rng.standard_normal((16384, 2048), np.float32), rng.standard_normal((2048, 256), np.float32) * 0.02
+    da, db = torch.from_numpy(a).cuda().double(), torch.from_numpy(b).cuda().double()
+    got = torch.from_numpy(run(a, b, tile_n=tile_n, split_k=split_k, ctas=ctas)).cuda()
+    assert ((got - da @ db).abs() <= 4e-6 * (da.abs() @ db.abs())).all()  # norm-wise per element, as above
