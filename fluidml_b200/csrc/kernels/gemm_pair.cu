@@ -163,6 +163,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   }
   pdl_wait();
 
+  // A's ring in two parts, one per converter set (pair_stages)
+  const int ring_0 = (a.stages_a + 1) >> 1, ring_1 = a.stages_a >> 1;
   TileEpilogue<ACT, kConvThreads, true> epi;
   float row_inv = 1.0f;  // converter threads: undoes the scale of this thread's row
   if (warp == 0) {
@@ -170,8 +172,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     if (!g_drop_loads) {
       const int ca2 = a.p.a_b0 ? z0 : 0, ca3 = a.p.a_b1 ? z1 : 0;
       bool ok = true;
-      int issued_a = 0, issued_b = pre_b;  // counted over both attempts: ring positions go on
-      RingPos ra, rb;
+      int issued_0 = 0, issued_1 = 0, issued_b = pre_b;  // counted over both attempts: ring positions go on
+      RingPos ra0, ra1, rb;
       for (int it = 0; it < pre_b; ++it) rb.step(a.stages_b);
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
         if (attempt) {
@@ -182,14 +184,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         uint32_t idle = 0;
         while (ia < nkb || ib < nkb) {  // whichever ring has room
           bool moved = false;
-          if (ia < nkb && mbar_test_warp(bar_empty_a + 8u * ra.s, ra.ph ^ 1u)) {
-            const uint32_t bar = bar_full_a + 8u * ra.s;
+          const bool odd = ia & 1;
+          const uint32_t sa = (uint32_t)(odd ? ring_0 + ra1.s : ra0.s);
+          if (ia < nkb && mbar_test_warp(bar_empty_a + 8u * sa, (odd ? ra1.ph : ra0.ph) ^ 1u)) {
+            const uint32_t bar = bar_full_a + 8u * sa;
             if (leader) {
               mbar_expect_tx(bar, kPairA);
-              tma_load_4d(ring_a + (uint32_t)ra.s * kPairA, &map_a, bar, (kb0 + ia) * kPK, tile_m * kBM, ca2, ca3);
+              tma_load_4d(ring_a + sa * kPairA, &map_a, bar, (kb0 + ia) * kPK, tile_m * kBM, ca2, ca3);
             }
-            ++ia; ++issued_a; moved = true;
-            ra.step(a.stages_a);
+            ++ia; moved = true;
+            if (odd) { ++issued_1; ra1.step(ring_1); } else { ++issued_0; ra0.step(ring_0); }
           }
           if (ib < nkb && mbar_test_warp(bar_empty_b + 8u * rb.s, rb.ph ^ 1u)) {
             if (leader) load_b(ib, rb.s);
@@ -205,8 +209,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         *abort_flag = 1;
         // bounded drain of the loads already in flight before the CTA may exit
         volatile int never = 0;
-        for (int i = max(0, issued_a - a.stages_a); i < issued_a; ++i)
-          mbar_wait_warp(bar_full_a + 8u * (i % a.stages_a), (uint32_t)(i / a.stages_a) & 1u, &never);
+        for (int i = max(0, issued_0 - ring_0); i < issued_0; ++i)
+          mbar_wait_warp(bar_full_a + 8u * (i % ring_0), (uint32_t)(i / ring_0) & 1u, &never);
+        for (int i = max(0, issued_1 - ring_1); i < issued_1; ++i)
+          mbar_wait_warp(bar_full_a + 8u * (ring_0 + i % ring_1), (uint32_t)(i / ring_1) & 1u, &never);
         for (int i = max(0, issued_b - a.stages_b); i < issued_b; ++i)
           mbar_wait_warp(bar_full_b + 8u * (i % a.stages_b), (uint32_t)(i / a.stages_b) & 1u, &never);
       }
@@ -274,10 +280,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       for (int i = 0; i < 16; ++i) sampled = fmaxf(sampled, fmaxf(fmaxf(fabsf(y[i].x), fabsf(y[i].y)), fmaxf(fabsf(y[i].z), fabsf(y[i].w))));
     }
     __syncwarp();
+    const int ring_n = set ? ring_1 : ring_0;
+    const uint32_t slot0 = set ? (uint32_t)ring_0 : 0u;
+    RingPos ma;  // within this set's part of A's ring
     for (int attempt = 0; attempt < 2 && ok; ++attempt) {
-      // positions of this set's block in the two rings (the second attempt's blocks follow the first's)
+      // position of this set's block in B's ring (the second attempt's blocks follow the first's)
       const int at = attempt * nkb + set;
-      RingPos ma{at % a.stages_a, (uint32_t)(at / a.stages_a) & 1u}, mb{at % a.stages_b, (uint32_t)(at / a.stages_b) & 1u};
+      RingPos mb{at % a.stages_b, (uint32_t)(at / a.stages_b) & 1u};
       float4 x[8];
       bool have = false;
       if (attempt) {
@@ -293,9 +302,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         if (set == 0) {
           float m = sampled;
           if (nkb > 0) {
-            ok = mbar_wait_warp(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
+            ok = mbar_wait_warp(bar_full_a + 8u * (slot0 + ma.s), ma.ph, abort_flag);
             if (ok) {
-              load_row(ma.s, x);
+              load_row(slot0 + ma.s, x);
               have = true;
 #pragma unroll
               for (int c = 0; c < 8; ++c)
@@ -318,9 +327,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       const bool watch = attempt == 0 && __any_sync(0xffffffffu, guess);
       for (int it = set; it < nkb && ok; it += 2) {
         if (!have) {
-          ok = mbar_wait_warp(bar_full_a + 8u * ma.s, ma.ph, abort_flag);
+          ok = mbar_wait_warp(bar_full_a + 8u * (slot0 + ma.s), ma.ph, abort_flag);
           if (!ok) break;
-          load_row(ma.s, x);
+          load_row(slot0 + ma.s, x);
         }
         if (watch) {
 #pragma unroll
@@ -334,8 +343,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
           split_pair(x[c].z, x[c].w, s_mul, hi[2 * c + 1], lo[2 * c + 1]);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_empty_a + 8u * ma.s);  // the values are in registers
-        ma.step(a.stages_a); ma.step(a.stages_a);
+        if (lane == 0) mbar_arrive(bar_empty_a + 8u * (slot0 + ma.s));  // the values are in registers
+        ma.step(ring_n);
         // the MMAs that read this tensor-memory stage last are done
         ok = mbar_wait_warp(bar_empty_b + 8u * mb.s, mb.ph ^ 1u, abort_flag);
         if (!ok) break;
@@ -344,8 +353,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         tmem_st16(t_hi, hi);
         tmem_st16(t_hi + 16u, lo);
         // the next block of this set, if it is there: its shared-memory latency runs under these stores
-        have = it + 2 < nkb && __all_sync(0xffffffffu, mbar_test(bar_full_a + 8u * ma.s, ma.ph));
-        if (have) load_row(ma.s, x);
+        have = it + 2 < nkb && __all_sync(0xffffffffu, mbar_test(bar_full_a + 8u * (slot0 + ma.s), ma.ph));
+        if (have) load_row(slot0 + ma.s, x);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -466,11 +475,11 @@ constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;
 constexpr size_t kSmemHalf = kSmemSm / 2 - 1024;  // what lets two CTAs share an SM
 
 // Ring depths for a tile width: the deepest that fits the budget and the 512 TMEM columns.
-// A's ring is even, or holds every block: the converter sets take alternate blocks, so with an odd ring a set
-// sees every other phase of a slot.  Loads land out of order, and while the other set's block is still on its
-// way the parity of the phase before it reads as this set's own: the set would convert what the slot held
-// before and give the slot back a second time.  (B's barriers need no such rule from two stages on: MMAs end in
-// order, and a set's previous wait covers the phase before.)
+// A's ring is split between the converter sets, which take alternate blocks, so that a set sees every phase of
+// its slots.  In one common ring of odd depth it would see every other one: loads land out of order, and while
+// the other set's block is still on its way the parity of the phase before it reads as this set's own -- stale
+// values would be converted and the slot given back a second time.  (B's barriers need no such care from two
+// stages on: MMAs end in order, and a set's previous wait covers the phase before.)
 bool pair_stages(int tile_n, int per, bool two_ctas, int *stages_a, int *stages_b, size_t *smem) {
   const int acc = (tile_n + 31) / 32 * 32;
   const size_t budget = two_ctas ? kSmemHalf : kSmemCta;
@@ -481,7 +490,7 @@ bool pair_stages(int tile_n, int per, bool two_ctas, int *stages_a, int *stages_
     for (int sa = 1; sa <= 8; ++sa) {
       if (pair_smem(tile_n, sa, sb) > budget) continue;
       if (sa > per || sb > per) continue;   // no deeper than the k loop
-      if ((sa & 1 && sa < per) || (sb == 1 && per > 1)) continue;
+      if (std::min(sa, sb) == 1 && per > 1) continue;
       // both rings count; the shallower one limits
       const double score = std::min(sa, sb) * 8 + sa + sb;
       if (score > best) { best = score; best_a = sa; best_b = sb; }
