@@ -60,8 +60,8 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   uint64_t *const bars = reinterpret_cast<uint64_t *>(max_s + 8);
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t bar_raw_full = bar0, bar_raw_empty = bar0 + 16, bar_s = bar0 + 32, bar_q_full = bar0 + 48, bar_q_ready = bar0 + 56,
-                 bar_k_ready = bar0 + 64, bar_k_free = bar0 + 72, bar_v_ready = bar0 + 80, bar_p_ready = bar0 + 88, bar_pv = bar0 + 104;
-  uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(bars + 14);
+                 bar_k_ready = bar0 + 64, bar_k_free = bar0 + 72, bar_v_ready = bar0 + 80, bar_p_ready = bar0 + 88, bar_pv = bar0 + 104, bar_final = bar0 + 112;
+  uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(bars + 15);
   volatile int *const abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -81,6 +81,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     mbar_init(bar_k_free, 1);
     mbar_init(bar_v_ready, 4);
     mbar_init(bar_pv, 1);
+    mbar_init(bar_final, 1);
     *abort_flag = 0;
     for (int i = 0; i < 6; ++i) max_s[i] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -171,6 +172,9 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         __syncwarp();
       }
     }
+    if (!ok) *abort_flag = 1;
+    if (leader) umma_drain(bar_final);
+    __syncwarp();
   } else if (warp < 6) {
     // ------------------------------------------------------------ softmax: thread = query row
     const int q = warp & 3, row = q * 32 + lane;
@@ -432,7 +436,7 @@ int launch_attention_pair(int64_t nb1, int64_t nb0, int64_t Sq, int64_t Sk, cons
   if (st == FML_OK) st = attention_map(&mk, k, Sk, k_s[3], nb0, k_s[1], nb1, k_s[0], kKeys);
   if (st == FML_OK) st = attention_map(&mv, v, Sk, v_s[2], nb0, v_s[1], nb1, v_s[0], kKeys);
   if (st != FML_OK) return st;
-  const size_t smem = 2 * kRawStage + 2 * kSplit + 2 * kKeys * 4 + 4 * 4 + 8 * 4 + 14 * 8 + 16;
+  const size_t smem = 2 * kRawStage + 2 * kSplit + 2 * kKeys * 4 + 4 * 4 + 8 * 4 + 15 * 8 + 16;
   using KernelFn = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const AttnPairArgs);
   static const KernelFn kernels[4] = {attention_pair_kernel<kNoMask>, attention_pair_kernel<kKeyMask>, attention_pair_kernel<kFullMask>,
                                       attention_pair_kernel<kCausal>};

@@ -61,8 +61,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   uint8_t *v_hi = k_lo + k_bytes, *v_lo = v_hi + v_bytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(v_lo + v_bytes);
   const uint32_t bar_q = smem_u32(bars), bar_kv = bar_q + 8, bar_conv = bar_q + 16, bar_s = bar_q + 24,
-                 bar_p = bar_q + 32, bar_o = bar_q + 40;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 6);
+                 bar_p = bar_q + 32, bar_o = bar_q + 40, bar_final = bar_q + 48;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 7);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   // a 128-row x 32-key piece of a mask that differs between query rows (pitch 33: the piece is
   // written with lanes along the keys and read with lanes along the rows)
@@ -85,6 +85,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     mbar_init(bar_s, 1);
     mbar_init(bar_p, 4);
     mbar_init(bar_o, 1);
+    mbar_init(bar_final, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -172,6 +173,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         atomicOr(a.status, kStatusTimeout);
         *abort_flag = 1;
       }
+      umma_drain(bar_final);
     }
   } else {
     // ------------------------------------------------------------ workers: one query row each
@@ -410,7 +412,7 @@ int launch_attention_tc(int64_t nb1, int64_t nb0, int64_t Sq, int64_t Sk, int64_
   if (st != FML_OK) return st;
   st = make_map4(&mv, v, Dv, Sk, v_s[2], nb0, v_s[1], nb1, v_s[0], 32, 32, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
   if (st != FML_OK) return st;
-  const size_t smem = (size_t)(D / 32) * 16384 * 4 + (size_t)(Dv / 32) * 4096 * 4 * 2 + 6 * 8 + 16 + 128 * 33 * 4 + 1024;
+  const size_t smem = (size_t)(D / 32) * 16384 * 4 + (size_t)(Dv / 32) * 4096 * 4 * 2 + 7 * 8 + 16 + 128 * 33 * 4 + 1024;
   static bool attr_set[64] = {false};
   int dev = 0;
   FML_CUDA(cudaGetDevice(&dev));

@@ -188,8 +188,8 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
   const uint32_t bar_bfull = smem_u32(bars), bar_bempty = bar_bfull + 8u * NB;
   const uint32_t bar_rfull = bar_bempty + 8u * NB, bar_rempty = bar_rfull + 8u * RB;
   const uint32_t bar_pfull = bar_rempty + 8u * RB, bar_pempty = bar_pfull + 16u;
-  const uint32_t bar_accum = bar_pempty + 16u, bar_decide = bar_accum + 8u;
-  uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NB + 2 * RB + 6);
+  const uint32_t bar_accum = bar_pempty + 16u, bar_decide = bar_accum + 8u, bar_final = bar_decide + 8u;
+  uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NB + 2 * RB + 8);
   volatile int *const abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   volatile int *const redo_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
   unsigned *const first_max = tmem_slot + 3;                             // bits of the first block's largest finite magnitude
@@ -234,6 +234,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
     for (int s = 0; s < 2; ++s) { mbar_init(bar_pfull + 8u * s, 8); mbar_init(bar_pempty + 8u * s, 1); }
     mbar_init(bar_accum, 1);
     mbar_init(bar_decide, 8);
+    mbar_init(bar_final, 1);
     *abort_flag = 0;
     *redo_flag = 0;
     *first_max = 0u;
@@ -252,7 +253,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
   pdl_launch_dependents();
   // The packed weights do not depend on the preceding kernel: the first stages are on their way while it drains.
   const int b_stages_total = (nkb + a.group - 1) / a.group, pre_b = min(NB, b_stages_total);
-  if (warp == 0 && leader && !g_drop_loads)
+  if (warp == 0 && leader && g_drop_loads != 1)
     for (int j = 0; j < pre_b; ++j) load_b(j * a.group, j);
   if (warp >= 2) {
     const int i = threadIdx.x - 64;
@@ -266,7 +267,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
 
   if (warp == 0) {
     // ------------------------------------------------------------ loads
-    if (!g_drop_loads) {
+    if (g_drop_loads != 1) {
       bool ok = true;
       int issued_r = 0, issued_b = pre_b;
       RingPos rr, rb;
@@ -276,7 +277,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
         if (attempt) {
           ok = mbar_wait_warp(bar_decide, (uint32_t)(attempt - 1) & 1u, abort_flag);
           if (attempt == 1) passes = (unsigned)*redo_flag;
-          if (!ok || !passes) break;
+          if (!ok || !passes || g_drop_loads) break;
           passes &= passes - 1u;
         }
         int ir = 0, jb = attempt ? 0 : pre_b;
@@ -389,6 +390,8 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
       if (leader) atomicOr(a.status, kStatusTimeout);
       *abort_flag = 1;
     }
+    if (leader) umma_drain(bar_final);
+    __syncwarp();
   } else {
     // ------------------------------------------------------------ patch split
     const int et = threadIdx.x - 64, set = et >> 7;
@@ -847,7 +850,7 @@ size_t finish_plan(ConvPairArgs &a, bool has_scale, size_t budget) {
   const size_t kb = (size_t)a.tile_n * kPairB;
   const int nkb = a.icb_per_split * a.taps;
   a.group = (int)std::max<size_t>(1, std::min<size_t>({(8 * 1024) / kb, (size_t)4, (size_t)nkb}));
-  const size_t fixed = (size_t)a.tile_n * 8 + 64 * 4 + (a.taps == 1 ? kRowWords * 4 : 0) + (has_scale ? (size_t)a.imgs * a.icb_per_split * kPK * 4 : 0) + 32 + (2 * 8 + 2 * 4 + 6) * 8;
+  const size_t fixed = (size_t)a.tile_n * 8 + 64 * 4 + (a.taps == 1 ? kRowWords * 4 : 0) + (has_scale ? (size_t)a.imgs * a.icb_per_split * kPK * 4 : 0) + 32 + (2 * 8 + 2 * 4 + 8) * 8;
   const size_t staging = a.split_k > 1 ? (size_t)kBM * a.mt * (a.tile_n + 4) * 4 + 128 : 0;
   const int nstages = (nkb + a.group - 1) / a.group;
   // Rings, no deeper than the work there is.  Without taps every k block waits for its own raw patch, which

@@ -145,8 +145,8 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const uint32_t bar_empty = bar_ready + 8u * NS;
   const uint32_t bar_rfull = bar_empty + 8u * NS;
   const uint32_t bar_rempty = bar_rfull + 8u * RS;
-  const uint32_t bar_accum = bar_rempty + 8u * RS;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * NS + 2 * RS + 1);
+  const uint32_t bar_accum = bar_rempty + 8u * RS, bar_final = bar_accum + 8u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * NS + 2 * RS + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   float *bias_s = reinterpret_cast<float *>(tmem_slot + 4);  // this tile's slice of the bias, [BN]
   float *scale_s = bias_s + 256;                             // this image's input scale, [n_icb * ICB] (when a.scale)
@@ -188,6 +188,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       mbar_init(bar_rempty + 8u * s, 8);  // both converter sets must have left the patch
     }
     mbar_init(bar_accum, 1);
+    mbar_init(bar_final, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -284,6 +285,7 @@ conv_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         atomicOr(a.status, kStatusTimeout);
         *abort_flag = 1;
       }
+      umma_drain(bar_final);
     }
   } else {
     // ------------------------------------------------------------ A gather + operand split, then epilogue
@@ -698,7 +700,7 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
   }
   const size_t ring = (size_t)stages * stage + a.raw_stages * raw_pitch;
   const size_t staging = a.split_k > 1 ? (((size_t)kBM * (a.tile_n + 4) * 4 + 127) & ~(size_t)127) : 0;
-  size_t smem = std::max(ring, staging) + (3 * stages + 2 * a.raw_stages + 1) * 8 + 16 + 256 * 4 /* bias slice */ +
+  size_t smem = std::max(ring, staging) + (3 * stages + 2 * a.raw_stages + 2) * 8 + 16 + 256 * 4 /* bias slice */ +
                 (a.scale ? (size_t)a.n_icb * icb * 4 : 0) /* input scale */ + 1024;
   {  // co-residency capped by TMEM columns, as in the GEMM
     unsigned need = (unsigned)((a.tile_n + 31) / 32 * 32 + a_cols * stages), cols = 32;

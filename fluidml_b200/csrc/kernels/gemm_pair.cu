@@ -76,8 +76,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   const uint32_t bar_full_a = smem_u32(bars), bar_empty_a = bar_full_a + 8u * a.stages_a;
   const uint32_t bar_full_b = bar_empty_a + 8u * a.stages_a, bar_conv = bar_full_b + 8u * a.stages_b;
   const uint32_t bar_empty_b = bar_conv + 8u * a.stages_b, bar_accum = bar_empty_b + 8u * a.stages_b;
-  const uint32_t bar_decide = bar_accum + 8u;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * a.stages_a + 3 * a.stages_b + 2);
+  const uint32_t bar_decide = bar_accum + 8u, bar_final = bar_decide + 8u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * a.stages_a + 3 * a.stages_b + 3);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   volatile int *redo_flag = reinterpret_cast<volatile int *>(tmem_slot + 2);
   unsigned *row_seen = reinterpret_cast<unsigned *>(tmem_slot + 4);          // [128], rows on the default scale: largest scaled magnitude
@@ -135,6 +135,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     }
     mbar_init(bar_accum, 1);
     mbar_init(bar_decide, 8);
+    mbar_init(bar_final, 1);
     *abort_flag = 0;
     *redo_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -150,7 +151,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   pdl_launch_dependents();
   // Weights do not depend on the preceding kernel: the first stages are on their way while it drains.
   const int pre_b = min(a.stages_b, nkb);
-  if (threadIdx.x == 0 && !g_drop_loads)
+  if (threadIdx.x == 0 && g_drop_loads != 1)
     for (int it = 0; it < pre_b; ++it) load_b(it, it);
   // vectors the epilogue will ask for, cold in HBM: into L2 now
   if (warp == 2) {
@@ -169,7 +170,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   float row_inv = 1.0f;  // converter threads: undoes the scale of this thread's row
   if (warp == 0) {
     // ------------------------------------------------------------ loads
-    if (!g_drop_loads) {
+    if (g_drop_loads != 1) {
       const int ca2 = a.p.a_b0 ? z0 : 0, ca3 = a.p.a_b1 ? z1 : 0;
       bool ok = true;
       int issued_0 = 0, issued_1 = 0, issued_b = pre_b;  // counted over both attempts: ring positions go on
@@ -178,7 +179,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       for (int attempt = 0; attempt < 2 && ok; ++attempt) {
         if (attempt) {
           ok = mbar_wait_warp(bar_decide, 0u, abort_flag);
-          if (!ok || !*redo_flag) break;
+          if (!ok || !*redo_flag || g_drop_loads) break;
         }
         int ia = 0, ib = attempt ? 0 : pre_b;
         uint32_t idle = 0;
@@ -255,6 +256,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
       if (leader) atomicOr(a.status, kStatusTimeout);
       *abort_flag = 1;
     }
+    if (leader) umma_drain(bar_final);
+    __syncwarp();
   } else {
     // ------------------------------------------------------------ converter
     const int q = warp & 3, row = q * 32 + lane, set = (warp - 2) >> 2, swz = row & 7;
@@ -468,7 +471,7 @@ size_t atoms_bytes(int64_t k, int64_t n) { return (size_t)k_blocks(k) * n_padded
 size_t pair_smem(int tile_n, int stages_a, int stages_b) {
   const size_t ring = (size_t)stages_a * kPairA + (size_t)stages_b * tile_n * kPairB;
   const size_t staging = ((size_t)kBM * (tile_n + 4) * 4 + 1023) / 1024 * 1024;
-  return std::max(ring, staging) + (2 * stages_a + 3 * stages_b + 2) * 8 + 16 + kBM * 5;
+  return std::max(ring, staging) + (2 * stages_a + 3 * stages_b + 3) * 8 + 16 + kBM * 5;
 }
 
 constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;

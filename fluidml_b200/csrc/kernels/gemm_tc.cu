@@ -105,8 +105,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const uint32_t bar_full = smem_u32(bars);
   const uint32_t bar_conv = bar_full + 8u * a.stages;
   const uint32_t bar_empty = bar_conv + 8u * a.stages;
-  const uint32_t bar_accum = bar_empty + 8u * a.stages;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * a.stages + 1);
+  const uint32_t bar_accum = bar_empty + 8u * a.stages, bar_final = bar_accum + 8u;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * a.stages + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -159,6 +159,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(bar_empty + 8u * s, 1);
     }
     mbar_init(bar_accum, 1);
+    mbar_init(bar_final, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -299,6 +300,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         atomicOr(a.status, kStatusTimeout);
         *abort_flag = 1;
       }
+      umma_drain(bar_final);
     }
   } else {
     // ------------------------------------------------------------ converter, then TMEM -> staging
@@ -438,7 +440,7 @@ size_t smem_for(int tile_n, int stages, int three_pass, int a_tmem) {
   const size_t stage = stage_bytes_for(tile_n, three_pass, a_tmem);
   const size_t staging = ((size_t)kBM * (tile_n + 4) * 4 + 1023) / 1024 * 1024;
   const size_t data = std::max(stage * stages, staging);
-  return data + (3 * stages + 1) * 8 + 16 + 1024;
+  return data + (3 * stages + 2) * 8 + 16 + 1024;
 }
 
 #ifdef FML_GEMM_PHASE_TRACE

@@ -12,7 +12,7 @@ constexpr uint32_t kSpinLimit = 1u << 22;
 // Test hook for the bounded waits (fml_debug_wait_test): a shorter iteration limit, and a switch
 // that makes the producers of the tensor-core kernels issue no loads, so that every wait of a
 // launch runs out, the kernel reports kStatusTimeout and returns -- nothing faults, nothing hangs,
-// no copy is in flight.  Each translation unit has its own copy; the setter sets them all.
+// no copy is in flight.  2: the packed-weight kernels drop the loads of repeated attempts only.  Each translation unit has its own copy; the setter sets them all.
 static __device__ uint32_t g_wait_limit = kSpinLimit;
 static __device__ int g_drop_loads = 0;
 void register_wait_test_setter(cudaError_t (*setter)(uint32_t, int));
@@ -262,6 +262,13 @@ __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                ::"r"(bar) : "memory");
+}
+// By the thread that issued the CTA's MMAs, last of all, whatever became of the pipeline: nothing may still be
+// executing when tensor memory and the rings are given back (after an abort the others do not wait for it).
+__device__ __forceinline__ void umma_drain(uint32_t bar) {
+  umma_commit(bar);
+  volatile int never = 0;
+  mbar_wait(bar, 0u, &never);
 }
 // 32 consecutive fp32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {

@@ -108,7 +108,8 @@ int fml_check_device(void *stream);
 /* Test hook for the failure path: sets the iteration limit of every bounded wait in the
  * tensor-core kernels (0 = default) and, with drop_loads != 0, makes their producers issue no
  * loads, so that a launch's waits run out, the kernel reports the timeout through the status
- * word and returns.  Nothing faults or hangs.  Restore with (0, 0). */
+ * word and returns (2: only the loads with which the packed-weight kernels repeat a tile).  Nothing faults or
+ * hangs.  Restore with (0, 0). */
 int fml_debug_wait_test(unsigned limit, int drop_loads);
 
 /* ---------------------------------------------------------------- elementwise

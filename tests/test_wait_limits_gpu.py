@@ -19,11 +19,11 @@ def rnd(*shape):
     return RNG.standard_normal(shape).astype(np.float32)
 
 
-def expect_timeout_then_recover(launch, verify):
+def expect_timeout_then_recover(launch, verify, drop=1):
     lib = cabi.lib()
     cabi.check_device()  # start from a clean status word
     try:
-        cabi.check(lib.fml_debug_wait_test(2000, 1))
+        cabi.check(lib.fml_debug_wait_test(2000, drop))
         launch()
         with pytest.raises(cabi.FmlError) as e:
             cabi.check_device()
@@ -81,3 +81,35 @@ def test_depthwise_waits_run_out_and_the_context_survives():
     ref = orc.conv(x, w, b, np.empty((2, 24, 28, 28), np.float32), (1, 1, 1, 1), (1, 1), (1, 1), 24)
     expect_timeout_then_recover(lambda: cabi.conv(dx, dw, db, dy, (1, 1), (1, 1), (1, 1), 24),
                                 lambda: np.testing.assert_allclose(dy.numpy(), ref, atol=1e-5 * np.abs(ref).max()))
+
+
+@pytest.mark.parametrize("drop", [1, 2])  # all loads; those of a repeated attempt, with the first one's MMAs behind it
+@pytest.mark.parametrize("split_k", [1, 8])
+def test_packed_gemm_waits_run_out_and_the_context_survives(split_k, drop):
+    a, b = rnd(300, 1024), rnd(1024, 768) * np.float32(0.05)
+    a[:, 40:] *= np.float32(1e6)  # every row outgrows the scale of its first block: in the first rank, at least
+    da, db, dc = DT.from_numpy(a), DT.from_numpy(b), DT((300, 768), np.float32)
+    packed = cabi.gemm_pack(db)
+    p = cabi.gemm_params(tile_n=64, split_k=split_k)
+    p.b_constant, p.b_packed = 1, packed.ptr
+    assert cabi.gemm_plan(da, db, dc, p).uses_packed
+    ref = a.astype(np.float64) @ b.astype(np.float64)
+    expect_timeout_then_recover(lambda: cabi.gemm(da, db, dc, params=p),
+                                lambda: np.testing.assert_allclose(dc.numpy(), ref, atol=1e-5 * np.abs(ref).max()), drop)
+
+
+@pytest.mark.parametrize("drop", [1, 2])
+@pytest.mark.parametrize("n,ic,oc,hw,k", [(2, 64, 64, 28, 3), (1, 512, 512, 14, 3), (2, 96, 24, 28, 1), (5, 192, 64, 7, 1), (1, 3, 32, 32, 3)])
+def test_packed_conv_waits_run_out_and_the_context_survives(n, ic, oc, hw, k, drop):
+    if drop == 2 and ic == 3:
+        pytest.skip("one k block: its scale is exact, nothing is repeated")
+    import torch
+    x, w = rnd(n, ic, hw, hw), rnd(oc, ic, k, k) * np.float32(0.05)
+    x[:, 1] *= np.float32(1e-7)
+    x[:, 8 if ic == 512 else 40:] *= np.float32(1e6)  # (512 channels: split over ranks of few blocks)
+    x[:, :, : hw // 2] *= np.float32(1e-9)            # two bands where there are taps
+    dx, dw, dy = DT.from_numpy(x), DT.from_numpy(w, [3, 2, 0, 1]), DT((n, oc, hw, hw), np.float32)
+    packed, pad = cabi.conv_pack(dw), [k // 2, k // 2]
+    ref = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(w).double(), padding=k // 2).numpy()
+    expect_timeout_then_recover(lambda: cabi.conv(dx, dw, None, dy, pad, [1, 1], [1, 1], packed=packed),
+                                lambda: np.testing.assert_allclose(dy.numpy(), ref, atol=1e-5 * np.abs(ref).max()), drop)
