@@ -20,7 +20,7 @@
 //            plane, side padding masked when the patch is split
 //   kRun     pointwise: 128 or 256 consecutive pixels of the plane
 //   kImages  pointwise over planes that are no multiple of 16 bytes (7 x 7): whole planes of several images
-//   kIm2col  few input channels (IC * KH * KW <= 64, any stride up to 4): K = (channel, tap) flattened, the
+//   kIm2col  few input channels (IC * KH * KW <= 64): K = (channel, tap) flattened, the
 //            split gathers the taps itself, so that a 3 x 3 layer over 3 channels is one k block, not nine
 //
 // Range of fp16.  A product's row must not lose bits to a large value that it does not contain: pixels of one
@@ -65,7 +65,7 @@ constexpr size_t kSmemSm = 228 * 1024, kSmemCta = 227 * 1024;
 
 struct ConvPairArgs {
   int mode, N, IC, OC, OH, OW, KH, KW, taps;
-  int strides[2], ph, pw;
+  int ph, pw;
   int n_icb, kb_total, icb_per_split, split_k;  // split over the cluster (1, 1, split_k)
   int mt, tile_n, stages_b, group;              // strips per CTA; k blocks per B stage
   int tiles_w, tiles_h, tiles_img;              // pixel tiles (kRun: tiles_h = 1; kImages: tiles_img groups of images)
@@ -288,12 +288,9 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
             const uint32_t bar = bar_rfull + 8u * rr.s, dst = raw0 + (uint32_t)rr.s * a.raw_pitch;
             const int c0 = (icb_lo + ir) * kPK;
             if (leader) {
-              if (a.mode == kBox) {
+              if (a.mode == kBox || a.mode == kIm2col) {  // (kIm2col: every k block cuts its k values from the same few channels)
                 mbar_expect_tx(bar, a.raw_bytes);
-                tma_load_4d(dst, &map_x, bar, ow0 - a.pw - a.xoff, oh0 - a.ph, c0, n0);
-              } else if (a.mode == kIm2col) {  // every k block cuts its k values from the same few channels
-                mbar_expect_tx(bar, a.raw_bytes);
-                tma_load_4d(dst, &map_x, bar, ow0 * a.strides[1] - a.pw - a.xoff, oh0 * a.strides[0] - a.ph, 0, n0);
+                tma_load_4d(dst, &map_x, bar, ow0 - a.pw - a.xoff, oh0 - a.ph, a.mode == kIm2col ? 0 : c0, n0);
               } else if (a.mode == kFlat) {
                 mbar_expect_tx(bar, a.raw_bytes);
                 tma_3d(dst, &map_x, bar, (oh0 - a.ph) * a.IW + ow0 - a.pw - a.xoff, c0, n0);
@@ -423,8 +420,7 @@ conv_pair_kernel(const __grid_constant__ CUtensorMap map_x, const ConvPairArgs a
         gate[u] = im < n_img ? im * n_icb * kPK : 0;
       } else {
         const int pr = (int)(((uint32_t)p * a.cw_magic) >> 16), pc = p - pr * a.cw;
-        if (a.mode == kIm2col) roff[u] = pr * a.strides[0] * a.raw_w + pc * a.strides[1] + a.xoff;
-        else if (a.mode == kBox) roff[u] = pr * a.raw_w + pc + a.xoff;
+        if (a.mode != kFlat) roff[u] = pr * a.raw_w + pc + a.xoff;
         else roff[u] = (unsigned)(ow0 + pc - a.pw) < (unsigned)a.IW ? pr * a.raw_w + pc + a.xoff : -1;
       }
     }
@@ -821,7 +817,7 @@ size_t finish_plan(ConvPairArgs &a, bool has_scale, size_t budget) {
   }
   a.cw_magic = (uint32_t)((65536 + a.cw - 1) / a.cw);
   a.imgs = 1;
-  const int rows = (a.TH - 1) * a.strides[0] + a.KH;
+  const int rows = a.TH - 1 + a.KH;
   a.xoff = 0;
   switch (a.mode) {
   case kRun: a.raw_w = a.TW; a.raw_ch = a.TW; break;
@@ -839,7 +835,7 @@ size_t finish_plan(ConvPairArgs &a, bool has_scale, size_t budget) {
   }
   default:
     a.xoff = (4 - a.pw % 4) % 4;
-    a.raw_w = ((a.TW - 1) * a.strides[1] + a.KW + a.xoff + 3) / 4 * 4;
+    a.raw_w = (a.TW - 1 + a.KW + a.xoff + 3) / 4 * 4;
     a.raw_ch = rows * a.raw_w;
     break;
   }
@@ -896,7 +892,6 @@ std::vector<Candidate> conv_pair_candidates(const fml_tensor *x, const fml_tenso
   a.OC = (int)w->shape[0]; a.KH = (int)w->shape[2]; a.KW = (int)w->shape[3];
   a.OH = (int)y->shape[2]; a.OW = (int)y->shape[3];
   a.ph = (int)p->pads_begin[0]; a.pw = (int)p->pads_begin[1];
-  a.strides[0] = a.strides[1] = 1;
   a.plane = a.IH * a.IW;
   a.n_pad = conv_n_pad(a.OC);
   const int taps = a.KH * a.KW;

@@ -66,9 +66,6 @@ struct RingPos {
   __device__ __forceinline__ void step(int n) {
     if (++s == n) { s = 0; ph ^= 1u; }
   }
-  __device__ __forceinline__ void back(int n) {
-    if (--s < 0) { s = n - 1; ph ^= 1u; }
-  }
 };
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t done;
