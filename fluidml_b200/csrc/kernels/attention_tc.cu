@@ -386,8 +386,14 @@ bool attention_tc_eligible(int64_t nb1, int64_t nb0, int64_t Sq, int64_t Sk, int
     return false;
   if (nb0 * nb1 > 65535 || nb0 * nb1 < 1) return false;
   if (mode == 1) return true;
-  // below ~200 Mflop, or with fewer tiles than two thirds of the SMs, the CUDA-core kernel's many
-  // small CTAs finish sooner than a few large tiles (8 x 6 heads x 128 rows: 25 us against 30)
+  // Head size 64: attention_pair_kernel is the faster one at every size measured (12 heads x 77: 7.3 us against
+  // 7.8 of the CUDA-core kernel; 48 x 128: 8.2 against 22.9; 12 x 256: 11.7 against 30.5; 96 x 128: 9.4 against
+  // 43.8), but its products are less precise: 7e-7 against fp64 where fp32 FMA has 1.9e-7 (12 heads x 128,
+  // 2-norm).  So it takes what came from tensor cores before it, fused or as 3xTF32 products around a softmax,
+  // and smaller blocks stay in fp32.
+  // Other head sizes (32): attention_tc_kernel needs 128-row tiles on two thirds of the SMs and 200 Mflop to
+  // come near the CUDA-core kernel's many small CTAs (96 heads x 128: 24.7 us against 22.2; 48 x 128: 24.3
+  // against 12.2) and wins with long rows (128 tiles of 1024 keys: 174 against 215).
   const double flops = 4.0 * (double)nb0 * (double)nb1 * (double)Sq * (double)Sk * (double)D;
   // (blocks beyond 256 Mflop that the pair kernel takes come here from the fusion pass whatever their tile count)
   if (D == 64 && Dv == 64 && flops > 256e6) return true;

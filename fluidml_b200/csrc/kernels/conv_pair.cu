@@ -907,8 +907,8 @@ std::vector<Candidate> conv_pair_candidates(const fml_tensor *x, const fml_tenso
   a.n_icb = a.mode == kIm2col ? conv_k_blocks(a.IC, taps) : (a.IC + kPK - 1) / kPK;
   a.kb_total = a.n_icb * a.taps;
   // Candidates scored in clocks of the busiest SM.  A CTA: set-up and pipeline fill, then per channel block
-  // the slowest of the MMAs (6 per k block and strip, 44 clocks or N / 2), the fill path (45 bytes per
-  // clock) and the split of the patch; then the stores (and the cluster's exchange with split-K).  Two CTAs
+  // the slowest of the MMAs (6 per k block and strip, charged 48 clocks or N / 2), the fill path (45 bytes
+  // per clock) and the split of the patch; then the stores (and the cluster's exchange with split-K).  Two CTAs
   // on an SM overlap each other's fixed parts but share the rest.
   for (int mt = 1; mt <= 2; ++mt) {
     if (mt == 2 && a.mode != kRun && a.mode != kImages && a.OW <= 8) continue;

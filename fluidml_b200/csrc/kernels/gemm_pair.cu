@@ -2,12 +2,13 @@
 // operand x is scaled by a power of two and split into hi = fp16(x), lo = fp16(x - hi), 22 significant
 // bits together, and lo*hi + hi*lo + hi*hi are accumulated in fp32 (kind::f16).  The same products as
 // the 3xTF32 kernel (gemm_tc.cu), whose truncated hi / lo carry 21 to 22 bits, but a kind::f16
-// instruction consumes 16 k values where kind::tf32 consumes 8 and both cost the same (47 clocks up to
-// N = 96, N / 2 beyond): half the tensor time.
+// instruction consumes 16 k values where kind::tf32 consumes 8 and both take N / 2 clocks: half the
+// tensor time.
 //
 // Range.  fp16 has 5 exponent bits, so both sides are scaled by powers of two (exact):
 //   B  per column, at packing time (fml_gemm_pack): the column's largest magnitude lands in
-//      [2^14, 2^15); elements 2^-28 below it still have all 22 bits.
+//      [2^14, 2^15); elements 2^-17 below it still have all 22 bits, and below that an absolute error of
+//      2^-39 of it.
 //   A  per row and k slice, on the fly: the first k block (32 values) of the row puts its largest
 //      magnitude into [2^3, 2^4).  Elements far below it keep an absolute error of 2^-28 of that
 //      magnitude, below fp32's own rounding of the sum; 2^12 of headroom is left for larger values
@@ -535,8 +536,10 @@ bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &p
   const int kb_total = k_blocks(p.K);
   const int64_t tiles_m = (p.M + kBM - 1) / kBM, batch = p.nb0 * p.nb1;
   // Default tile and split (the tuner measures the alternatives): time of a CTA = set-up and epilogue
-  // plus its k blocks at the slower of the MMAs (6 per block, 47 clocks each or N / 2) and one SM's
-  // fill path; waves of CTAs at one or two per SM.
+  // plus its k blocks at one SM's fill path (80 bytes per ns: slower than the block's 6 MMAs of N / 2 clocks
+  // at every width); waves of CTAs at one or two per SM.  Against the best of all tiles and splits, over 23
+  // products of 32 to 6144 rows in captured graphs: 1.27x in the geometric mean (77 x 1024 x 4096: 21.5 us
+  // for 11.4, a wide tile split eight ways; from 1024 rows on within 1.06x).
   const int tn_opts[] = {32, 64, 96, 128, 192, 256};
   const int sk_opts[] = {1, 2, 4, 8};
   double best = 1e30;
@@ -557,7 +560,7 @@ bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &p
         const int64_t ctas = tiles_m * ((p.N + tn - 1) / tn) * batch * sk;
         const int slots = (two ? 296 : 148) * (sk == 8 ? 0.87 : sk == 4 ? 0.97 : 1.0);
         const double waves = (double)((ctas + slots - 1) / slots);
-        const double t_kb = std::max(6 * std::max(47.0, tn / 2.0) / 1.9e3, (double)(kPairA + tn * kPairB) / 80e3);
+        const double t_kb = (double)(kPairA + tn * kPairB) / 80e3;
         const double t_fixed = 3.0 + (double)kBM * tn / sk * 4.0 / 20e3 + (sk > 1 ? 0.6 : 0.0);
         const double t = waves * (t_fixed + per * t_kb * (two && ctas > 148 ? 2.0 : 1.0));
         if (t < best) {
