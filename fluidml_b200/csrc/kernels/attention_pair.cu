@@ -16,8 +16,8 @@
 //   warps 6-9   split K and V: unswizzled core matrices [8 k values][row][16 bytes] in shared memory, K as
 //               (key, 8 of d), V transposed as (d, 8 keys), so that both are K-major B operands
 //
-// Scales (powers of two).  Q per row, K and V per block, all from exact maxima (largest in [2^14, 2^15)); Q's
-// and K's are divided out with the attention scale.  P is exp(s - m) times 2^x, x = (scale of O) - (scale of
+// Scales (powers of two).  Q per row, K and V per block, all from exact finite maxima (largest in [2^14, 2^15):
+// 22 bits down to 2^-17 of it, below that an absolute error of 2^-39 of it); Q's and K's are divided out with the attention scale.  P is exp(s - m) times 2^x, x = (scale of O) - (scale of
 // this block's V): O is one accumulator.  O is rescaled, by a round trip through registers, only when a
 // block's maximum exceeds the reference m of a row by more than 4 in log2 or V's scale moves by more than 3:
 // the largest P of a row is then within 2^-3 .. 2^7, and what its pair leaves out is below 2^-22 of it.
@@ -343,7 +343,9 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
           xv[i] = *reinterpret_cast<const float *>(rv + key * 128 + ((cv ^ (key & 7)) << 4));
           mv = fmaxf(mv, fabsf(xv[i]));
         }
-        const unsigned wk = __reduce_max_sync(0xffffffffu, __float_as_uint(mk)), wv = __reduce_max_sync(0xffffffffu, __float_as_uint(mv));
+        // (an infinity is in no maximum: it would flush the block's other keys and columns to zero)
+        const unsigned wk = __reduce_max_sync(0xffffffffu, mk <= FLT_MAX ? __float_as_uint(mk) : 0u);
+        const unsigned wv = __reduce_max_sync(0xffffffffu, mv <= FLT_MAX ? __float_as_uint(mv) : 0u);
         if (lane == 0) { atomicMax(max_s + 2 * slot, wk); atomicMax(max_s + 2 * slot + 1, wv); }
         if (MASK == kKeyMask && t < kKeys) {
           const int key = j * kKeys + t;

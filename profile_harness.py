@@ -2,8 +2,8 @@
 through the C ABI.  These are the small, self-contained commands to put under `ncu`; the
 summaries under profiles/ name them.
 
-    python profile_harness.py gemm --m 128 --k 3072 --n 768 --reps 3 [--precision 3xtf32]
-    python profile_harness.py conv --batch 8 --ic 256 --oc 256 --hw 56 [--k 3] [--precision 3xtf32]
+    python profile_harness.py gemm --m 128 --k 3072 --n 768 --reps 3 [--precision 3xtf32 | --packed [--tuned]]
+    python profile_harness.py conv --batch 8 --ic 256 --oc 256 --hw 56 [--k 3] [--precision 3xtf32 | --packed]
     python profile_harness.py attention --heads 12 --seq 128 --dim 64 [--batch 1]
     python profile_harness.py membound [--only layernorm]
     python profile_harness.py resident --layers 2 [--trace]
@@ -104,6 +104,7 @@ def main() -> None:
     c.add_argument("--reps", type=int, default=3)
     c.add_argument("--act", default="relu", choices=["none", "relu", "silu"])
     c.add_argument("--stride", type=int, default=1)
+    c.add_argument("--packed", action="store_true", help="constant weights, packed: the half-precision-pair kernel")
     c.add_argument("--depthwise", action="store_true", help="group = channels (oc is ignored)")
     a = sub.add_parser("attention")
     a.add_argument("--batch", type=int, default=1)
@@ -120,6 +121,9 @@ def main() -> None:
     g.add_argument("--precision", default="3xtf32", choices=["fp32", "3xtf32", "tf32"])
     g.add_argument("--tile-n", type=int, default=0)
     g.add_argument("--split-k", type=int, default=0)
+    g.add_argument("--ctas", type=int, default=0, help="with --packed: CTAs per SM of the tile")
+    g.add_argument("--packed", action="store_true", help="constant right-hand side, packed: the half-precision-pair kernel")
+    g.add_argument("--tuned", action="store_true", help="with --packed: the tiles fml_gemm_autotune finds")
     g.add_argument("--b-kmajor", action="store_true", help="B stored [n, k] (a Gemm with transB = 1: a classifier's weights)")
     r = sub.add_parser("resident")
     r.add_argument("--layers", type=int, default=2)
@@ -145,10 +149,15 @@ def main() -> None:
         else:
             b = DT.from_numpy(rng.standard_normal((*lead, args.k, args.n)).astype(np.float32))
         c = DT((*lead, args.m, args.n), np.float32)
-        p = cabi.gemm_params(precision=prec, tile_n=args.tile_n, split_k=args.split_k)
+        p = cabi.gemm_params(precision=cabi.GEMM_AUTO if args.packed else prec, tile_n=args.tile_n, split_k=args.split_k)
+        if args.packed:
+            blob = cabi.gemm_pack(b)
+            p.b_constant, p.b_packed, p.ctas_per_sm = 1, blob.ptr, args.ctas
+            if args.tuned:
+                p = cabi.gemm_autotune(a, b, c, p)
         info = cabi.gemm_plan(a, b, c, p)
         print(f"plan: tensor_cores={info.uses_tensor_cores} tile_n={info.tile_n} split_k={info.split_k} "
-              f"stages={info.stages} smem={info.shared_memory_bytes}")
+              f"stages={info.stages} smem={info.shared_memory_bytes} packed={info.uses_packed} stages_a={info.stages_a}")
         us = _time(lambda: cabi.gemm(a, b, c, params=p), args.reps)
         nbytes = (args.m * args.k + args.k * args.n + args.m * args.n) * 4 * args.batch
         print(f"{us:.2f} us per launch, {nbytes / us / 1e3:.1f} GB/s algorithmic, "
@@ -195,7 +204,11 @@ def main() -> None:
         b = DT.from_numpy(np.zeros(oc, np.float32))
         y = DT((args.batch, oc, ohw, ohw), np.float32)
         print("tensor cores:", (not args.depthwise) and cabi.conv_uses_tensor_cores(x, w, y, [pad, pad], prec))
-        us = _time(lambda: cabi.conv(x, w, b, y, [pad, pad], [st, st], [1, 1], group, act=act, precision=prec), args.reps)
+        packed = cabi.conv_pack(w) if args.packed else None
+        if packed is not None:
+            prec = cabi.GEMM_AUTO
+            print("packed:", cabi.conv_uses_packed(x, w, y, [pad, pad]))
+        us = _time(lambda: cabi.conv(x, w, b, y, [pad, pad], [st, st], [1, 1], group, act=act, precision=prec, packed=packed), args.reps)
         flop = 2.0 * args.batch * oc * (args.ic // group) * args.k * args.k * ohw * ohw
         nbytes = 4.0 * (args.batch * (args.ic * args.hw * args.hw + oc * ohw * ohw) + wh.size)
         print(f"{us:.2f} us per launch, {flop / us / 1e6:.1f} TFLOP/s, {nbytes / us / 1e3:.1f} GB/s algorithmic")

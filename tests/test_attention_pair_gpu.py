@@ -51,3 +51,23 @@ def test_attention_pair(b, h, sq, sk, kind, values):
         got = out.numpy()
         assert np.linalg.norm(got - ref) <= 8e-6 * np.linalg.norm(ref)
         assert np.abs(got - ref).max() <= 2e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_infinities_stay_in_their_keys_and_columns(value):
+    """A key with an infinity leaves the rows that do not see it alone, a value with one the other columns."""
+    rng = np.random.default_rng(5)
+    b, h, s = 2, 64, 256
+    q, k, v = (rng.standard_normal((b, h, s, 64)).astype(np.float32) for _ in range(3))
+    k[0, 1, 70, 3] = k[1, 7, 250, 60] = v[0, 5, 100, 9] = v[1, 60, 3, 40] = value
+    mask = np.where(np.tril(np.ones((s, s), np.bool_)), 0.0, LOWEST).astype(np.float32)[None, None]
+    kd = DT.from_numpy(k)
+    st = list(kd.strides)
+    out = DT((b, h, s, 64), np.float32)
+    cabi.attention(DT.from_numpy(q), kd.view((b, h, 64, s), [*st[:2], st[3], st[2]], 0), DT.from_numpy(v), DT.from_numpy(mask), 8.0, out, causal=True)
+    cabi.check_device()
+    got, fine = out.numpy(), np.ones((b, h, s, 64), bool)
+    fine[0, 1, 70:], fine[1, 7, 250:], fine[0, 5, :, 9], fine[1, 60, :, 40] = False, False, False, False
+    ref = oracle(q, np.where(np.isfinite(k), k, 0), np.where(np.isfinite(v), v, 0), mask, 8.0)
+    assert not np.isfinite(got[0, 1, 70:]).any() and not np.isfinite(got[0, 5, 100:, 9]).any() and not np.isfinite(got[1, 60, 3:, 40]).any()
+    assert np.abs(np.where(fine, got - ref, 0)).max() <= 2e-5 * np.abs(ref).max()
