@@ -161,8 +161,8 @@ def gemm_algorithmic_bytes():
 
 def captured_traffic_ratio():
     """DRAM bytes per algorithmic byte of the tensor-core GEMM, read from the committed ncu summary
-    (first capture column): (dram read + dram write) / (A + B + C bytes of that launch)."""
-    path = os.path.join(ROOT, "profiles", "gemm_tc_kernel_ffn2_m128_k3072_n768.md")
+    (first capture column): (dram read + dram write) / (A + packed B + C bytes of that launch)."""
+    path = os.path.join(ROOT, "profiles", "gemm_pair_kernel_ffn2_m128_k3072_n768.md")
     try:
         text = open(path).read()
         rd = re.search(r"`dram__bytes_read\.sum`\s*\|\s*([0-9.]+)\s*MB", text)
@@ -485,7 +485,7 @@ def run_ours(args):
         achieved = alg_bytes / (gemm_us * 1e-6) / 1e9 if gemm_us else None
         ratio, ratio_src = captured_traffic_ratio()
         line["roofline"] = {
-            "bound": "hbm", "kernel": "gemm_tc_kernel (FusedGemmKernel launches)",
+            "bound": "hbm", "kernel": "gemm_pair_kernel (FusedGemmKernel launches)",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak if achieved else None,
             "peak_source": peak_kind,
             "traffic": ratio * alg_bytes / alg_launches if ratio else None,
