@@ -98,7 +98,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   bool ok = true;
   if (warp == 0) {
     // ------------------------------------------------------------ loads: Q lands in raw stage 1, block j in stage j & 1
-    if (!g_drop_loads) {
+    if (g_drop_loads != 1) {
       if (leader) {
         mbar_expect_tx(bar_q_full, kRawStage);
         for (int i = 0; i < 2; ++i)

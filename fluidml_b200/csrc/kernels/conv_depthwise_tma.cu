@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_tma_kernel(const __
   const int pl = d.PP == 1 ? 0 : tid / per_plane, rem = tid - pl * per_plane;
   const int tr = rem / d.SW, j = rem - tr * d.SW;
   const bool worker = pl < d.PP && tr < d.TR;
-  const int drop = g_drop_loads;
+  const int drop = g_drop_loads == 1;
 
   auto issue = [&](int item, int stage) {  // thread 0 only
     const int tile = item / d.row_tiles, band = item - tile * d.row_tiles;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_planes_kernel(const
   const int pl = tid / per_plane, rem = tid - pl * per_plane;
   const int tr = rem / d.SW, j = rem - tr * d.SW;
   const bool worker = pl < d.PP;
-  const int drop = g_drop_loads;
+  const int drop = g_drop_loads == 1;
   const int per_plane_elems = d.PH * d.PWn, patch_elems = d.PP * per_plane_elems;
 
   auto issue = [&](int item, int stage) {  // thread 0 only: the planes [item * PP, ...) of the tensor

@@ -269,8 +269,8 @@ std::vector<cudaError_t (*)(uint32_t, int)> &wait_test_setters() {
 void register_wait_test_setter(cudaError_t (*setter)(uint32_t, int)) { wait_test_setters().push_back(setter); }
 }  // namespace fml
 // Test hook: iteration limit of every bounded mbarrier wait of the tensor-core kernels (0 restores
-// the default) and whether their producers skip their loads.  With (small limit, 1) a launch's
-// waits all run out: the kernel sets the status bit fml_check_device reports as
+// the default) and whether their producers skip their loads (2: those of repeated attempts only).  With
+// (small limit, 1) a launch's waits all run out: the kernel sets the status bit fml_check_device reports as
 // FML_DEVICE_TIMEOUT and returns; the context stays usable.  Synchronises the device.
 extern "C" int fml_debug_wait_test(unsigned limit, int drop_loads) {
   FML_CUDA(cudaDeviceSynchronize());

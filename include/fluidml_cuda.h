@@ -236,15 +236,18 @@ int fml_softmax(const fml_tensor *in, const fml_tensor *mask, float divisor,
  * (matmul.cpp:5-44, softmax.cpp:22-139).  q [.., S_q, D], kt [.., D, S_k] (the transposed
  * keys, as the MatMul receives them), v [.., S_k, D_v], out [.., S_q, D_v], ranks 2 to 4 with
  * equal leading dims; mask (may be NULL) broadcasts to [.., S_q, S_k].  Any strides: the
- * head-split transposes can stay views.  fp32 FMA throughout; the scores never leave the SM.
- * K and V of a head are staged once when they fit in shared memory; longer key sequences stream
+ * head-split transposes can stay views.  The scores never leave the SM.  Blocks that
+ * fml_attention_uses_tensor_cores names run there; the others in fp32 FMA, where K and V of a head
+ * are staged once when they fit in shared memory and longer key sequences stream
  * through it in chunks of 128 keys with a running-maximum softmax.  fml_attention_supported
  * tells whether a shape is taken (head sizes multiples of 4 up to 128); fml_attention returns
  * FML_UNSUPPORTED otherwise. */
 int fml_attention_supported(int64_t s_q, int64_t s_k, int64_t d, int64_t d_v);
-/* 1 when blocks of these head sizes run on the tensor cores (tcgen05, scores in tensor memory,
- * 3xTF32) once they are large enough (about 200 Mflop) and their operands are 16-byte aligned
- * views with unit innermost stride; smaller or unaligned blocks take the CUDA-core kernel. */
+/* 1 when blocks of these head sizes run on the tensor cores (tcgen05, scores in tensor memory;
+ * head size 64 as pairs of half-precision numbers, others in 3xTF32) once they are large enough
+ * (about 200 Mflop and 96 tiles of 128 rows, head size 64 from 256 Mflop on whatever the tiles) and
+ * their operands are 16-byte aligned views with unit innermost stride; smaller or unaligned blocks
+ * take the CUDA-core kernel. */
 int fml_attention_on_tensor_cores(int64_t s_q, int64_t s_k, int64_t d, int64_t d_v);
 /* The same question for concrete operands (shapes, strides, alignment, size). */
 int fml_attention_uses_tensor_cores(const fml_tensor *q, const fml_tensor *kt, const fml_tensor *v, int *uses);
@@ -291,7 +294,8 @@ typedef enum fml_gemm_act {
 } fml_gemm_act;
 
 typedef enum fml_gemm_precision {
-  FML_GEMM_AUTO = 0,   /* 3xTF32 tensor-core path when operands allow it, else fp32 FMA   */
+  FML_GEMM_AUTO = 0,   /* tensor cores when operands allow it -- pairs of half-precision numbers
+                        * with packed constant weights, else 3xTF32 --, else fp32 FMA       */
   FML_GEMM_FP32 = 1,   /* CUDA-core fp32 FMA, any strides                                 */
   FML_GEMM_3XTF32 = 2, /* tcgen05, hi/lo split: error ~2^-21 relative per product         */
   FML_GEMM_TF32 = 3    /* tcgen05, single pass: error ~2^-11 relative per product         */

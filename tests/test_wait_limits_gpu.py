@@ -113,3 +113,22 @@ def test_packed_conv_waits_run_out_and_the_context_survives(n, ic, oc, hw, k, dr
     ref = torch.nn.functional.conv2d(torch.from_numpy(x).double(), torch.from_numpy(w).double(), padding=k // 2).numpy()
     expect_timeout_then_recover(lambda: cabi.conv(dx, dw, None, dy, pad, [1, 1], [1, 1], packed=packed),
                                 lambda: np.testing.assert_allclose(dy.numpy(), ref, atol=1e-5 * np.abs(ref).max()), drop)
+
+
+def test_dropping_repeats_leaves_the_other_kernels_alone():
+    """The hook's value 2 is for the packed-weight kernels: attention, depthwise and unpacked products load as ever."""
+    q, x, a, b = rnd(8, 12, 128, 64), rnd(2, 24, 28, 28), rnd(128, 256), rnd(256, 96)
+    w = rnd(24, 1, 3, 3)
+    dq, da, db, out, c, y = DT.from_numpy(q), DT.from_numpy(a), DT.from_numpy(b), DT(q.shape, np.float32), DT((128, 96), np.float32), DT(x.shape, np.float32)
+    st = list(dq.strides)
+    kt = dq.view((8, 12, 64, 128), [st[0], st[1], st[3], st[2]], 0)
+    cabi.check_device()
+    try:
+        cabi.check(cabi.lib().fml_debug_wait_test(0, 2))
+        cabi.attention(dq, kt, dq, None, 8.0, out)
+        cabi.conv(DT.from_numpy(x), DT.from_numpy(w), None, y, (1, 1, 1, 1), (1, 1), (1, 1), 24)
+        cabi.gemm(da, db, c)
+        cabi.check_device()
+    finally:
+        cabi.check(cabi.lib().fml_debug_wait_test(0, 0))
+    np.testing.assert_allclose(c.numpy(), a.astype(np.float64) @ b, atol=1e-4)
