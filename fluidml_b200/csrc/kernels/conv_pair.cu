@@ -37,6 +37,9 @@
 //   in the last one), at the scale that puts them into [2^1, 2^15), and a row's accumulator is rescaled when
 //   the row's window has pixels in the band at hand.  One band is the usual case (a tile that outgrew its
 //   scale); a range beyond 2^14 within a tile costs one pass for every 2^14 in use.
+//   Time when every tile is repeated, in captured graphs: 8 x 256 x 56 x 56, 3 x 3 to 256 channels, 81 us
+//   usually, 146 repeated, 214 in two bands; 64 x 480 x 14 x 14, pointwise to 112, 15.9 and 24.6.  One scale for
+//   a whole tile in every mode was 1 % slower over VGG-16 and EfficientNet-B0 (batch 32: 3976 us, now 3922).
 //
 // Roles, 320 threads: warp 0 loads, warp 1 issues MMAs, warps 2-9 split the patches and do the epilogue.
 #include "gemm_common.cuh"

@@ -18,7 +18,8 @@
 //      2^7.  A row that outgrows its scale overflows to infinity, which the finished accumulator shows
 //      in every column, and one whose magnitudes stay below the default scale's reach is noticed by
 //      their maximum: the CTA then finds the exact row maxima and does its tile a second time with
-//      them.  Infinities and NaNs of the input come out as NaN, as in the 3xTF32 kernel.
+//      them (in captured graphs 128 x 768 x 3072: 10.7 us usually, 13.5 when one row is, 29.9 when all are).
+//      Infinities and NaNs of the input come out as NaN, as in the 3xTF32 kernel.
 // The powers of two are divided out again when the accumulator leaves tensor memory (rows) and in the
 // epilogue (columns).
 //
