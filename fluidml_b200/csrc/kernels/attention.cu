@@ -456,6 +456,284 @@ __global__ void __launch_bounds__(kThreads) attention_flash_kernel(AttnArgs a) {
   }
 }
 
+// Head sizes 32 and 64 whose rows are 16-byte-aligned runs (every model of the benchmark): the same
+// computation as attention_kernel, arranged so that a call of a few microseconds is not spent on its own
+// bookkeeping.  What bounds it is latency: one L2 round trip for Q and K, the shared-memory reads of the two
+// products (about 1,300 + 400 clocks per 16 x 128 x 64 block) and one drain; attention_kernel took 10.4 us for 12
+// heads of 128 x 128 of which 3.1 went into issuing the copies (a division per 16 bytes), 2.5 into the scores
+// (partial sums added through shared memory in turns), 1.8 into the softmax and 2.0 into the context.  Here
+//   - a thread's copies are a pointer and a step, worked out before the dependency wait;
+//   - products are fma.rn.f32x2: the scores' pairs run along the head dimension (their two sums are added at
+//     the end), the context's along the output columns;
+//   - the halves of the head dimension leave their scores side by side and the softmax, four keys per read,
+//     adds them; weights stay unnormalised and the finished row is divided once;
+//   - keys beyond 128 come in chunks under a running maximum, the next chunk's K on its way during the softmax and
+//     the context, its V during the next scores;
+//   - 87 KB of shared memory for head size 64 (the partial contexts lie over K) and at most 128 registers: two
+//     CTAs per SM overlap each other's phases where there are many (8 x 6 heads of 128: 384 CTAs).
+// Captured graphs of one call after another, attention_kernel / attention_flash_kernel -> this one, us: 12 heads of
+// 128 x 128 8.4 -> 7.3 (inside a BERT-base pass 10.4 -> 7.2), 36 of 77 9.8 -> 7.0, 48 of 128 22.6 -> 12.6, 16 of 77
+// causal 10.5 -> 5.9, 12 of 256 30.2 -> 14.2, 8 of 300 38.7 -> 17.7, 64 of 128 x 32 16.7 -> 10.4, 2 of 16 5.3 -> 3.6.
+// Left of a 7 us launch: 1.4 us to the first scores, 2.0 scores, 1.2 softmax, 1.1 context, 0.6 sum and store.
+constexpr int kRowsKeys = 128;              // keys per chunk
+constexpr int kRowsPP = kRowsKeys + 4;      // score pitch: 16-byte reads of four rows in different banks
+
+__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void cp_async16_or_zero(unsigned dst, const float *src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+
+template <int D> constexpr size_t attn_rows_smem() {
+  return (size_t)(kRows * (D + 4) + kRowsKeys * (D + 4) + kRowsKeys * D + 2 * kRows * kRowsPP + kRows) * sizeof(float);
+}
+
+// Scores of one chunk: rows rq, rq + 4, .. of Q against keys lane, lane + 32, .. over d4 in [d_lo, d_lo + N4).
+template <int NU, int N4>
+__device__ __forceinline__ void rows_scores(const float *q, const float *k, int pk, float *dst) {
+  unsigned long long acc[4][NU];
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int u = 0; u < NU; ++u) acc[x][u] = 0ull;
+#pragma unroll 2
+  for (int d = 0; d < N4; ++d) {
+    ulonglong2 qv[4], kv[NU];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) qv[x] = *reinterpret_cast<const ulonglong2 *>(q + 4 * x * pk + 4 * d);
+#pragma unroll
+    for (int u = 0; u < NU; ++u) kv[u] = *reinterpret_cast<const ulonglong2 *>(k + 32 * u * pk + 4 * d);
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int u = 0; u < NU; ++u) {
+        fma2(acc[x][u], qv[x].x, kv[u].x);
+        fma2(acc[x][u], qv[x].y, kv[u].y);
+      }
+  }
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+      const float2 t = unpack2(acc[x][u]);
+      dst[4 * x * kRowsPP + 32 * u] = t.x + t.y;
+    }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kThreads, 2) attention_rows_kernel(AttnArgs a, int causal) {
+  constexpr int pk = D + 4, NV = D / 32, kPerRow = D / 4, kStep = kThreads / kPerRow;
+  extern __shared__ __align__(16) float smem[];
+  float *const Qs = smem;                      // [kRows][pk]
+  float *const Ks = Qs + kRows * pk;           // [128][pk]; at the end the eight partial contexts [8][kRows][D]
+  float *const Vs = Ks + kRowsKeys * pk;       // [128][D]
+  float *const Ps = Vs + kRowsKeys * D;        // [2][kRows][kRowsPP]: scores of either half of d, then weights in the first
+  float *const row_scale = Ps + 2 * kRows * kRowsPP;
+  const ExactDivisor div(a.divisor);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int z0 = (int)(blockIdx.y % (unsigned)a.nb0), z1 = (int)(blockIdx.y / (unsigned)a.nb0);
+  const int row0 = blockIdx.x * kRows, rows = min(kRows, (int)a.Sq - row0);
+  const int Sk = causal ? min((int)a.Sk, row0 + kRows) : (int)a.Sk;  // no row of this block sees more
+  // copies: this thread's 16-byte column and first row
+  const int cr = threadIdx.x / kPerRow, cc = (threadIdx.x % kPerRow) * 4;
+  const float *const q = a.q + z1 * a.q_s[0] + z0 * a.q_s[1] + (int64_t)row0 * a.q_s[2] + cc;
+  const float *const k = a.k + z1 * a.k_s[0] + z0 * a.k_s[1] + cc;
+  const float *const v = a.v + z1 * a.v_s[0] + z0 * a.v_s[1] + cc;
+  const unsigned qd = (unsigned)__cvta_generic_to_shared(Qs + cr * pk + cc);
+  const unsigned kd = (unsigned)__cvta_generic_to_shared(Ks + cr * pk + cc);
+  const unsigned vd = (unsigned)__cvta_generic_to_shared(Vs + cr * D + cc);
+  // softmax: sixteen threads per row, four adjacent keys at a time
+  const int sr = threadIdx.x >> 4, sc4 = (threadIdx.x & 15) * 4;
+  const bool live = sr < rows;
+  const float *const mr = a.mask ? a.mask + z1 * a.m_s[0] + z0 * a.m_s[1] + (int64_t)(row0 + (live ? sr : 0)) * a.m_s[2] : nullptr;
+  const bool m_vec = a.m_s[3] == 1 && (reinterpret_cast<uintptr_t>(mr) & 15) == 0;
+  float *const o = a.out + z1 * a.o_s[0] + z0 * a.o_s[1] + (int64_t)(row0 + sr) * a.o_s[2];
+  const bool o_vec = a.o_s[3] == 1 && (reinterpret_cast<uintptr_t>(o) & 15) == 0;
+
+  auto load_k = [&](int j0) {  // rows up to the next multiple of 32; those that do not exist are zero
+    const int kc = min(kRowsKeys, Sk - j0), kz = (kc + 31) & ~31;
+    const float *src = k + (int64_t)j0 * a.k_s[3];
+#pragma unroll 4
+    for (int r = cr; r < kz; r += kStep) cp_async16_or_zero(kd + (unsigned)((r - cr) * pk * 4), src + (r < kc ? r : 0) * a.k_s[3], r < kc);
+    cp_async_commit();
+  };
+  auto load_v = [&](int j0) {
+    const int kc = min(kRowsKeys, Sk - j0), kz = (kc + 31) & ~31;
+    const float *src = v + (int64_t)j0 * a.v_s[2];
+#pragma unroll 4
+    for (int r = cr; r < kz; r += kStep) cp_async16_or_zero(vd + (unsigned)((r - cr) * D * 4), src + (r < kc ? r : 0) * a.v_s[2], r < kc);
+    cp_async_commit();
+  };
+  pdl_prologue();
+#pragma unroll
+  for (int r = cr; r < kRows; r += kStep) cp_async16_or_zero(qd + (unsigned)((r - cr) * pk * 4), q + (r < rows ? r : 0) * a.q_s[2], r < rows);
+  load_k(0);
+  load_v(0);
+
+  float m_run = -3.402823466e+38f, l_run = 0.0f;  // of row sr, the same in its sixteen threads
+  unsigned long long acc[4][NV][2];               // context: rows rg + 4x, columns cg * 4 + 32 v, over this warp's keys
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int n = 0; n < NV; ++n) acc[x][n][0] = acc[x][n][1] = 0ull;
+  const int rg = lane >> 3, cg = (lane & 7) * 4;
+
+  for (int j0 = 0; j0 < Sk; j0 += kRowsKeys) {
+    const int kc = min(kRowsKeys, Sk - j0), nu = (kc + 31) >> 5;
+    const bool more = j0 + kRowsKeys < Sk;
+    float4 mv[2];  // this thread's mask values, on their way during the scores
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int j = sc4 + 64 * i;
+      mv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!mr || j >= kc) continue;
+      const float *src = mr + (int64_t)(j0 + j) * a.m_s[3];
+      if (m_vec && j + 3 < kc) mv[i] = *reinterpret_cast<const float4 *>(src);
+      else {
+        mv[i].x = src[0];
+        if (j + 1 < kc) mv[i].y = src[a.m_s[3]];
+        if (j + 2 < kc) mv[i].z = src[2 * a.m_s[3]];
+        if (j + 3 < kc) mv[i].w = src[3 * a.m_s[3]];
+      }
+    }
+    cp_async_wait<1>();  // K (and Q); V may still be on its way
+    __syncthreads();
+    {
+      const int half = warp >> 2, rq = warp & 3;
+      const float *q_at = Qs + rq * pk + half * (D / 2), *k_at = Ks + lane * pk + half * (D / 2);
+      float *dst = Ps + (half * kRows + rq) * kRowsPP + lane;
+      if (nu == 4) rows_scores<4, D / 8>(q_at, k_at, pk, dst);
+      else if (nu == 3) rows_scores<3, D / 8>(q_at, k_at, pk, dst);
+      else if (nu == 2) rows_scores<2, D / 8>(q_at, k_at, pk, dst);
+      else rows_scores<1, D / 8>(q_at, k_at, pk, dst);
+    }
+    __syncthreads();
+    if (more) load_k(j0 + kRowsKeys);
+    {
+      float4 s[2];
+      float mx = m_run;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int j = sc4 + 64 * i;
+        if (j >= 32 * nu) continue;
+        const float *p = Ps + sr * kRowsPP + j;
+        const float4 p0 = *reinterpret_cast<const float4 *>(p), p1 = *reinterpret_cast<const float4 *>(p + kRows * kRowsPP);
+        s[i] = make_float4(p0.x + p1.x, p0.y + p1.y, p0.z + p1.z, p0.w + p1.w);
+        if (a.divisor != 1.0f) s[i] = make_float4(div(s[i].x), div(s[i].y), div(s[i].z), div(s[i].w));
+        s[i].x += mv[i].x; s[i].y += mv[i].y; s[i].z += mv[i].z; s[i].w += mv[i].w;
+        if (j < kc) mx = fmaxf(mx, s[i].x);
+        if (j + 1 < kc) mx = fmaxf(mx, s[i].y);
+        if (j + 2 < kc) mx = fmaxf(mx, s[i].z);
+        if (j + 3 < kc) mx = fmaxf(mx, s[i].w);
+      }
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+      float sum = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int j = sc4 + 64 * i;
+        if (j >= 32 * nu) continue;
+        float4 e = make_float4(0.f, 0.f, 0.f, 0.f);  // keys that do not exist weigh nothing
+        if (j < kc) e.x = expf(s[i].x - mx);
+        if (j + 1 < kc) e.y = expf(s[i].y - mx);
+        if (j + 2 < kc) e.z = expf(s[i].z - mx);
+        if (j + 3 < kc) e.w = expf(s[i].w - mx);
+        *reinterpret_cast<float4 *>(Ps + sr * kRowsPP + j) = e;
+        sum += (e.x + e.y) + (e.z + e.w);
+      }
+#pragma unroll
+      for (int d = 8; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+      const float scale = j0 ? expf(m_run - mx) : 0.0f;
+      m_run = mx;
+      l_run = l_run * scale + sum;
+      if (j0 && (threadIdx.x & 15) == 0) row_scale[sr] = scale;
+    }
+    if (more) cp_async_wait<1>();  // V; the next K may still be on its way
+    else cp_async_wait<0>();
+    __syncthreads();
+    {
+      if (j0) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const float t = row_scale[rg + 4 * x];
+          const unsigned long long t2 = pack2(t, t);
+#pragma unroll
+          for (int n = 0; n < NV; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[x][n][h]) : "l"(t2));
+        }
+      }
+      const float *p = Ps + rg * kRowsPP + warp * 4 * nu, *vr = Vs + warp * 4 * nu * D + cg;  // 4 nu keys per warp
+      for (int g = 0; g < nu; ++g, p += 4, vr += 4 * D) {
+        float4 pv[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) pv[x] = *reinterpret_cast<const float4 *>(p + 4 * x * kRowsPP);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          ulonglong2 vv[NV];
+#pragma unroll
+          for (int n = 0; n < NV; ++n) vv[n] = *reinterpret_cast<const ulonglong2 *>(vr + jj * D + 32 * n);
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            const float w = jj == 0 ? pv[x].x : jj == 1 ? pv[x].y : jj == 2 ? pv[x].z : pv[x].w;
+            const unsigned long long w2 = pack2(w, w);
+#pragma unroll
+            for (int n = 0; n < NV; ++n) { fma2(acc[x][n][0], w2, vv[n].x); fma2(acc[x][n][1], w2, vv[n].y); }
+          }
+        }
+      }
+    }
+    if (more) {
+      __syncthreads();  // V, weights and scales of this chunk are no longer read
+      load_v(j0 + kRowsKeys);
+    }
+  }
+  // the warps' partial contexts, added in warp order (K was read before the last barrier but one)
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+      *reinterpret_cast<ulonglong2 *>(Ks + (warp * kRows + rg + 4 * x) * D + cg + 32 * n) = make_ulonglong2(acc[x][n][0], acc[x][n][1]);
+  __syncthreads();
+  if (!live) return;
+#pragma unroll
+  for (int c = sc4; c < D; c += 64) {
+    float4 t = *reinterpret_cast<const float4 *>(Ks + sr * D + c);
+#pragma unroll
+    for (int w = 1; w < 8; ++w) {
+      const float4 u = *reinterpret_cast<const float4 *>(Ks + (w * kRows + sr) * D + c);
+      t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+    }
+    t = make_float4(t.x / l_run, t.y / l_run, t.z / l_run, t.w / l_run);
+    float *dst = o + c * a.o_s[3];
+    if (o_vec) *reinterpret_cast<float4 *>(dst) = t;
+    else { dst[0] = t.x; dst[a.o_s[3]] = t.y; dst[2 * a.o_s[3]] = t.z; dst[3 * a.o_s[3]] = t.w; }
+  }
+}
+
+// What attention_rows_kernel takes: head size 32 or 64 on both sides, rows of Q, K and V contiguous and on 16-byte
+// boundaries (its copies are 16 bytes wide), offsets within a tile in 32 bits.
+bool attn_rows_eligible(const AttnArgs &a) {
+  if (a.D != a.Dv || (a.D != 32 && a.D != 64)) return false;
+  if (a.q_s[3] != 1 || a.k_s[2] != 1 || a.v_s[3] != 1) return false;
+  if (!aligned16(a.q) || !aligned16(a.k) || !aligned16(a.v)) return false;
+  for (int i = 0; i < 2; ++i)
+    if (a.q_s[i] % 4 || a.k_s[i] % 4 || a.v_s[i] % 4) return false;
+  if (a.q_s[2] % 4 || a.k_s[3] % 4 || a.v_s[2] % 4) return false;
+  return a.Sq < (1ll << 30) && a.Sk < (1ll << 30);
+}
+
 size_t attn_flash_smem_bytes(int64_t D, int64_t Dv) {
   return (size_t)(kRows * (D + 4) + kChunk * (D + 4) + kChunk * Dv + 8 * kRows * Dv + kRows * (kChunk | 1) +
                   kRows * kChunk + 3 * kRows) * sizeof(float);
@@ -560,12 +838,17 @@ static int attention_impl(const fml_tensor *q, const fml_tensor *kt, const fml_t
   int dev = 0;
   FML_CUDA(cudaGetDevice(&dev));
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    FML_CUDA(cudaFuncSetAttribute(attention_rows_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_rows_smem<32>()));
+    FML_CUDA(cudaFuncSetAttribute(attention_rows_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_rows_smem<64>()));
     FML_CUDA(cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
     FML_CUDA(cudaFuncSetAttribute(attention_flash_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit));
     attr_set[dev] = true;
   }
   const dim3 grid((unsigned)((a.Sq + kRows - 1) / kRows), (unsigned)(a.nb0 * a.nb1));
-  if (whole) FML_LAUNCH((attention_kernel), grid, kThreads, smem, as_stream(stream), a);
+  if (attn_rows_eligible(a)) {
+    if (a.D == 64) FML_LAUNCH((attention_rows_kernel<64>), grid, kThreads, attn_rows_smem<64>(), as_stream(stream), a, causal ? 1 : 0);
+    else FML_LAUNCH((attention_rows_kernel<32>), grid, kThreads, attn_rows_smem<32>(), as_stream(stream), a, causal ? 1 : 0);
+  } else if (whole) FML_LAUNCH((attention_kernel), grid, kThreads, smem, as_stream(stream), a);
   else FML_LAUNCH((attention_flash_kernel), grid, kThreads, smem, as_stream(stream), a);
   return FML_OK;
 }
