@@ -47,7 +47,9 @@ class GemmParams(ctypes.Structure):
                 ("divisor", ctypes.c_float), ("alpha", ctypes.c_float), ("beta", ctypes.c_float),
                 ("act_param", ctypes.c_float * 3), ("split_k", ctypes.c_int32),
                 ("tile_n", ctypes.c_int32), ("b_constant", ctypes.c_int32), ("l2_prefetch", ctypes.c_void_p),
-                ("l2_prefetch_bytes", ctypes.c_uint64), ("b_packed", ctypes.c_void_p), ("ctas_per_sm", ctypes.c_int32)]
+                ("l2_prefetch_bytes", ctypes.c_uint64), ("b_packed", ctypes.c_void_p), ("ctas_per_sm", ctypes.c_int32),
+                ("act_from", ctypes.c_int32), ("rot", ctypes.c_int32), ("rot_head", ctypes.c_int32), ("rot_cols", ctypes.c_int32),
+                ("rot_len", ctypes.c_int32), ("rot_cos", ctypes.c_void_p), ("rot_sin", ctypes.c_void_p), ("a2", Tensor)]
 
 
 class ConvParams(ctypes.Structure):

@@ -146,7 +146,12 @@ size_t CostModel::GetTimeCost(const flow::Node &n, const std::vector<Layout> &in
     cost = alias ? 0.0 : kLaunchNs + 2.0 * obytes / (kHbmBytesPerNs * 0.5);
     break;
   }
-  case Kind::Dropout: case Kind::Identity: {
+  case Kind::Dropout: case Kind::Identity: case Kind::Rotary: {
+    if (n.inputs.size() > 1) {  // a rotation that is a launch
+      cost = kLaunchNs + write_cost;
+      for (size_t i = 0; i < n.inputs.size(); ++i) cost += read_cost(*n.inputs[i], is[i]);
+      break;
+    }
     cost = (is[0] == os && o.kind == flow::Region::kInner) ? 0.0 : kLaunchNs + 2.0 * obytes / (kHbmBytesPerNs * kTileEfficiency);
     break;
   }
@@ -174,13 +179,14 @@ size_t CostModel::GetTimeCost(const flow::Node &n, const std::vector<Layout> &in
     if (n.trans_a) std::swap(a_sm, a_sk);
     if (n.trans_b) std::swap(b_sk, b_sn);
     const int64_t M = o.meta.GetShape()[ro - 2], N = o.meta.GetShape()[ro - 1];
-    const int64_t K = n.trans_a ? a.meta.GetShape()[ra - 2] : a.meta.GetShape()[ra - 1];
+    const int64_t K = n.two_a ? b.meta.GetShape()[0] : n.trans_a ? a.meta.GetShape()[ra - 2] : a.meta.GetShape()[ra - 1];
     double batch = 1;
     for (size_t i = 0; i + 2 < ro; ++i) batch *= (double)o.meta.GetShape()[i];
     const double flops = 2.0 * batch * (double)M * (double)N * (double)K;
-    const double bytes = (double)a.meta.GetSize() + (double)b.meta.GetSize() + obytes;
+    const double bytes = (double)a.meta.GetSize() + (n.two_a ? (double)n.inputs[1]->meta.GetSize() : 0.0) + (double)b.meta.GetSize() + obytes;
+    const bool a2_ok = !n.two_a || (is[1][ra - 1] == 1 && is[1][ra - 2] % 4 == 0);
     const bool const_b = b.kind == flow::Region::kConstant;  // baked in whatever layout suits
-    const bool tc = precision_ != FML_GEMM_FP32 && a_sk == 1 && a_sm % 4 == 0 &&
+    const bool tc = precision_ != FML_GEMM_FP32 && a_sk == 1 && a_sm % 4 == 0 && a2_ok &&
                     (const_b || ((b_sk == 1 && b_sn % 4 == 0) || (b_sn == 1 && b_sk % 4 == 0))) &&
                     M >= 32 && N >= 16 && K >= 16;
     const double passes = precision_ == FML_GEMM_TF32 ? 1.0 : 3.0;

@@ -54,7 +54,7 @@ enum class Kind {
   FusedAttention,  // softmax(Q K^T / divisor + mask) V; inputs: Q, K^T, V, [mask]
   FusedMulAdd,     // a * b + c, broadcast; inputs: a, b, c
   FusedMulAddChain,   // a0*b0 + a1*b1 + ... in the rounding order of the Mul / Add chain it replaces; inputs: a0, b0, a1, b1, ...
-  Rotary,             // rotary position embedding over the first `value` features; inputs: x, cos, sin
+  Rotary,             // rotary position embedding over the first `value` features; inputs: x, cos, sin, or x alone when its product has rotated it
   SqueezeExciteGate,  // act2(W2 act1(W1 mean_hw(x) + b1) + b2); consts: W1, [b1], W2, [b2]; has_bias / has_bias2 = b1 / b2 present; act, act2
 };
 const char *KindName(Kind k);
@@ -87,6 +87,11 @@ struct Node {
   float act_param[3] = {1.4142135381698608f, 1.0f, 0.5f};
   bool has_bias = false, has_residual = false, has_mask = false;
   bool causal = false;      // FusedSoftmax, FusedAttention: the mask is lower-triangular, 0 / lowest
+  // FusedGemm, joined products: the activation from column act_from on (0: everywhere); the first rot features of
+  // every head of rot_head columns below rot_cols rotated by tables of rot_len rows (the last two consts); A's
+  // columns followed by those of inputs[1].
+  int64_t act_from = 0, rot = 0, rot_head = 0, rot_cols = 0, rot_len = 1;
+  bool two_a = false;
   bool b_is_const = false;  // FusedGemm: B is a captured constant (consts[0]) rather than inputs[1]
   // Scratch bytes the REFERENCE kernel of this kind needs (one float per row for Softmax and
   // LayerNorm, a padded copy for ConvWithPadding); used to report the reference-equivalent

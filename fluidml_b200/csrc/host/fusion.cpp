@@ -597,6 +597,200 @@ bool FuseRotary(Rewriter &rw, const NodePtr &cat) {
   return true;
 }
 
+// A constant of our own making.
+RegionPtr MakeConstant(flow::Flow &f, const std::string &name, std::vector<int64_t> shape, std::vector<uint8_t> bytes) {
+  auto r = std::make_shared<flow::Region>();
+  r->kind = flow::Region::kConstant;
+  r->name = name;
+  r->meta = Meta(Type::kFloat32, shape);
+  r->layout = utils::GenDefaultLayout(shape.size());
+  r->constant = std::make_shared<Tensor>(r->meta, std::move(bytes));
+  f.regions.push_back(r);
+  f.by_name[name] = r;
+  return r;
+}
+
+bool HoldsFloats(const RegionPtr &r, size_t rank, size_t count) {
+  return r->kind == flow::Region::kConstant && r->meta.GetType() == Type::kFloat32 && r->meta.GetRank() == rank && r->constant &&
+         r->constant->Bytes().size() == count * 4 && utils::IsDefaultLayout(r->layout);
+}
+
+// A product with a captured weight [K, N] and bias [N] (or none) in logical row-major order, nothing but an
+// activation on top of it: what the passes below may join.  `rows` of it at least 32: fewer stay separate, on the
+// weight-streaming kernel.
+bool IsPlainProduct(const NodePtr &n) {
+  if (n->kind != Kind::FusedGemm || !n->b_is_const || n->trans_a || n->trans_b || n->has_mask || n->two_a || n->divisor != 1.0f ||
+      n->alpha != 1.0f || n->beta != 1.0f)
+    return false;
+  const RegionPtr &w = n->consts[0];
+  if (w->meta.GetRank() != 2) return false;
+  const int64_t K = w->meta.GetShape()[0], N = w->meta.GetShape()[1];
+  return HoldsFloats(w, 2, (size_t)K * (size_t)N) && (!n->has_bias || (n->consts.size() >= 2 && HoldsFloats(n->consts[1], 1, (size_t)N)));
+}
+bool IsJoinable(const NodePtr &n) {
+  if (!IsPlainProduct(n)) return false;
+  const int64_t K = n->consts[0]->meta.GetShape()[0], N = n->consts[0]->meta.GetShape()[1];
+  return K % 4 == 0 && K >= 16 && N % 4 == 0 && N >= 16 && (int64_t)n->output->meta.GetElementsNum() / N >= 32;
+}
+
+// ---- product -> Reshape [b, s, heads, size] -> Transpose (0, 2, 1, 3) -> Rotary: the rotation in the product's epilogue.
+// The Rotary node stays, with one input and no launch.
+bool FuseRotaryIntoGemm(Rewriter &rw, const NodePtr &rot) {
+  if (rot->kind != Kind::Rotary || rot->inputs.size() != 3) return false;
+  auto made_by = [&](const RegionPtr &r, Kind k) -> NodePtr {
+    auto it = rw.producer.find(r.get());
+    return it != rw.producer.end() && it->second->kind == k && rw.Sole(r) ? it->second : nullptr;
+  };
+  const NodePtr tr = made_by(rot->inputs[0], Kind::Transpose);
+  if (!tr || tr->perm != std::vector<int64_t>{0, 2, 1, 3}) return false;
+  const NodePtr rs = made_by(tr->inputs[0], Kind::Reshape);
+  if (!rs) return false;
+  const NodePtr mm = made_by(rs->inputs[0], Kind::FusedGemm);
+  if (!mm || !IsJoinable(mm) || mm->act != 0 || mm->has_residual || mm->rot) return false;
+  const auto &flat = mm->output->meta.GetShape(), &split = rs->output->meta.GetShape();
+  if (flat.size() != 3 || split.size() != 4 || split[0] != flat[0] || split[1] != flat[1] || split[2] * split[3] != flat[2]) return false;
+  const int64_t width = (int64_t)rot->value, length = flat[1];
+  for (size_t i = 1; i < 3; ++i) {
+    const RegionPtr &t = rot->inputs[i];
+    const auto &ts = t->meta.GetShape();
+    if (ts.size() < 2 || ts[ts.size() - 1] != width || ts[ts.size() - 2] != length || !HoldsFloats(t, ts.size(), (size_t)(width * length))) return false;
+  }
+  RegionPtr tables[2];
+  for (size_t i = 0; i < 2; ++i) {  // rows of this node's own: the layout search may permute what other nodes read
+    const RegionPtr &t = rot->inputs[1 + i];
+    auto it = rw.f.by_name.find(t->name + "_rows");
+    tables[i] = it != rw.f.by_name.end() ? it->second : MakeConstant(rw.f, t->name + "_rows", {length, width}, t->constant->Bytes());
+  }
+  mm->consts.push_back(tables[0]);
+  mm->consts.push_back(tables[1]);
+  mm->rot = width;
+  mm->rot_head = split[3];
+  mm->rot_cols = flat[2];
+  mm->rot_len = length;
+  rot->inputs = {rot->inputs[0]};  // what the product has rotated: a view
+  return true;
+}
+
+// ---- LayerNorms of one tensor that feed products only (the two halves of a parallel-residual block): scale and
+// shift move into the products, (x^ g + b) W + c = x^ (g W) + (b W + c), worked out in 64 bits, and one LayerNorm
+// without them serves all.  Its readers are then siblings and merge.
+bool FoldSharedLayerNorms(Rewriter &rw) {
+  for (const NodePtr &first : rw.f.nodes) {
+    if (first->kind != Kind::LayerNormalizationConstantScaleBias || first->inputs.size() != 1) continue;
+    const RegionPtr x = first->inputs[0];
+    const auto &shape = x->meta.GetShape();
+    const int64_t last = (int64_t)shape.size() - 1;
+    std::vector<NodePtr> norms;
+    for (const NodePtr &n : rw.consumers[x.get()]) {
+      if (n->kind != Kind::LayerNormalizationConstantScaleBias || n->inputs.size() != 1 || n->axis != first->axis || n->epsilon != first->epsilon) continue;
+      if (n->axis != last && n->axis != -1) continue;
+      bool ok = n->output->kind == flow::Region::kInner && n->consts.size() == 2 && HoldsFloats(n->consts[0], 1, (size_t)shape[last]) &&
+                HoldsFloats(n->consts[1], 1, (size_t)shape[last]);
+      const auto &readers = rw.consumers[n->output.get()];
+      ok = ok && !readers.empty();
+      for (const NodePtr &r : readers) {
+        size_t uses = 0;
+        for (const RegionPtr &in : r->inputs) uses += in == n->output;
+        ok = ok && IsJoinable(r) && uses == 1 && r->inputs[0] == n->output && r->consts[0]->meta.GetShape()[0] == shape[last];
+      }
+      if (ok) norms.push_back(n);
+    }
+    if (norms.size() < 2) continue;
+    const int64_t K = shape[last];
+    std::vector<uint8_t> ones((size_t)K * 4), zeros((size_t)K * 4);
+    for (int64_t k = 0; k < K; ++k) reinterpret_cast<float *>(ones.data())[k] = 1.0f;
+    for (const NodePtr &n : norms) {
+      const float *g = reinterpret_cast<const float *>(n->consts[0]->constant->Bytes().data());
+      const float *b = reinterpret_cast<const float *>(n->consts[1]->constant->Bytes().data());
+      for (const NodePtr &r : rw.consumers[n->output.get()]) {
+        const int64_t N = r->consts[0]->meta.GetShape()[1];
+        const float *w = reinterpret_cast<const float *>(r->consts[0]->constant->Bytes().data());
+        const float *c = r->has_bias ? reinterpret_cast<const float *>(r->consts[1]->constant->Bytes().data()) : nullptr;
+        std::vector<uint8_t> wb((size_t)K * N * 4), cb((size_t)N * 4);
+        std::vector<double> shift((size_t)N);
+        for (int64_t j = 0; j < N; ++j) shift[j] = c ? (double)c[j] : 0.0;
+        float *wo = reinterpret_cast<float *>(wb.data()), *co = reinterpret_cast<float *>(cb.data());
+        for (int64_t k = 0; k < K; ++k)
+          for (int64_t j = 0; j < N; ++j) {
+            wo[k * N + j] = (float)((double)g[k] * (double)w[k * N + j]);
+            shift[j] += (double)b[k] * (double)w[k * N + j];
+          }
+        for (int64_t j = 0; j < N; ++j) co[j] = (float)shift[j];
+        r->consts[0] = MakeConstant(rw.f, r->name + "_normed.w", {K, N}, std::move(wb));
+        const RegionPtr nc = MakeConstant(rw.f, r->name + "_normed.b", {N}, std::move(cb));
+        if (r->has_bias) r->consts[1] = nc;
+        else r->consts.insert(r->consts.begin() + 1, nc);
+        r->has_bias = true;
+        r->inputs[0] = norms[0]->output;
+      }
+      if (n != norms[0]) rw.Kill(n);
+    }
+    norms[0]->consts = {MakeConstant(rw.f, norms[0]->name + "_plain.g", {K}, std::move(ones)),
+                        MakeConstant(rw.f, norms[0]->name + "_plain.b", {K}, std::move(zeros))};
+    rw.Commit();
+    return true;
+  }
+  return false;
+}
+
+// [W1; W2] and the sum of the biases: what a product over two left-hand sides reads.
+void JoinWeights(flow::Flow &f, const NodePtr &into, const NodePtr &top, const NodePtr &bottom) {
+  const int64_t N = top->consts[0]->meta.GetShape()[1], K = top->consts[0]->meta.GetShape()[0] + bottom->consts[0]->meta.GetShape()[0];
+  std::vector<uint8_t> w = top->consts[0]->constant->Bytes();
+  const std::vector<uint8_t> &w2 = bottom->consts[0]->constant->Bytes();
+  w.insert(w.end(), w2.begin(), w2.end());
+  std::vector<uint8_t> bias;
+  for (const NodePtr &n : {top, bottom}) {
+    if (!n->has_bias) continue;
+    const std::vector<uint8_t> &b = n->consts[1]->constant->Bytes();
+    if (bias.empty()) { bias = b; continue; }
+    for (int64_t j = 0; j < N; ++j) reinterpret_cast<float *>(bias.data())[j] += reinterpret_cast<const float *>(b.data())[j];
+  }
+  const std::string base = into->name + "_joined";
+  into->consts = {MakeConstant(f, base + ".w", {K, N}, std::move(w))};
+  into->has_bias = !bias.empty();
+  if (into->has_bias) into->consts.push_back(MakeConstant(f, base + ".b", {N}, std::move(bias)));
+}
+
+// ---- A1 W1 + (A2 W2 + x) -> [A1 | A2] [W1; W2] + x: one launch, one reduction and one pass over the result for both
+// halves of a parallel-residual block.
+bool JoinSummedProducts(Rewriter &rw, const NodePtr &mm) {
+  if (!IsJoinable(mm) || mm->act != 0 || mm->rot || !mm->has_residual || mm->inputs.size() != 2) return false;
+  const RegionPtr r = mm->inputs[1];
+  auto it = rw.producer.find(r.get());
+  if (it == rw.producer.end() || rw.Sole(r) != mm) return false;
+  const NodePtr g = it->second;
+  if (!IsJoinable(g) || g->act != 0 || g->rot || g->inputs.size() != (g->has_residual ? 2u : 1u) || g->output->meta != mm->output->meta) return false;
+  if (g->inputs[0]->meta.GetRank() != mm->inputs[0]->meta.GetRank() || g->act_from || mm->act_from) return false;
+  const bool swap = mm->consts[0]->meta.GetShape()[0] % 32 != 0;  // k blocks must not straddle the seam
+  const NodePtr &top = swap ? g : mm, &bottom = swap ? mm : g;
+  if (top->consts[0]->meta.GetShape()[0] % 32 != 0) return false;
+  std::vector<RegionPtr> inputs = {top->inputs[0], bottom->inputs[0]};
+  if (g->has_residual) inputs.push_back(g->inputs[1]);
+  JoinWeights(rw.f, mm, top, bottom);
+  mm->inputs = inputs;
+  mm->has_residual = g->has_residual;
+  mm->two_a = true;
+  rw.Kill(g);
+  return true;
+}
+
+// ---- Concat(A1, A2) along the features -> product: the product reads both where they are.
+bool JoinConcatenatedProduct(Rewriter &rw, const NodePtr &cat) {
+  if (cat->kind != Kind::Concat2 || cat->inputs.size() != 2 || IsConst(cat->inputs[0]) || IsConst(cat->inputs[1])) return false;
+  const int64_t rank = (int64_t)cat->output->meta.GetRank();
+  if (rank < 2 || (cat->axis != rank - 1 && cat->axis != -1)) return false;
+  const NodePtr mm = rw.SoleOfKind(cat->output, Kind::FusedGemm);
+  if (!mm || !IsJoinable(mm) || mm->act != 0 || mm->rot || mm->act_from || mm->inputs[0] != cat->output) return false;
+  const int64_t k1 = cat->inputs[0]->meta.GetShape()[rank - 1], k2 = cat->inputs[1]->meta.GetShape()[rank - 1];
+  if (k1 % 32 != 0 || k2 % 4 != 0) return false;
+  mm->inputs[0] = cat->inputs[0];
+  mm->inputs.insert(mm->inputs.begin() + 1, cat->inputs[1]);
+  mm->two_a = true;
+  rw.Kill(cat);
+  return true;
+}
+
 // ---- Conv -> SiLU: the activation rides in the convolution's epilogue
 bool FuseSiluIntoConv(Rewriter &rw, const NodePtr &cv) {
   if ((cv->kind != Kind::ConvWithPadding && cv->kind != Kind::ConvWithoutPadding) || cv->act != 0) return false;
@@ -610,25 +804,22 @@ bool FuseSiluIntoConv(Rewriter &rw, const NodePtr &cv) {
 
 // ---- GEMMs that read the same activations with constant weights (the Q, K, V projections):
 // one GEMM over the concatenated weights, the original outputs become column slices of its
-// result (views, no copy).  Fewer launches and one pass over the shared A operand.
-bool MergeSiblingGemms(flow::Flow &f) {
-  auto eligible = [](const NodePtr &n) {
-    if (n->kind != Kind::FusedGemm || !n->b_is_const || n->trans_a || n->trans_b || n->act != 0 ||
-        n->has_residual || n->has_mask || n->divisor != 1.0f || n->alpha != 1.0f || n->beta != 1.0f)
-      return false;
-    if (n->inputs.size() != 1 || n->output->kind != flow::Region::kInner) return false;
-    const RegionPtr &w = n->consts[0];
-    if (w->meta.GetRank() != 2 || w->meta.GetType() != Type::kFloat32 || !utils::IsDefaultLayout(w->layout)) return false;
-    // the merge copies K * N weights and N bias values per sibling: both constants must hold exactly that
-    const int64_t K = w->meta.GetShape()[0], N = w->meta.GetShape()[1];
-    if (!w->constant || w->constant->Bytes().size() != (size_t)K * (size_t)N * 4) return false;
-    if (n->has_bias) {
-      if (n->consts.size() < 2 || n->consts[1]->meta.GetRank() != 1 || n->consts[1]->meta.GetShape()[0] != N) return false;
-      if (n->consts[1]->meta.GetType() != Type::kFloat32 || !n->consts[1]->constant ||
-          n->consts[1]->constant->Bytes().size() != (size_t)N * 4)
-        return false;
-    }
-    return true;
+// result (views, no copy).  Fewer launches and one pass over the shared A operand.  With `join` (the packed-weight
+// kernel will run them) rotated projections and those with a GELU come along, the former in front, the latter last.
+bool MergeSiblingGemms(flow::Flow &f, bool join) {
+  auto eligible = [&](const NodePtr &n) {
+    if (!IsPlainProduct(n) || n->has_residual || n->inputs.size() != 1 || n->output->kind != flow::Region::kInner || n->act_from) return false;
+    if (n->act == 0 && !n->rot) return true;
+    if (n->rot && n->rot_cols != n->consts[0]->meta.GetShape()[1]) return false;  // already merged
+    return join && IsJoinable(n) && !(n->act && n->rot) && (n->act == 0 || n->act == FML_ACT_GELU_ERF);
+  };
+  auto place = [](const NodePtr &n) { return n->rot ? 0 : n->act ? 2 : 1; };
+  auto together = [&](const NodePtr &a, const NodePtr &b) {  // same tables, same constants of the activation
+    if (a->rot && b->rot)
+      return a->rot == b->rot && a->rot_head == b->rot_head && a->rot_len == b->rot_len && a->consts[a->consts.size() - 2] == b->consts[b->consts.size() - 2] &&
+             a->consts.back() == b->consts.back();
+    if (a->act && b->act) return a->act == b->act && std::equal(a->act_param, a->act_param + 3, b->act_param);
+    return (place(a) == 1 && place(b) == 1) || (IsJoinable(a) && IsJoinable(b));
   };
   for (size_t i = 0; i < f.nodes.size(); ++i) {
     const NodePtr &first = f.nodes[i];
@@ -640,9 +831,12 @@ bool MergeSiblingGemms(flow::Flow &f) {
       if (n->consts[0]->meta.GetShape()[0] != first->consts[0]->meta.GetShape()[0]) continue;
       const auto &sa = n->output->meta.GetShape(), &sb = first->output->meta.GetShape();
       if (sa.size() != sb.size() || !std::equal(sa.begin(), sa.end() - 1, sb.begin())) continue;
-      group.push_back(n);
+      bool ok = true;
+      for (const NodePtr &g : group) ok = ok && together(g, n);
+      if (ok) group.push_back(n);
     }
     if (group.size() < 2) continue;
+    std::stable_sort(group.begin(), group.end(), [&](const NodePtr &a, const NodePtr &b) { return place(a) < place(b); });
     const int64_t K = first->consts[0]->meta.GetShape()[0];
     int64_t total = 0;
     for (const auto &n : group) total += n->consts[0]->meta.GetShape()[1];
@@ -656,20 +850,9 @@ bool MergeSiblingGemms(flow::Flow &f) {
       if (n->has_bias) memcpy(bbytes.data() + (size_t)col * 4, n->consts[1]->constant->Bytes().data(), (size_t)N * 4);
       col += N;
     }
-    auto make_const = [&](const std::string &name, std::vector<int64_t> shape, std::vector<uint8_t> bytes) {
-      auto r = std::make_shared<flow::Region>();
-      r->kind = flow::Region::kConstant;
-      r->name = name;
-      r->meta = Meta(Type::kFloat32, shape);
-      r->layout = utils::GenDefaultLayout(shape.size());
-      r->constant = std::make_shared<Tensor>(r->meta, std::move(bytes));
-      f.regions.push_back(r);
-      f.by_name[name] = r;
-      return r;
-    };
     const std::string base = first->name + "_merged";
-    RegionPtr wcat = make_const(base + ".w", {K, total}, std::move(wbytes));
-    RegionPtr bcat = first->has_bias ? make_const(base + ".b", {total}, std::move(bbytes)) : nullptr;
+    RegionPtr wcat = MakeConstant(f, base + ".w", {K, total}, std::move(wbytes));
+    RegionPtr bcat = first->has_bias ? MakeConstant(f, base + ".b", {total}, std::move(bbytes)) : nullptr;
     auto merged = std::make_shared<flow::Region>();
     merged->kind = flow::Region::kInner;
     merged->name = base;
@@ -693,12 +876,31 @@ bool MergeSiblingGemms(flow::Flow &f) {
       col += n->consts[0]->meta.GetShape()[1];
       slices.push_back(sl);
     }
+    // what rides in the epilogue: the rotation of the columns in front, the activation of those at the end
+    std::vector<RegionPtr> tables;
+    int64_t rot_cols = 0, act_from = total;
+    NodePtr with_rot, with_act;
+    for (const auto &n : group) {
+      const int64_t N = n->consts[0]->meta.GetShape()[1];
+      if (n->rot) { with_rot = n; rot_cols += N; }
+      if (n->act) { with_act = n; act_from -= N; }
+    }
+    if (with_rot) tables = {with_rot->consts[with_rot->consts.size() - 2], with_rot->consts.back()};
+    const int64_t rot = with_rot ? with_rot->rot : 0, rot_head = with_rot ? with_rot->rot_head : 0, rot_len = with_rot ? with_rot->rot_len : 1;
+    if (with_act) {
+      first->act = with_act->act;
+      std::copy(with_act->act_param, with_act->act_param + 3, first->act_param);
+      first->act_from = act_from;  // 0: all of them
+    }
+    first->rot = rot; first->rot_head = rot_head; first->rot_cols = rot_cols; first->rot_len = rot_len;
     first->consts.clear();
     first->consts.push_back(wcat);
     if (bcat) first->consts.push_back(bcat);
+    first->consts.insert(first->consts.end(), tables.begin(), tables.end());
     first->output = merged;
     std::unordered_set<const flow::Node *> gone;
-    for (size_t g = 1; g < group.size(); ++g) gone.insert(group[g].get());
+    for (const auto &n : group)
+      if (n != first) gone.insert(n.get());
     std::vector<NodePtr> next;
     for (const auto &n : f.nodes) {
       if (gone.count(n.get())) continue;
@@ -713,25 +915,34 @@ bool MergeSiblingGemms(flow::Flow &f) {
 
 }  // namespace
 
-size_t FusionPasses::Run(flow::Flow &flow) {
+size_t FusionPasses::Run(flow::Flow &flow, bool join) {
   const size_t before = flow.nodes.size();
   Rewriter rw(flow);
   using Pass = bool (*)(Rewriter &, const NodePtr &);
   // order matters: bias before GELU / activation before residual, residual before Add+LN
   const Pass passes[] = {FuseEmbedding, FuseMask, FuseBias, FuseGeluIntoGemm, FuseBiasGelu, FuseActivation,
                          FuseResidual, FuseSecondResidual, FuseAddLayerNorm, FuseScaledMaskedSoftmax, FuseAttention, FuseSilu, FuseSiluIntoConv, FuseSqueezeExcite, FuseGateIntoConv, FuseResidualIntoConv, FuseMulAdd, FuseRotary, FuseMulAddChain};
-  for (Pass pass : passes) {
+  auto until_done = [&](Pass pass) {
     bool again = true;
     while (again) {
       again = false;
       for (size_t i = 0; i < flow.nodes.size(); ++i) {
         const NodePtr n = flow.nodes[i];
-        if (rw.dead.count(n.get())) continue;
         if (pass(rw, n)) { rw.Commit(); again = true; break; }
       }
     }
+  };
+  for (Pass pass : passes) until_done(pass);
+  if (join) {
+    until_done(FuseRotaryIntoGemm);
+    while (FoldSharedLayerNorms(rw)) {}
   }
-  while (MergeSiblingGemms(flow)) {}
+  while (MergeSiblingGemms(flow, join)) {}
+  if (join) {
+    rw.Index();
+    until_done(JoinSummedProducts);
+    until_done(JoinConcatenatedProduct);
+  }
   // drop tensors nothing refers to any more
   std::unordered_set<const flow::Region *> live;
   for (const auto &n : flow.nodes) {

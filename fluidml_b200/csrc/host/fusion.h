@@ -11,8 +11,10 @@ namespace worker {
 
 class FusionPasses {
 public:
-  // Rewrites `flow` in place; returns the number of nodes removed.
-  static size_t Run(flow::Flow &flow);
+  // Rewrites `flow` in place; returns the number of nodes removed.  `join`: products may be joined beyond what every
+  // GEMM kernel takes in one launch (rotations and activations of some columns, two left-hand sides), which pays
+  // where the packed-weight kernel runs them.
+  static size_t Run(flow::Flow &flow, bool join);
 };
 
 }  // namespace worker

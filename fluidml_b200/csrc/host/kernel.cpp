@@ -551,7 +551,7 @@ public:
     fml_gemm_params params;
     bool has_const_b = false, has_bias = false, has_residual = false, bias_is_input = false;
     fml_tensor const_b{}, bias{};
-    bool trans_a = false, trans_b = false, autotune = false;
+    bool trans_a = false, trans_b = false, autotune = false, two_a = false;
   };
   explicit GemmLikeKernel(Config c) : c_(c) {}
   std::string GetKernelName() const override { return c_.name; }
@@ -574,6 +574,7 @@ public:
     Resolve(in, a, b, bias, res);
     if (b.rank != 2) return 0;
     fml_gemm_params p = c_.params;
+    if (c_.two_a) p.a2 = in.at(1);
     p.b_packed = b.data;  // any aligned address: would the library take the packed path?
     fml_gemm_plan_info info;
     if (fml_gemm_plan(&a, &b, &output, &p, &info) != FML_OK || !info.uses_packed) return 0;
@@ -605,6 +606,7 @@ public:
                fml_tensor &res) const {
     size_t k = 0;
     a = in.at(k++);
+    if (c_.two_a) ++k;  // inputs[1] continues A's columns
     b = c_.has_const_b ? c_.const_b : in.at(k++);
     if (c_.trans_a) std::swap(a.shape[a.rank - 2], a.shape[a.rank - 1]), std::swap(a.stride[a.rank - 2], a.stride[a.rank - 1]);
     if (c_.trans_b) std::swap(b.shape[b.rank - 2], b.shape[b.rank - 1]), std::swap(b.stride[b.rank - 2], b.stride[b.rank - 1]);
@@ -614,7 +616,7 @@ public:
   }
   bool DescribeResident(const std::vector<fml_tensor> &in, const fml_tensor &output, fml_resident_stage *st) const override {
     const fml_gemm_params &p = c_.params;
-    if (!c_.has_const_b || c_.trans_a || c_.bias_is_input) return false;
+    if (!c_.has_const_b || c_.trans_a || c_.bias_is_input || c_.two_a || p.act_from || p.rot) return false;
     if (p.alpha != 1.0f || (c_.has_bias && p.beta != 1.0f) || (p.divisor != 1.0f && p.divisor != 0.0f)) return false;
     if (p.precision == FML_GEMM_FP32 || p.precision == FML_GEMM_TF32) return false;  // the resident GEMM is 3xTF32
     if (p.act < FML_ACT_NONE || p.act > FML_ACT_SIGMOID) return false;
@@ -636,6 +638,7 @@ public:
     Resolve(in, a, b, bias, res);
     Config c = c_;
     c.params.b_constant = c.has_const_b ? 1 : 0;
+    if (c.two_a) c.params.a2 = in.at(1);
     if (c.autotune) {  // device buffers are live while the builder records: try the candidates now
       fml_gemm_params tuned;
       if (fml_gemm_autotune(&a, &b, &output, c.has_bias ? &bias : nullptr, c.has_residual ? &res : nullptr,
@@ -763,7 +766,9 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
   case Kind::Silu: return std::make_unique<SiluKernel>();
   case Kind::FusedMulAdd: return std::make_unique<FusedMulAddKernel>();
   case Kind::FusedMulAddChain: return std::make_unique<FusedMulAddChainKernel>();
-  case Kind::Rotary: return std::make_unique<RotaryKernel>((int64_t)n.value);
+  case Kind::Rotary:
+    if (n.inputs.size() == 1) return std::make_unique<DropoutKernel>();  // rotated by its product: a view
+    return std::make_unique<RotaryKernel>((int64_t)n.value);
   case Kind::SqueezeExciteGate: {
     size_t k = 0;
     const fml_tensor w1 = C(k++);
@@ -846,12 +851,21 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
     c.trans_a = n.trans_a;
     c.trans_b = n.trans_b;
     size_t k = 0;
-    // inputs: A, [B if variable], [variable addend if has_mask], [residual];
-    // consts: [B if captured], [bias if has_bias]
+    // inputs: A, [A2 if two_a], [B if variable], [variable addend if has_mask], [residual];
+    // consts: [B if captured], [bias if has_bias], [cos, sin if rot]
     if (n.b_is_const) { c.has_const_b = true; c.const_b = C(k++); }
     if (n.has_bias) { c.has_bias = true; c.bias = C(k++); }
     if (n.has_mask) { c.has_bias = true; c.bias_is_input = true; }  // a variable addend (attention mask)
     c.has_residual = n.has_residual;
+    c.two_a = n.two_a;
+    c.params.act_from = (int32_t)n.act_from;
+    if (n.rot) {
+      if (!utils::IsDefaultLayout(n.consts.at(k)->layout) || !utils::IsDefaultLayout(n.consts.at(k + 1)->layout)) throw Error("rotary tables must be row-major");
+      c.params.rot = (int32_t)n.rot; c.params.rot_head = (int32_t)n.rot_head;
+      c.params.rot_cols = (int32_t)n.rot_cols; c.params.rot_len = (int32_t)n.rot_len;
+      c.params.rot_cos = (const float *)C(k).data;
+      c.params.rot_sin = (const float *)C(k + 1).data;
+    }
     return std::make_unique<GemmLikeKernel>(c);
   }
   case Kind::ConvWithoutPadding:

@@ -5,7 +5,7 @@
 // innermost collapsed dimension is contiguous (or broadcast) and 16-byte aligned the kernel
 // moves float4 per thread; otherwise it falls back to one element per thread with the
 // offsets rebuilt from the collapsed shape.
-#include "common.cuh"
+#include "gemm_common.cuh"
 
 namespace fml {
 namespace {
@@ -464,7 +464,33 @@ bool vec4_ok(const Iter<3> &it, const void *out, const void *a, const void *b) {
   return true;
 }
 
+// The rotary embedding in place, for products whose kernel does not apply it itself: a thread owns both features
+// of a pair, and only the rotated features are touched.
+__global__ void rotary_in_place_kernel(GemmProblem p, GemmExtras x) {
+  pdl_prologue();
+  const int half = x.rot >> 1, heads = x.rot_cols / x.rot_head;
+  const int64_t per_z = p.M * heads * half, total = per_z * p.nb0 * p.nb1;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t z = i / per_z, z1 = z / p.nb0, z0 = z - z1 * p.nb0, in_z = i - z * per_z, mh = in_z / half;
+    const int d = (int)(in_z - mh * half), head = (int)(mh % heads);
+    const int64_t m = mh / heads;
+    float *lo = p.c + z0 * p.c_b0 + z1 * p.c_b1 + m * p.c_sm + ((int64_t)head * x.rot_head + d) * p.c_sn, *hi = lo + half * p.c_sn;
+    const float *c = x.rot_cos + (m % x.rot_len) * x.rot + d, *s = x.rot_sin + (m % x.rot_len) * x.rot + d;
+    const float a = *lo, b = *hi;
+    *lo = __fadd_rn(__fmul_rn(a, c[0]), __fmul_rn(-b, s[0]));
+    *hi = __fadd_rn(__fmul_rn(b, c[half]), __fmul_rn(a, s[half]));
+  }
+}
+
 }  // namespace
+
+int launch_rotary_in_place(const GemmProblem &p, const GemmExtras &x, cudaStream_t s) {
+  const int64_t total = p.M * (x.rot_cols / x.rot_head) * (x.rot / 2) * p.nb0 * p.nb1;
+  if (total == 0) return FML_OK;
+  FML_LAUNCH((rotary_in_place_kernel), grid_for(total, 256), 256, 0, s, p, x);
+  return FML_OK;
+}
+
 }  // namespace fml
 
 using namespace fml;

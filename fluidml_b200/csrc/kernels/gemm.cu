@@ -190,17 +190,68 @@ struct Choice {
   Path path;
   TcPlan tc;
   PairPlan pair;
+  GemmExtras x;
+  bool parts = false;  // joined by the caller (a2, act_from) but not one launch here: fml_gemm runs the parts
 };
+
+// Dims [from, to) of dim `dim` of t.
+fml_tensor part_of(const fml_tensor *t, int dim, int64_t from, int64_t to) {
+  fml_tensor v = *t;
+  v.shape[dim] = to - from;
+  v.data = (char *)t->data + from * t->stride[dim] * 4;
+  return v;
+}
 }  // namespace
 
 static int resolve(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
                    const fml_tensor *bias, const fml_tensor *res, const fml_gemm_params *gp,
                    GemmProblem &p, Choice &ch) {
   FML_REQUIRE(gp, FML_BAD_ARG, "fml_gemm: null params");
-  int st = analyse_gemm(a, b, c, bias, res, p);
-  if (st != FML_OK) return st;
+  GemmExtras &x = ch.x;
+  x = GemmExtras();
+  ch.parts = false;
+  bool joined = true;  // A2's rows are walked as A's are
+  fml_tensor whole;
+  if (gp->a2.data) {
+    const fml_tensor *a2 = &gp->a2;
+    FML_REQUIRE(valid_tensor(a) && valid_tensor(a2) && valid_tensor(b) && a2->dtype == FML_F32 && a->rank >= 2 && b->rank == 2 && a2->rank == a->rank,
+                FML_BAD_ARG, "fml_gemm: A2 needs A's rank and a B of rank 2");
+    for (int i = 0; i + 1 < a->rank; ++i) FML_REQUIRE(a2->shape[i] == a->shape[i], FML_BAD_ARG, "fml_gemm: A2's shape");
+    const int64_t k1 = a->shape[a->rank - 1], k2 = a2->shape[a->rank - 1];
+    FML_REQUIRE(k1 > 0 && k2 > 0 && b->shape[0] == k1 + k2, FML_BAD_ARG, "fml_gemm: the columns of A and A2 are not the rows of B");
+    FML_REQUIRE(gp->act == FML_ACT_NONE && gp->alpha == 1.0f && gp->beta == 1.0f && (gp->divisor == 1.0f || gp->divisor == 0.0f) && !gp->act_from && !gp->rot,
+                FML_UNSUPPORTED, "fml_gemm: A2 with an activation, a scale or a rotation");
+    const fml_tensor b2 = part_of(b, 0, k1, k1 + k2);
+    GemmProblem p2;
+    const int st = analyse_gemm(a2, &b2, c, bias, res, p2);
+    if (st != FML_OK) return st;
+    x.a2 = p2.a; x.a2_sm = p2.a_sm; x.a2_b0 = p2.a_b0; x.a2_b1 = p2.a_b1; x.k1 = k1;
+    whole = *a;
+    whole.shape[a->rank - 1] = k1 + k2;
+    a = &whole;
+    joined = p2.a_sk == 1;
+    const int st1 = analyse_gemm(a, b, c, bias, res, p);
+    if (st1 != FML_OK) return st1;
+    joined = joined && p2.M == p.M && p2.nb0 == p.nb0 && p2.nb1 == p.nb1;
+  } else {
+    const int st = analyse_gemm(a, b, c, bias, res, p);
+    if (st != FML_OK) return st;
+  }
+  if (gp->act_from) {
+    FML_REQUIRE(gp->act_from > 0 && gp->act_from < p.N, FML_BAD_ARG, "fml_gemm: act_from is not a column");
+    x.act_from = gp->act_from;
+  }
+  if (gp->rot) {
+    FML_REQUIRE(gp->rot > 0 && gp->rot % 2 == 0 && gp->rot <= gp->rot_head && gp->rot_cols > 0 && gp->rot_cols <= p.N &&
+                    gp->rot_cols % gp->rot_head == 0 && gp->rot_len > 0 && p.M % gp->rot_len == 0 && gp->rot_cos && gp->rot_sin && !res,
+                FML_BAD_ARG, "fml_gemm: rotary embedding");
+    FML_REQUIRE(gp->act_from ? gp->rot_cols <= gp->act_from : gp->act == FML_ACT_NONE, FML_UNSUPPORTED, "fml_gemm: an activation on rotated columns");
+    x.rot = gp->rot; x.rot_head = gp->rot_head; x.rot_cols = gp->rot_cols; x.rot_len = gp->rot_len;
+    x.rot_cos = gp->rot_cos; x.rot_sin = gp->rot_sin;
+  }
   ch.path = Path::kSimt;
-  if (plan_gemm_pair(p, *gp, ch.pair)) ch.path = Path::kPair;
+  if (joined && plan_gemm_pair(p, x, *gp, ch.pair)) ch.path = Path::kPair;
+  else if (x.a2 || x.act_from) { ch.parts = true; return FML_OK; }
   else if (gp->precision != FML_GEMM_FP32 && plan_gemm_tc(p, *gp, ch.tc)) ch.path = Path::kTc;
   FML_REQUIRE(ch.path != Path::kSimt || gp->precision == FML_GEMM_AUTO || gp->precision == FML_GEMM_FP32,
               FML_MISALIGNED,
@@ -217,6 +268,7 @@ extern "C" int fml_gemm_plan(const fml_tensor *a, const fml_tensor *b, const fml
   int st = resolve(a, b, c, nullptr, nullptr, gp, p, ch);
   if (st != FML_OK) return st;
   memset(info, 0, sizeof(*info));
+  if (ch.parts) return FML_OK;
   info->uses_tensor_cores = ch.path != Path::kSimt ? 1 : 0;
   if (ch.path == Path::kPair) {
     info->tile_n = ch.pair.tile_n; info->split_k = ch.pair.split_k; info->stages = ch.pair.stages_b;
@@ -250,6 +302,35 @@ extern "C" int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tens
   int st = resolve(a, b, c, bias, residual, gp, p, ch);
   if (st != FML_OK) return st;
   if (p.M == 0 || p.N == 0 || p.nb0 * p.nb1 == 0) return FML_OK;
+  if (ch.parts) {  // the parts one after the other, each with the tiles the library chooses for it
+    fml_gemm_params q = *gp;
+    q.tile_n = q.split_k = q.ctas_per_sm = 0;
+    q.b_packed = nullptr;
+    q.act_from = 0;
+    memset(&q.a2, 0, sizeof(q.a2));
+    const int rb = b->rank, rc = c->rank;
+    if (gp->a2.data) {  // A's part with bias and residual, then A2's on top of it
+      const int64_t k1 = a->shape[a->rank - 1];
+      const fml_tensor b1 = part_of(b, 0, 0, k1), b2 = part_of(b, 0, k1, b->shape[0]);
+      st = fml_gemm(a, &b1, c, bias, residual, &q, stream);
+      return st != FML_OK ? st : fml_gemm(&gp->a2, &b2, c, nullptr, c, &q, stream);
+    }
+    for (int part = 0; part < 2; ++part) {  // the columns without the activation, then those with it
+      const int64_t from = part ? gp->act_from : 0, to = part ? p.N : gp->act_from;
+      const fml_tensor bp = part_of(b, rb - 1, from, to), cp = part_of(c, rc - 1, from, to);
+      auto columns = [&](const fml_tensor *t, fml_tensor *v) -> const fml_tensor * {
+        if (!t || t->rank == 0 || t->shape[t->rank - 1] == 1) return t;
+        *v = part_of(t, t->rank - 1, from, to);
+        return v;
+      };
+      fml_tensor bias_part, res_part;
+      q.act = part ? gp->act : FML_ACT_NONE;
+      if (part) q.rot = 0;
+      st = fml_gemm(a, &bp, &cp, columns(bias, &bias_part), columns(residual, &res_part), &q, stream);
+      if (st != FML_OK) return st;
+    }
+    return FML_OK;
+  }
   GemmEpilogue e = make_epilogue(*gp, bias != nullptr, residual != nullptr);
   p.b_constant = gp->b_constant ? 1 : 0;
   if (gp->l2_prefetch && gp->l2_prefetch_bytes) {
@@ -258,19 +339,19 @@ extern "C" int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tens
     p.prefetch = static_cast<const char *>(gp->l2_prefetch);
     p.prefetch_bytes = gp->l2_prefetch_bytes;
   }
-  if (ch.path == Path::kPair) return launch_gemm_pair(p, e, ch.pair, gp->b_packed, as_stream(stream));
-  if (ch.path == Path::kTc) return launch_gemm_tc(p, e, ch.tc, as_stream(stream));
-  if (skinny_eligible(p)) return launch_gemm_skinny(p, e, as_stream(stream));
-  return launch_gemm_simt(p, e, as_stream(stream));
+  if (ch.path == Path::kPair) return launch_gemm_pair(p, e, ch.x, ch.pair, gp->b_packed, as_stream(stream));
+  st = ch.path == Path::kTc ? launch_gemm_tc(p, e, ch.tc, as_stream(stream))
+       : skinny_eligible(p) ? launch_gemm_skinny(p, e, as_stream(stream)) : launch_gemm_simt(p, e, as_stream(stream));
+  return st == FML_OK && ch.x.rot ? launch_rotary_in_place(p, ch.x, as_stream(stream)) : st;
 }
 
 // What a remembered choice of tiles belongs to: the device, the problem and its epilogue.
 static std::string tuning_key(int device, const GemmProblem &p, const Choice &ch, const fml_gemm_params &gp, bool bias, bool residual) {
   const bool pair = ch.path == Path::kPair;
   char key[256];
-  snprintf(key, sizeof(key), "%d|%lld,%lld,%lld,%lld,%lld|%d%d%d|%d,%d,%d,%d|%lld,%lld", device, (long long)p.M, (long long)p.N, (long long)p.K,
+  snprintf(key, sizeof(key), "%d|%lld,%lld,%lld,%lld,%lld|%d%d%d|%d,%d,%d,%d|%lld,%lld|%d,%d,%lld", device, (long long)p.M, (long long)p.N, (long long)p.K,
            (long long)p.nb0, (long long)p.nb1, pair, pair ? 0 : ch.tc.b_mn_major, pair ? 1 : ch.tc.three_pass, gp.act, bias, residual,
-           gp.divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn);
+           gp.divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn, ch.x.act_from, ch.x.rot ? ch.x.rot_cols : 0, (long long)ch.x.k1);
   return key;
 }
 
@@ -281,7 +362,7 @@ extern "C" int fml_gemm_tuning_key(const fml_tensor *a, const fml_tensor *b, con
   Choice ch;
   const int st = resolve(a, b, c, bias, residual, gp, p, ch);
   if (st != FML_OK) return st;
-  snprintf(key, bytes, "%s", ch.path == Path::kSimt ? "" : tuning_key(device, p, ch, *gp, bias != nullptr, residual != nullptr).c_str());
+  snprintf(key, bytes, "%s", ch.parts || ch.path == Path::kSimt ? "" : tuning_key(device, p, ch, *gp, bias != nullptr, residual != nullptr).c_str());
   return FML_OK;
 }
 
@@ -298,7 +379,7 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
   Choice ch;
   int st = resolve(a, b, c, bias, residual, gp, p, ch);
   if (st != FML_OK) return st;
-  if (ch.path == Path::kSimt || gp->tile_n != 0 || gp->split_k != 0) return FML_OK;  // nothing to choose
+  if (ch.parts || ch.path == Path::kSimt || gp->tile_n != 0 || gp->split_k != 0) return FML_OK;  // nothing to choose
   const bool pair = ch.path == Path::kPair;
   int device = 0;
   FML_CUDA(cudaGetDevice(&device));
@@ -338,7 +419,7 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
         q.split_k = sk;
         q.ctas_per_sm = ctas;
         Choice cand;
-        if (pair ? !plan_gemm_pair(p, q, cand.pair) : !plan_gemm_tc(p, q, cand.tc)) continue;
+        if (pair ? !plan_gemm_pair(p, ch.x, q, cand.pair) : !plan_gemm_tc(p, q, cand.tc)) continue;
         const Tiles id = pair ? Tiles{cand.pair.tile_n, cand.pair.split_k, cand.pair.ctas_per_sm}
                               : Tiles{cand.tc.tile_n, cand.tc.split_k, 0};
         bool dup = false;
@@ -347,7 +428,7 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
         if (dup) continue;
         seen.push_back(id);
         auto launch = [&] {
-          return pair ? launch_gemm_pair(p, epi, cand.pair, gp->b_packed, s) : launch_gemm_tc(p, epi, cand.tc, s);
+          return pair ? launch_gemm_pair(p, epi, ch.x, cand.pair, gp->b_packed, s) : launch_gemm_tc(p, epi, cand.tc, s);
         };
         float one = 0.0f;
         bool ok = launch() == FML_OK;  // warm-up; skip what cannot launch

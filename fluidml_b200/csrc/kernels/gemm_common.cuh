@@ -47,6 +47,16 @@ __device__ __forceinline__ float gemm_epilogue(const GemmEpilogue &e, float acc,
   return v;
 }
 
+// What only the packed-weight kernel does inside one launch (fml_gemm_params: a2, act_from, rot_*); fml_gemm runs the
+// other kernels once per part instead.
+struct GemmExtras {
+  const float *a2 = nullptr;  // columns k1 .. K of A, with strides of their own
+  int64_t a2_sm = 0, a2_b0 = 0, a2_b1 = 0, k1 = 0;
+  int act_from = 0;           // the activation is applied from this column on
+  int rot = 0, rot_head = 0, rot_cols = 0, rot_len = 1;  // rotary embedding of columns below rot_cols
+  const float *rot_cos = nullptr, *rot_sin = nullptr;    // [rot_len][rot]
+};
+
 // Fills `p` from the tensors; returns FML_UNSUPPORTED when more than two batch dims remain
 // after collapsing (the caller then loops or falls back).
 int analyse_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
@@ -81,8 +91,13 @@ struct PairPlan {
 };
 size_t pair_packed_bytes(int64_t K, int64_t N);
 int pair_pack(const float *b, int64_t K, int64_t N, int64_t sk, int64_t sn, void *dst, cudaStream_t s);
-bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &plan);
-int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const PairPlan &plan, const void *packed, cudaStream_t s);
+bool plan_gemm_pair(const GemmProblem &p, const GemmExtras &x, const fml_gemm_params &gp, PairPlan &plan);
+// Whether this plan's epilogue can apply the rotary embedding (else fml_gemm launches it on its own).
+bool pair_rotates(const GemmProblem &p, const GemmExtras &x, const PairPlan &plan);
+int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const GemmExtras &x, const PairPlan &plan, const void *packed, cudaStream_t s);
+
+// x[m, head * rot_head + d] for d < rot, in place, by the rotary embedding (elementwise.cu)
+int launch_rotary_in_place(const GemmProblem &p, const GemmExtras &x, cudaStream_t s);
 
 // pipelined depthwise convolution over dense NCHW planes (conv_depthwise_tma.cu); false = not taken
 bool launch_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,

@@ -58,7 +58,9 @@ inline EpilogueShape epilogue_shape(int tile_n, int threads) {
 // the loads that do not depend on it -- bias, column scales, the first row's residual -- whose L2 round
 // trip is then off the critical path of a launch that does each phase once.  Only those values stay in
 // registers; finish() works the geometry out again (kept live across the accumulator reads it spilled).
-template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
+// PROJ: the columns are several projections side by side: those below x.rot_cols are heads whose first x.rot features
+// get the rotary embedding (pair_rotates), those from x.act_from on the activation.
+template <int ACT, int NT, bool COL_SCALE, bool PROJ = false> struct TileEpilogue {
   float4 bvec, cs, rvec;
 
   // Where this thread works.
@@ -107,7 +109,7 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
   }
 
   __device__ __forceinline__ void finish(const GemmProblem &p, const GemmEpilogue &e, const EpilogueShape &shape, float *staging, int pitch, int BN, int tile_m,
-                                         int tile_n, int split, int S, int z0, int z1, int et, const float *col_scale) {
+                                         int tile_n, int split, int S, int z0, int z1, int et, const float *col_scale, const GemmExtras &x = {}) {
     asm volatile("" : "+r"(tile_m), "+r"(tile_n), "+r"(et));  // recompute: nothing of preload()'s geometry is kept
     const Where w(p, shape, BN, tile_m, tile_n, split, S, z0, z1, et);
     const float *bias = w.bias, *res = w.res;
@@ -130,7 +132,14 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
       const int64_t r_step = (int64_t)rows_pass * p.res_sm;
       const float *bp = bias ? bias + (m_base + r) * p.bias_sm + (p.bias_sn ? n : 0) : nullptr;
       const int64_t b_step = (int64_t)rows_pass * p.bias_sm;
-      auto one = [&](float4 acc, float4 bq, float4 rq) {
+      const bool act_here = !PROJ || n >= x.act_from;
+      // The rotary embedding pairs feature d with d +- rot / 2: the thread rot / 8 quads away in the same row, which is
+      // in this warp because rot / 4 quads are an aligned power of two.
+      const int feature = PROJ && x.rot && n < x.rot_cols ? (int)n % x.rot_head : 1 << 30;
+      const bool rotate = PROJ && feature < x.rot;
+      const int span = PROJ ? x.rot >> 2 : 1;
+      const unsigned peers = PROJ && rotate ? (span == 32 ? 0xffffffffu : ((1u << span) - 1u) << ((et & 31) & ~(span - 1))) : 0u;
+      auto one = [&](float4 acc, float4 bq, float4 rq, int row) {
         if (COL_SCALE) { acc.x *= cs.x; acc.y *= cs.y; acc.z *= cs.z; acc.w *= cs.w; }
         float v[4] = {acc.x, acc.y, acc.z, acc.w};
         const float bv[4] = {bq.x, bq.y, bq.z, bq.w}, rv[4] = {rq.x, rq.y, rq.z, rq.w};
@@ -143,7 +152,26 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
           } else {
             y += bv[j];
           }
-          v[j] = act_op<ACT>(e, y) + rv[j];
+          v[j] = PROJ ? y : act_op<ACT>(e, y) + rv[j];
+        }
+        if (PROJ) {
+          if (rotate) {  // two rounded products and a rounded sum, as rotary_kernel
+            const int at = (int)((unsigned)(m_base + row) % (unsigned)x.rot_len) * x.rot + feature;
+            const float4 cq = __ldg(reinterpret_cast<const float4 *>(x.rot_cos + at)), sq = __ldg(reinterpret_cast<const float4 *>(x.rot_sin + at));
+            const float co[4] = {cq.x, cq.y, cq.z, cq.w}, si[4] = {sq.x, sq.y, sq.z, sq.w};
+            const float sgn = feature < (x.rot >> 1) ? -1.0f : 1.0f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float other = __shfl_xor_sync(peers, v[j], span >> 1);
+              v[j] = __fadd_rn(__fmul_rn(v[j], co[j]), __fmul_rn(sgn * other, si[j]));
+            }
+          }
+          if (act_here) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = act_op<ACT>(e, v[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] += rv[j];
         }
         return make_float4(v[0], v[1], v[2], v[3]);
       };
@@ -159,7 +187,7 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
             rq[u] = res ? *reinterpret_cast<const float4 *>(rp + u * r_step) : make_float4(0.f, 0.f, 0.f, 0.f);
           }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) *reinterpret_cast<float4 *>(cp + u * c_step) = one(acc[u], bvec, rq[u]);
+          for (int u = 0; u < 4; ++u) *reinterpret_cast<float4 *>(cp + u * c_step) = one(acc[u], bvec, rq[u], r + u * rows_pass);
           r += 4 * rows_pass; sp += 4 * sp_step; cp += 4 * c_step; rp += 4 * r_step;
         }
         if (res && r < r_end) rvec = *reinterpret_cast<const float4 *>(rp);
@@ -175,7 +203,7 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
           if (bias && !bias_per_col) bvec = column_bias();
           rp += r_step;
           if (res && r + rows_pass < r_end) rvec = *reinterpret_cast<const float4 *>(rp);  // the next row's, under this row's arithmetic
-          *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq);
+          *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq, r);
           sp += sp_step; cp += c_step; bp += b_step;
         }
       } else {
@@ -208,7 +236,7 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
 #pragma unroll
               for (int k = 0; k < kRanks; ++k) { acc.x += t[u][k].x; acc.y += t[u][k].y; acc.z += t[u][k].z; acc.w += t[u][k].w; }
               if (bias && !bias_per_col) bvec = column_bias();
-              *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq[u]);
+              *reinterpret_cast<float4 *>(cp) = one(acc, bvec, rq[u], r + u * rows_pass);
               cp += c_step; bp += b_step;
             }
             r += kRows * rows_pass;
@@ -248,7 +276,7 @@ template <int ACT, int NT, bool COL_SCALE> struct TileEpilogue {
           } else {
             y += bv;
           }
-          C[m * p.c_sm + n * p.c_sn] = act_op<ACT>(e, y) + rv;
+          C[m * p.c_sm + n * p.c_sn] = (PROJ && n < x.act_from ? y : act_op<ACT>(e, y)) + rv;
         }
       }
     }

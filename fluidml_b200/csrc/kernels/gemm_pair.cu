@@ -52,6 +52,7 @@ constexpr int kConvThreads = 256;
 struct PairArgs {
   GemmProblem p;
   GemmEpilogue e;
+  GemmExtras x;
   EpilogueShape shape;
   const char *packed;       // B atoms
   const float *col_scale;   // 2^-s of each column
@@ -61,9 +62,16 @@ struct PairArgs {
   int *status;
 };
 
-template <int ACT>
+// MODE: what else a launch does.  kProj: several projections of the same rows side by side (the queries, keys and
+// values of an attention block and the first product of a feed-forward layer), with the rotary embedding on the
+// first columns and the activation on the last (TileEpilogue).  kTwoA: A's columns come from two tensors, [A | A2] * B:
+// the sum of two products (both halves of a parallel-residual block) or a concatenation's product, one launch
+// and one reduction for both; k blocks do not straddle the seam (k1 is a multiple of 32).
+enum { kPlain = 0, kProj = 1, kTwoA = 2 };
+
+template <int ACT, int MODE>
 __global__ void __launch_bounds__(kPairThreads, 2)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_a2, const PairArgs a) {
   // (no static shared memory in this kernel: the dynamic part starts on a 1024-byte boundary)
   extern __shared__ __align__(1024) uint8_t smem[];
   const int BN = a.tile_n;
@@ -113,6 +121,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   };
 
   if (threadIdx.x == 0) tma_prefetch_map(&map_a);
+  if (MODE == kTwoA && threadIdx.x == 0) tma_prefetch_map(&map_a2);
+  const int kb_seam = MODE == kTwoA ? (int)(a.x.k1 / kPK) : 0;  // first k block of A2
   if (a.p.prefetch_bytes && threadIdx.x == 64) {  // the next launch's weights (gemm_tc.cu)
     const uint64_t pf_policy = l2_policy_evict_first();
     const unsigned long long ctas = (unsigned long long)gridDim.x * gridDim.y * gridDim.z;
@@ -168,7 +178,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
 
   // A's ring in two parts, one per converter set (pair_stages)
   const int ring_0 = (a.stages_a + 1) >> 1, ring_1 = a.stages_a >> 1;
-  TileEpilogue<ACT, kConvThreads, true> epi;
+  TileEpilogue<ACT, kConvThreads, true, MODE == kProj> epi;
   float row_inv = 1.0f;  // converter threads: undoes the scale of this thread's row
   if (warp == 0) {
     // ------------------------------------------------------------ loads
@@ -193,7 +203,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
             const uint32_t bar = bar_full_a + 8u * sa;
             if (leader) {
               mbar_expect_tx(bar, kPairA);
-              tma_load_4d(ring_a + sa * kPairA, &map_a, bar, (kb0 + ia) * kPK, tile_m * kBM, ca2, ca3);
+              if (MODE == kTwoA && kb0 + ia >= kb_seam)
+                tma_load_4d(ring_a + sa * kPairA, &map_a2, bar, (kb0 + ia - kb_seam) * kPK, tile_m * kBM, a.x.a2_b0 ? z0 : 0, a.x.a2_b1 ? z1 : 0);
+              else
+                tma_load_4d(ring_a + sa * kPairA, &map_a, bar, (kb0 + ia) * kPK, tile_m * kBM, ca2, ca3);
             }
             ++ia; moved = true;
             if (odd) { ++issued_1; ra1.step(ring_1); } else { ++issued_0; ra0.step(ring_0); }
@@ -276,11 +289,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
     float seen = 0.0f;   // largest scaled magnitude this thread converted (kept while a row of its warp has the default scale)
     bool bad = false;    // this row needs a second attempt
     const float *const a_row = a.p.a + (int64_t)z0 * a.p.a_b0 + (int64_t)z1 * a.p.a_b1 + ((int64_t)tile_m * kBM + row) * a.p.a_sm;
+    auto a2_row = [&](int r) { return a.x.a2 + (int64_t)z0 * a.x.a2_b0 + (int64_t)z1 * a.x.a2_b1 + ((int64_t)tile_m * kBM + r) * a.x.a2_sm; };
     float sampled = 0.0f;
     if (nkb >= kSampleBlocks && set == 0 && real_row) {
       float4 y[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) y[i] = *reinterpret_cast<const float4 *>(a_row + (kb0 + (int64_t)i * (nkb - 1) / 16) * kPK);
+      for (int i = 0; i < 16; ++i) {
+        const int kb = kb0 + i * (nkb - 1) / 16;
+        y[i] = *reinterpret_cast<const float4 *>(MODE == kTwoA && kb >= kb_seam ? a2_row(row) + (int64_t)(kb - kb_seam) * kPK : a_row + (int64_t)kb * kPK);
+      }
 #pragma unroll
       for (int i = 0; i < 16; ++i) sampled = fmaxf(sampled, fmaxf(fmaxf(fabsf(y[i].x), fabsf(y[i].y)), fmaxf(fabsf(y[i].z), fabsf(y[i].w))));
     }
@@ -299,7 +316,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
         for (uint32_t left = __ballot_sync(0xffffffffu, bad); left; left &= left - 1) {
           const int r = __ffs((int)left) - 1;
           const float *src = a_row + (int64_t)(r - lane) * a.p.a_sm;
-          const float m = warp_row_max(src, (int64_t)kb0 * kPK, min((int64_t)kb1 * kPK, a.p.K), lane);
+          const int64_t k_end = min((int64_t)kb1 * kPK, a.p.K);
+          float m;
+          if (MODE == kTwoA) {
+            m = kb0 < kb_seam ? warp_row_max(src, (int64_t)kb0 * kPK, min(k_end, a.x.k1), lane) : 0.0f;
+            if (kb1 > kb_seam) m = fmaxf(m, warp_row_max(a2_row(q * 32 + r), (int64_t)max(kb0 - kb_seam, 0) * kPK, k_end - a.x.k1, lane));
+          } else {
+            m = warp_row_max(src, (int64_t)kb0 * kPK, k_end, lane);
+          }
           if (lane == r) k_row = scale_exponent(m, 14);
         }
       } else {
@@ -417,7 +441,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const PairArgs a) {
   const int S = a.split_k;
   if (S > 1) cluster_sync_all();
   if (warp >= 2)
-    epi.finish(a.p, a.e, a.shape, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, threadIdx.x - 64, a.col_scale);
+    epi.finish(a.p, a.e, a.shape, staging, pitch, BN, tile_m, tile_n, split, S, z0, z1, threadIdx.x - 64, a.col_scale, a.x);
   if (S > 1) cluster_sync_relaxed();
   __syncthreads();
   if (warp == 1) {
@@ -525,13 +549,29 @@ int pair_pack(const float *b, int64_t K, int64_t N, int64_t sk, int64_t sn, void
   return FML_OK;
 }
 
-bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &plan) {
+bool pair_rotates(const GemmProblem &p, const GemmExtras &x, const PairPlan &plan) {
+  if (!x.rot) return false;
+  // groups of rot columns lie within a tile and, four columns to a lane, within a warp
+  const bool pow2 = (x.rot & (x.rot - 1)) == 0;
+  if (!pow2 || x.rot < 8 || x.rot > 128 || x.rot_head % x.rot || plan.tile_n % x.rot) return false;
+  if (!aligned16(x.rot_cos) || !aligned16(x.rot_sin)) return false;
+  // tiles of rotated columns take the epilogue's 16-byte path (TileEpilogue::Where)
+  if ((x.rot_cols + plan.tile_n - 1) / plan.tile_n * (int64_t)plan.tile_n > p.N) return false;
+  if (p.c_sn != 1 || p.c_sm % 4 || p.c_b0 % 4 || p.c_b1 % 4 || !aligned16(p.c) || p.res) return false;
+  return !p.bias || (p.bias_sn == 1 && p.bias_sm % 4 == 0 && p.bias_b0 % 4 == 0 && p.bias_b1 % 4 == 0 && aligned16(p.bias));
+}
+
+bool plan_gemm_pair(const GemmProblem &p, const GemmExtras &x, const fml_gemm_params &gp, PairPlan &plan) {
   if (!gp.b_packed || gp.precision != FML_GEMM_AUTO) return false;
   // A goes through a tensor map (K contiguous, 16-byte aligned rows); fewer than 32 rows stay on the
   // weight-streaming fp32 kernel, as with the 3xTF32 kernel
   if (p.M < 32 || p.N < 16 || p.K < 16 || p.a_sk != 1 || !aligned16(p.a) || p.a_sm <= 0 || p.a_sm % 4) return false;
   auto stride_ok = [](int64_t s) { return s == 0 || (s > 0 && s % 4 == 0); };
   if (!stride_ok(p.a_b0) || !stride_ok(p.a_b1) || p.b_b0 || p.b_b1) return false;
+  if (x.a2 && (!aligned16(x.a2) || x.a2_sm <= 0 || x.a2_sm % 4 || !stride_ok(x.a2_b0) || !stride_ok(x.a2_b1) || x.k1 % kPK)) return false;
+  if ((x.act_from || x.rot) && gp.act != FML_ACT_GELU_ERF && gp.act != FML_ACT_NONE) return false;  // the instantiations there are
+  if (x.a2 && gp.act != FML_ACT_NONE) return false;
+  if ((x.act_from || x.rot) && x.a2) return false;
   if (p.M > (1ll << 30) || p.N > (1ll << 24) || p.K > (1ll << 30) || p.nb0 * p.nb1 > 65535) return false;
   if (!aligned16(gp.b_packed)) return false;
   const int kb_total = k_blocks(p.K);
@@ -578,9 +618,12 @@ bool plan_gemm_pair(const GemmProblem &p, const fml_gemm_params &gp, PairPlan &p
   return found;
 }
 
-int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const PairPlan &plan, const void *packed, cudaStream_t s) {
+int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const GemmExtras &x, const PairPlan &plan, const void *packed, cudaStream_t s) {
   PairArgs a;
-  a.p = p; a.e = e;
+  a.p = p; a.e = e; a.x = x;
+  const bool rotates = pair_rotates(p, x, plan);
+  if (!rotates) a.x.rot = 0;
+  const int mode = x.a2 ? kTwoA : x.act_from || rotates ? kProj : kPlain;
   a.shape = epilogue_shape(plan.tile_n, kConvThreads);
   a.packed = static_cast<const char *>(packed);
   a.col_scale = reinterpret_cast<const float *>(a.packed + atoms_bytes(p.K, p.N));
@@ -592,13 +635,21 @@ int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const PairPlan
   a.kb_per_split = (a.kb_total + plan.split_k - 1) / plan.split_k;
   a.status = device_status_word();
   FML_REQUIRE(a.status, FML_CUDA_ERROR, "fml_gemm: no device status word");
-  CUtensorMap map_a;
-  int st = make_gemm_map(&map_a, p.a, p.K, p.M, p.a_sm, p.nb0, p.a_b0, p.nb1, p.a_b1, 32, kBM, CU_TENSOR_MAP_SWIZZLE_128B);
+  CUtensorMap map_a, map_a2;
+  int st = make_gemm_map(&map_a, p.a, x.a2 ? x.k1 : p.K, p.M, p.a_sm, p.nb0, p.a_b0, p.nb1, p.a_b1, 32, kBM, CU_TENSOR_MAP_SWIZZLE_128B);
   if (st != FML_OK) return st;
-  using KernelFn = void (*)(const CUtensorMap, const PairArgs);
-  static const KernelFn kernels[6] = {gemm_pair_kernel<FML_ACT_NONE>, gemm_pair_kernel<FML_ACT_GELU_ERF>, gemm_pair_kernel<FML_ACT_RELU>,
-                                      gemm_pair_kernel<FML_ACT_TANH>, gemm_pair_kernel<FML_ACT_SIGMOID>, gemm_pair_kernel<FML_ACT_SILU>};
+  map_a2 = map_a;
+  if (x.a2) {
+    st = make_gemm_map(&map_a2, x.a2, p.K - x.k1, p.M, x.a2_sm, p.nb0, x.a2_b0, p.nb1, x.a2_b1, 32, kBM, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (st != FML_OK) return st;
+  }
+  using KernelFn = void (*)(const CUtensorMap, const CUtensorMap, const PairArgs);
+  static const KernelFn kernels[9] = {gemm_pair_kernel<FML_ACT_NONE, kPlain>, gemm_pair_kernel<FML_ACT_GELU_ERF, kPlain>, gemm_pair_kernel<FML_ACT_RELU, kPlain>,
+                                      gemm_pair_kernel<FML_ACT_TANH, kPlain>, gemm_pair_kernel<FML_ACT_SIGMOID, kPlain>, gemm_pair_kernel<FML_ACT_SILU, kPlain>,
+                                      gemm_pair_kernel<FML_ACT_NONE, kProj>, gemm_pair_kernel<FML_ACT_GELU_ERF, kProj>, gemm_pair_kernel<FML_ACT_NONE, kTwoA>};
   FML_REQUIRE(e.act >= 0 && e.act <= FML_ACT_SILU, FML_BAD_ARG, "fml_gemm: unknown activation %d", e.act);
+  FML_REQUIRE(mode == kPlain || e.act == FML_ACT_NONE || (mode == kProj && e.act == FML_ACT_GELU_ERF), FML_UNSUPPORTED, "fml_gemm: activation %d in a joined product", e.act);
+  const KernelFn kernel = kernels[mode == kPlain ? e.act : mode == kTwoA ? 8 : e.act == FML_ACT_NONE ? 6 : 7];
   static bool attr_set[64] = {false};
   int dev = 0;
   FML_CUDA(cudaGetDevice(&dev));
@@ -621,8 +672,8 @@ int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const PairPlan
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  FML_CUDA(cudaLaunchKernelEx(&cfg, kernels[e.act], map_a, a));
-  return FML_OK;
+  FML_CUDA(cudaLaunchKernelEx(&cfg, kernel, map_a, map_a2, a));
+  return x.rot && !rotates ? launch_rotary_in_place(p, x, s) : FML_OK;
 }
 
 }  // namespace fml

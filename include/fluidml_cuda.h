@@ -325,6 +325,19 @@ typedef struct fml_gemm_params {
    * on the 16-bit tensor-core path at half the cost of 3xTF32.  NULL = not packed. */
   const void *b_packed;
   int32_t ctas_per_sm; /* tuning choice that goes with tile_n (packed B only); 0 = library    */
+  /* Several projections of the same rows in one product, their weights side by side in B:
+   * the activation is applied to columns act_from .. N - 1 only (0 = all of them). */
+  int32_t act_from;
+  /* Rotary position embedding of columns 0 .. rot_cols - 1, heads of rot_head columns of which the first
+   * `rot` are rotated, after bias and before anything else: fml_rotary's arithmetic with cos / sin row
+   * (m mod rot_len) of the constant tables [rot_len, rot].  rot 0 = none.  The rotated columns lie below
+   * act_from or there is no activation; no residual. */
+  int32_t rot, rot_head, rot_cols, rot_len;
+  const float *rot_cos, *rot_sin;
+  /* [A | A2] * B: the columns of A followed by those of A2 (data NULL = none; the same shape but for the last
+   * dim).  No activation, divisor, alpha or beta.  What the packed path does not take in one launch runs as
+   * two or more products (act_from, a2) or as a product and a rotation in place. */
+  fml_tensor a2;
 } fml_gemm_params;
 
 /* Packs a constant right-hand side [K, N] (any strides) for fml_gemm_params::b_packed: about 4 bytes

@@ -1,0 +1,179 @@
+"""Products joined into one launch: several projections side by side (rotation of the first columns, activation of the
+last) and two left-hand sides, against fp64 and against the parts run one by one; and the rewrites that make them.
+
+Tolerance 2e-5 of the largest magnitude, as for every product of the packed-weight kernel (operands of 22 bits,
+fp32 accumulation in chunks); a rotation or a GELU of it adds two roundings.
+"""
+import math
+
+import numpy as np
+import pytest
+
+from fluidml_b200 import cabi, models
+from fluidml_b200.cabi import DeviceTensor as DT
+from fluidml_b200.executor import Executor
+from fluidml_b200.onnx_lite import FLOAT
+
+TOL = 2e-5
+erf = np.vectorize(math.erf)
+
+
+def close(got, ref):
+    return np.abs(got.astype(np.float64) - ref).max() <= TOL * np.abs(ref).max()
+
+
+def params(b, packed, **kw):
+    p = cabi.gemm_params(act=kw.pop("act", cabi.ACT_NONE), tile_n=kw.pop("tile", 0), split_k=kw.pop("split", 0))
+    blob = cabi.gemm_pack(b) if packed else None
+    if packed:
+        p.b_constant, p.b_packed = 1, blob.ptr
+    for k, v in kw.items():
+        setattr(p, k, v)
+    return p, blob
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 31, 32, 33, 128, 129, 300])
+@pytest.mark.parametrize("k1,k2", [(32, 32), (64, 20), (96, 160), (1024, 256), (40, 64)])
+@pytest.mark.parametrize("n,tile,split", [(16, 0, 0), (96, 32, 2), (200, 256, 1), (768, 128, 8), (130, 64, 4)])
+def test_two_left_hand_sides(m, k1, k2, n, tile, split):
+    rng = np.random.default_rng(m * 7 + k1 + n)
+    a1, a2 = rng.standard_normal((m, k1)).astype(np.float32), rng.standard_normal((m, k2)).astype(np.float32)
+    a2[:: 3] *= 1e-3          # rows whose parts differ in magnitude,
+    a2[1:: 4] *= 3e4          # and rows whose second part outgrows the scale of the first
+    b, bias, res = (rng.standard_normal(s).astype(np.float32) for s in ((k1 + k2, n), (n,), (m, n)))
+    ref = np.concatenate([a1, a2], 1).astype(np.float64) @ b + bias + res
+    db, c = DT.from_numpy(b), DT((m, n), np.float32)
+    wide = DT.from_numpy(np.concatenate([np.ones((m, 4), np.float32), a2], 1))  # a view with a row stride of its own
+    a2v = wide.view((m, k2), [k2 + 4, 1], 4)
+    for packed in (True, False):
+        p, blob = params(db, packed, tile=tile if packed else 0, split=split if packed else 0)
+        p.a2 = a2v.c()
+        cabi.gemm(DT.from_numpy(a1), db, c, DT.from_numpy(bias), DT.from_numpy(res), p)
+        cabi.check_device()
+        rows = np.abs(ref).max(1, keepdims=True)  # each row by its own magnitude
+        assert (np.abs(c.numpy() - ref) <= TOL * np.maximum(rows, 1.0)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,length", [(1, 5), (1, 32), (3, 77), (2, 128)])
+@pytest.mark.parametrize("heads,size,rot", [(2, 64, 16), (3, 32, 32), (2, 64, 64), (2, 48, 12), (4, 16, 8)])
+@pytest.mark.parametrize("tile,split", [(0, 0), (16, 1), (48, 2), (96, 4), (256, 8)])
+def test_projections_side_by_side(batch, length, heads, size, rot, tile, split):
+    """[Q | K | V | GELU(F)] of the same rows: rotated, plain and activated columns."""
+    rng = np.random.default_rng(batch * 1000 + length + size)
+    m, k, h, ffn = batch * length, 256, heads * size, 80
+    a = rng.standard_normal((m, k)).astype(np.float32)
+    b, bias = (rng.standard_normal((k, 3 * h + ffn)) * 0.1).astype(np.float32), rng.standard_normal(3 * h + ffn).astype(np.float32)
+    ang = rng.standard_normal((length, rot))
+    cos, sin = np.cos(ang).astype(np.float32), np.sin(ang).astype(np.float32)
+    y = a.astype(np.float64) @ b + bias
+    qk = y[:, :2 * h].reshape(batch, length, 2 * heads, size)
+    x = qk[..., :rot].copy()
+    half = np.concatenate([-x[..., rot // 2:], x[..., :rot // 2]], -1)
+    qk[..., :rot] = x * cos[None, :, None] + half * sin[None, :, None]
+    f = y[:, 3 * h:]
+    ref = np.concatenate([qk.reshape(m, 2 * h), y[:, 2 * h:3 * h], f * (erf(f / np.sqrt(2.0)) + 1) * 0.5], 1)
+    db, c, dc, ds = DT.from_numpy(b), DT((m, 3 * h + ffn), np.float32), DT.from_numpy(cos), DT.from_numpy(sin)
+    for packed in (True, False):
+        p, blob = params(db, packed, act=cabi.ACT_GELU_ERF, tile=tile if packed else 0, split=split if packed else 0, act_from=3 * h, rot=rot, rot_head=size,
+                         rot_cols=2 * h, rot_len=length, rot_cos=dc.c().data, rot_sin=ds.c().data)
+        cabi.gemm(DT.from_numpy(a), db, c, DT.from_numpy(bias), None, p)
+        cabi.check_device()
+        assert close(c.numpy(), ref)
+
+
+def refused(a, b, c, **kw):
+    p = cabi.gemm_params(act=kw.pop("act", cabi.ACT_NONE))
+    for k, v in kw.items():
+        setattr(p, k, v)
+    with pytest.raises(cabi.FmlError):
+        cabi.gemm_plan(a, b, c, p)
+
+
+class Host:
+    """A tensor of host memory: planning looks at shapes, strides and addresses only."""
+    def __init__(self, *shape):
+        self.array = np.zeros(shape, np.float32)
+        self.shape = shape
+
+    def c(self):
+        t = cabi.Tensor()
+        t.data, t.dtype, t.rank = self.array.ctypes.data, cabi.F32, len(self.shape)
+        for i, (s, st) in enumerate(zip(self.shape, self.array.strides)):
+            t.shape[i], t.stride[i] = s, st // 4
+        return t
+
+
+def test_what_does_not_chain_is_refused():
+    a, b, c, a2, t = Host(64, 32), Host(96, 48), Host(64, 48), Host(64, 64), Host(64, 16)
+    rot = dict(rot=16, rot_head=16, rot_cols=32, rot_len=64, rot_cos=t.array.ctypes.data, rot_sin=t.array.ctypes.data)
+    refused(a, b, c, a2=Host(64, 60).c())                      # columns do not add up
+    refused(a, b, c, a2=Host(63, 64).c())                      # other rows
+    refused(a, b, c, a2=a2.c(), act=cabi.ACT_RELU)
+    refused(a, b, c, a2=a2.c(), alpha=2.0)
+    a = Host(64, 96)
+    refused(a, b, c, act_from=48, act=cabi.ACT_GELU_ERF)       # no such column
+    refused(a, b, c, act=cabi.ACT_GELU_ERF, **rot)             # an activation on rotated columns
+    refused(a, b, c, **{**rot, "rot_cols": 40})                # part of a head
+    refused(a, b, c, **{**rot, "rot_len": 60})                 # rows are no multiple of the tables'
+    refused(a, b, c, **{**rot, "rot_cos": None})
+    cabi.gemm_plan(a, b, c, cabi.gemm_params())
+
+
+def block(m, gamma_seed, rows=2):
+    """Two LayerNorms of x with scales and shifts of their own: (x + gelu(ln2(x) W1 + b1) W2) + ln1(x) W3."""
+    rng = np.random.default_rng(gamma_seed)
+    g = models.GraphBuilder("block")
+    x = g.input("x", FLOAT, (rows, m, 64))
+    f32 = lambda *s, scale=0.1: (rng.standard_normal(s) * scale).astype(np.float32)
+    ln = lambda i: g.layernorm(x, g.const(f"g{i}", 1 + f32(64, scale=0.5)), g.const(f"b{i}", f32(64, scale=0.5)), -1, 1e-5)
+    h1, h2 = ln(1), ln(2)
+    f = g.add(g.const("c1", f32(96)), g.matmul(h2, g.const("w1", f32(64, 96))))
+    e = g.erf(g.div(f, g.scalar(math.sqrt(2.0))))
+    f = g.mul(g.mul(f, g.add(e, g.scalar(1.0))), g.scalar(0.5))
+    f = g.matmul(f, g.const("w2", f32(96, 64)))
+    a = g.add(g.const("c3", f32(64)), g.matmul(h1, g.const("w3", f32(64, 64))))
+    g.add(g.add(a, f), x, out="y")
+    g.output("y")
+    return g.finish()
+
+
+def test_a_parallel_block_is_three_launches():
+    kinds = [n["kind"] for n in Executor.make_plain_greedy("t").plan(block(40, 0).to_bytes())["sequence"]]
+    assert kinds.count("LayerNormalizationConstantScaleBias") == 1 and kinds.count("FusedGemm") == 2
+    few = [n["kind"] for n in Executor.make_plain_greedy("t").plan(block(5, 0).to_bytes())["sequence"]]
+    assert few.count("FusedGemm") == 3 and few.count("LayerNormalizationConstantScaleBias") == 2  # ten rows: as before
+    exact = [n["kind"] for n in Executor.make_plain_greedy("t").set_option("gemm_precision", "fp32").plan(block(40, 0).to_bytes())["sequence"]]
+    assert exact.count("FusedGemm") == 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [5, 16, 17, 77])
+@pytest.mark.parametrize("make", [Executor.make_dp_greedy, Executor.make_plain_greedy])
+def test_a_parallel_block_against_the_oracle(m, make):
+    from oracle import oracle as orc
+    model = block(m, m)
+    x = {"x": np.random.default_rng(1).standard_normal((2, m, 64)).astype(np.float32)}
+    out = {"y": np.zeros((2, m, 64), np.float32)}
+    make("t").compile(model.to_bytes()).invoke({**x, **out})
+    assert close(out["y"], orc.run_model(model, x, acc64=True)["y"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k1,k2", [(32, 64), (96, 20), (20, 64)])
+@pytest.mark.parametrize("m", [3, 40, 140])
+def test_a_concatenation_in_front_of_a_product(k1, k2, m):
+    from oracle import oracle as orc
+    rng = np.random.default_rng(k1 + m)
+    g = models.GraphBuilder("cat")
+    a, b = g.input("a", FLOAT, (m, k1)), g.input("b", FLOAT, (m, k2))
+    w = g.const("w", rng.standard_normal((k1 + k2, 48)).astype(np.float32))
+    g.matmul(g.concat(g.relu(a), g.relu(b), 1), w, out="y")
+    g.output("y")
+    model = g.finish()
+    x = {"a": rng.standard_normal((m, k1)).astype(np.float32), "b": rng.standard_normal((m, k2)).astype(np.float32)}
+    out = {"y": np.zeros((m, 48), np.float32)}
+    ex = Executor.make_dp_greedy("t").compile(model.to_bytes())
+    ex.invoke({**x, **out})
+    assert close(out["y"], orc.run_model(model, x, acc64=True)["y"])
