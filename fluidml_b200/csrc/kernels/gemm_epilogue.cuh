@@ -17,14 +17,19 @@ namespace fml {
 // i.e. a GELU value off by at most 5e-7 |v| -- far below the 3xTF32 product it is applied to.
 // The exact erff is ~45 dependent instructions per element; with one epilogue warp per scheduler
 // that was 35 us of a 134 us FFN launch at 2048 rows (4096 columns each).
+// The reciprocal and the exponential in their flushing forms: the reciprocal's argument is at least 1 and an exponential
+// below 2^-126 vanishes beside 1, so the values are those of __fdividef and __expf without the instructions that look after
+// denormals (1024 x 768 x 3072 in tiles of 192 with GELU 22.3 -> 20.8 us).
 __device__ __forceinline__ float erf_fast(float x) {
   const float ax = fabsf(x);
-  const float t = __fdividef(1.0f, fmaf(0.3275911f, ax, 1.0f));
+  float t, g;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.3275911f, ax, 1.0f)));
   float p = fmaf(1.061405429f, t, -1.453152027f);
   p = fmaf(p, t, 1.421413741f);
   p = fmaf(p, t, -0.284496736f);
   p = fmaf(p, t, 0.254829592f);
-  return copysignf(fmaf(-p * t, __expf(-ax * ax), 1.0f), x);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(-ax * ax * 1.4426950408889634f));
+  return copysignf(fmaf(-p * t, g, 1.0f), x);
 }
 
 template <int ACT>
