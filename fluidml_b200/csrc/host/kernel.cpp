@@ -663,12 +663,15 @@ private:
 fml_conv_params TuneConv(const char *name, const fml_tensor &x, const fml_tensor *scale, const fml_tensor &w, const fml_tensor *bias,
                          const fml_tensor *res, const fml_tensor &y, const fml_conv_params &p, bool autotune) {
   fml_conv_params tuned = p;
+  int prefers = 0;
+  if (p.tile_n == 0 && (!autotune || !p.w_packed) && fml_conv_prefers_fma(&x, &w, &y, &p, scale != nullptr, &prefers) == FML_OK) tuned.pointwise_fma = prefers;
   if (autotune && p.w_packed && fml_conv_autotune_residual(&x, scale, &w, bias, res, &y, &p, nullptr, &tuned) != FML_OK)
     throw Error(std::string(name) + ": " + fml_last_error());
   return tuned;
 }
 void PresetConvTiles(const GemmTiles &t, fml_conv_params *p) {
   p->tile_n = t.tile_n; p->split_k = t.split_k; p->ctas_per_sm = t.ctas_per_sm; p->strips = t.strips;
+  p->pointwise_fma = t.strips < 0 ? 1 : 0;  // (what fml_conv_autotune reports for the FMA kernel)
 }
 bool TunedConvTiles(const fml_conv_params &p, GemmTiles *t) {
   if (p.tile_n <= 0) return false;

@@ -662,6 +662,8 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
   const int64_t M = a.N * a.OH * a.OW;
   if (M == 0 || a.OC == 0) return FML_OK;
   cudaStream_t s = as_stream(stream);
+  if (double us; p->pointwise_fma && nd == 2 && a.IH * a.IW > 1 && pointwise_fma_plan(x, w, y, p, a.scale != nullptr, &us))
+    return launch_pointwise_fma(x, w, bias, y, p, s, a.scale, a.scale_sn, a.scale_sc, residual);
   if (a.scale) {
     // the tensor-core kernel applies the scale while it splits the operand; every other case
     // takes the general implicit GEMM (the specialised CUDA-core paths below read x unscaled)
@@ -832,6 +834,8 @@ extern "C" int fml_conv_residual(const fml_tensor *x, const fml_tensor *x_scale,
   bool same = false;  // then the packed-weight kernel adds it in its epilogue
   if (const int rs = residual_laid_out_as(residual, y, &same); rs != FML_OK) return rs;
   int uses = 0;
+  if (double us; same && p->pointwise_fma && pointwise_fma_plan(x, w, y, p, x_scale != nullptr, &us))
+    return conv_impl(x, x_scale, w, bias, y, p, stream, (const float *)residual->data);
   if (same && y->rank == 4 && p->w_packed) {
     const int st = fml_conv_uses_packed(x, w, y, p, x_scale != nullptr, &uses);
     if (st != FML_OK) return st;
@@ -854,6 +858,7 @@ extern "C" int fml_conv_uses_tensor_cores(const fml_tensor *x, const fml_tensor 
 extern "C" int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p,
                                     int scaled, int *uses) {
   FML_REQUIRE(valid_tensor(x) && valid_tensor(w) && valid_tensor(y) && p && uses, FML_BAD_ARG, "fml_conv_uses_packed: bad argument");
+  if (double us; p->pointwise_fma && pointwise_fma_plan(x, w, y, p, scaled != 0, &us)) { *uses = 0; return FML_OK; }
   if (Planes pl; !scaled && as_planes(x, w, y, p, &pl)) {
     const fml_conv_params q = plane_params(p);
     *uses = x->dtype == FML_F32 && w->dtype == FML_F32 && y->dtype == FML_F32 && conv_pair_eligible(&pl.x, &pl.w, &pl.y, &q, false) ? 1 : 0;
@@ -863,6 +868,13 @@ extern "C" int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, co
                   p->group <= 1 && x->shape[2] * x->shape[3] > 1 && (!scaled || x->shape[1] <= 4096) &&
                   conv_pair_eligible(x, w, y, p, scaled != 0)
               ? 1 : 0;
+  return FML_OK;
+}
+
+extern "C" int fml_conv_prefers_fma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int scaled, int *prefers) {
+  FML_REQUIRE(valid_tensor(x) && valid_tensor(w) && valid_tensor(y) && p && prefers, FML_BAD_ARG, "fml_conv_prefers_fma: bad argument");
+  double us;
+  *prefers = pointwise_fma_plan(x, w, y, p, scaled != 0, &us) && (us < 6.0 || !conv_pair_eligible(x, w, y, p, scaled != 0)) ? 1 : 0;
   return FML_OK;
 }
 
@@ -881,13 +893,13 @@ extern "C" int fml_conv_autotune_residual(const fml_tensor *x, const fml_tensor 
   if (Planes pl; !x_scale && as_planes(x, w, y, p, &pl)) {
     const fml_conv_params q = plane_params(p);
     fml_conv_params t = q;
-    const int ts = tune_conv_pair(&pl.x, &pl.w, bias, &pl.y, &q, nullptr, 0, 0, nullptr, &t);
+    const int ts = tune_conv_pair(&pl.x, &pl.w, bias, &pl.y, &q, nullptr, 0, 0, nullptr, false, &t);
     tuned->tile_n = t.tile_n; tuned->strips = t.strips; tuned->split_k = t.split_k; tuned->ctas_per_sm = t.ctas_per_sm;
     return ts;
   }
   return tune_conv_pair(x, w, bias, y, p, x_scale ? (const float *)x_scale->data : nullptr,
                         x_scale && x_scale->shape[0] != 1 ? x_scale->stride[0] : 0, x_scale && x_scale->shape[1] != 1 ? x_scale->stride[1] : 0,
-                        same ? (const float *)residual->data : nullptr, tuned);
+                        same ? (const float *)residual->data : nullptr, !residual || same, tuned);
 }
 
 extern "C" int fml_conv_autotune(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,

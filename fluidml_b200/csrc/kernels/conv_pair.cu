@@ -1076,15 +1076,16 @@ std::string conv_tuning_key(int device, const fml_tensor *x, const fml_tensor *w
 // Times the candidates the model ranks highest as captured graphs of back-to-back launches and keeps the
 // fastest, per device and problem signature (as fml_gemm_autotune).
 int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
-                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, fml_conv_params *tuned) {
+                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, bool pointwise_fma, fml_conv_params *tuned) {
   int device = 0;
   FML_CUDA(cudaGetDevice(&device));
   const std::string key = conv_tuning_key(device, x, w, y, p, x_scale != nullptr, residual != nullptr);
-  struct Choice { int tile_n, strips, split_k, occ; };
+  struct Choice { int tile_n, strips, split_k, occ, fma; };
   static std::map<std::string, Choice> cache;
   static std::mutex mu;
   auto take = [&](const Choice &c) {
     tuned->tile_n = c.tile_n; tuned->strips = c.strips; tuned->split_k = c.split_k; tuned->ctas_per_sm = c.occ;
+    tuned->pointwise_fma = c.fma;
   };
   {
     std::lock_guard<std::mutex> lock(mu);
@@ -1099,9 +1100,19 @@ int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
   FML_CUDA(cudaEventCreate(&e0));
   FML_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
-  const Candidate *chosen = &all[0];
-  for (size_t i = 0; i < all.size() && i < 16; ++i) {
-    auto launch = [&] { return launch_planned(all[i].a, all[i].smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc, residual); };
+  Choice c{all[0].a.tile_n, all[0].a.mt, all[0].a.split_k, all[0].occ, 0};
+  // a pointwise layer with little arithmetic: the FMA kernel's splits too (conv_pointwise.cu)
+  static const int fma_splits[][2] = {{1, 1}, {2, 1}, {4, 1}, {8, 1}, {8, 2}, {8, 4}, {8, 8}};
+  double fma_us = 0.0;
+  const bool fma = pointwise_fma && pointwise_fma_plan(x, w, y, p, x_scale != nullptr, &fma_us) && fma_us < 24.0;
+  const size_t pairs = std::min<size_t>(all.size(), 16);
+  for (size_t i = 0; i < pairs + (fma ? 7 : 0); ++i) {
+    fml_conv_params q = *p;
+    if (i >= pairs) { q.pointwise_fma = 1; q.tile_n = fma_splits[i - pairs][0]; q.split_k = fma_splits[i - pairs][1]; }
+    auto launch = [&] {
+      return i < pairs ? launch_planned(all[i].a, all[i].smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc, residual)
+                       : launch_pointwise_fma(x, w, bias, y, &q, s, x_scale, x_scale_sn, x_scale_sc, residual);
+    };
     float one = 0;
     bool ok = launch() == FML_OK;  // warm-up
     cudaEventRecord(e0, s);
@@ -1129,12 +1140,14 @@ int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
     }
     if (exec) cudaGraphExecDestroy(exec);
     if (!ok) { cudaGetLastError(); continue; }
-    if (ms < best) { best = ms; chosen = &all[i]; }
+    if (ms < best) {
+      best = ms;
+      c = i < pairs ? Choice{all[i].a.tile_n, all[i].a.mt, all[i].a.split_k, all[i].occ, 0} : Choice{q.tile_n, -1, q.split_k, 0, 1};
+    }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaStreamDestroy(s);
-  const Choice c{chosen->a.tile_n, chosen->a.mt, chosen->a.split_k, chosen->occ};
   take(c);
   std::lock_guard<std::mutex> lock(mu);
   cache[key] = c;

@@ -109,6 +109,11 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
                    const fml_conv_params *p, cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0,
                    int64_t x_scale_sc = 0);
 
+// pointwise convolution in fp32 FMA (conv_pointwise.cu): whether it takes the layer, with the microseconds its model gives
+bool pointwise_fma_plan(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled, double *us);
+int launch_pointwise_fma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p, cudaStream_t s,
+                         const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual);
+
 // half-precision-pair convolution with packed weights (conv_pair.cu)
 bool conv_pair_eligible(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool has_scale);
 size_t conv_packed_bytes(const fml_tensor *w);
@@ -118,7 +123,7 @@ int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor 
                      cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0, int64_t x_scale_sc = 0,
                      const float *residual = nullptr);
 int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
-                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, fml_conv_params *tuned);
+                   const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, bool pointwise_fma, fml_conv_params *tuned);
 std::string conv_tuning_key(int device, const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled,
                             bool residual);
 

@@ -409,7 +409,15 @@ typedef struct fml_conv_params {
    * fml_conv_uses_packed accepts: half-precision-pair products as with fml_gemm_params::b_packed. */
   const void *w_packed;
   int32_t tile_n, strips, split_k, ctas_per_sm; /* tuning choices with packed weights; 0 = library */
+  /* Non-zero: a pointwise layer that the fp32 FMA kernel takes (2-D, unit strides, dense planes, weights with the
+   * output channels innermost, a multiple of 4 of them) runs there, whatever w_packed says; tile_n = slices of k
+   * among the warps of a CTA and split_k = CTAs per tile may then be given.  See fml_conv_prefers_fma. */
+  int32_t pointwise_fma;
 } fml_conv_params;
+
+/* Whether pointwise_fma is the faster choice for this layer (scaled: with the gate of fml_conv_scaled): little
+ * arithmetic, where the tensor-core kernel's fixed phases are most of its time.  Pure host computation. */
+int fml_conv_prefers_fma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int scaled, int *prefers);
 
 /* Packs constant weights [OC, IC, KH, KW] (any strides) for fml_conv_params::w_packed. */
 size_t fml_conv_packed_bytes(const fml_tensor *w);
