@@ -303,6 +303,7 @@ private:
     kernel::KernelOptions ko;
     ko.gemm_precision = options_.gemm_precision;
     const AliasMap aliases = Lowering::ComputeAliases(sequence, ko);
+    Lowering::AttachPlaneSums(sequence, aliases, ko);
     Lowering::ComputeScratch(sequence, ko);
     const std::vector<memory::Info> infos = Lowering::Lifetimes(sequence, aliases);
     const memory::Index index = Planner::Plan(infos, plan_, options_.alignment);

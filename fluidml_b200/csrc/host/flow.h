@@ -70,6 +70,7 @@ struct Node {
   // condition / y, Conv weights / bias, embedding addends, fused bias.
   std::vector<RegionPtr> consts;
   RegionPtr output;
+  RegionPtr side_output;  // Conv: the sums of the output's planes, for the SqueezeExciteGate that reads them as its inputs[1] (Lowering::AttachPlaneSums)
 
   // parameters (which ones are meaningful depends on the kind)
   Type scalar_type = Type::kFloat32;

@@ -264,16 +264,19 @@ public:
 
 // ReduceMean over H, W -> 1 x 1 Conv -> 1 x 1 Conv (the gate of a squeeze-and-excite block) in one
 // launch (reduce_mean.cpp + conv.cpp twice in the reference)
-class SqueezeExciteGateKernel : public SingleInputWithoutBufferKernel {
+class SqueezeExciteGateKernel : public Kernel {
 public:
   SqueezeExciteGateKernel(fml_tensor w1, bool has_b1, fml_tensor b1, fml_tensor w2, bool has_b2, fml_tensor b2, int act1, int act2)
       : w1_(w1), b1_(b1), w2_(w2), b2_(b2), has_b1_(has_b1), has_b2_(has_b2), act1_(act1), act2_(act2) {}
   std::string GetKernelName() const override { return "SqueezeExciteGateKernel"; }
-  void Run(LaunchRecorder &rec, const fml_tensor &input, const fml_tensor &output) const override {
-    const fml_tensor w1 = w1_, b1 = b1_, w2 = w2_, b2 = b2_;
-    const bool hb1 = has_b1_, hb2 = has_b2_;
+  void Launch(LaunchRecorder &rec, const std::vector<fml_tensor> &in, const fml_tensor &output, const Buffer &) const override {
+    const fml_tensor input = in.at(0), w1 = w1_, b1 = b1_, w2 = w2_, b2 = b2_;
+    const bool hb1 = has_b1_, hb2 = has_b2_, from_sums = in.size() > 1;  // inputs[1]: the sums of the planes (Lowering::AttachPlaneSums)
+    const fml_tensor sums = from_sums ? in.at(1) : fml_tensor{};
     const int a1 = act1_, a2 = act2_;
     rec.Add(GetKernelName(), [=](void *s) {
+      if (from_sums)
+        return fml_squeeze_excite_gate_from_sums(&sums, input.shape[2] * input.shape[3], &w1, hb1 ? &b1 : nullptr, &w2, hb2 ? &b2 : nullptr, a1, a2, &output, s);
       return fml_squeeze_excite_gate(&input, &w1, hb1 ? &b1 : nullptr, &w2, hb2 ? &b2 : nullptr, a1, a2, &output, s);
     });
   }
@@ -694,13 +697,19 @@ public:
   }
   int Pack(const fml_tensor &source, void *packed, size_t bytes) const override { return fml_conv_pack(&source, packed, bytes, nullptr); }
   void SetPacked(const void *packed, size_t) override { p_.w_packed = packed; }
+  int PlaneSumParts(const std::vector<fml_tensor> &in, const fml_tensor &output) const override {
+    int parts = 0;
+    if (has_scale_ || has_residual_ || fml_conv_plane_sum_parts(&in.at(0), &w_, &output, &p_, &parts) != FML_OK) return 0;
+    return parts;
+  }
   void PresetTiles(const GemmTiles &t) override { PresetConvTiles(t, &p_); }
   bool TunedTiles(GemmTiles *t) const override { return TunedConvTiles(tuned_, t); }
-  void Launch(LaunchRecorder &rec, const std::vector<fml_tensor> &in, const fml_tensor &output, const Buffer &) const override {
+  void Launch(LaunchRecorder &rec, const std::vector<fml_tensor> &in, const fml_tensor &output, const Buffer &sums) const override {
     const fml_tensor x = in.at(0), w = w_, b = bias_;
     const fml_tensor scale = has_scale_ ? in.at(1) : fml_tensor{}, res = has_residual_ ? in.back() : fml_tensor{};
     const bool hb = has_bias_, hs = has_scale_, hr = has_residual_;
-    const fml_conv_params p = tuned_ = TuneConv(name_, x, hs ? &scale : nullptr, w, hb ? &b : nullptr, hr ? &res : nullptr, output, p_, autotune_);
+    fml_conv_params p = tuned_ = TuneConv(name_, x, hs ? &scale : nullptr, w, hb ? &b : nullptr, hr ? &res : nullptr, output, p_, autotune_);
+    p.plane_sums = (float *)sums.data;
     rec.Add(name_, [=](void *s) {
       const fml_tensor *bias = hb ? &b : nullptr;
       if (hr) return fml_conv_residual(&x, hs ? &scale : nullptr, &w, bias, &res, &output, &p, s);

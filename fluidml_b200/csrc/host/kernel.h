@@ -56,6 +56,12 @@ public:
     (void)output;
     return 0;
   }
+  // Partial sums per output plane that the kernel can leave in the buffer it is launched with (a depthwise convolution in
+  // front of a squeeze-and-excite gate); 0 = none.
+  virtual int PlaneSumParts(const std::vector<fml_tensor> &inputs, const fml_tensor &output) const {
+    (void)inputs; (void)output;
+    return 0;
+  }
   // When the output is just another way of addressing the input's bytes (a reshape that
   // splits or merges contiguous dims, a transpose, a slice), fills `view` with the output's
   // shape and the strides / data pointer that realise it over `input`, and returns true: the

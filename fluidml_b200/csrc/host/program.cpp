@@ -90,6 +90,33 @@ void Lowering::ComputeScratch(const flow::Sequence &sequence, const kernel::Kern
   }
 }
 
+void Lowering::AttachPlaneSums(flow::Sequence &sequence, const AliasMap &aliases, const kernel::KernelOptions &ko) {
+  const kernel::ConstResolver resolve = PlaceholderResolver();
+  std::unordered_map<const flow::Region *, flow::NodePtr> producer;
+  for (const auto &node : sequence.nodes) producer[node->output.get()] = node;
+  for (const auto &gate : sequence.nodes) {
+    if (gate->kind != flow::Kind::SqueezeExciteGate || gate->inputs.size() != 1) continue;
+    const flow::RegionPtr x = gate->inputs[0];
+    auto it = producer.find(x.get());
+    if (it == producer.end() || aliases.count(x.get()) || it->second->side_output) continue;
+    const flow::NodePtr &conv = it->second;
+    std::unique_ptr<kernel::Kernel> k = kernel::SelectKernel(*conv, resolve, ko);
+    std::vector<fml_tensor> ins;
+    for (const auto &r : conv->inputs) ins.push_back(kernel::MakeTensor(*r, kPlaceholder));
+    const int parts = k->PlaneSumParts(ins, kernel::MakeTensor(*x, kPlaceholder));
+    if (parts <= 0) continue;
+    const auto &shape = x->meta.GetShape();
+    auto sums = std::make_shared<flow::Region>();
+    sums->kind = flow::Region::kInner;
+    sums->name = conv->name + "_plane_sums";
+    sums->meta = Meta(Type::kFloat32, {shape[0], shape[1], (int64_t)parts});
+    sums->layout = utils::GenDefaultLayout(3);
+    sequence.regions.push_back(sums);
+    conv->side_output = sums;
+    gate->inputs.push_back(sums);
+  }
+}
+
 std::vector<memory::Info> Lowering::Lifetimes(const flow::Sequence &sequence, const AliasMap &aliases) {
   std::unordered_map<const flow::Region *, std::pair<size_t, size_t>> life;
   auto touch = [&](const flow::RegionPtr &r0, size_t i) {
@@ -102,6 +129,7 @@ std::vector<memory::Info> Lowering::Lifetimes(const flow::Sequence &sequence, co
   for (size_t i = 0; i < sequence.nodes.size(); ++i) {
     for (const auto &r : sequence.nodes[i]->inputs) touch(r, i);
     touch(sequence.nodes[i]->output, i);
+    if (sequence.nodes[i]->side_output) touch(sequence.nodes[i]->side_output, i);
   }
   std::vector<memory::Info> infos;
   for (const auto &r : sequence.regions) {
@@ -381,6 +409,10 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
     if (need > 0) {
       buf.data = (char *)prog->arena + index.Get(node->name);
       buf.bytes = node->buffer_size;
+    }
+    if (node->side_output) {
+      buf.data = base_of(node->side_output);
+      buf.bytes = node->side_output->meta.GetSize();
     }
     if (options.gemm_tiles) {
       auto it = options.gemm_tiles->find(node->name);

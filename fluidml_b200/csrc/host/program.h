@@ -55,6 +55,9 @@ public:
   // addresses: planned offsets are multiples of the alignment, so the real operands take the
   // same path.
   static void ComputeScratch(const flow::Sequence &sequence, const kernel::KernelOptions &ko);
+  // A depthwise convolution in front of a squeeze-and-excite gate, both over the same tensor, leaves the sums of its planes
+  // where its kernel can: a tensor of a few kilobytes with a place in the arena, the gate's second input.
+  static void AttachPlaneSums(flow::Sequence &sequence, const AliasMap &aliases, const kernel::KernelOptions &ko);
   // Lifetimes with aliases merged into their owners.
   static std::vector<memory::Info> Lifetimes(const flow::Sequence &sequence, const AliasMap &aliases);
 };

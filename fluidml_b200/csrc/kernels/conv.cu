@@ -632,6 +632,12 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
   a.ys[0] = y->stride[0]; a.ys[1] = y->stride[1]; a.ys[2] = nd == 2 ? y->stride[2] : 0; a.ys[3] = y->stride[nd + 1];
   a.x = (const float *)x->data; a.w = (const float *)w->data; a.y = (float *)y->data;
   a.bias = nullptr; a.bias_stride = 0;
+  if (p->plane_sums) {
+    int parts = 0;
+    const int ps = fml_conv_plane_sum_parts(x, w, y, p, &parts);
+    if (ps != FML_OK) return ps;
+    FML_REQUIRE(parts > 0, FML_UNSUPPORTED, "fml_conv: this layer's kernel leaves no plane sums");
+  }
   if (bias) {
     FML_REQUIRE(valid_tensor(bias) && bias->dtype == FML_F32 && numel(bias) == a.OC, FML_BAD_ARG,
                 "fml_conv: bias must hold one value per output channel");
@@ -868,6 +874,17 @@ extern "C" int fml_conv_uses_packed(const fml_tensor *x, const fml_tensor *w, co
                   p->group <= 1 && x->shape[2] * x->shape[3] > 1 && (!scaled || x->shape[1] <= 4096) &&
                   conv_pair_eligible(x, w, y, p, scaled != 0)
               ? 1 : 0;
+  return FML_OK;
+}
+
+extern "C" int fml_conv_plane_sum_parts(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int *parts) {
+  FML_REQUIRE(valid_tensor(x) && valid_tensor(w) && valid_tensor(y) && p && parts, FML_BAD_ARG, "fml_conv_plane_sum_parts: bad argument");
+  *parts = 0;
+  if (x->rank != 4 || w->rank != 4 || y->rank != 4 || x->dtype != FML_F32 || w->dtype != FML_F32 || y->dtype != FML_F32) return FML_OK;
+  const int64_t C = x->shape[1];
+  if (C < 2 || p->group != C || w->shape[0] != C || w->shape[1] != 1 || y->shape[1] != C || y->shape[0] != x->shape[0]) return FML_OK;
+  if (x->stride[1] == 1 && y->stride[1] == 1) return FML_OK;  // channel-innermost operands have kernels of their own
+  *parts = depthwise_sum_parts(x, w, y, p);
   return FML_OK;
 }
 

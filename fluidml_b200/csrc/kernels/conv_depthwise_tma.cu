@@ -47,6 +47,8 @@ struct DwTmaArgs {
   int64_t bias_stride;
   float *y;
   int64_t ys[4];
+  float *sums;             // [planes][row_tiles], or null
+  int sum_shift;
   int act;
   int *status;
 };
@@ -60,16 +62,40 @@ __device__ __forceinline__ float dwt_act(int act, float v) {
   default: return v;
   }
 }
+// Stores a row of a micro-tile; returns the sum of what it stored.
 template <int ACT>
-__device__ __forceinline__ void dwt_store_row(float *yp, const float *v, float bias, bool vec, int valid, int64_t ys3) {
+__device__ __forceinline__ float dwt_store_row(float *yp, const float *v, float bias, bool vec, int valid, int64_t ys3) {
+  const float r[4] = {dwt_act(ACT, v[0] + bias), dwt_act(ACT, v[1] + bias), dwt_act(ACT, v[2] + bias), dwt_act(ACT, v[3] + bias)};
   if (vec) {
-    *reinterpret_cast<float4 *>(yp) = make_float4(dwt_act(ACT, v[0] + bias), dwt_act(ACT, v[1] + bias),
-                                                  dwt_act(ACT, v[2] + bias), dwt_act(ACT, v[3] + bias));
-  } else {
-#pragma unroll
-    for (int o = 0; o < 4; ++o)
-      if (o < valid) yp[o * ys3] = dwt_act(ACT, v[o] + bias);
+    *reinterpret_cast<float4 *>(yp) = make_float4(r[0], r[1], r[2], r[3]);
+    return (r[0] + r[1]) + (r[2] + r[3]);
   }
+  float sum = 0.0f;
+#pragma unroll
+  for (int o = 0; o < 4; ++o)
+    if (o < valid) { yp[o * ys3] = r[o]; sum += r[o]; }
+  return sum;
+}
+// Plane sums of a tile, for the squeeze-and-excite gate behind the layer (it then reads a few kilobytes where it read the
+// whole tensor): threads of a plane are adjacent, `part` holds their sums; 2^shift lanes (about a quarter of a
+// plane's threads) add a plane's in a fixed order.  From the last warps down, so that the copies' issuer, thread 0, has
+// the least of it; a warp per plane whatever its size cost 4 to 10 us of a 35 to 60 us layer at 64 images, this 3 to 5;
+// the gate behind it saves 6 to 22.
+__device__ __forceinline__ void dwt_plane_sums(const float *part, int per_plane, int planes, int shift, float *dst, int64_t dst_step) {
+  const int u = kDwThreads - 1 - (int)threadIdx.x, lanes = 1 << shift, li = u & (lanes - 1);
+  for (int base = 0; base + ((u & ~31) >> shift) < planes; base += kDwThreads >> shift) {  // (whole warps)
+    const int pl = base + (u >> shift);
+    float s = 0.0f;
+    if (pl < planes)
+      for (int i = li; i < per_plane; i += lanes) s += part[pl * per_plane + i];
+    for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (pl < planes && li == 0) dst[pl * dst_step] = s;
+  }
+}
+inline int dwt_sum_shift(int per_plane) {
+  int shift = 0;
+  while (shift < 5 && (4 << shift) < per_plane) ++shift;
+  return shift;
 }
 __device__ __forceinline__ void dwt_tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2) {
   asm volatile(
@@ -89,6 +115,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_tma_kernel(const __
   __shared__ __align__(8) uint64_t bars[kDwMaxStages];
   const int NS = d.stages;
   __shared__ int abort_flag;
+  __shared__ float part[kDwThreads];
   const uint32_t stage_floats = (uint32_t)(d.PP * d.PH * d.PWt);
   const uint32_t stage_bytes = stage_floats * 4u;
   const uint32_t stage_pitch = (stage_bytes + 127u) & ~127u;  // a tensor-map copy lands on a 128-byte boundary
@@ -148,6 +175,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_tma_kernel(const __
     ok = __syncthreads_and(mbar_wait(smem_u32(&bars[stage]), ((uint32_t)(k / NS)) & 1u, &abort_flag) ? 1 : 0) != 0;
     if (!ok) break;
     if (tid == 0) consumed = k + 1;
+    float sum = 0.0f;
     if (active) {
       float acc[RT][4];
 #pragma unroll
@@ -182,7 +210,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_tma_kernel(const __
       switch (d.act) {  // one dispatch per thread, outside the store loops
 #define FML_DWT_ROWS(ACT)                                                                 \
   _Pragma("unroll") for (int rr = 0; rr < RT; ++rr)                                          \
-    if (rr < rows) dwt_store_row<ACT>(yp + rr * d.ys[2], acc[rr], bias, vec, valid, d.ys[3]);
+    if (rr < rows) sum += dwt_store_row<ACT>(yp + rr * d.ys[2], acc[rr], bias, vec, valid, d.ys[3]);
       case FML_ACT_RELU: FML_DWT_ROWS(FML_ACT_RELU) break;
       case FML_ACT_TANH: FML_DWT_ROWS(FML_ACT_TANH) break;
       case FML_ACT_SIGMOID: FML_DWT_ROWS(FML_ACT_SIGMOID) break;
@@ -191,7 +219,10 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_tma_kernel(const __
 #undef FML_DWT_ROWS
       }
     }
+    part[tid] = sum;
     __syncthreads();  // every thread has read this buffer: the copy after next may overwrite it
+    // (part is written again behind the next tile's barrier)
+    if (d.sums) dwt_plane_sums(part, per_plane, min(d.PP, d.planes - tile * d.PP), d.sum_shift, d.sums + (int64_t)tile * d.PP * d.row_tiles + band, d.row_tiles);
   }
   if (!ok) {
     // a bounded wait ran out: report it, and (thread 0) give the copies already issued a bounded
@@ -226,6 +257,8 @@ struct DwFlatArgs {
   int64_t bias_stride;
   float *y;
   int64_t ys[4];
+  float *sums;               // [planes], or null
+  int sum_shift;
   int act;
   int *status;
 };
@@ -243,6 +276,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_planes_kernel(const
   extern __shared__ __align__(128) uint8_t dwt_smem[];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ int abort_flag;
+  __shared__ float part[kDwThreads];
   const int HW = d.IH * d.IW;
   const uint32_t raw_pitch = ((uint32_t)(d.PP * HW) * 4u + 127u) & ~127u;
   uint8_t *smem = dwt_smem + ((128u - (smem_u32(dwt_smem) & 127u)) & 127u);
@@ -328,6 +362,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_planes_kernel(const
     // the previous tile's results have left shared memory before this tile's are written
     if (d.dense_y && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     __syncthreads();
+    float sum = 0.0f;
     if (active) {
       float acc[RT][4];
 #pragma unroll
@@ -361,7 +396,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_planes_kernel(const
         switch (d.act) {  // one dispatch per thread, outside the store loops
 #define FML_DWT_SROWS(ACT)                                                                \
   _Pragma("unroll") for (int rr = 0; rr < RT; ++rr)                                          \
-    if (rr < rows) dwt_store_row<ACT>(op + rr * d.OW, acc[rr], bias, false, valid, 1);
+    if (rr < rows) sum += dwt_store_row<ACT>(op + rr * d.OW, acc[rr], bias, false, valid, 1);
         case FML_ACT_RELU: FML_DWT_SROWS(FML_ACT_RELU) break;
         case FML_ACT_TANH: FML_DWT_SROWS(FML_ACT_TANH) break;
         case FML_ACT_SIGMOID: FML_DWT_SROWS(FML_ACT_SIGMOID) break;
@@ -375,7 +410,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_planes_kernel(const
         switch (d.act) {
 #define FML_DWT_ROWS(ACT)                                                                 \
   _Pragma("unroll") for (int rr = 0; rr < RT; ++rr)                                          \
-    if (rr < rows) dwt_store_row<ACT>(yp + rr * d.ys[2], acc[rr], bias, vec, valid, d.ys[3]);
+    if (rr < rows) sum += dwt_store_row<ACT>(yp + rr * d.ys[2], acc[rr], bias, vec, valid, d.ys[3]);
         case FML_ACT_RELU: FML_DWT_ROWS(FML_ACT_RELU) break;
         case FML_ACT_TANH: FML_DWT_ROWS(FML_ACT_TANH) break;
         case FML_ACT_SIGMOID: FML_DWT_ROWS(FML_ACT_SIGMOID) break;
@@ -385,6 +420,7 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_planes_kernel(const
         }
       }
     }
+    part[tid] = sum;
     __syncthreads();  // the patch may be rebuilt; the tile's results are complete
     if (d.dense_y && tid == 0) {
       const int count = min(d.PP, d.planes - item * d.PP);
@@ -393,8 +429,9 @@ __global__ void __launch_bounds__(kDwThreads) conv_depthwise_planes_kernel(const
                    ::"l"(d.y + (size_t)item * d.PP * OHW), "r"(smem_u32(out_s)), "r"((uint32_t)(count * OHW) * 4u) : "memory");
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
+    if (d.sums) dwt_plane_sums(part, per_plane, min(d.PP, d.planes - item * d.PP), d.sum_shift, d.sums + (int64_t)item * d.PP, 1);
   }
-  if (d.dense_y && tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // stores complete before the CTA leaves
+  if (d.dense_y && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory stays until the copies have read it
   if (!ok && tid == 0) {
     atomicOr(d.status, kStatusTimeout);
     abort_flag = 1;
@@ -423,15 +460,13 @@ int launch_planes_variant(const DwFlatArgs &d, size_t smem, cudaStream_t s) {
 // The narrow-plane variant: dense NCHW x on a 16-byte base, planes of at most 1024 elements that
 // fit one CTA's threads, a plane count that is a multiple of 4 (so that every copy is a multiple
 // of 16 bytes).
-bool launch_depthwise_planes(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,
-                             const fml_conv_params *p, cudaStream_t s, int *status) {
+bool plan_depthwise_planes(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, DwFlatArgs &d, size_t *smem) {
   const int64_t N = x->shape[0], C = x->shape[1], IH = x->shape[2], IW = x->shape[3];
   const int64_t OH = y->shape[2], OW = y->shape[3], KH = w->shape[2], KW = w->shape[3];
   const int64_t S = p->strides[0], HW = IH * IW;
   if (HW > 1024 || ((N * C) & 3) || N * C >= (1ll << 30)) return false;
   if (p->pads_begin[0] < 0 || p->pads_begin[0] > 8 || p->pads_begin[1] < 0 || p->pads_begin[1] > 8) return false;
   constexpr int RT = 4;
-  DwFlatArgs d;
   memset(&d, 0, sizeof(d));
   d.C = (int)C; d.IH = (int)IH; d.IW = (int)IW; d.OH = (int)OH; d.OW = (int)OW;
   d.ph = (int)p->pads_begin[0]; d.pw = (int)p->pads_begin[1];
@@ -456,6 +491,15 @@ bool launch_depthwise_planes(const fml_tensor *x, const fml_tensor *w, const fml
   };
   while (d.PP > 4 && smem_of() > 56 * 1024) d.PP -= 4;
   if (smem_of() > 100 * 1024 || (int64_t)d.PP * d.PH * d.PWn >= 65536) return false;
+  *smem = smem_of();
+  return true;
+}
+bool launch_depthwise_planes(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,
+                             const fml_conv_params *p, cudaStream_t s, int *status) {
+  const int64_t KH = w->shape[2], S = p->strides[0];
+  DwFlatArgs d;
+  size_t smem;
+  if (!plan_depthwise_planes(x, w, y, p, d, &smem)) return false;
   d.items = (d.planes + d.PP - 1) / d.PP;
   auto magic = [](int64_t dv) { return (uint32_t)((0x100000000ull + (uint64_t)dv - 1) / (uint64_t)dv); };
   d.m_plane = magic((int64_t)d.PH * d.PWn); d.m_pwn = magic(d.PWn);
@@ -468,9 +512,10 @@ bool launch_depthwise_planes(const fml_tensor *x, const fml_tensor *w, const fml
   d.y = (float *)y->data;
   for (int i = 0; i < 4; ++i) d.ys[i] = y->stride[i];
   d.act = p->act;
+  d.sums = p->plane_sums;
+  d.sum_shift = dwt_sum_shift(d.TR * d.SW);
   d.status = device_status_word();
   if (!d.status) return false;
-  const size_t smem = smem_of();
   const int key = (int)(KH * 10 + S);
   switch (key) {
   case 31: *status = launch_planes_variant<3, 3, 1>(d, smem, s); break;
@@ -499,17 +544,13 @@ int launch_variant(const CUtensorMap &map, const DwTmaArgs &d, size_t smem, cuda
   return FML_OK;
 }
 
-}  // namespace
-
-// Takes the layer when it can: x dense NCHW with rows of a multiple of four floats on a 16-byte
-// base, y with unit column stride, 3 x 3 or 5 x 5 window with "same" column padding, stride 1 or
-// 2 in both directions, dilation 1.  Returns false (nothing launched, *status untouched) otherwise.
-bool launch_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,
-                          const fml_conv_params *p, cudaStream_t s, int *status) {
+// What both kernels ask of a layer: x dense NCHW on a 16-byte base, y with unit column stride, 3 x 3 or 5 x 5 window,
+// stride 1 or 2 in both directions, dilation 1.
+bool depthwise_pipelined(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p) {
   static const bool enabled = [] { const char *e = getenv("FLUIDML_DEPTHWISE_TMA"); return !(e && e[0] == '0'); }();
   if (!enabled || x->rank != 4 || y->rank != 4 || w->rank != 4) return false;
   const int64_t N = x->shape[0], C = x->shape[1], IH = x->shape[2], IW = x->shape[3];
-  const int64_t OH = y->shape[2], OW = y->shape[3], KH = w->shape[2], KW = w->shape[3];
+  const int64_t KH = w->shape[2], KW = w->shape[3];
   const int64_t S = p->strides[0];
   if (p->strides[1] != S || (S != 1 && S != 2) || p->dilations[0] != 1 || p->dilations[1] != 1) return false;
   if (!((KH == 3 && KW == 3) || (KH == 5 && KW == 5))) return false;
@@ -518,10 +559,17 @@ bool launch_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_te
     return false;
   if (N * C >= (1ll << 30) || IH >= (1 << 20) || y->stride[3] != 1) return false;
   for (int i = 0; i < 4; ++i) if (y->stride[i] < 0) return false;
-  if ((IW & 3) || IW < 16) return launch_depthwise_planes(x, w, bias, y, p, s, status);
+  return true;
+}
+
+// ... and the tensor-map one: rows of a multiple of four floats, at least 16; "same" column padding.
+bool plan_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, DwTmaArgs &d, size_t *stage) {
+  const int64_t N = x->shape[0], C = x->shape[1], IW = x->shape[3];
+  const int64_t OH = y->shape[2], OW = y->shape[3], KH = w->shape[2], KW = w->shape[3];
+  const int64_t S = p->strides[0];
+  if ((IW & 3) || IW < 16) return false;
   if (p->pads_begin[1] != (KW - 1) / 2 || p->pads_begin[0] < 0 || p->pads_begin[0] > 8) return false;
   constexpr int RT = 4;
-  DwTmaArgs d;
   memset(&d, 0, sizeof(d));
   d.C = (int)C; d.OH = (int)OH; d.OW = (int)OW; d.ph = (int)p->pads_begin[0];
   d.SW = (int)((OW + 3) / 4);
@@ -555,10 +603,34 @@ bool launch_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_te
     d.TR = (RW + d.row_tiles - 1) / d.row_tiles;
   }
   d.row_tiles = (RW + d.TR - 1) / d.TR;
-  const size_t stage = stage_bytes();
+  *stage = stage_bytes();
   const int64_t items = (int64_t)((d.planes + d.PP - 1) / d.PP) * d.row_tiles;
   if (items > 0x7fffffff) return false;
   d.items = (int)items;
+  return true;
+}
+
+}  // namespace
+
+// Partial sums per plane that the layer's kernel can leave (fml_conv_params::plane_sums), 0 when it is another kernel's.
+int depthwise_sum_parts(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p) {
+  if (!depthwise_pipelined(x, w, y, p)) return 0;
+  DwTmaArgs t;
+  DwFlatArgs f;
+  size_t bytes;
+  if ((x->shape[3] & 3) || x->shape[3] < 16) return plan_depthwise_planes(x, w, y, p, f, &bytes) ? 1 : 0;
+  return plan_depthwise_tma(x, w, y, p, t, &bytes) ? t.row_tiles : 0;
+}
+
+// Takes the layer when it can; returns false (nothing launched, *status untouched) otherwise.
+bool launch_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y,
+                          const fml_conv_params *p, cudaStream_t s, int *status) {
+  if (!depthwise_pipelined(x, w, y, p)) return false;
+  const int64_t N = x->shape[0], C = x->shape[1], IH = x->shape[2], IW = x->shape[3], KH = w->shape[2], S = p->strides[0];
+  if ((IW & 3) || IW < 16) return launch_depthwise_planes(x, w, bias, y, p, s, status);
+  DwTmaArgs d;
+  size_t stage;
+  if (!plan_depthwise_tma(x, w, y, p, d, &stage)) return false;
   d.w = (const float *)w->data; d.ws0 = w->stride[0]; d.ws2 = w->stride[2]; d.ws3 = w->stride[3];
   if (bias) {
     d.bias = (const float *)bias->data;
@@ -567,6 +639,8 @@ bool launch_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_te
   d.y = (float *)y->data;
   for (int i = 0; i < 4; ++i) d.ys[i] = y->stride[i];
   d.act = p->act;
+  d.sums = p->plane_sums;
+  d.sum_shift = dwt_sum_shift(d.TR * d.SW);
   d.status = device_status_word();
   if (!d.status) return false;
   CUtensorMap map;

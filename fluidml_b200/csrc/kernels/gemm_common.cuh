@@ -109,6 +109,8 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
                    const fml_conv_params *p, cudaStream_t s, const float *x_scale = nullptr, int64_t x_scale_sn = 0,
                    int64_t x_scale_sc = 0);
 
+int depthwise_sum_parts(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p);
+
 // pointwise convolution in fp32 FMA (conv_pointwise.cu): whether it takes the layer, with the microseconds its model gives
 bool pointwise_fma_plan(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled, double *us);
 int launch_pointwise_fma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p, cudaStream_t s,

@@ -10,6 +10,11 @@
 // CTA pulls the other shares through distributed shared memory (at most a few KB), computes
 // the whole hidden vector (redundantly: it is tiny) and then the gate of its own channels.
 // No scratch memory, no atomics; the summation order is fixed, so results are bit-stable.
+//
+// Where the depthwise layer in front leaves the sums of its planes (fml_conv_params::plane_sums) the gate starts from
+// those: every CTA adds up all of the image's (a few kilobytes), so the tensor is not read again and the first exchange
+// between the CTAs falls away.  A pass of EfficientNet-B0, sixteen gates: one image 129 -> 69 us, 64 images 306 -> 104 (of
+// which the second layer's weights, staged with an even pitch that put a warp's 32 rows into two banks, were 46).
 #include <algorithm>
 
 #include "common.cuh"
@@ -44,6 +49,9 @@ struct SeArgs {
   int parts;        // pieces a plane is cut into
   int part_len;     // elements (float4 when vec, else float) per piece
   int stage_w;      // the CTA's weight rows fit in shared memory
+  const float *sums; // [N][C][sum_parts]
+  int sum_parts;
+  int images;       // per cluster; 1 unless from sums
 };
 
 __device__ __forceinline__ float se_act(int act, float v) {
@@ -88,58 +96,72 @@ __device__ __forceinline__ float se_ldg1(const float *p) {
   return v;
 }
 __device__ __forceinline__ void se_keep(float4 &v) { asm volatile("" : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)); }
-// rows x cols block of a strided matrix into dense shared memory; 16-byte loads when the rows allow
-__device__ __forceinline__ void se_stage(float *dst, const float *src, int rows, int cols, int64_t row_stride, int64_t col_stride) {
+// rows x cols block of a strided matrix into shared memory, `pitch` floats to a row; 16-byte loads when the rows allow
+__device__ __forceinline__ void se_stage(float *dst, int pitch, const float *src, int rows, int cols, int64_t row_stride, int64_t col_stride) {
   const bool v4 = col_stride == 1 && (cols & 3) == 0 && (row_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
   if (v4) {
     const int c4 = cols >> 2, total = rows * c4;
 #pragma unroll 8
     for (int i = threadIdx.x; i < total; i += kSeThreads) {
       const int r = i / c4, c = i - r * c4;
-      reinterpret_cast<float4 *>(dst)[i] = __ldg(reinterpret_cast<const float4 *>(src + (int64_t)r * row_stride) + c);
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(src + (int64_t)r * row_stride) + c);
+      float *const at = dst + r * pitch + 4 * c;
+      if (pitch & 3) { at[0] = v.x; at[1] = v.y; at[2] = v.z; at[3] = v.w; }
+      else *reinterpret_cast<float4 *>(at) = v;
     }
   } else {
     const int total = rows * cols;
 #pragma unroll 8
     for (int i = threadIdx.x; i < total; i += kSeThreads) {
       const int r = i / cols, c = i - r * cols;
-      dst[i] = __ldg(src + (int64_t)r * row_stride + (int64_t)c * col_stride);
+      dst[r * pitch + c] = __ldg(src + (int64_t)r * row_stride + (int64_t)c * col_stride);
     }
   }
 }
 
+template <bool SUMS>
 __global__ void __launch_bounds__(kSeThreads) squeeze_excite_gate_kernel(const SeArgs a) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) float se_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t rank = se_cluster_rank();
-  const int n = blockIdx.y;
+  const int n = (int)blockIdx.y * a.images, ims = min(a.images, a.N - n);  // images n .. n + ims - 1
   const int c0 = min(a.C, (int)rank * a.per_rank), c1 = min(a.C, c0 + a.per_rank), planes = c1 - c0;
   const int j0 = min(a.Cr, (int)rank * a.hid_per_rank), j1 = min(a.Cr, j0 + a.hid_per_rank), hids = j1 - j0;
   const int HW = a.H * a.W;
   // shared-memory map (every CTA of the cluster uses the same offsets: peers address `own` and `hid_own`)
   float *w1_s = se_smem;                                                   // [hid_per_rank][C]     (stage_w)
   float *w2_s = w1_s + (a.stage_w ? (size_t)a.hid_per_rank * a.C : 0);     // [per_rank][Cr]        (stage_w)
-  float *own = w2_s + (a.stage_w ? (size_t)a.per_rank * a.Cr : 0);         // [per_rank] means of this CTA's channels
-  float *hid_own = own + a.per_rank;                                       // [hid_per_rank] this CTA's hidden units
-  float *mean_s = hid_own + a.hid_per_rank;                                // [C]
-  float *hid_s = mean_s + a.C;                                             // [Cr]
-  float *b1_s = hid_s + a.Cr;                                              // [hid_per_rank]
+  float *own = w2_s + (a.stage_w ? (size_t)a.per_rank * (a.Cr | 1) : 0);  // (an odd pitch: a thread has a row in the last phase)         // [per_rank] means of this CTA's channels
+  float *hid_own = own + a.per_rank;                                       // [images][hid_per_rank] this CTA's hidden units
+  float *mean_s = hid_own + a.hid_per_rank * a.images;                     // [images][C]
+  float *hid_s = mean_s + a.C * a.images;                                  // [images][Cr]
+  float *b1_s = hid_s + a.Cr * a.images;                                   // [hid_per_rank]
   float *b2_s = b1_s + a.hid_per_rank;                                     // [per_rank]
   float *part_s = b2_s + a.per_rank;                                       // [planes * parts]
 
   // ---- 0. this CTA's weight rows and biases: constants, fetched before the dependency wait
   if (a.stage_w) {
-    se_stage(w1_s, a.w1 + (int64_t)j0 * a.w1s[0], hids, a.C, a.w1s[0], a.w1s[1]);
-    se_stage(w2_s, a.w2 + (int64_t)c0 * a.w2s[0], planes, a.Cr, a.w2s[0], a.w2s[1]);
+    se_stage(w1_s, a.C, a.w1 + (int64_t)j0 * a.w1s[0], hids, a.C, a.w1s[0], a.w1s[1]);
+    se_stage(w2_s, a.Cr | 1, a.w2 + (int64_t)c0 * a.w2s[0], planes, a.Cr, a.w2s[0], a.w2s[1]);
   }
   for (int j = threadIdx.x; j < hids; j += kSeThreads) b1_s[j] = a.b1 ? __ldg(a.b1 + (int64_t)(j0 + j) * a.b1s) : 0.0f;
   for (int c = threadIdx.x; c < planes; c += kSeThreads) b2_s[c] = a.b2 ? __ldg(a.b2 + (int64_t)(c0 + c) * a.b2s) : 0.0f;
   pdl_wait();
 
+  if (SUMS) {
+    const float *sn = a.sums + (int64_t)n * a.C * a.sum_parts;
+    for (int c = threadIdx.x; c < a.C * ims; c += kSeThreads) {  // images lie side by side
+      float t = 0.0f;
+#pragma unroll 4
+      for (int q = 0; q < a.sum_parts; ++q) t += sn[c * a.sum_parts + q];
+      mean_s[c] = t / (float)HW;
+    }
+  }
+
   // ---- 1. means of the CTA's channels.  A unit is one piece of one plane, summed by `lanes`
   // lanes with all their loads in flight at once; the pieces of a plane are then added in order.
-  {
+  if (!SUMS) {
     const float *xn = a.x + (int64_t)n * a.xs[0];
     const int L = a.lanes, groups = 32 / L, units = planes * a.parts;
     const int E = a.vec ? HW >> 2 : HW;
@@ -202,9 +224,9 @@ __global__ void __launch_bounds__(kSeThreads) squeeze_excite_gate_kernel(const S
   }
 
   // ---- 2. every CTA gathers all means of the image
-  se_cluster_arrive();
-  se_cluster_wait();
-  {
+  if (!SUMS) {
+    se_cluster_arrive();
+    se_cluster_wait();
     const uint32_t own_addr = (uint32_t)__cvta_generic_to_shared(own);
     for (int c = threadIdx.x; c < a.C; c += kSeThreads) {
       const int q = c / a.per_rank;
@@ -214,31 +236,35 @@ __global__ void __launch_bounds__(kSeThreads) squeeze_excite_gate_kernel(const S
   __syncthreads();
 
   // ---- 3. this CTA's hidden units: one warp per unit, lanes along the channels
-  for (int j = warp; j < hids; j += kSeWarps) {
+  for (int im = 0, u = warp; im < ims;) {  // (image, unit) pairs
+    if (u >= hids) { u -= hids; ++im; continue; }
+    const int j = u;
+    const float *const mean = mean_s + im * a.C;
     float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
     int k = lane;
     if (a.stage_w) {
       const float *wr = w1_s + (size_t)j * a.C;
       for (; k + 96 < a.C; k += 128) {
-        s0 = fmaf(wr[k], mean_s[k], s0);
-        s1 = fmaf(wr[k + 32], mean_s[k + 32], s1);
-        s2 = fmaf(wr[k + 64], mean_s[k + 64], s2);
-        s3 = fmaf(wr[k + 96], mean_s[k + 96], s3);
+        s0 = fmaf(wr[k], mean[k], s0);
+        s1 = fmaf(wr[k + 32], mean[k + 32], s1);
+        s2 = fmaf(wr[k + 64], mean[k + 64], s2);
+        s3 = fmaf(wr[k + 96], mean[k + 96], s3);
       }
-      for (; k < a.C; k += 32) s0 = fmaf(wr[k], mean_s[k], s0);
+      for (; k < a.C; k += 32) s0 = fmaf(wr[k], mean[k], s0);
     } else {
       const float *wr = a.w1 + (int64_t)(j0 + j) * a.w1s[0];
 #pragma unroll 2
       for (; k + 96 < a.C; k += 128) {
-        s0 = fmaf(__ldg(wr + (int64_t)k * a.w1s[1]), mean_s[k], s0);
-        s1 = fmaf(__ldg(wr + (int64_t)(k + 32) * a.w1s[1]), mean_s[k + 32], s1);
-        s2 = fmaf(__ldg(wr + (int64_t)(k + 64) * a.w1s[1]), mean_s[k + 64], s2);
-        s3 = fmaf(__ldg(wr + (int64_t)(k + 96) * a.w1s[1]), mean_s[k + 96], s3);
+        s0 = fmaf(__ldg(wr + (int64_t)k * a.w1s[1]), mean[k], s0);
+        s1 = fmaf(__ldg(wr + (int64_t)(k + 32) * a.w1s[1]), mean[k + 32], s1);
+        s2 = fmaf(__ldg(wr + (int64_t)(k + 64) * a.w1s[1]), mean[k + 64], s2);
+        s3 = fmaf(__ldg(wr + (int64_t)(k + 96) * a.w1s[1]), mean[k + 96], s3);
       }
-      for (; k < a.C; k += 32) s0 = fmaf(__ldg(wr + (int64_t)k * a.w1s[1]), mean_s[k], s0);
+      for (; k < a.C; k += 32) s0 = fmaf(__ldg(wr + (int64_t)k * a.w1s[1]), mean[k], s0);
     }
     const float s = se_warp_sum((s0 + s1) + (s2 + s3));
-    if (lane == 0) hid_own[j] = se_act(a.act1, s + b1_s[j]);
+    if (lane == 0) hid_own[im * a.hid_per_rank + j] = se_act(a.act1, s + b1_s[j]);
+    u += kSeWarps;
   }
 
   // ---- 4. every CTA gathers the hidden vector (the barrier also tells the peers that this CTA
@@ -247,27 +273,29 @@ __global__ void __launch_bounds__(kSeThreads) squeeze_excite_gate_kernel(const S
   se_cluster_wait();
   {
     const uint32_t hid_addr = (uint32_t)__cvta_generic_to_shared(hid_own);
-    for (int j = threadIdx.x; j < a.Cr; j += kSeThreads) {
-      const int q = j / a.hid_per_rank;
-      hid_s[j] = se_peer_load(hid_addr, j - q * a.hid_per_rank, (uint32_t)q);
+    for (int i = threadIdx.x; i < a.Cr * ims; i += kSeThreads) {
+      const int im = i / a.Cr, j = i - im * a.Cr, q = j / a.hid_per_rank;
+      hid_s[i] = se_peer_load(hid_addr, im * a.hid_per_rank + j - q * a.hid_per_rank, (uint32_t)q);
     }
   }
   // nobody leaves while a peer may still read its hidden units: arrive now, wait at the end
   se_cluster_arrive();
   __syncthreads();
 
-  // ---- 5. gate of the CTA's channels: one thread per channel
-  for (int c = threadIdx.x; c < planes; c += kSeThreads) {
+  // ---- 5. gates of the CTA's channels: one thread per channel and image
+  for (int i = threadIdx.x; i < planes * ims; i += kSeThreads) {
+    const int im = i / planes, c = i - im * planes;
+    const float *const hid = hid_s + im * a.Cr;
     float s = 0.0f;
     if (a.stage_w) {
-      const float *wr = w2_s + (size_t)c * a.Cr;
-      for (int j = 0; j < a.Cr; ++j) s = fmaf(wr[j], hid_s[j], s);
+      const float *wr = w2_s + (size_t)c * (a.Cr | 1);
+      for (int j = 0; j < a.Cr; ++j) s = fmaf(wr[j], hid[j], s);
     } else {
       const float *wr = a.w2 + (int64_t)(c0 + c) * a.w2s[0];
 #pragma unroll 8
-      for (int j = 0; j < a.Cr; ++j) s = fmaf(__ldg(wr + (int64_t)j * a.w2s[1]), hid_s[j], s);
+      for (int j = 0; j < a.Cr; ++j) s = fmaf(__ldg(wr + (int64_t)j * a.w2s[1]), hid[j], s);
     }
-    a.gate[(int64_t)n * a.gs[0] + (int64_t)(c0 + c) * a.gs[1]] = se_act(a.act2, s + b2_s[c]);
+    a.gate[(int64_t)(n + im) * a.gs[0] + (int64_t)(c0 + c) * a.gs[1]] = se_act(a.act2, s + b2_s[c]);
   }
   se_cluster_wait();
 }
@@ -277,20 +305,20 @@ __global__ void __launch_bounds__(kSeThreads) squeeze_excite_gate_kernel(const S
 
 using namespace fml;
 
-extern "C" int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1, const fml_tensor *b1,
-                                       const fml_tensor *w2, const fml_tensor *b2, int act1, int act2,
-                                       const fml_tensor *gate, void *stream) {
+// x: the tensor, or with `plane` > 0 the sums [N, C, parts] of its planes of that many elements.
+static int gate_impl(const fml_tensor *x, int64_t plane, const fml_tensor *w1, const fml_tensor *b1, const fml_tensor *w2, const fml_tensor *b2, int act1,
+                     int act2, const fml_tensor *gate, void *stream) {
   FML_REQUIRE(valid_tensor(x) && valid_tensor(w1) && valid_tensor(w2) && valid_tensor(gate), FML_BAD_ARG,
               "fml_squeeze_excite_gate: bad argument");
   FML_REQUIRE(x->dtype == FML_F32 && w1->dtype == FML_F32 && w2->dtype == FML_F32 && gate->dtype == FML_F32,
               FML_UNSUPPORTED, "fml_squeeze_excite_gate: fp32 only");
-  FML_REQUIRE(x->rank == 4 && gate->rank == 4 && w1->rank >= 2 && w2->rank >= 2, FML_BAD_ARG,
+  FML_REQUIRE(x->rank == (plane ? 3 : 4) && gate->rank == 4 && w1->rank >= 2 && w2->rank >= 2, FML_BAD_ARG,
               "fml_squeeze_excite_gate: x and gate are [N, C, H, W] / [N, C, 1, 1], weights [out, in(, 1, 1)]");
   for (int i = 2; i < w1->rank; ++i) FML_REQUIRE(w1->shape[i] == 1, FML_BAD_ARG, "fml_squeeze_excite_gate: w1 must be 1 x 1");
   for (int i = 2; i < w2->rank; ++i) FML_REQUIRE(w2->shape[i] == 1, FML_BAD_ARG, "fml_squeeze_excite_gate: w2 must be 1 x 1");
   SeArgs a;
   memset(&a, 0, sizeof(a));
-  a.N = (int)x->shape[0]; a.C = (int)x->shape[1]; a.H = (int)x->shape[2]; a.W = (int)x->shape[3];
+  a.N = (int)x->shape[0]; a.C = (int)x->shape[1]; a.H = plane ? 1 : (int)x->shape[2]; a.W = (int)(plane ? plane : x->shape[3]);
   a.Cr = (int)w1->shape[0];
   FML_REQUIRE(w1->shape[1] == a.C && w2->shape[0] == a.C && w2->shape[1] == a.Cr, FML_BAD_ARG,
               "fml_squeeze_excite_gate: weight shapes must be [Cr, C] and [C, Cr]");
@@ -304,8 +332,15 @@ extern "C" int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1
                   (int64_t)a.H * a.W >= 1 && (int64_t)a.H * a.W < (1ll << 31),
               FML_UNSUPPORTED, "fml_squeeze_excite_gate: at most %d channels, %d hidden units, 65535 images",
               kSeMaxChannels, kSeMaxHidden);
-  for (int i = 0; i < 4; ++i) a.xs[i] = x->stride[i];
-  a.x = (const float *)x->data;
+  if (plane) {
+    FML_REQUIRE(x->shape[2] >= 1 && x->shape[2] < (1 << 20) && x->stride[2] == 1 && x->stride[1] == x->shape[2] && (a.N == 1 || x->stride[0] == a.C * x->shape[2]),
+                FML_UNSUPPORTED, "fml_squeeze_excite_gate_from_sums: the sums must be dense");
+    a.sums = (const float *)x->data;
+    a.sum_parts = (int)x->shape[2];
+  } else {
+    for (int i = 0; i < 4; ++i) a.xs[i] = x->stride[i];
+    a.x = (const float *)x->data;
+  }
   a.w1 = (const float *)w1->data; a.w1s[0] = w1->stride[0]; a.w1s[1] = w1->stride[1];
   a.w2 = (const float *)w2->data; a.w2s[0] = w2->stride[0]; a.w2s[1] = w2->stride[1];
   if (b1) {
@@ -320,7 +355,7 @@ extern "C" int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1
   }
   a.gate = (float *)gate->data; a.gs[0] = gate->stride[0]; a.gs[1] = gate->stride[1];
   a.act1 = act1; a.act2 = act2;
-  a.plane_dense = (a.W == 1 || x->stride[3] == 1) && (a.H == 1 || x->stride[2] == a.W) ? 1 : 0;
+  a.plane_dense = !plane && (a.W == 1 || x->stride[3] == 1) && (a.H == 1 || x->stride[2] == a.W) ? 1 : 0;
   const int64_t HW = (int64_t)a.H * a.W;
   a.vec = a.plane_dense && (HW & 3) == 0 && aligned16(a.x) && (x->stride[0] & 3) == 0 && (x->stride[1] & 3) == 0 ? 1 : 0;
   // cluster size: eight CTAs per image unless the image has fewer than eight channels
@@ -338,23 +373,39 @@ extern "C" int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1
     if (a.parts < 1) a.parts = 1;
   }
   a.part_len = (int)((E + a.parts - 1) / a.parts);
-  const size_t stage_bytes = ((size_t)a.hid_per_rank * a.C + (size_t)a.per_rank * a.Cr) * sizeof(float);
+  const size_t stage_bytes = ((size_t)a.hid_per_rank * a.C + (size_t)a.per_rank * (a.Cr | 1)) * sizeof(float);
   a.stage_w = (((size_t)a.hid_per_rank * a.C) & 3) == 0 && stage_bytes <= kSeStageBytes ? 1 : 0;
-  const size_t smem = (a.stage_w ? stage_bytes : 0) +
-                      ((size_t)2 * a.per_rank + 2 * a.hid_per_rank + a.C + a.Cr + (size_t)a.per_rank * a.parts) * sizeof(float);
+  a.images = 1;
+  auto smem_of = [&] {
+    return (a.stage_w ? stage_bytes : 0) + ((size_t)2 * a.per_rank + a.hid_per_rank + (size_t)a.images * (a.hid_per_rank + a.C + a.Cr) +
+                                            (plane ? 0 : (size_t)a.per_rank * a.parts)) * sizeof(float);
+  };
+  // From sums, more clusters than the SMs hold at once: two or four images to a cluster, which share its staged weights
+  // and its exchange (64 images of 1152 channels: 15.0 -> 10.0 us).  No sooner: a cluster does its images one after the
+  // other (672 channels, where all clusters fit: 5.4 us with one image, 6.7 with two, 10.1 with four).
+  auto waves = [&] {
+    const int64_t per_sm = std::min<int64_t>(2048 / kSeThreads, (int64_t)(228 * 1024 / (smem_of() + 1024)));
+    return (double)((a.N + a.images - 1) / a.images) * ranks / (148.0 * (double)std::max<int64_t>(1, per_sm));
+  };
+  while (plane && a.images < 4 && waves() > 1.0) {
+    a.images *= 2;
+    if (smem_of() > 100 * 1024) { a.images /= 2; break; }
+  }
+  const size_t smem = smem_of();
   {
     static bool attr_set[64] = {false};
     int dev = 0;
     FML_CUDA(cudaGetDevice(&dev));
     if (!attr_set[dev & 63]) {
-      FML_CUDA(cudaFuncSetAttribute(squeeze_excite_gate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+      FML_CUDA(cudaFuncSetAttribute(squeeze_excite_gate_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+      FML_CUDA(cudaFuncSetAttribute(squeeze_excite_gate_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
       attr_set[dev & 63] = true;
     }
   }
 
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)ranks, (unsigned)a.N, 1);
+  cfg.gridDim = dim3((unsigned)ranks, (unsigned)((a.N + a.images - 1) / a.images), 1);
   cfg.blockDim = dim3(kSeThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = as_stream(stream);
@@ -367,6 +418,17 @@ extern "C" int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  FML_CUDA(cudaLaunchKernelEx(&cfg, squeeze_excite_gate_kernel, a));
+  FML_CUDA(cudaLaunchKernelEx(&cfg, plane ? squeeze_excite_gate_kernel<true> : squeeze_excite_gate_kernel<false>, a));
   return FML_OK;
+}
+
+extern "C" int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1, const fml_tensor *b1, const fml_tensor *w2, const fml_tensor *b2, int act1,
+                                       int act2, const fml_tensor *gate, void *stream) {
+  return gate_impl(x, 0, w1, b1, w2, b2, act1, act2, gate, stream);
+}
+
+extern "C" int fml_squeeze_excite_gate_from_sums(const fml_tensor *sums, int64_t plane, const fml_tensor *w1, const fml_tensor *b1, const fml_tensor *w2,
+                                                 const fml_tensor *b2, int act1, int act2, const fml_tensor *gate, void *stream) {
+  FML_REQUIRE(plane > 0 && plane < (1ll << 31), FML_BAD_ARG, "fml_squeeze_excite_gate_from_sums: plane size");
+  return gate_impl(sums, plane, w1, b1, w2, b2, act1, act2, gate, stream);
 }

@@ -186,6 +186,11 @@ int fml_sum_of_products(int n, const fml_tensor *const *a, const fml_tensor *con
 int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1, const fml_tensor *b1,
                             const fml_tensor *w2, const fml_tensor *b2, int act1, int act2,
                             const fml_tensor *gate, void *stream);
+/* The same from plane sums: `sums` [N, C, parts] (dense; the parts of a plane are added in order), planes of
+ * `plane` elements. */
+int fml_squeeze_excite_gate_from_sums(const fml_tensor *sums, int64_t plane, const fml_tensor *w1, const fml_tensor *b1,
+                                      const fml_tensor *w2, const fml_tensor *b2, int act1, int act2, const fml_tensor *gate,
+                                      void *stream);
 
 /* WhereConstantCond{ConstantScalarY,ConstantTensorY}Kernel (where.cpp:30-80, :90-150):
  * out = cond ? x : y, all broadcast to out.  y == NULL takes the scalar y_scalar. */
@@ -413,7 +418,14 @@ typedef struct fml_conv_params {
    * output channels innermost, a multiple of 4 of them) runs there, whatever w_packed says; tile_n = slices of k
    * among the warps of a CTA and split_k = CTAs per tile may then be given.  See fml_conv_prefers_fma. */
   int32_t pointwise_fma;
+  /* Depthwise layers: where to leave the sums of y's planes (after bias and activation), [N * C][parts] floats with the
+   * parts that fml_conv_plane_sum_parts names; NULL = not wanted.  FML_UNSUPPORTED where it names none. */
+  float *plane_sums;
 } fml_conv_params;
+
+/* Partial sums per output plane that fml_conv leaves in plane_sums for this layer, 0 when its kernel leaves none.  Pure
+ * host computation. */
+int fml_conv_plane_sum_parts(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, int *parts);
 
 /* Whether pointwise_fma is the faster choice for this layer (scaled: with the gate of fml_conv_scaled): little
  * arithmetic, where the tensor-core kernel's fixed phases are most of its time.  Pure host computation. */

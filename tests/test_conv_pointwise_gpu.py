@@ -35,7 +35,8 @@ def run(x, w, bias, gate, res, act, wk=0, split=0, pad=0):
     if res is not None:
         wide = np.zeros((n, oc + pad, h, wd), np.float32)
         wide[:, :oc] = res
-        cabi.check(cabi.lib().fml_conv_residual(_ref(dx), _ref(dg), _ref(dw), _ref(db), _ref(view(DT.from_numpy(wide))), _ref(y), ctypes.byref(p), None))
+        dr = view(DT.from_numpy(wide))
+        cabi.check(cabi.lib().fml_conv_residual(_ref(dx), _ref(dg), _ref(dw), _ref(db), _ref(dr), _ref(y), ctypes.byref(p), None))
     elif gate is not None:
         cabi.check(cabi.lib().fml_conv_scaled(_ref(dx), _ref(dg), _ref(dw), _ref(db), _ref(y), ctypes.byref(p), None))
     else:
