@@ -53,7 +53,7 @@ enum class Kind {
   Silu,            // x * sigmoid(x)
   FusedAttention,  // softmax(Q K^T / divisor + mask) V; inputs: Q, K^T, V, [mask]
   FusedMulAdd,     // a * b + c, broadcast; inputs: a, b, c
-  FusedMulAddChain,   // a0*b0 + a1*b1 + ... in the rounding order of the Mul / Add chain it replaces; inputs: a0, b0, a1, b1, ...
+  FusedMulAddChain,   // a0*b0 + a1*b1 + ... in the rounding order of the Mul / Add chain it replaces; inputs: a0, b0, a1, b1, ...; with span > 0 (ConvBERT): x, logits of `span` taps
   Rotary,             // rotary position embedding over the first `value` features; inputs: x, cos, sin, or x alone when its product has rotated it
   SqueezeExciteGate,  // act2(W2 act1(W1 mean_hw(x) + b1) + b2); consts: W1, [b1], W2, [b2]; has_bias / has_bias2 = b1 / b2 present; act, act2
 };
@@ -93,6 +93,7 @@ struct Node {
   // columns followed by those of inputs[1].
   int64_t act_from = 0, rot = 0, rot_head = 0, rot_cols = 0, rot_len = 1;
   bool two_a = false;
+  int64_t span = 0;  // FusedMulAddChain: a span convolution of that many taps, pads[0] rows of padding in front
   bool b_is_const = false;  // FusedGemm: B is a captured constant (consts[0]) rather than inputs[1]
   // Scratch bytes the REFERENCE kernel of this kind needs (one float per row for Softmax and
   // LayerNorm, a padded copy for ConvWithPadding); used to report the reference-equivalent

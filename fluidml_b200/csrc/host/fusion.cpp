@@ -526,6 +526,61 @@ bool FuseMulAddChain(Rewriter &rw, const NodePtr &last) {
   return true;
 }
 
+// ---- FusedMulAddChain over windows of a Pad along the sequence and the taps of a Softmax: x [b, s, h, d], padded with zeros
+// along s, its windows starting at 0, 1, .., each times one tap of softmax(logits [b, s, h, taps]).  Four launches in one.
+bool FuseSpanConvolution(Rewriter &rw, const NodePtr &chain) {
+  if (chain->kind != Kind::FusedMulAddChain || chain->span || chain->inputs.size() % 2) return false;
+  const int64_t taps = (int64_t)chain->inputs.size() / 2;
+  if (!fml_span_convolution_supported(taps)) return false;
+  const auto &os = chain->output->meta.GetShape();
+  if (os.size() != 4 || chain->output->meta.GetType() != Type::kFloat32) return false;
+  auto slice_of = [&](const RegionPtr &r) -> NodePtr {
+    auto it = rw.producer.find(r.get());
+    return it != rw.producer.end() && it->second->kind == Kind::Slice && it->second->inputs.size() == 1 && it->second->starts.size() == 4 && rw.Sole(r) == chain
+               ? it->second : nullptr;
+  };
+  RegionPtr padded, weights;
+  std::vector<NodePtr> slices;
+  for (int64_t j = 0; j < taps; ++j) {
+    NodePtr win = slice_of(chain->inputs[2 * j]), tap = slice_of(chain->inputs[2 * j + 1]);
+    if (!win || !tap) return false;
+    if (win->output->meta.GetShape() != os) std::swap(win, tap);  // a product may be written either way round
+    const auto &ws = win->output->meta.GetShape(), &ts = tap->output->meta.GetShape();
+    if (ws != os || ts.size() != 4 || ts[0] != os[0] || ts[1] != os[1] || ts[2] != os[2] || ts[3] != 1) return false;
+    const int64_t at = win->starts[1];
+    // (the chain's first sum, a product plus a product, has no order)
+    if (at != j && !(j < 2 && at == 1 - j)) return false;
+    if (j == 1 && at == slices[0]->starts[1]) return false;
+    if (win->starts != std::vector<int64_t>{0, at, 0, 0} || tap->starts != std::vector<int64_t>{0, 0, 0, at}) return false;
+    if (j == 0) { padded = win->inputs[0]; weights = tap->inputs[0]; }
+    if (win->inputs[0] != padded || tap->inputs[0] != weights) return false;
+    slices.push_back(win);
+    slices.push_back(tap);
+  }
+  auto made_by = [&](const RegionPtr &r, Kind k) -> NodePtr {  // read by the slices only
+    auto it = rw.producer.find(r.get());
+    auto readers = rw.consumers.find(r.get());
+    return it != rw.producer.end() && it->second->kind == k && r->kind == flow::Region::kInner && readers != rw.consumers.end() &&
+                   (int64_t)readers->second.size() == taps ? it->second : nullptr;
+  };
+  const NodePtr pad = made_by(padded, Kind::Pad), sm = made_by(weights, Kind::Softmax);
+  if (!pad || !sm || pad->inputs.size() != 1 || sm->inputs.size() != 1 || (sm->axis != 3 && sm->axis != -1)) return false;
+  const RegionPtr &x = pad->inputs[0], &logits = sm->inputs[0];
+  if (x->meta.GetShape() != os || x->meta.GetType() != Type::kFloat32 || logits->meta.GetType() != Type::kFloat32 || IsConst(x) || IsConst(logits)) return false;
+  if (logits->meta.GetShape() != std::vector<int64_t>{os[0], os[1], os[2], taps} || pad->pads.size() != 8) return false;
+  for (size_t i = 0; i < 8; ++i)
+    if (i % 4 != 1 && pad->pads[i] != 0) return false;
+  if (pad->pads[1] < 0 || pad->pads[5] < 0 || pad->pads[1] + pad->pads[5] != taps - 1) return false;
+  if (os[0] > 65535 || os[2] * taps > 1024 || os[2] > 512) return false;  // limits of fml_span_convolution
+  chain->inputs = {x, logits};
+  chain->span = taps;
+  chain->pads = {pad->pads[1]};
+  for (const NodePtr &n : slices) rw.Kill(n);
+  rw.Kill(pad);
+  rw.Kill(sm);
+  return true;
+}
+
 // ---- Rotary position embedding as exported (GPT-NeoX):
 //   xr = x[..., :rot]; xp = x[..., rot:]
 //   out = Concat(xr * cos + Concat(-xr[..., rot/2:], xr[..., :rot/2]) * sin, xp)
@@ -921,7 +976,7 @@ size_t FusionPasses::Run(flow::Flow &flow, bool join) {
   using Pass = bool (*)(Rewriter &, const NodePtr &);
   // order matters: bias before GELU / activation before residual, residual before Add+LN
   const Pass passes[] = {FuseEmbedding, FuseMask, FuseBias, FuseGeluIntoGemm, FuseBiasGelu, FuseActivation,
-                         FuseResidual, FuseSecondResidual, FuseAddLayerNorm, FuseScaledMaskedSoftmax, FuseAttention, FuseSilu, FuseSiluIntoConv, FuseSqueezeExcite, FuseGateIntoConv, FuseResidualIntoConv, FuseMulAdd, FuseRotary, FuseMulAddChain};
+                         FuseResidual, FuseSecondResidual, FuseAddLayerNorm, FuseScaledMaskedSoftmax, FuseAttention, FuseSilu, FuseSiluIntoConv, FuseSqueezeExcite, FuseGateIntoConv, FuseResidualIntoConv, FuseMulAdd, FuseRotary, FuseMulAddChain, FuseSpanConvolution};
   auto until_done = [&](Pass pass) {
     bool again = true;
     while (again) {

@@ -247,6 +247,21 @@ private:
   int64_t rot_;
 };
 
+// Softmax, Pad, Slices and the chain of products over them (ConvBERT's span convolution) in one launch
+class SpanConvolutionKernel : public Kernel {
+public:
+  explicit SpanConvolutionKernel(int64_t pad) : pad_(pad) {}
+  std::string GetKernelName() const override { return "SpanConvolutionKernel"; }
+  void Launch(LaunchRecorder &rec, const std::vector<fml_tensor> &in, const fml_tensor &output, const Buffer &) const override {
+    const fml_tensor x = in.at(0), logits = in.at(1);
+    const int64_t pad = pad_;
+    rec.Add(GetKernelName(), [=](void *s) { return fml_span_convolution(&x, &logits, pad, &output, s); });
+  }
+
+private:
+  int64_t pad_;
+};
+
 // A chain MulCommon -> FusedMulAdd -> FusedMulAdd ... that sums products, in one launch
 class FusedMulAddChainKernel : public Kernel {
 public:
@@ -777,7 +792,9 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
   case Kind::Sigmoid: return std::make_unique<SigmoidKernel>();
   case Kind::Silu: return std::make_unique<SiluKernel>();
   case Kind::FusedMulAdd: return std::make_unique<FusedMulAddKernel>();
-  case Kind::FusedMulAddChain: return std::make_unique<FusedMulAddChainKernel>();
+  case Kind::FusedMulAddChain:
+    if (n.span) return std::make_unique<SpanConvolutionKernel>(n.pads.at(0));
+    return std::make_unique<FusedMulAddChainKernel>();
   case Kind::Rotary:
     if (n.inputs.size() == 1) return std::make_unique<DropoutKernel>();  // rotated by its product: a view
     return std::make_unique<RotaryKernel>((int64_t)n.value);

@@ -192,6 +192,13 @@ int fml_squeeze_excite_gate_from_sums(const fml_tensor *sums, int64_t plane, con
                                       const fml_tensor *w2, const fml_tensor *b2, int act1, int act2, const fml_tensor *gate,
                                       void *stream);
 
+/* Softmax over the taps, zero Pad along the sequence, Slices, Mul / Add chain of a span-based dynamic convolution in one
+ * launch: out[b, s, h, :] = sum_j softmax(logits[b, s, h, :])[j] * x[b, s + j - pad, h, :], x and out
+ * [batch, length, heads, features], logits [batch, length, heads, taps]; products and partial sums rounded in tap order
+ * (softmax.cpp:22-139, pad.cpp:15-51, mul.cpp, add.cpp). */
+int fml_span_convolution_supported(int64_t taps);
+int fml_span_convolution(const fml_tensor *x, const fml_tensor *logits, int64_t pad, const fml_tensor *out, void *stream);
+
 /* WhereConstantCond{ConstantScalarY,ConstantTensorY}Kernel (where.cpp:30-80, :90-150):
  * out = cond ? x : y, all broadcast to out.  y == NULL takes the scalar y_scalar. */
 int fml_where(const fml_tensor *cond, const fml_tensor *x, const fml_tensor *y, float y_scalar,
