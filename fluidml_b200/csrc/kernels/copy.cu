@@ -246,30 +246,55 @@ __global__ void gather_generic(GatherArgs g, T *out, const T *data, const int64_
   }
 }
 
-// Embedding rows: one warp per output row, 16-byte lanes.  table rows contiguous.
-__global__ void embedding_rows(int64_t rows, int64_t width, int64_t vocab, float *out,
-                               const float *table, int64_t table_row_stride, const int64_t *ids,
-                               const float *add0, int64_t add0_row_stride,
-                               const float *add1, int64_t add1_row_stride, int64_t add_rows,
-                               int *status) {
+// Rows of a table by index, with up to two addends whose rows follow the output's (position and token-type embeddings):
+// one warp per row, 16-byte lanes, four of each operand's loads in flight before the first store.  Leading dims of the
+// output are two (outer, inner) at most; an addend's row is outer * s[0] + inner * s[1].  (6144 rows of 768 with two
+// addends: 69 us in embedding_generic, whose threads work 64-bit divisions out per element, 10 us here.)
+struct EmbedRows {
+  int64_t rows, inner, vocab, table_stride;
+  int width4;
+  const float *table, *add[2];
+  int64_t add_s[2][2];
+  const int64_t *ids;
+  float *out;
+  int *status;
+};
+__global__ void __launch_bounds__(256) embedding_rows(const EmbedRows a) {
   pdl_prologue();
   const int lane = threadIdx.x & 31;
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (warp >= rows) return;
-  int64_t id = ids[warp];
-  if (id < 0 || id >= vocab) {
-    if (lane == 0) atomicOr(status, kStatusIndexRange);
-    id = id < 0 ? 0 : vocab - 1;
+  const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (row >= a.rows) return;
+  int64_t id = a.ids[row];
+  if (id < 0 || id >= a.vocab) {
+    if (lane == 0) atomicOr(a.status, kStatusIndexRange);
+    id = id < 0 ? 0 : a.vocab - 1;
   }
-  const float4 *src = reinterpret_cast<const float4 *>(table + id * table_row_stride);
-  const float4 *a0 = add0 ? reinterpret_cast<const float4 *>(add0 + (warp % add_rows) * add0_row_stride) : nullptr;
-  const float4 *a1 = add1 ? reinterpret_cast<const float4 *>(add1 + (warp % add_rows) * add1_row_stride) : nullptr;
-  float4 *dst = reinterpret_cast<float4 *>(out + warp * width);
-  for (int64_t c = lane; c < width / 4; c += 32) {
-    float4 v = src[c];
-    if (a0) { float4 t = a0[c]; v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w; }
-    if (a1) { float4 t = a1[c]; v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w; }
-    dst[c] = v;
+  const int64_t outer = row / a.inner, in = row - outer * a.inner;
+  const float4 *src = reinterpret_cast<const float4 *>(a.table + id * a.table_stride);
+  const float4 *add[2];
+#pragma unroll
+  for (int o = 0; o < 2; ++o) add[o] = a.add[o] ? reinterpret_cast<const float4 *>(a.add[o] + outer * a.add_s[o][0] + in * a.add_s[o][1]) : nullptr;
+  float4 *dst = reinterpret_cast<float4 *>(a.out) + row * a.width4;
+  for (int c0 = lane; c0 < a.width4; c0 += 128) {
+    float4 v[4], t[2][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = c0 + 32 * u;
+      v[u] = t[0][u] = t[1][u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c >= a.width4) continue;
+      v[u] = src[c];
+      if (add[0]) t[0][u] = add[0][c];
+      if (add[1]) t[1][u] = add[1][c];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int c = c0 + 32 * u;
+      if (c >= a.width4) continue;
+#pragma unroll
+      for (int o = 0; o < 2; ++o)
+        if (add[o]) { v[u].x += t[o][u].x; v[u].y += t[o][u].y; v[u].z += t[o][u].z; v[u].w += t[o][u].w; }
+      dst[c] = v[u];
+    }
   }
 }
 
@@ -407,9 +432,11 @@ extern "C" int fml_gather(const fml_tensor *data, const fml_tensor *indices, con
       data->shape[1] % 4 == 0 && data->stride[0] % 4 == 0 && is_row_major(out) &&
       is_row_major(indices) && aligned16(data->data) && aligned16(out->data)) {
     int64_t rows = numel(indices);
-    FML_LAUNCH((embedding_rows), (unsigned)((rows * 32 + 255) / 256), 256, 0, s, 
-        rows, data->shape[1], data->shape[0], (float *)out->data, (const float *)data->data,
-        data->stride[0], (const int64_t *)indices->data, nullptr, 0, nullptr, 0, 1, status);
+    EmbedRows e;
+    memset(&e, 0, sizeof(e));
+    e.rows = rows; e.inner = 1; e.vocab = data->shape[0]; e.table_stride = data->stride[0]; e.width4 = (int)(data->shape[1] / 4);
+    e.table = (const float *)data->data; e.ids = (const int64_t *)indices->data; e.out = (float *)out->data; e.status = status;
+    FML_LAUNCH((embedding_rows), (unsigned)((rows * 32 + 255) / 256), 256, 0, s, e);
     FML_CUDA(cudaGetLastError());
     return FML_OK;
   }
@@ -441,6 +468,30 @@ extern "C" int fml_embedding(const fml_tensor *table, const fml_tensor *ids, con
     FML_REQUIRE(valid_tensor(adds[o]) && adds[o]->dtype == FML_F32, FML_BAD_ARG, "fml_embedding: bad addend");
     FML_REQUIRE(broadcast_strides(adds[o], out, add.stride[o + 1]), FML_BAD_ARG,
                 "fml_embedding: addend does not broadcast to the output");
+  }
+  // whole rows of 16-byte groups: table rows contiguous, indices and output row-major, addends contiguous along the last dim
+  const int r = out->rank;
+  bool by_rows = table->rank == 2 && r >= 2 && r <= 3 && ids->rank == r - 1 && table->stride[1] == 1 && table->shape[1] % 4 == 0 && table->stride[0] % 4 == 0 &&
+                 table->shape[1] < (1ll << 30) && is_row_major(out) && is_row_major(ids) && aligned16(table->data) && aligned16(out->data);
+  EmbedRows e;
+  memset(&e, 0, sizeof(e));
+  for (int o = 0; o < 2 && by_rows; ++o) {
+    if (!adds[o]) continue;
+    const int64_t *st = add.stride[o + 1];
+    by_rows = (st[r - 1] == 1 || out->shape[r - 1] == 1) && aligned16(adds[o]->data);
+    for (int i = 0; i + 1 < r; ++i) by_rows = by_rows && st[i] % 4 == 0;
+    e.add[o] = (const float *)adds[o]->data;
+    e.add_s[o][0] = r == 3 ? st[0] : 0;
+    e.add_s[o][1] = st[r - 2];
+  }
+  if (by_rows) {
+    e.inner = out->shape[r - 2];
+    e.rows = numel(ids); e.vocab = table->shape[0]; e.table_stride = table->stride[0]; e.width4 = (int)(table->shape[1] / 4);
+    e.table = (const float *)table->data; e.ids = (const int64_t *)ids->data; e.out = (float *)out->data; e.status = status;
+    if (e.rows * 32 < (1ll << 31) * 256) {
+      FML_LAUNCH((embedding_rows), (unsigned)((e.rows * 32 + 255) / 256), 256, 0, as_stream(stream), e);
+      return FML_OK;
+    }
   }
   FML_LAUNCH((embedding_generic), grid_for(g.total, 256), 256, 0, as_stream(stream), 
       g, add, (float *)out->data, (const float *)table->data, (const int64_t *)ids->data,
