@@ -348,6 +348,116 @@ __global__ void __launch_bounds__(kThreads, MR == 32 ? 1 : 2) gemm_skinny_rows_k
   if (a.splits > 1 && threadIdx.x == 0) a.counters[tile_id] = 0u;  // ready for the next launch
 }
 
+// K-major B, without a second CTA on any output: a CTA has four columns, its eight warps share out the rows (`groups` of R)
+// and, 8 / groups of them, alternate chunks of 128 k values, DEPTH chunks in flight (sixteen 16-byte weight loads per lane
+// with few rows); the sums meet in shared memory.  A classifier head is then one memory round trip and one block barrier, where the slices
+// above meet through scratch memory: fence, counter and a second pass over the partial sums, 3 to 4 us of a small launch,
+// and 32 columns x 8 slices a CTA were too few bytes in flight (1 x 4096 x 1000: 1.1 TB/s).  Weights that no earlier
+// launch writes are asked for before the dependency wait.
+// Captured graphs, us, slices -> this: 1 x 4096 x 1000 12.3 (weights from HBM 14.8) -> 3.2 (4.3), 1 x 1280 x 1000 6.8 -> 2.7,
+// 1 x 25088 x 4096 66 -> 65, 3 x 768 x 768 6.8 -> 2.6, 8 x 4096 x 4096 39 -> 29; against N-major weights on
+// gemm_skinny_rows_kernel 16 x 128 x 512 3.5 -> 2.2, 16 x 512 x 128 7.1 -> 3.9, 24 x 256 x 1024 6.8 -> 4.5, 31 x 768 x 768
+// 11.9 -> 9.9, but 16 x 768 x 3072 9.9 -> 16: there every CTA reads all rows again, so a compiled model's weights are
+// stored K-major only below 16 million multiply-adds.
+constexpr int kCtaCols = 4;
+
+template <int V> __device__ __forceinline__ void warp_reduce_scatter(float (&v)[V], int lane) {
+  // V sums over the warp in V - 1 exchanges and what is left of five: lane l ends with sums l * V / 32 .. (V >= 32), or
+  // l * V / 32 alone (V < 32: lanes share)
+  int n = V;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    if (n > 1) {
+      const bool up = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i)
+        if (i < n / 2) {
+          const float keep = up ? v[i + n / 2] : v[i], send = up ? v[i] : v[i + n / 2];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+      n >>= 1;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+}
+
+template <int R, int DEPTH>
+__global__ void __launch_bounds__(kThreads, 2) gemm_skinny_columns_kernel(const GemmProblem p, const GemmEpilogue e, const int groups) {
+  constexpr int COLS = kCtaCols, V = R * COLS;
+  pdl_launch_dependents();
+  __shared__ float red[kThreads / 32][V];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per = (kThreads / 32) / groups;  // warps of a row group
+  const int z = blockIdx.z, row0 = warp / per * R, M = min(R, (int)p.M - row0);                // this warp's rows
+  const int64_t z0 = z % p.nb0, z1 = z / p.nb0, n0 = (int64_t)blockIdx.x * COLS;
+  const float *const A = p.a + z0 * p.a_b0 + z1 * p.a_b1 + row0 * p.a_sm;
+  const float *const B = p.b + z0 * p.b_b0 + z1 * p.b_b1;
+  const int step = per * 32, quads = (int)(p.K >> 2);  // (K is a multiple of 4)
+  const float4 *bcol[COLS];           // columns past the edge read the last one again
+#pragma unroll
+  for (int j = 0; j < COLS; ++j) bcol[j] = reinterpret_cast<const float4 *>(B + min(n0 + j, p.N - 1) * p.b_sn);
+  float4 w[DEPTH][COLS];
+  auto load = [&](int q0) {
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u) {
+      const int q = q0 + u * step;
+#pragma unroll
+      for (int j = 0; j < COLS; ++j) w[u][j] = q < quads ? __ldcs(bcol[j] + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  int q0 = warp % per * 32 + lane;
+  if (p.b_constant) load(q0);
+  pdl_wait();
+  if (!p.b_constant) load(q0);
+  // what the last phase adds, asked for now: output i = row * COLS + column
+  const int fj = threadIdx.x % COLS, fm = threadIdx.x / COLS;
+  const bool last = fm < (int)p.M && n0 + fj < p.N;
+  float bias = 0.0f, res = 0.0f;
+  if (last && p.bias) bias = p.bias[z0 * p.bias_b0 + z1 * p.bias_b1 + fm * p.bias_sm + (n0 + fj) * p.bias_sn];
+  if (last && p.res) res = p.res[z0 * p.res_b0 + z1 * p.res_b1 + fm * p.res_sm + (n0 + fj) * p.res_sn];
+  float acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = 0.0f;
+  for (; q0 < quads; q0 += DEPTH * step) {
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u) {
+      const int q = q0 + u * step;
+      if (q >= quads) break;
+#pragma unroll
+      for (int m = 0; m < R; ++m)
+        if (m < M) {
+          const float4 x = reinterpret_cast<const float4 *>(A + m * p.a_sm)[q];
+#pragma unroll
+          for (int j = 0; j < COLS; ++j) {
+            float &t = acc[m * COLS + j];
+            t = fmaf(x.x, w[u][j].x, fmaf(x.y, w[u][j].y, fmaf(x.z, w[u][j].z, fmaf(x.w, w[u][j].w, t))));
+          }
+        }
+    }
+    if (q0 + DEPTH * step < quads) load(q0 + DEPTH * step);
+  }
+  warp_reduce_scatter<V>(acc, lane);
+  if (V >= 32) {
+#pragma unroll
+    for (int i = 0; i < (V + 31) / 32; ++i) red[warp][lane * (V / 32) + i] = acc[i];
+  } else if (lane % (32 / (V < 32 ? V : 32)) == 0) {
+    red[warp][lane * V / 32] = acc[0];
+  }
+  __syncthreads();
+  if (!last) return;
+  const int group = fm / R;
+  float v = 0.0f;
+  for (int k = 0; k < per; ++k) v += red[group * per + k][threadIdx.x - group * V];
+  p.c[z0 * p.c_b0 + z1 * p.c_b1 + fm * p.c_sm + (n0 + fj) * p.c_sn] = gemm_epilogue(e, v, bias, res);
+}
+
+// Which products: rows and columns of B on 16-byte boundaries, k in one sweep of a few batches.
+bool by_columns(const GemmProblem &p) {
+  if (p.b_sk != 1 || p.b_sn == 1 || p.a_sk != 1 || p.K % 4 || p.K > (1 << 20)) return false;
+  if (p.a_sm % 4 || p.b_sn % 4 || !aligned16(p.a) || !aligned16(p.b) || p.a_b0 % 4 || p.a_b1 % 4 || p.b_b0 % 4 || p.b_b1 % 4) return false;
+  return p.N < (1ll << 31);
+}
+
 struct SkinnyPlan {
   int splits, tiles_n;
   int64_t k_per_split;
@@ -440,7 +550,25 @@ bool skinny_eligible(const GemmProblem &p) {
          (p.N + kColsPerCta - 1) / kColsPerCta <= 0x7fffffff;
 }
 
+static int launch_columns(const GemmProblem &p, const GemmEpilogue &e, cudaStream_t s) {
+  const unsigned z = (unsigned)(p.nb0 * p.nb1);
+  // row groups: as many as leave every warp a chunk of k, and enough that a warp has at most sixteen rows
+  int groups = p.M > 16 ? 2 : 1;
+  while (groups < 8 && p.M > groups && p.K * groups <= 4 * 128) groups *= 2;
+  const int64_t rows = (p.M + groups - 1) / groups;
+  auto columns = [&](auto kernel) -> int {
+    FML_LAUNCH(kernel, dim3((unsigned)((p.N + kCtaCols - 1) / kCtaCols), 1, z), kThreads, 0, s, p, e, groups);
+    return FML_OK;
+  };
+  if (rows == 1) return columns(gemm_skinny_columns_kernel<1, 4>);
+  if (rows == 2) return columns(gemm_skinny_columns_kernel<2, 4>);
+  if (rows <= 4) return columns(gemm_skinny_columns_kernel<4, 4>);
+  if (rows <= 8) return columns(gemm_skinny_columns_kernel<8, 4>);
+  return columns(gemm_skinny_columns_kernel<16, 2>);
+}
+
 int launch_gemm_skinny(const GemmProblem &p, const GemmEpilogue &e, cudaStream_t s) {
+  if (by_columns(p)) return launch_columns(p, e, s);
   const SkinnyPlan pl = plan_skinny(p);
   void *scratch = nullptr;
   if (pl.scratch_bytes) {
@@ -527,5 +655,6 @@ extern "C" int fml_gemm_skinny_noalloc(const fml_tensor *a, const fml_tensor *b,
     }
     scratch = g_static_scratch_addr[dev];
   }
+  if (by_columns(p)) return launch_columns(p, e, s);  // as fml_gemm (the capacity is checked all the same)
   return launch_skinny(p, e, pl, scratch, s);
 }
