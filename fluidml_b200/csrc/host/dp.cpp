@@ -239,7 +239,7 @@ size_t CostModel::GetTimeCost(const flow::Node &n, const std::vector<Layout> &in
     if (!n.consts.empty()) {
       double w = 1;
       for (size_t i = 1; i < n.consts[0]->meta.GetRank(); ++i) w *= (double)n.consts[0]->meta.GetShape()[i];
-      flops = 2.0 * (double)o.meta.GetElementsNum() * w;
+      flops = 2.0 * (double)o.meta.GetElementsNum() * w * (n.pooled ? 4.0 : 1.0);
     }
     const double bytes = obytes * (n.has_residual ? 2.0 : 1.0) + (double)n.inputs[0]->meta.GetSize();
     cost = kLaunchNs + std::max(flops / kFp32FlopsPerNs, bytes / kHbmBytesPerNs) * (dflt ? 1.0 : 8.0);

@@ -307,6 +307,7 @@ private:
     kernel::KernelOptions ko;
     ko.gemm_precision = options_.gemm_precision;
     const AliasMap aliases = Lowering::ComputeAliases(sequence, ko);
+    Lowering::FoldPools(sequence, aliases, ko);
     Lowering::AttachPlaneSums(sequence, aliases, ko);
     Lowering::ComputeScratch(sequence, ko);
     const std::vector<memory::Info> infos = Lowering::Lifetimes(sequence, aliases);

@@ -71,6 +71,7 @@ struct Node {
   std::vector<RegionPtr> consts;
   RegionPtr output;
   RegionPtr side_output;  // Conv: the sums of the output's planes, for the SqueezeExciteGate that reads them as its inputs[1] (Lowering::AttachPlaneSums)
+  bool pooled = false;    // Conv: output is the 2 x 2 / stride 2 maximum of the convolution (Lowering::FoldPools)
 
   // parameters (which ones are meaningful depends on the kind)
   Type scalar_type = Type::kFloat32;

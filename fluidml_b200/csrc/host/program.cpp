@@ -117,6 +117,38 @@ void Lowering::AttachPlaneSums(flow::Sequence &sequence, const AliasMap &aliases
   }
 }
 
+void Lowering::FoldPools(flow::Sequence &sequence, const AliasMap &aliases, const kernel::KernelOptions &ko) {
+  const kernel::ConstResolver resolve = PlaceholderResolver();
+  std::unordered_map<const flow::Region *, flow::NodePtr> producer;
+  std::unordered_map<const flow::Region *, int> readers;
+  for (const auto &node : sequence.nodes) {
+    producer[node->output.get()] = node;
+    for (const auto &r : node->inputs) ++readers[r.get()];
+  }
+  const std::vector<int64_t> two = {2, 2};
+  std::vector<flow::NodePtr> kept;
+  for (const auto &pool : sequence.nodes) {
+    kept.push_back(pool);
+    if (pool->kind != flow::Kind::MaxPoolWithoutPadding || pool->kernel_shape != two || pool->strides != two) continue;
+    const flow::RegionPtr x = pool->inputs.at(0), y = pool->output;
+    auto it = producer.find(x.get());
+    if (it == producer.end() || x->kind != flow::Region::kInner || readers[x.get()] != 1 || aliases.count(x.get()) || aliases.count(y.get())) continue;
+    const flow::NodePtr &conv = it->second;
+    if ((conv->kind != flow::Kind::ConvWithPadding && conv->kind != flow::Kind::ConvWithoutPadding) || conv->has_in_scale || conv->has_residual) continue;
+    const auto &xs = x->meta.GetShape(), &ys = y->meta.GetShape();
+    if (xs.size() != 4 || xs[2] != 2 * ys[2] || xs[3] != 2 * ys[3]) continue;
+    conv->pooled = true;
+    std::unique_ptr<kernel::Kernel> k = kernel::SelectKernel(*conv, resolve, ko);
+    std::vector<fml_tensor> ins;
+    for (const auto &r : conv->inputs) ins.push_back(kernel::MakeTensor(*r, kPlaceholder));
+    fml_tensor source;
+    if (k->PackedBytes(ins, kernel::MakeTensor(*y, kPlaceholder), &source) == 0) { conv->pooled = false; continue; }
+    conv->output = y;
+    kept.pop_back();
+  }
+  sequence.nodes = std::move(kept);
+}
+
 std::vector<memory::Info> Lowering::Lifetimes(const flow::Sequence &sequence, const AliasMap &aliases) {
   std::unordered_map<const flow::Region *, std::pair<size_t, size_t>> life;
   auto touch = [&](const flow::RegionPtr &r0, size_t i) {

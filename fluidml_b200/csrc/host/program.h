@@ -58,6 +58,9 @@ public:
   // A depthwise convolution in front of a squeeze-and-excite gate, both over the same tensor, leaves the sums of its planes
   // where its kernel can: a tensor of a few kilobytes with a place in the arena, the gate's second input.
   static void AttachPlaneSums(flow::Sequence &sequence, const AliasMap &aliases, const kernel::KernelOptions &ko);
+  // A 2 x 2 / stride 2 max pooling behind a convolution that nothing else reads becomes part of it where the convolution's
+  // kernel pools: the convolution writes the pooled tensor, the other one never exists.
+  static void FoldPools(flow::Sequence &sequence, const AliasMap &aliases, const kernel::KernelOptions &ko);
   // Lifetimes with aliases merged into their owners.
   static std::vector<memory::Info> Lifetimes(const flow::Sequence &sequence, const AliasMap &aliases);
 };

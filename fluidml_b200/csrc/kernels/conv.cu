@@ -548,8 +548,8 @@ __global__ void pool2d_kernel(PoolArgs a) {
   }
 }
 
-// 2 x 2 / stride 2 pooling over dense NCHW planes whose rows are a multiple of 4 long (every
-// pooling layer of VGG-16): a thread reads 16 bytes from each of the two input rows and writes two
+// 2 x 2 / stride 2 pooling over dense NCHW planes whose rows are a multiple of 4 long, where no convolution pools its own
+// result (fml_conv_params::max_pool): a thread reads 16 bytes from each of the two input rows and writes two
 // outputs; 32-bit index arithmetic with two divisions per thread.
 __global__ void __launch_bounds__(256) pool2x2_kernel(const float *__restrict__ x, float *__restrict__ y, unsigned planes,
                                                      unsigned OH, unsigned OW2, unsigned IW, unsigned in_plane, int mode) {
@@ -637,6 +637,12 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
     const int ps = fml_conv_plane_sum_parts(x, w, y, p, &parts);
     if (ps != FML_OK) return ps;
     FML_REQUIRE(parts > 0, FML_UNSUPPORTED, "fml_conv: this layer's kernel leaves no plane sums");
+  }
+  if (p->max_pool) {
+    int uses = 0;
+    const int ps = fml_conv_uses_packed(x, w, y, p, x_scale != nullptr, &uses);
+    if (ps != FML_OK) return ps;
+    FML_REQUIRE(uses && p->w_packed && !residual && !p->plane_sums, FML_UNSUPPORTED, "fml_conv: this layer's kernel does not pool");
   }
   if (bias) {
     FML_REQUIRE(valid_tensor(bias) && bias->dtype == FML_F32 && numel(bias) == a.OC, FML_BAD_ARG,
@@ -837,6 +843,7 @@ static int residual_laid_out_as(const fml_tensor *residual, const fml_tensor *y,
 extern "C" int fml_conv_residual(const fml_tensor *x, const fml_tensor *x_scale, const fml_tensor *w, const fml_tensor *bias,
                                  const fml_tensor *residual, const fml_tensor *y, const fml_conv_params *p, void *stream) {
   FML_REQUIRE(p, FML_BAD_ARG, "fml_conv_residual: bad argument");
+  FML_REQUIRE(!p->max_pool, FML_UNSUPPORTED, "fml_conv_residual: no residual behind a pooled convolution");
   bool same = false;  // then the packed-weight kernel adds it in its epilogue
   if (const int rs = residual_laid_out_as(residual, y, &same); rs != FML_OK) return rs;
   int uses = 0;

@@ -428,6 +428,10 @@ typedef struct fml_conv_params {
   /* Depthwise layers: where to leave the sums of y's planes (after bias and activation), [N * C][parts] floats with the
    * parts that fml_conv_plane_sum_parts names; NULL = not wanted.  FML_UNSUPPORTED where it names none. */
   float *plane_sums;
+  /* Non-zero: y is the 2 x 2 / stride 2 maximum of the convolution (whose height and width are twice y's), pooled before it
+   * leaves the chip.  With packed weights, FML_ACT_RELU, more than one tap, no scale and no residual, where
+   * fml_conv_uses_packed says so for these parameters; FML_UNSUPPORTED otherwise. */
+  int32_t max_pool;
 } fml_conv_params;
 
 /* Partial sums per output plane that fml_conv leaves in plane_sums for this layer, 0 when its kernel leaves none.  Pure
