@@ -108,15 +108,21 @@ __global__ void softmax_rows_generic(RowArgs a, float *out, const float *in, con
 }
 
 // ---- LayerNorm ---------------------------------------------------------------------
-// EARLY: for a few rows (a latency-bound launch) gamma and beta are fetched together with the
-// row instead of after the two reductions, so that their latency overlaps the row's; with many
-// rows the 8 * NV extra registers would cost occupancy and the vectors are cache hits anyway.
-template <int NV, bool EARLY>
-__global__ void layernorm_rows_vec(RowArgs a, float *out, const float *in, const float *res,
+constexpr int kLnThreads = 128;
+// A warp has a row in registers.  EARLY: while one wave of CTAs holds all rows, gamma and beta are fetched together with
+// the row instead of after the two reductions, so that their latency overlaps the row's; with more rows their 8 NV
+// registers would cost occupancy and the vectors are cache hits anyway.  MB: CTAs of kLnThreads per SM, as many as the rows
+// ask for in one wave and no more (at 40 registers the row spills a little).  What a row's address takes in divisions is done
+// before the dependency wait, rows are spread over all SMs first, and NV is 6 for the common 768.  Captured graphs, us,
+// before (8 warps a CTA, NV 8 for 768, addresses after the wait) -> now: 16 x 256 2.17 -> 1.92, 128 x 768 2.87 -> 2.19,
+// 77 x 1024 3.22 -> 2.32, 1024 x 768 3.47 -> 3.18, 2048 x 1024 4.47 -> 3.98, 4100 x 768 7.15 -> 4.86, 6144 x 768 7.60 -> 6.89
+// (5.5 TB/s), 6144 x 1024 10.7 -> 10.2, 12288 x 768 15.6 -> 15.2, 16384 x 384 9.85 -> 9.09.
+template <int NV, bool EARLY, int MB>
+__global__ void __launch_bounds__(kLnThreads, MB) layernorm_rows_vec(RowArgs a, float *out, const float *in, const float *res,
                                    const float *gamma, const float *beta, float eps) {
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
-  const int64_t n4 = a.len >> 2;
+  const int n4 = (int)(a.len >> 2);
   const float4 *g4 = reinterpret_cast<const float4 *>(gamma), *b4 = reinterpret_cast<const float4 *>(beta);
   // While the preceding kernel drains: pull gamma and beta (weights: cold in a pass that
   // streams more weights than L2 holds) into L2.  A prefetch reads nothing into the SM, so it
@@ -129,19 +135,19 @@ __global__ void layernorm_rows_vec(RowArgs a, float *out, const float *in, const
         asm volatile("prefetch.global.L2 [%0];" ::"l"(b4 + lane + 32 * i));
       }
   }
-  pdl_wait();
   const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (row >= a.rows.total) return;
   int64_t off[3];
-  offsets_of(a.rows, row, off);
+  offsets_of(a.rows, min(row, a.rows.total - 1), off);  // (its divisions run while the preceding kernel drains)
   const float4 *x4 = reinterpret_cast<const float4 *>(in + off[1]);
   const float4 *r4 = res ? reinterpret_cast<const float4 *>(res + off[2]) : nullptr;
+  pdl_wait();
+  if (row >= a.rows.total) return;
   float4 v[NV];
   float4 ge[EARLY ? NV : 1], be[EARLY ? NV : 1];
   float s = 0.0f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    int64_t c = lane + 32 * i;
+    const int c = lane + 32 * i;
     if (c < n4) {
       float4 t = x4[c];
       if (r4) { float4 r = r4[c]; t.x += r.x; t.y += r.y; t.z += r.z; t.w += r.w; }
@@ -164,7 +170,7 @@ __global__ void layernorm_rows_vec(RowArgs a, float *out, const float *in, const
   float4 *y4 = reinterpret_cast<float4 *>(out + off[0]);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    int64_t c = lane + 32 * i;
+    const int c = lane + 32 * i;
     if (c < n4) {
       const float4 g = EARLY ? ge[EARLY ? i : 0] : g4[c], b = EARLY ? be[EARLY ? i : 0] : b4[c];
       y4[c] = make_float4(v[i].x * inv * g.x + b.x, v[i].y * inv * g.y + b.y,
@@ -360,17 +366,6 @@ using namespace fml;
     else FML_LAUNCH((KERNEL<32>), grid, 256, 0, stream, __VA_ARGS__);                      \
   } while (0)
 
-// The same ladder for a kernel family named through a macro K(NV).
-#define DISPATCH_NV_FN(per_lane, K, grid, stream, ...)                                     \
-  do {                                                                                     \
-    if ((per_lane) <= 1) FML_LAUNCH((K(1)), grid, 256, 0, stream, __VA_ARGS__);            \
-    else if ((per_lane) <= 2) FML_LAUNCH((K(2)), grid, 256, 0, stream, __VA_ARGS__);       \
-    else if ((per_lane) <= 4) FML_LAUNCH((K(4)), grid, 256, 0, stream, __VA_ARGS__);       \
-    else if ((per_lane) <= 8) FML_LAUNCH((K(8)), grid, 256, 0, stream, __VA_ARGS__);       \
-    else if ((per_lane) <= 16) FML_LAUNCH((K(16)), grid, 256, 0, stream, __VA_ARGS__);     \
-    else FML_LAUNCH((K(32)), grid, 256, 0, stream, __VA_ARGS__);                           \
-  } while (0)
-
 extern "C" int fml_softmax(const fml_tensor *in, const fml_tensor *mask, float divisor,
                            const fml_tensor *out, int axis, void *stream) {
   FML_REQUIRE(in && out, FML_BAD_ARG, "fml_softmax: null tensor");
@@ -405,7 +400,6 @@ extern "C" int fml_layernorm(const fml_tensor *in, const fml_tensor *residual,
               FML_BAD_ARG, "fml_layernorm: scale/bias must hold one value per normalised element");
   if (a.rows.total == 0 || a.len == 0) return FML_OK;
   cudaStream_t s = as_stream(stream);
-  const unsigned grid = (unsigned)((a.rows.total * 32 + 255) / 256);
   const float *rp = residual ? (const float *)residual->data : nullptr;
   // stride of the (single) non-unit dim of scale / bias
   auto vec_stride = [](const fml_tensor *t) {
@@ -416,17 +410,29 @@ extern "C" int fml_layernorm(const fml_tensor *in, const fml_tensor *residual,
   const bool res_vec = !residual || a.axis_stride[2] == 1;
   if (rows_vec_ok(a, out->data, in->data, rp) && res_vec && gs == 1 && bs == 1 &&
       aligned16(scale->data) && aligned16(bias->data)) {
-#define LN_EARLY(NV) layernorm_rows_vec<NV, true>
-#define LN_LATE(NV) layernorm_rows_vec<NV, false>
     const int64_t per_lane = (a.len / 4 + 31) / 32;
-    if (a.rows.total <= 4096 && per_lane <= 8)
-      DISPATCH_NV_FN(per_lane, LN_EARLY, grid, s, a, (float *)out->data, (const float *)in->data, rp, (const float *)scale->data, (const float *)bias->data, eps);
-    else
-      DISPATCH_NV_FN(per_lane, LN_LATE, grid, s, a, (float *)out->data, (const float *)in->data, rp, (const float *)scale->data, (const float *)bias->data, eps);
-#undef LN_EARLY
-#undef LN_LATE
+    const int threads = a.rows.total <= 148 ? 32 : a.rows.total <= 296 ? 64 : kLnThreads;
+    const unsigned ctas = (unsigned)((a.rows.total * 32 + threads - 1) / threads);
+#define LN_GO(NV, EARLY, MB) \
+  FML_LAUNCH((layernorm_rows_vec<NV, EARLY, MB>), ctas, threads, 0, s, a, (float *)out->data, (const float *)in->data, rp, (const float *)scale->data, (const float *)bias->data, eps)
+    const auto one_wave = [&](int per_sm) { return a.rows.total <= 148ll * per_sm * (kLnThreads / 32); };
+    if (per_lane <= 6 && one_wave(5)) {
+      if (per_lane <= 1) LN_GO(1, true, 5);
+      else if (per_lane <= 2) LN_GO(2, true, 5);
+      else if (per_lane <= 4) LN_GO(4, true, 5);
+      else LN_GO(6, true, 5);
+    } else if (per_lane <= 1) LN_GO(1, false, 12);
+    else if (per_lane <= 2) LN_GO(2, false, 12);
+    else if (per_lane <= 4) LN_GO(4, false, 12);
+    else if (per_lane <= 6 && one_wave(8)) LN_GO(6, false, 8);  // (3072-4100 rows of 768: 4.8-5.0 us, 5.9-6.4 with 12)
+    else if (per_lane <= 6) LN_GO(6, false, 12);                // (6144 rows: 6.8, 8.2 with 8)
+    else if (per_lane <= 8 && one_wave(4)) LN_GO(8, true, 4);
+    else if (per_lane <= 8) LN_GO(8, false, 7);                 // (6144 x 1024: 10.1, 10.5 with 9, 11.2 with 10)
+    else if (per_lane <= 16) LN_GO(16, false, 1);
+    else LN_GO(32, false, 1);
+#undef LN_GO
   } else {
-    FML_LAUNCH((layernorm_rows_generic), grid, 256, 0, s, a, (float *)out->data, (const float *)in->data, rp,
+    FML_LAUNCH((layernorm_rows_generic), (unsigned)((a.rows.total * 32 + 255) / 256), 256, 0, s, a, (float *)out->data, (const float *)in->data, rp,
                                                 (const float *)scale->data, gs,
                                                 (const float *)bias->data, bs, eps);
   }
