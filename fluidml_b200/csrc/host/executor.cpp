@@ -226,7 +226,7 @@ private:
       reference_linear = Planner::Plan(infos, MemoryPlanKind::kLinear, 1).GetMaximum();
     }
     const size_t nodes_before_fusion = flow.nodes.size();
-    if (options_.fusion) FusionPasses::Run(flow, options_.gemm_precision == FML_GEMM_AUTO && !options_.resident);
+    if (options_.fusion) FusionPasses::Run(flow, options_.gemm_precision == FML_GEMM_AUTO && !options_.resident, layout_ == LayoutMode::kDP);
 
     flow::Sequence sequence = Planner::TopologicalSort(flow);
     json::Value dp_json = json::Value::Object();

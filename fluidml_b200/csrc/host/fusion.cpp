@@ -846,6 +846,57 @@ bool JoinConcatenatedProduct(Rewriter &rw, const NodePtr &cat) {
   return true;
 }
 
+// ---- 1-D pointwise convolution -> Transpose (0, 2, 1): the product [B, L, C] x [C, OC] it is, read and written with the
+// channels innermost, where what stands in front is a depthwise convolution over a transposed view, whose result the layout
+// search can leave in that order too (ConvBERT: nothing changes between the orders any more, and the product with the
+// queries behind it reads rows).  Only layers that the packed convolution takes: the arithmetic stays half-precision pairs.
+bool PointwiseAsProduct(Rewriter &rw, const NodePtr &cv) {
+  if (cv->kind != Kind::ConvWithoutPadding || cv->inputs.size() != 1 || cv->group != 1 || cv->act != 0 || cv->has_in_scale || cv->has_residual) return false;
+  const auto &xs = cv->inputs[0]->meta.GetShape();
+  if (xs.size() != 3 || IsConst(cv->inputs[0]) || cv->strides != std::vector<int64_t>{1} || cv->dilations != std::vector<int64_t>{1}) return false;
+  auto made_by = [&](const RegionPtr &r) -> NodePtr {
+    auto it = rw.producer.find(r.get());
+    return it == rw.producer.end() ? nullptr : it->second;
+  };
+  const NodePtr dw = made_by(cv->inputs[0]);
+  if (!dw || rw.Sole(dw->output) != cv || (dw->kind != Kind::ConvWithPadding && dw->kind != Kind::ConvWithoutPadding) || dw->group != xs[1] || dw->group < 2) return false;
+  const NodePtr before = made_by(dw->inputs[0]);
+  if (!before || before->kind != Kind::Transpose || before->perm != std::vector<int64_t>{0, 2, 1}) return false;
+  const NodePtr tr = rw.SoleOfKind(cv->output, Kind::Transpose);
+  if (!tr || tr->perm != std::vector<int64_t>{0, 2, 1}) return false;
+  const int64_t B = xs[0], IC = xs[1], L = xs[2];
+  const auto &ws = cv->consts.at(0)->meta.GetShape();
+  if (ws.size() != 3 || ws[1] != IC || ws[2] != 1) return false;
+  const int64_t OC = ws[0];
+  if (L % 4 != 0 || L < 32 || IC % 4 != 0 || IC < 32 || OC % 4 != 0 || OC < 64) return false;
+  if (!HoldsFloats(cv->consts[0], 3, (size_t)(OC * IC)) || (cv->has_bias && !HoldsFloats(cv->consts.at(1), 1, (size_t)OC))) return false;
+  std::vector<uint8_t> bytes((size_t)(OC * IC) * 4);
+  const float *w = reinterpret_cast<const float *>(cv->consts[0]->constant->Bytes().data());
+  float *wt = reinterpret_cast<float *>(bytes.data());
+  for (int64_t o = 0; o < OC; ++o)
+    for (int64_t c = 0; c < IC; ++c) wt[c * OC + o] = w[o * IC + c];
+  std::vector<RegionPtr> consts = {MakeConstant(rw.f, cv->name + "_columns", {IC, OC}, std::move(bytes))};
+  if (cv->has_bias) consts.push_back(cv->consts[1]);
+  auto rows = std::make_shared<flow::Region>();
+  rows->kind = flow::Region::kInner;
+  rows->name = cv->name + "_rows";
+  rows->meta = Meta(Type::kFloat32, {B, L, IC});
+  rows->layout = utils::GenDefaultLayout(3);
+  rw.f.regions.push_back(rows);
+  rw.f.by_name[rows->name] = rows;
+  tr->kind = Kind::FusedGemm;
+  tr->inputs = {rows};
+  tr->consts = std::move(consts);
+  tr->b_is_const = true;
+  tr->has_bias = cv->has_bias;
+  cv->kind = Kind::Transpose;
+  cv->perm = {0, 2, 1};
+  cv->consts.clear();
+  cv->has_bias = false;
+  cv->output = rows;
+  return true;
+}
+
 // ---- Conv -> SiLU: the activation rides in the convolution's epilogue
 bool FuseSiluIntoConv(Rewriter &rw, const NodePtr &cv) {
   if ((cv->kind != Kind::ConvWithPadding && cv->kind != Kind::ConvWithoutPadding) || cv->act != 0) return false;
@@ -970,7 +1021,7 @@ bool MergeSiblingGemms(flow::Flow &f, bool join) {
 
 }  // namespace
 
-size_t FusionPasses::Run(flow::Flow &flow, bool join) {
+size_t FusionPasses::Run(flow::Flow &flow, bool join, bool relayout) {
   const size_t before = flow.nodes.size();
   Rewriter rw(flow);
   using Pass = bool (*)(Rewriter &, const NodePtr &);
@@ -991,6 +1042,7 @@ size_t FusionPasses::Run(flow::Flow &flow, bool join) {
   if (join) {
     until_done(FuseRotaryIntoGemm);
     while (FoldSharedLayerNorms(rw)) {}
+    if (relayout) until_done(PointwiseAsProduct);
   }
   while (MergeSiblingGemms(flow, join)) {}
   if (join) {

@@ -14,7 +14,7 @@ public:
   // Rewrites `flow` in place; returns the number of nodes removed.  `join`: products may be joined beyond what every
   // GEMM kernel takes in one launch (rotations and activations of some columns, two left-hand sides), which pays
   // where the packed-weight kernel runs them.
-  static size_t Run(flow::Flow &flow, bool join);
+  static size_t Run(flow::Flow &flow, bool join, bool relayout);
 };
 
 }  // namespace worker
