@@ -177,3 +177,56 @@ def test_a_concatenation_in_front_of_a_product(k1, k2, m):
     ex = Executor.make_dp_greedy("t").compile(model.to_bytes())
     ex.invoke({**x, **out})
     assert close(out["y"], orc.run_model(model, x, acc64=True)["y"])
+
+
+def two_halves(apart, top, rows=64, k1=256, k2=512, n=64):
+    """(a1 W1 + a2 W2) + x whose halves contribute alike, W of one half (0: the first) `apart` times the other's."""
+    rng = np.random.default_rng(int(np.log2(apart)) * 2 + top)
+    f32 = lambda *s: rng.standard_normal(s).astype(np.float32)
+    w1, w2, feeds = f32(k1, n), f32(k2, n), {"a1": f32(rows, k1), "a2": f32(rows, k2), "x": f32(rows, n)}
+    if top:
+        w2, feeds["a2"] = w2 * np.float32(apart), feeds["a2"] / np.float32(apart)
+    else:
+        w1, feeds["a1"] = w1 * np.float32(apart), feeds["a1"] / np.float32(apart)
+    g = models.GraphBuilder("halves")
+    a1, a2, x = (g.input(name, FLOAT, v.shape) for name, v in feeds.items())
+    g.add(g.add(g.matmul(a1, g.const("w1", w1)), g.matmul(a2, g.const("w2", w2))), x, out="y")
+    g.output("y")
+    wide = {k: v.astype(np.float64) for k, v in feeds.items()}
+    ref = wide["a1"] @ w1 + wide["a2"] @ w2 + wide["x"]
+    size = np.abs(wide["a1"]) @ np.abs(w1) + np.abs(wide["a2"]) @ np.abs(w2) + np.abs(wide["x"])
+    return g.finish(), feeds, ref, size
+
+
+def products(model):
+    return [n["kind"] for n in Executor.make_plain_greedy("t").plan(model.to_bytes())["sequence"]].count("FusedGemm")
+
+
+@pytest.mark.parametrize("top", [0, 1])
+def test_halves_are_joined_where_their_weights_are_of_one_magnitude(top):
+    assert products(two_halves(1, top)[0]) == 1
+    assert products(two_halves(2, top)[0]) == 1
+    for apart in (2.0 ** 6, 2.0 ** 12, 2.0 ** 20):
+        assert products(two_halves(apart, top)[0]) == 2
+    # one column is enough
+    rng = np.random.default_rng(0)
+    w = [rng.standard_normal((64, 64)).astype(np.float32) for _ in range(2)]
+    w[top][:, 17] = 0.0
+    g = models.GraphBuilder("column")
+    a, b, x = (g.input(name, FLOAT, (64, 64)) for name in "abx")
+    g.add(g.add(g.matmul(a, g.const("w1", w[0])), g.matmul(b, g.const("w2", w[1]))), x, out="y")
+    g.output("y")
+    assert products(g.finish()) == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("top", [0, 1])
+@pytest.mark.parametrize("apart", [1.0, 2.0, 2.0 ** 6, 2.0 ** 12, 2.0 ** 20])
+def test_halves_that_differ_in_magnitude(apart, top):
+    """Operands of 22 bits are off by 2^-22 each.  An accumulator takes sixteen products at a time, three times over, and
+    each time cuts its sum to 24 bits: 2^-23 of it.  Bias and residual round twice more."""
+    model, feeds, ref, size = two_halves(apart, top)
+    out = {"y": np.zeros(ref.shape, np.float32)}
+    Executor.make_dp_greedy("t").compile(model.to_bytes()).invoke({**feeds, **out})
+    steps = 3 * (256 + 512) // 16
+    assert (np.abs(out["y"] - ref) <= (2.0 ** -21 + (steps + 2) * 2.0 ** -23) * size).all()
