@@ -100,8 +100,9 @@ struct Node {
   // LayerNorm, a padded copy for ConvWithPadding); used to report the reference-equivalent
   // arena.  The CUDA kernels need none of it.
   size_t reference_buffer_size = 0;
-  // Scratch bytes this back end needs (split-K partial tiles), filled by the planner.
+  // Scratch bytes this back end needs (split-K partial tiles), and the arena tenant they are, both filled by the planner.
   size_t buffer_size = 0;
+  std::string buffer_name;
 };
 using NodePtr = std::shared_ptr<Node>;
 
@@ -115,6 +116,23 @@ struct Flow {
     auto it = by_name.find(n);
     if (it == by_name.end()) throw Error("flow has no region '" + n + "'");
     return it->second;
+  }
+  // `base`, or `base` and a number where a tensor has that name: interface tensors, the arena and saved plans go by name.
+  std::string NewName(const std::string &base) const {
+    std::string name = base;
+    for (size_t i = 2; by_name.count(name); ++i) name = base + "#" + std::to_string(i);
+    return name;
+  }
+  // A region of this back end's own making.
+  RegionPtr NewRegion(Region::Kind kind, const std::string &base, Meta meta) {
+    auto r = std::make_shared<Region>();
+    r->kind = kind;
+    r->name = NewName(base);
+    r->meta = std::move(meta);
+    r->layout = utils::GenDefaultLayout(r->meta.GetRank());
+    regions.push_back(r);
+    by_name[r->name] = r;
+    return r;
   }
 };
 

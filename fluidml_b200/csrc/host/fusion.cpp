@@ -19,6 +19,7 @@ struct Rewriter {
   std::unordered_map<const flow::Region *, std::vector<NodePtr>> consumers;
   std::unordered_map<const flow::Region *, NodePtr> producer;
   std::unordered_set<const flow::Node *> dead;
+  std::unordered_map<RegionPtr, RegionPtr> table_rows;  // the rows of a rotary table (FuseRotaryIntoGemm)
 
   explicit Rewriter(flow::Flow &flow) : f(flow) { Index(); }
 
@@ -303,14 +304,8 @@ bool FuseScaledMaskedSoftmax(Rewriter &rw, const NodePtr &div) {
     float *m = reinterpret_cast<float *>(bytes.data());
     const float y = (float)where->value;
     for (int64_t i = 0; i < n; ++i) m[i] = cond->constant->AsInt(i) ? 0.0f : y;
-    mask = std::make_shared<flow::Region>();
-    mask->kind = flow::Region::kConstant;
-    mask->name = where->name + "_additive_mask";
-    mask->meta = Meta(Type::kFloat32, cond->meta.GetShape());
-    mask->layout = utils::GenDefaultLayout(cond->meta.GetRank());
+    mask = rw.f.NewRegion(flow::Region::kConstant, where->name + "_additive_mask", Meta(Type::kFloat32, cond->meta.GetShape()));
     mask->constant = std::make_shared<Tensor>(mask->meta, std::move(bytes));
-    rw.f.regions.push_back(mask);
-    rw.f.by_name[mask->name] = mask;
   }
   sm->kind = Kind::FusedSoftmax;
   sm->divisor = (float)div->value;
@@ -655,14 +650,8 @@ bool FuseRotary(Rewriter &rw, const NodePtr &cat) {
 
 // A constant of our own making.
 RegionPtr MakeConstant(flow::Flow &f, const std::string &name, std::vector<int64_t> shape, std::vector<uint8_t> bytes) {
-  auto r = std::make_shared<flow::Region>();
-  r->kind = flow::Region::kConstant;
-  r->name = name;
-  r->meta = Meta(Type::kFloat32, shape);
-  r->layout = utils::GenDefaultLayout(shape.size());
+  const RegionPtr r = f.NewRegion(flow::Region::kConstant, name, Meta(Type::kFloat32, shape));
   r->constant = std::make_shared<Tensor>(r->meta, std::move(bytes));
-  f.regions.push_back(r);
-  f.by_name[name] = r;
   return r;
 }
 
@@ -714,8 +703,9 @@ bool FuseRotaryIntoGemm(Rewriter &rw, const NodePtr &rot) {
   RegionPtr tables[2];
   for (size_t i = 0; i < 2; ++i) {  // rows of this node's own: the layout search may permute what other nodes read
     const RegionPtr &t = rot->inputs[1 + i];
-    auto it = rw.f.by_name.find(t->name + "_rows");
-    tables[i] = it != rw.f.by_name.end() ? it->second : MakeConstant(rw.f, t->name + "_rows", {length, width}, t->constant->Bytes());
+    RegionPtr &rows = rw.table_rows[t];
+    if (!rows) rows = MakeConstant(rw.f, t->name + "_rows", {length, width}, t->constant->Bytes());
+    tables[i] = rows;
   }
   mm->consts.push_back(tables[0]);
   mm->consts.push_back(tables[1]);
@@ -904,13 +894,7 @@ bool PointwiseAsProduct(Rewriter &rw, const NodePtr &cv) {
     for (int64_t c = 0; c < IC; ++c) wt[c * OC + o] = w[o * IC + c];
   std::vector<RegionPtr> consts = {MakeConstant(rw.f, cv->name + "_columns", {IC, OC}, std::move(bytes))};
   if (cv->has_bias) consts.push_back(cv->consts[1]);
-  auto rows = std::make_shared<flow::Region>();
-  rows->kind = flow::Region::kInner;
-  rows->name = cv->name + "_rows";
-  rows->meta = Meta(Type::kFloat32, {B, L, IC});
-  rows->layout = utils::GenDefaultLayout(3);
-  rw.f.regions.push_back(rows);
-  rw.f.by_name[rows->name] = rows;
+  const RegionPtr rows = rw.f.NewRegion(flow::Region::kInner, cv->name + "_rows", Meta(Type::kFloat32, {B, L, IC}));
   tr->kind = Kind::FusedGemm;
   tr->inputs = {rows};
   tr->consts = std::move(consts);
@@ -986,15 +970,9 @@ bool MergeSiblingGemms(flow::Flow &f, bool join) {
     const std::string base = first->name + "_merged";
     RegionPtr wcat = MakeConstant(f, base + ".w", {K, total}, std::move(wbytes));
     RegionPtr bcat = first->has_bias ? MakeConstant(f, base + ".b", {total}, std::move(bbytes)) : nullptr;
-    auto merged = std::make_shared<flow::Region>();
-    merged->kind = flow::Region::kInner;
-    merged->name = base;
     std::vector<int64_t> mshape = first->output->meta.GetShape();
     mshape.back() = total;
-    merged->meta = Meta(Type::kFloat32, mshape);
-    merged->layout = utils::GenDefaultLayout(mshape.size());
-    f.regions.push_back(merged);
-    f.by_name[base] = merged;
+    const RegionPtr merged = f.NewRegion(flow::Region::kInner, base, Meta(Type::kFloat32, mshape));
     // slices that hand the original outputs back
     std::vector<NodePtr> slices;
     col = 0;

@@ -29,6 +29,22 @@ const flow::RegionPtr &Owner(const AliasMap &aliases, const flow::RegionPtr &r) 
   return it == aliases.end() ? r : it->second;
 }
 
+// Names of the arena's tenants that are no tensors of the model: unlike every tensor's and every other's.
+class Names {
+public:
+  explicit Names(const flow::Sequence &sequence) {
+    for (const auto &r : sequence.regions) taken_.insert(r->name);
+  }
+  std::string New(const std::string &base) {
+    std::string name = base;
+    for (size_t i = 2; !taken_.insert(name).second; ++i) name = base + "#" + std::to_string(i);
+    return name;
+  }
+
+private:
+  std::unordered_set<std::string> taken_;
+};
+
 // Row-major logical bytes -> bytes in the region's physical order (builder.cpp:280-296).
 std::vector<uint8_t> PermuteConstant(const flow::Region &r) {
   const std::vector<uint8_t> &src = r.constant->Bytes();
@@ -94,6 +110,7 @@ void Lowering::AttachPlaneSums(flow::Sequence &sequence, const AliasMap &aliases
   const kernel::ConstResolver resolve = PlaceholderResolver();
   std::unordered_map<const flow::Region *, flow::NodePtr> producer;
   for (const auto &node : sequence.nodes) producer[node->output.get()] = node;
+  Names names(sequence);
   for (const auto &gate : sequence.nodes) {
     if (gate->kind != flow::Kind::SqueezeExciteGate || gate->inputs.size() != 1) continue;
     const flow::RegionPtr x = gate->inputs[0];
@@ -108,7 +125,7 @@ void Lowering::AttachPlaneSums(flow::Sequence &sequence, const AliasMap &aliases
     const auto &shape = x->meta.GetShape();
     auto sums = std::make_shared<flow::Region>();
     sums->kind = flow::Region::kInner;
-    sums->name = conv->name + "_plane_sums";
+    sums->name = names.New(conv->name + "_plane_sums");
     sums->meta = Meta(Type::kFloat32, {shape[0], shape[1], (int64_t)parts});
     sums->layout = utils::GenDefaultLayout(3);
     sequence.regions.push_back(sums);
@@ -169,9 +186,13 @@ std::vector<memory::Info> Lowering::Lifetimes(const flow::Sequence &sequence, co
     if (it == life.end()) continue;
     infos.push_back({r->name, it->second.first, it->second.second, r->meta.GetSize()});
   }
-  for (size_t i = 0; i < sequence.nodes.size(); ++i)
-    if (sequence.nodes[i]->buffer_size > 0)
-      infos.push_back({sequence.nodes[i]->name, i, i, sequence.nodes[i]->buffer_size});
+  Names names(sequence);
+  for (size_t i = 0; i < sequence.nodes.size(); ++i) {
+    const flow::NodePtr &node = sequence.nodes[i];
+    if (node->buffer_size == 0) continue;
+    node->buffer_name = names.New(node->name);
+    infos.push_back({node->buffer_name, i, i, node->buffer_size});
+  }
   return infos;
 }
 
@@ -439,7 +460,7 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
     if (need > node->buffer_size)
       throw Error("node '" + node->name + "' needs more scratch than was planned for it");
     if (need > 0) {
-      buf.data = (char *)prog->arena + index.Get(node->name);
+      buf.data = (char *)prog->arena + index.Get(node->buffer_name);
       buf.bytes = node->buffer_size;
     }
     if (node->side_output) {
