@@ -860,6 +860,8 @@ static int conv_impl(const fml_tensor *x, const fml_tensor *x_scale, const fml_t
       int st = FML_OK;
       if (launch_depthwise_tma(x, w, bias, y, p, s, &st)) return st;
     }
+    // (the kernel is the right one, but its tensor map or status word could not be had; the ones below leave no sums)
+    FML_REQUIRE(!p->plane_sums, FML_CUDA_ERROR, "fml_conv: the kernel that leaves plane sums cannot be launched");
     if (a.dh == 1 && a.dw == 1 && a.sh == a.sw && (a.sh == 1 || a.sh == 2) && a.xs[3] == 1) {
       int st = FML_OK;
       bool done = false;

@@ -2,6 +2,9 @@
 
 Tolerance: a sum of K fp32 terms, in any order, is off by at most K 2^-24 sum|terms|; carried through the gate's layers."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -94,6 +97,28 @@ def test_where_there_are_no_sums():
     last = [0, 3, 1, 2]
     p = params(8, 3, 1, cabi.ACT_NONE)
     assert parts_of(Host((1, 8, 32, 32), last), w, Host((1, 8, 32, 32), last), p) == 0  # channels innermost
+
+
+def test_a_layer_that_cannot_leave_its_sums_is_an_error():
+    """Without a device there is no status word: the layer must not go on to a kernel that ignores the sums."""
+    code = """if True:
+        import ctypes, sys
+        sys.path[:0] = ["tests"]
+        from test_plane_sums_gpu import Host, cabi, params
+        for size in (32, 7):   # either of the kernels that leave sums
+            x, w, y, sums = Host((1, 8, size, size)), Host((8, 1, 3, 3)), Host((1, 8, size, size)), Host((8, 1))
+            p = params(8, 3, 1, cabi.ACT_NONE)
+            p.plane_sums = sums.c().data
+            try:
+                cabi.check(cabi.lib().fml_conv(ctypes.byref(x.c()), ctypes.byref(w.c()), None, ctypes.byref(y.c()), ctypes.byref(p), None))
+            except cabi.FmlError as e:
+                assert "plane sums" in str(e), e
+            else:
+                raise SystemExit("no error")
+    """
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, env={**os.environ, "CUDA_VISIBLE_DEVICES": "", "PYTHONPATH": root}, capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
 
 
 def test_the_plan_gives_the_sums_a_place():
