@@ -618,7 +618,7 @@ bool plan_depthwise_tma(const fml_tensor *x, const fml_tensor *w, const fml_tens
 
 // Partial sums per plane that the layer's kernel can leave (fml_conv_params::plane_sums), 0 when it is another kernel's.
 int depthwise_sum_parts(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p) {
-  if (!depthwise_pipelined(x, w, y, p)) return 0;
+  if (!depthwise_pipelined(x, w, y, p) || numel(x) == 0 || numel(y) == 0) return 0;  // (nothing is launched over empty planes)
   DwTmaArgs t;
   DwFlatArgs f;
   size_t bytes;

@@ -30,6 +30,13 @@ def parts_of(x, w, y, p):
     return n.value
 
 
+def alone(code):
+    """What a process of its own, without a device, has to say about `code`: nothing when it ends well."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, env={**os.environ, "CUDA_VISIBLE_DEVICES": "", "PYTHONPATH": root}, capture_output=True, text=True)
+    return "" if done.returncode == 0 else f"{done.returncode}: {done.stderr}"
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("k", [3, 5])
 @pytest.mark.parametrize("stride", [1, 2])
@@ -99,6 +106,18 @@ def test_where_there_are_no_sums():
     assert parts_of(Host((1, 8, 32, 32), last), w, Host((1, 8, 32, 32), last), p) == 0  # channels innermost
 
 
+@pytest.mark.parametrize("x,y", [((1, 8, 32, 32), (1, 8, 0, 32)), ((1, 8, 7, 7), (1, 8, 7, 0)), ((1, 8, 0, 32), (1, 8, 0, 32)), ((0, 8, 32, 32), (0, 8, 32, 32)),
+                                 ((0, 8, 7, 7), (0, 8, 7, 7))])
+def test_empty_planes_have_no_sums(x, y):
+    code = f"""if True:
+        import sys
+        sys.path[:0] = ["tests"]
+        from test_plane_sums_gpu import Host, params, parts_of
+        assert parts_of(Host({x}), Host((8, 1, 3, 3)), Host({y}), params(8, 3, 1, 0)) == 0
+    """
+    assert alone(code) == ""  # a process of its own: a division by zero would end this one
+
+
 def test_a_layer_that_cannot_leave_its_sums_is_an_error():
     """Without a device there is no status word: the layer must not go on to a kernel that ignores the sums."""
     code = """if True:
@@ -116,9 +135,7 @@ def test_a_layer_that_cannot_leave_its_sums_is_an_error():
             else:
                 raise SystemExit("no error")
     """
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    done = subprocess.run([sys.executable, "-c", code], cwd=root, env={**os.environ, "CUDA_VISIBLE_DEVICES": "", "PYTHONPATH": root}, capture_output=True, text=True)
-    assert done.returncode == 0, done.stderr
+    assert alone(code) == ""
 
 
 def test_the_plan_gives_the_sums_a_place():
