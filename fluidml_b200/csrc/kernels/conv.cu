@@ -1010,8 +1010,8 @@ extern "C" int fml_conv_tuning_key(const fml_tensor *x, const fml_tensor *w, con
   Planes pl;
   const bool planes = !scaled && as_planes(x, w, y, p, &pl);
   const fml_conv_params q = planes ? plane_params(p) : *p;
-  snprintf(key, bytes, "%s", !uses ? "" : planes ? conv_tuning_key(device, &pl.x, &pl.w, &pl.y, &q, false, false).c_str()
-                                                 : conv_tuning_key(device, x, w, y, &q, scaled != 0, residual != 0).c_str());
+  snprintf(key, bytes, "%s", !uses ? "" : planes ? conv_tuning_key(device, &pl.x, &pl.w, &pl.y, &q, false, false, false).c_str()
+                                                 : conv_tuning_key(device, x, w, y, &q, scaled != 0, residual != 0, conv_tunes_fma(x, w, y, &q, scaled != 0)).c_str());
   return FML_OK;
 }
 

@@ -1116,15 +1116,22 @@ int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor 
   return launch_planned(a, smem, x, bias, y, p, s, x_scale, x_scale_sn, x_scale_sc, residual);
 }
 
-// What a remembered choice of tiles belongs to: the device, the layer, the layout it writes and its epilogue.
+// Whether the FMA kernel's splits are among a layer's candidates: a pointwise layer with little arithmetic (conv_pointwise.cu).
+bool conv_tunes_fma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled) {
+  double us = 0.0;
+  return pointwise_fma_plan(x, w, y, p, scaled, &us) && us < 24.0;
+}
+
+// What a remembered choice of tiles belongs to: the device, the layer, the layout it writes, its epilogue and whether it
+// may name the FMA kernel (a 1-D layer seen as planes may not).
 std::string conv_tuning_key(int device, const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled,
-                            bool residual) {
+                            bool residual, bool fma) {
   char key[320];
   snprintf(key, sizeof(key), "%d|%lld,%lld,%lld,%lld|%lld,%lld,%lld|%lld,%lld|%lld,%lld,%lld,%lld|%d,%d,%d", device, (long long)x->shape[0],
            (long long)x->shape[1], (long long)x->shape[2], (long long)x->shape[3], (long long)w->shape[0], (long long)w->shape[2],
            (long long)w->shape[3], (long long)p->pads_begin[0], (long long)p->pads_begin[1], (long long)y->stride[0], (long long)y->stride[1],
            (long long)y->stride[2], (long long)y->stride[3], p->act, scaled, residual);
-  return p->max_pool ? std::string(key) + "|pool" : key;
+  return std::string(key) + (p->max_pool ? "|pool" : "") + (fma ? "|fma" : "");
 }
 
 // Times the candidates the model ranks highest as captured graphs of back-to-back launches and keeps the
@@ -1133,7 +1140,8 @@ int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
                    const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, bool pointwise_fma, fml_conv_params *tuned) {
   int device = 0;
   FML_CUDA(cudaGetDevice(&device));
-  const std::string key = conv_tuning_key(device, x, w, y, p, x_scale != nullptr, residual != nullptr);
+  const bool fma = pointwise_fma && conv_tunes_fma(x, w, y, p, x_scale != nullptr);
+  const std::string key = conv_tuning_key(device, x, w, y, p, x_scale != nullptr, residual != nullptr, fma);
   struct Choice { int tile_n, strips, split_k, occ, fma; };
   static std::map<std::string, Choice> cache;
   static std::mutex mu;
@@ -1155,10 +1163,7 @@ int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
   FML_CUDA(cudaEventCreate(&e1));
   float best = 1e30f;
   Choice c{all[0].a.tile_n, all[0].a.mt, all[0].a.split_k, all[0].occ, 0};
-  // a pointwise layer with little arithmetic: the FMA kernel's splits too (conv_pointwise.cu)
   static const int fma_splits[][2] = {{1, 1}, {2, 1}, {4, 1}, {8, 1}, {8, 2}, {8, 4}, {8, 8}};
-  double fma_us = 0.0;
-  const bool fma = pointwise_fma && pointwise_fma_plan(x, w, y, p, x_scale != nullptr, &fma_us) && fma_us < 24.0;
   const size_t pairs = std::min<size_t>(all.size(), 16);
   for (size_t i = 0; i < pairs + (fma ? 7 : 0); ++i) {
     fml_conv_params q = *p;

@@ -127,6 +127,7 @@ int launch_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor 
 int tune_conv_pair(const fml_tensor *x, const fml_tensor *w, const fml_tensor *bias, const fml_tensor *y, const fml_conv_params *p,
                    const float *x_scale, int64_t x_scale_sn, int64_t x_scale_sc, const float *residual, bool pointwise_fma, fml_conv_params *tuned);
 std::string conv_tuning_key(int device, const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled,
-                            bool residual);
+                            bool residual, bool fma);
+bool conv_tunes_fma(const fml_tensor *x, const fml_tensor *w, const fml_tensor *y, const fml_conv_params *p, bool scaled);
 
 }  // namespace fml

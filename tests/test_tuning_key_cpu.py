@@ -47,6 +47,21 @@ def test_every_part_of_the_signature_counts(key, changes):
     assert keys[0] and len(set(keys)) == len(keys) and key() == keys[0]
 
 
+def test_who_may_not_choose_the_fma_kernel_has_a_key_of_its_own():
+    """The same planes as a 1-D layer (packed kernel only) and as a 2-D one."""
+    def key(x, w, y):
+        p = cabi.ConvParams()
+        for i in range(2):
+            p.strides[i] = p.dilations[i] = 1
+        p.group = 1
+        buf = ctypes.create_string_buffer(512)
+        cabi.check(cabi.lib().fml_conv_tuning_key(ctypes.byref(x), ctypes.byref(w), ctypes.byref(y), ctypes.byref(p), 0, 0, 0, buf, ctypes.c_size_t(512)))
+        return buf.value
+    line = key(tensor((2, 96, 64)), tensor((64, 96, 1)), tensor((2, 64, 64)))
+    plane = key(tensor((2, 96, 1, 64)), tensor((64, 96, 1, 1), [1, 64, 96 * 64, 96 * 64]), tensor((2, 64, 1, 64)))
+    assert line and plane and line != plane
+
+
 def test_nothing_to_choose():
     assert conv_key(hw=1) == b""
     assert gemm_key(m=4) == b""
