@@ -51,8 +51,44 @@ std::optional<Meta> BroadcastMatMulShape(const Meta &lhs, const Meta &rhs, Type 
   return Meta(type, std::move(out));
 }
 
+void Tensor::WriteRow(int64_t row, float *dst) const {
+  if (blocks_.empty()) {
+    const size_t n = (size_t)meta_.GetShape().at(1);
+    memcpy(dst, bytes_.data() + (size_t)row * n * 4, n * 4);
+    return;
+  }
+  for (const Block &b : blocks_) {
+    const int64_t r = row - b.row;
+    if (r < 0 || r >= b.source->meta_.GetShape()[0]) continue;
+    float *to = dst + b.col;
+    b.source->WriteRow(r, to);
+    if (!b.row_scale) continue;
+    float scale;
+    memcpy(&scale, b.row_scale->Bytes().data() + r * 4, 4);
+    for (int64_t j = 0; j < b.source->meta_.GetShape()[1]; ++j) to[j] *= scale;
+  }
+}
+
+void Tensor::WriteTo(uint8_t *dst) const {
+  if (blocks_.empty() || !bytes_.empty()) {
+    if (!bytes_.empty()) memcpy(dst, bytes_.data(), bytes_.size());
+    return;
+  }
+  const int64_t rows = meta_.GetShape().at(0), cols = meta_.GetShape().at(1);
+  for (int64_t r = 0; r < rows; ++r) WriteRow(r, reinterpret_cast<float *>(dst) + r * cols);
+}
+
+const std::vector<uint8_t> &Tensor::Bytes() const {
+  if (!blocks_.empty() && bytes_.empty()) {
+    std::vector<uint8_t> bytes(meta_.GetSize());
+    WriteTo(bytes.data());
+    bytes_ = std::move(bytes);
+  }
+  return bytes_;
+}
+
 double Tensor::AsDouble(int64_t i) const {
-  const uint8_t *p = bytes_.data();
+  const uint8_t *p = Bytes().data();
   switch (meta_.GetType()) {
   case Type::kFloat32: { float v; memcpy(&v, p + 4 * i, 4); return v; }
   case Type::kFloat64: { double v; memcpy(&v, p + 8 * i, 8); return v; }
@@ -64,7 +100,7 @@ double Tensor::AsDouble(int64_t i) const {
 }
 
 int64_t Tensor::AsInt(int64_t i) const {
-  if (meta_.GetType() == Type::kInt64) { int64_t v; memcpy(&v, bytes_.data() + 8 * i, 8); return v; }
+  if (meta_.GetType() == Type::kInt64) { int64_t v; memcpy(&v, Bytes().data() + 8 * i, 8); return v; }
   return (int64_t)AsDouble(i);
 }
 

@@ -67,14 +67,23 @@ private:
 std::optional<Meta> BroadcastShape(const Meta &lhs, const Meta &rhs, Type type);
 std::optional<Meta> BroadcastMatMulShape(const Meta &lhs, const Meta &rhs, Type type);
 
-// A constant: row-major bytes in its native dtype.
+// A constant: row-major bytes in its native dtype, or a matrix of floats put together from others.  The latter is written
+// where it is wanted and nowhere in between: a weight that is scaled, set beside others and put on top of others is copied once.
 class Tensor {
 public:
+  struct Block {  // rows row .., columns col .. are `source`, row r of it times row_scale[r] if there is one
+    std::shared_ptr<const Tensor> source;
+    int64_t row = 0, col = 0;
+    std::shared_ptr<const Tensor> row_scale;
+  };
   Tensor() = default;
   Tensor(Meta meta, std::vector<uint8_t> bytes) : meta_(std::move(meta)), bytes_(std::move(bytes)) {}
+  Tensor(Meta meta, std::vector<Block> blocks) : meta_(std::move(meta)), blocks_(std::move(blocks)) {}
   const Meta &GetMeta() const { return meta_; }
-  const std::vector<uint8_t> &Bytes() const { return bytes_; }
-  std::vector<uint8_t> &Bytes() { return bytes_; }
+  size_t ByteSize() const { return blocks_.empty() ? bytes_.size() : meta_.GetSize(); }
+  void WriteTo(uint8_t *dst) const;                   // all of it, row-major
+  void WriteRow(int64_t row, float *dst) const;       // a row of a matrix of floats
+  const std::vector<uint8_t> &Bytes() const;          // (of blocks: put together now, and kept)
   // Element `i` (row-major) converted to double / int64, whatever the dtype.
   double AsDouble(int64_t i = 0) const;
   int64_t AsInt(int64_t i = 0) const;
@@ -82,7 +91,8 @@ public:
 
 private:
   Meta meta_;
-  std::vector<uint8_t> bytes_;
+  mutable std::vector<uint8_t> bytes_;
+  std::vector<Block> blocks_;
 };
 
 namespace utils {

@@ -654,10 +654,16 @@ RegionPtr MakeConstant(flow::Flow &f, const std::string &name, std::vector<int64
   r->constant = std::make_shared<Tensor>(r->meta, std::move(bytes));
   return r;
 }
+// One that is put together from others when it is uploaded.
+RegionPtr MakeConstant(flow::Flow &f, const std::string &name, std::vector<int64_t> shape, std::vector<Tensor::Block> blocks) {
+  const RegionPtr r = f.NewRegion(flow::Region::kConstant, name, Meta(Type::kFloat32, shape));
+  r->constant = std::make_shared<Tensor>(r->meta, std::move(blocks));
+  return r;
+}
 
 bool HoldsFloats(const RegionPtr &r, size_t rank, size_t count) {
   return r->kind == flow::Region::kConstant && r->meta.GetType() == Type::kFloat32 && r->meta.GetRank() == rank && r->constant &&
-         r->constant->Bytes().size() == count * 4 && utils::IsDefaultLayout(r->layout);
+         r->constant->ByteSize() == count * 4 && utils::IsDefaultLayout(r->layout);
 }
 
 // A product with a captured weight [K, N] and bias [N] (or none) in logical row-major order, nothing but an
@@ -746,23 +752,19 @@ bool FoldSharedLayerNorms(Rewriter &rw) {
     std::vector<uint8_t> ones((size_t)K * 4), zeros((size_t)K * 4);
     for (int64_t k = 0; k < K; ++k) reinterpret_cast<float *>(ones.data())[k] = 1.0f;
     for (const NodePtr &n : norms) {
-      const float *g = reinterpret_cast<const float *>(n->consts[0]->constant->Bytes().data());
       const float *b = reinterpret_cast<const float *>(n->consts[1]->constant->Bytes().data());
       for (const NodePtr &r : rw.consumers[n->output.get()]) {
         const int64_t N = r->consts[0]->meta.GetShape()[1];
         const float *w = reinterpret_cast<const float *>(r->consts[0]->constant->Bytes().data());
         const float *c = r->has_bias ? reinterpret_cast<const float *>(r->consts[1]->constant->Bytes().data()) : nullptr;
-        std::vector<uint8_t> wb((size_t)K * N * 4), cb((size_t)N * 4);
+        std::vector<uint8_t> cb((size_t)N * 4);
         std::vector<double> shift((size_t)N);
         for (int64_t j = 0; j < N; ++j) shift[j] = c ? (double)c[j] : 0.0;
-        float *wo = reinterpret_cast<float *>(wb.data()), *co = reinterpret_cast<float *>(cb.data());
+        float *co = reinterpret_cast<float *>(cb.data());
         for (int64_t k = 0; k < K; ++k)
-          for (int64_t j = 0; j < N; ++j) {
-            wo[k * N + j] = (float)((double)g[k] * (double)w[k * N + j]);
-            shift[j] += (double)b[k] * (double)w[k * N + j];
-          }
+          for (int64_t j = 0; j < N; ++j) shift[j] += (double)b[k] * (double)w[k * N + j];
         for (int64_t j = 0; j < N; ++j) co[j] = (float)shift[j];
-        r->consts[0] = MakeConstant(rw.f, r->name + "_normed.w", {K, N}, std::move(wb));
+        r->consts[0] = MakeConstant(rw.f, r->name + "_normed.w", {K, N}, {{r->consts[0]->constant, 0, 0, n->consts[0]->constant}});
         const RegionPtr nc = MakeConstant(rw.f, r->name + "_normed.b", {N}, std::move(cb));
         if (r->has_bias) r->consts[1] = nc;
         else r->consts.insert(r->consts.begin() + 1, nc);
@@ -781,10 +783,8 @@ bool FoldSharedLayerNorms(Rewriter &rw) {
 
 // [W1; W2] and the sum of the biases: what a product over two left-hand sides reads.
 void JoinWeights(flow::Flow &f, const NodePtr &into, const NodePtr &top, const NodePtr &bottom) {
-  const int64_t N = top->consts[0]->meta.GetShape()[1], K = top->consts[0]->meta.GetShape()[0] + bottom->consts[0]->meta.GetShape()[0];
-  std::vector<uint8_t> w = top->consts[0]->constant->Bytes();
-  const std::vector<uint8_t> &w2 = bottom->consts[0]->constant->Bytes();
-  w.insert(w.end(), w2.begin(), w2.end());
+  const int64_t N = top->consts[0]->meta.GetShape()[1], K1 = top->consts[0]->meta.GetShape()[0], K = K1 + bottom->consts[0]->meta.GetShape()[0];
+  std::vector<Tensor::Block> w = {{top->consts[0]->constant, 0, 0, nullptr}, {bottom->consts[0]->constant, K1, 0, nullptr}};
   std::vector<uint8_t> bias;
   for (const NodePtr &n : {top, bottom}) {
     if (!n->has_bias) continue;
@@ -811,12 +811,14 @@ bool AlikeByColumns(const RegionPtr &a, const RegionPtr &b) {
   for (int i = 0; i < 2; ++i) {
     const RegionPtr &w = i ? b : a;
     most[i].assign((size_t)N, 0.0f);
-    const float *v = reinterpret_cast<const float *>(w->constant->Bytes().data());
-    for (int64_t k = 0; k < w->meta.GetShape()[0]; ++k, v += N)
+    std::vector<float> v((size_t)N);
+    for (int64_t k = 0; k < w->meta.GetShape()[0]; ++k) {
+      w->constant->WriteRow(k, v.data());
       for (int64_t j = 0; j < N; ++j) {
         const float m = std::fabs(v[j]);
         most[i][j] = m > most[i][j] ? m : most[i][j];
       }
+    }
   }
   for (int64_t j = 0; j < N; ++j)
     if (!(most[0][j] <= 4.0f * most[1][j] && most[1][j] <= 4.0f * most[0][j])) return false;
@@ -958,17 +960,17 @@ bool MergeSiblingGemms(flow::Flow &f, bool join) {
     int64_t total = 0;
     for (const auto &n : group) total += n->consts[0]->meta.GetShape()[1];
     // concatenated weights [K, total] and bias [total]
-    std::vector<uint8_t> wbytes((size_t)K * total * 4), bbytes((size_t)total * 4);
+    std::vector<Tensor::Block> weights;
+    std::vector<uint8_t> bbytes(first->has_bias ? (size_t)total * 4 : 0);
     int64_t col = 0;
     for (const auto &n : group) {
       const int64_t N = n->consts[0]->meta.GetShape()[1];
-      const uint8_t *src = n->consts[0]->constant->Bytes().data();
-      for (int64_t k = 0; k < K; ++k) memcpy(wbytes.data() + ((size_t)k * total + col) * 4, src + (size_t)k * N * 4, (size_t)N * 4);
+      weights.push_back({n->consts[0]->constant, 0, col, nullptr});
       if (n->has_bias) memcpy(bbytes.data() + (size_t)col * 4, n->consts[1]->constant->Bytes().data(), (size_t)N * 4);
       col += N;
     }
     const std::string base = first->name + "_merged";
-    RegionPtr wcat = MakeConstant(f, base + ".w", {K, total}, std::move(wbytes));
+    RegionPtr wcat = MakeConstant(f, base + ".w", {K, total}, std::move(weights));
     RegionPtr bcat = first->has_bias ? MakeConstant(f, base + ".b", {total}, std::move(bbytes)) : nullptr;
     std::vector<int64_t> mshape = first->output->meta.GetShape();
     mshape.back() = total;

@@ -45,27 +45,25 @@ private:
   std::unordered_set<std::string> taken_;
 };
 
-// Row-major logical bytes -> bytes in the region's physical order (builder.cpp:280-296).
-std::vector<uint8_t> PermuteConstant(const flow::Region &r) {
+// Row-major logical bytes -> bytes in the region's physical order (builder.cpp:280-296), at dst.
+void WriteConstant(const flow::Region &r, uint8_t *dst) {
+  if (utils::IsDefaultLayout(r.layout)) return r.constant->WriteTo(dst);
   const std::vector<uint8_t> &src = r.constant->Bytes();
-  if (utils::IsDefaultLayout(r.layout)) return src;
   const size_t es = GetSizeFromType(r.meta.GetType());
   const std::vector<int64_t> &shape = r.meta.GetShape();
   const std::vector<int64_t> strides = r.GetStrides();
-  std::vector<uint8_t> dst(src.size());
   const size_t rank = shape.size();
   std::vector<int64_t> idx(rank, 0);
   const int64_t n = r.meta.GetElementsNum();
   for (int64_t e = 0; e < n; ++e) {
     int64_t off = 0;
     for (size_t d = 0; d < rank; ++d) off += idx[d] * strides[d];
-    memcpy(dst.data() + off * es, src.data() + e * es, es);
+    memcpy(dst + off * es, src.data() + e * es, es);
     for (size_t d = rank; d-- > 0;) {
       if (++idx[d] < shape[d]) break;
       idx[d] = 0;
     }
   }
-  return dst;
 }
 
 }  // namespace
@@ -213,23 +211,30 @@ std::unique_ptr<Program> Builder::Run(const flow::Flow &flow, const flow::Sequen
 
   // ---- constants referenced by any node: one blob, each at a 256-byte boundary
   std::unordered_map<const flow::Region *, size_t> const_offset;
-  std::vector<uint8_t> blob;
+  std::vector<flow::RegionPtr> constants;
   auto add_const = [&](const flow::RegionPtr &r) {
     if (r->kind != flow::Region::kConstant || const_offset.count(r.get())) return;
-    const size_t off = AlignUp(blob.size(), 256);
-    const std::vector<uint8_t> bytes = PermuteConstant(*r);
-    blob.resize(off + std::max<size_t>(bytes.size(), 1));
-    memcpy(blob.data() + off, bytes.data(), bytes.size());
+    const size_t off = AlignUp(prog->weight_bytes, 256);
+    prog->weight_bytes = off + std::max<size_t>(r->constant->ByteSize(), 1);
     const_offset[r.get()] = off;
+    constants.push_back(r);
   };
   for (const auto &node : sequence.nodes) {
     for (const auto &r : node->inputs) add_const(r);
     for (const auto &r : node->consts) add_const(r);
   }
-  prog->weight_bytes = blob.size();
-  Check(fml_malloc(&prog->weights, blob.size()), "allocating the weight blob");
-  if (!blob.empty()) {
-    Check(fml_memcpy_h2d(prog->weights, blob.data(), blob.size(), nullptr), "uploading the weights");
+  Check(fml_malloc(&prog->weights, prog->weight_bytes), "allocating the weight blob");
+  if (prog->weight_bytes) {
+    const std::unique_ptr<uint8_t[]> blob(new uint8_t[prog->weight_bytes]);  // every byte is written below
+    size_t end = 0;
+    for (const auto &r : constants) {
+      const size_t off = const_offset[r.get()], size = r->constant->ByteSize();
+      memset(blob.get() + end, 0, off - end);
+      WriteConstant(*r, blob.get() + off);
+      if (!size) blob[off] = 0;
+      end = off + std::max<size_t>(size, 1);
+    }
+    Check(fml_memcpy_h2d(prog->weights, blob.get(), prog->weight_bytes, nullptr), "uploading the weights");
     Check(fml_stream_sync(nullptr), "uploading the weights");
   }
 
