@@ -298,10 +298,10 @@ private:
         if (!b || b->kind != flow::Region::kConstant || b->meta.GetRank() != 2 || n->trans_b) continue;
         const int64_t K = b->meta.GetShape()[0], N = b->meta.GetShape()[1];
         if (K % 4 != 0 || !utils::IsDefaultLayout(b->layout) || n->output->meta.GetRank() < 2) continue;
-        // ... and a product of fewer than 32 rows below 16 million multiply-adds is fastest with whole columns per CTA
-        // (gemm_skinny_columns_kernel: 16 x 512 x 128 3.9 us against 7.1, 16 x 768 x 3072 16 against 9.9)
+        // ... and a product of few rows may be fastest with whole columns per CTA (gemm_skinny_columns_kernel: 16 x 512 x 128
+        // 3.9 us against 7.1 with the weights as they are)
         const int64_t rows = (int64_t)n->output->meta.GetElementsNum() / N;
-        if (N % 4 != 0 || (options_.gemm_precision == FML_GEMM_AUTO && rows < 32 && rows * N * K <= (16ll << 20))) b->layout = {1, 0};
+        if (N % 4 != 0 || (options_.gemm_precision == FML_GEMM_AUTO && fml_gemm_prefers_k_major(rows, N, K))) b->layout = {1, 0};
       }
 
     kernel::KernelOptions ko;

@@ -200,7 +200,9 @@ inline cudaError_t launch_kernel(void (*kernel)(Exp...), dim3 grid, dim3 block, 
 #define FML_LAUNCH(kernel, grid, block, smem, stream, ...)                                 \
   FML_CUDA(::fml::launch_kernel(kernel, grid, block, smem, stream, __VA_ARGS__))
 
-inline int grid_for(int64_t work, int block, int max_blocks = 148 * 16) {
+constexpr int kSms = 148;  // of a B200: what the host plans count waves by
+
+inline int grid_for(int64_t work, int block, int max_blocks = kSms * 16) {
   int64_t g = (work + block - 1) / block;
   if (g < 1) g = 1;
   if (g > max_blocks) g = max_blocks;

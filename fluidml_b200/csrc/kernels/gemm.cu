@@ -294,6 +294,16 @@ extern "C" int fml_gemm_uses_tensor_cores(const fml_tensor *a, const fml_tensor 
   return FML_OK;
 }
 
+extern "C" int fml_gemm_uses_columns(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c, const fml_gemm_params *gp, int *uses) {
+  FML_REQUIRE(uses, FML_BAD_ARG, "fml_gemm_uses_columns: null argument");
+  GemmProblem p;
+  Choice ch;
+  const int st = resolve(a, b, c, nullptr, nullptr, gp, p, ch);
+  if (st != FML_OK) return st;
+  *uses = !ch.parts && ch.path == Path::kSimt && p.M > 0 && p.N > 0 && gemm_skinny_by_columns(p) ? 1 : 0;
+  return FML_OK;
+}
+
 extern "C" int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
                         const fml_tensor *bias, const fml_tensor *residual,
                         const fml_gemm_params *gp, void *stream) {

@@ -68,6 +68,7 @@ int launch_gemm_simt(const GemmProblem &p, const GemmEpilogue &e, cudaStream_t s
 // library-owned scratch memory (one buffer per device and stream).
 bool skinny_eligible(const GemmProblem &p);
 int launch_gemm_skinny(const GemmProblem &p, const GemmEpilogue &e, cudaStream_t s);
+bool gemm_skinny_by_columns(const GemmProblem &p);  // whole columns per CTA, no scratch
 
 // tcgen05 path -------------------------------------------------------------------------
 struct TcPlan {

@@ -15,6 +15,7 @@
 // the epilogue and resets the counter.  The scratch (counters first, then partials) is global
 // memory beyond the inputs and outputs, owned by the library per (device, stream).
 #include "gemm_common.cuh"
+#include <cmath>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -355,10 +356,8 @@ __global__ void __launch_bounds__(kThreads, MR == 32 ? 1 : 2) gemm_skinny_rows_k
 // and 32 columns x 8 slices a CTA were too few bytes in flight (1 x 4096 x 1000: 1.1 TB/s).  Weights that no earlier
 // launch writes are asked for before the dependency wait.
 // Captured graphs, us, slices -> this: 1 x 4096 x 1000 12.3 (weights from HBM 14.8) -> 3.2 (4.3), 1 x 1280 x 1000 6.8 -> 2.7,
-// 1 x 25088 x 4096 66 -> 65, 3 x 768 x 768 6.8 -> 2.6, 8 x 4096 x 4096 39 -> 29; against N-major weights on
-// gemm_skinny_rows_kernel 16 x 128 x 512 3.5 -> 2.2, 16 x 512 x 128 7.1 -> 3.9, 24 x 256 x 1024 6.8 -> 4.5, 31 x 768 x 768
-// 11.9 -> 9.9, but 16 x 768 x 3072 9.9 -> 16: there every CTA reads all rows again, so a compiled model's weights are
-// stored K-major only below 16 million multiply-adds.
+// 1 x 25088 x 4096 66 -> 65, 3 x 768 x 768 6.8 -> 2.6, 8 x 4096 x 4096 39 -> 29.  Every CTA reads all rows again and has
+// fixed phases of its own, so wide and flat products lose (1 x 256 x 50304 12 -> 77): columns_pay.
 constexpr int kCtaCols = 4;
 
 template <int V> __device__ __forceinline__ void warp_reduce_scatter(float (&v)[V], int lane) {
@@ -451,8 +450,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_skinny_columns_kernel(const 
   p.c[z0 * p.c_b0 + z1 * p.c_b1 + fm * p.c_sm + (n0 + fj) * p.c_sn] = gemm_epilogue(e, v, bias, res);
 }
 
-// Which products: rows and columns of B on 16-byte boundaries, k in one sweep of a few batches.
-bool by_columns(const GemmProblem &p) {
+// Rows and columns of B on 16-byte boundaries, k in one sweep of a few batches.
+bool columns_possible(const GemmProblem &p) {
   if (p.b_sk != 1 || p.b_sn == 1 || p.a_sk != 1 || p.K % 4 || p.K > (1 << 20)) return false;
   if (p.a_sm % 4 || p.b_sn % 4 || !aligned16(p.a) || !aligned16(p.b) || p.a_b0 % 4 || p.a_b1 % 4 || p.b_b0 % 4 || p.b_b1 % 4) return false;
   return p.N < (1ll << 31);
@@ -469,7 +468,7 @@ SkinnyPlan plan_skinny(const GemmProblem &p) {
   pl.tiles_n = (int)((p.N + kColsPerCta - 1) / kColsPerCta);
   const int64_t tiles = (int64_t)pl.tiles_n * p.nb0 * p.nb1;
   // enough CTAs for ~8 per SM, each split at least 256 k values long
-  int64_t s = (148 * 8 + tiles - 1) / tiles;
+  int64_t s = (kSms * 8 + tiles - 1) / tiles;
   // (with at most four rows the kernel is a chain of load latencies, not arithmetic: slices of
   // 128 k values already pay there; more rows keep slices of at least 256)
   s = std::min<int64_t>(s, std::max<int64_t>(1, p.K / (p.M <= 4 ? 128 : 256)));
@@ -485,6 +484,31 @@ SkinnyPlan plan_skinny(const GemmProblem &p) {
   pl.counter_bytes = pl.splits > 1 ? kCounterBytes : 0;
   pl.scratch_bytes = pl.splits > 1 ? pl.counter_bytes + (size_t)tiles * pl.splits * p.M * kColsPerCta * 4 : 0;
   return pl;
+}
+
+// Times of the three kernels in microseconds: fixed phases, then waves of CTAs at the SMs' rate, not below the weights'
+// bytes.  Fitted to captured graphs of 51 K-major shapes (K 256 to 8192, N 768 to 50304) and 61 N-major ones below 16 M
+// multiply-adds (K 128 to 4096, N 128 to 4096), 1 to 31 rows each, warm.  Taking the kernel with the smaller time costs 2 %
+// over taking the faster one (K-major: columns always 15 %, at worst 1 x 256 x 50304 77 us for 12; slices always 22 %) and
+// 0.3 % (columns or N-major rows; columns always 11 %, at worst 31 x 4096 x 128 2.7 times).
+double columns_us(double m, double n, double k, double batch) {
+  const double per_k = m <= 4 ? 0.3 + 0.058 * m : m <= 8 ? 0.31 + 0.186 * m : 0.78 + 0.205 * (m <= 16 ? m : 32);  // (a group of sixteen rows, or two)
+  const double waves = std::max(1.0, n / kCtaCols * batch / (2.0 * kSms));
+  return std::max(0.76 + waves * (1.76 + per_k * k / 1024), n * k * batch * 4 / 6.4e6);
+}
+double slices_us(const GemmProblem &p, const SkinnyPlan &pl) {
+  const double waves = (double)pl.tiles_n * pl.splits * (double)(p.nb0 * p.nb1) / ((p.M <= 4 ? 3.0 : 2.0) * kSms);
+  const double work = 2.85 + 2.2 * (double)p.M * (double)pl.k_per_split / 1024;
+  return 1.04 + (pl.splits > 1 ? 2.79 : 0.0) +
+         std::max((waves < 4 ? std::ceil(waves) : waves + 0.5) * work, 1.2 * (double)p.N * (double)p.K * (double)(p.nb0 * p.nb1) * 4 / 6.4e6);
+}
+double rows_us(const GemmProblem &p, const SkinnyPlan &pl) {
+  const double per_k = p.M <= 4 ? 9.2 : p.M <= 8 ? 7.4 : p.M <= 16 ? 12.6 : 23.3, per_sm = p.M <= 16 ? 2.0 : 1.0;
+  const double waves = std::max(1.0, (double)pl.tiles_n * pl.splits * (double)(p.nb0 * p.nb1) / (per_sm * kSms));
+  return (pl.splits > 1 ? 2.82 : 0.0) + waves * (2.2 + per_k * (double)pl.k_per_split / 1024);
+}
+bool columns_pay(const GemmProblem &p, const SkinnyPlan &pl) {
+  return columns_possible(p) && columns_us((double)p.M, (double)p.N, (double)p.K, (double)(p.nb0 * p.nb1)) <= slices_us(p, pl);
 }
 
 int launch_skinny(const GemmProblem &p, const GemmEpilogue &e, const SkinnyPlan &pl, void *scratch, cudaStream_t s) {
@@ -568,17 +592,20 @@ static int launch_columns(const GemmProblem &p, const GemmEpilogue &e, cudaStrea
 }
 
 int launch_gemm_skinny(const GemmProblem &p, const GemmEpilogue &e, cudaStream_t s) {
-  if (by_columns(p)) return launch_columns(p, e, s);
   const SkinnyPlan pl = plan_skinny(p);
+  if (columns_pay(p, pl)) return launch_columns(p, e, s);
   void *scratch = nullptr;
   if (pl.scratch_bytes) {
     int st = scratch_for(pl.scratch_bytes, s, &scratch);
+    if (st != FML_OK && columns_possible(p)) return launch_columns(p, e, s);  // (needs none: a stream that is being captured)
     if (st != FML_OK) return st;
   }
   return launch_skinny(p, e, pl, scratch, s);
 }
 
 size_t gemm_skinny_scratch_bytes(const GemmProblem &p) { return plan_skinny(p).scratch_bytes; }
+
+bool gemm_skinny_by_columns(const GemmProblem &p) { return skinny_eligible(p) && columns_pay(p, plan_skinny(p)); }
 
 
 // ---- the same product for callers that cannot let the library allocate ---------------------
@@ -655,6 +682,15 @@ extern "C" int fml_gemm_skinny_noalloc(const fml_tensor *a, const fml_tensor *b,
     }
     scratch = g_static_scratch_addr[dev];
   }
-  if (by_columns(p)) return launch_columns(p, e, s);  // as fml_gemm (the capacity is checked all the same)
+  if (columns_pay(p, pl)) return launch_columns(p, e, s);  // as fml_gemm (the capacity is checked all the same)
   return launch_skinny(p, e, pl, scratch, s);
+}
+
+// Declared in fluidml_cuda.h: measured below 16 M multiply-adds only.
+extern "C" int fml_gemm_prefers_k_major(int64_t rows, int64_t n, int64_t k) {
+  if (rows < 1 || rows >= kMaxM || n < 1 || k < 4 || k % 4 || rows * n * k > (16ll << 20)) return 0;
+  GemmProblem p;
+  memset(&p, 0, sizeof(p));
+  p.M = rows; p.N = n; p.K = k; p.nb0 = p.nb1 = 1;
+  return columns_us((double)rows, (double)n, (double)k, 1.0) <= rows_us(p, plan_skinny(p)) ? 1 : 0;
 }

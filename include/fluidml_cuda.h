@@ -408,6 +408,11 @@ int fml_gemm_skinny_noalloc(const fml_tensor *a, const fml_tensor *b, const fml_
 int fml_gemm_uses_tensor_cores(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c,
                                const fml_gemm_params *p, int *uses);
 
+/* Whether fml_gemm gives a product of at most 32 rows with K-major B (b_sk == 1) whole columns per CTA rather than slices
+ * of k, and whether a constant B is better stored that way in the first place.  Pure host computation. */
+int fml_gemm_uses_columns(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c, const fml_gemm_params *p, int *uses);
+int fml_gemm_prefers_k_major(int64_t rows, int64_t n, int64_t k);
+
 /* ---------------------------------------------------------------- convolution, pooling
  * ConvWithoutPaddingKernel / ConvWithPaddingKernel (conv.cpp:27-280): NCHW x OIHW, 1-D or
  * 2-D, group == 1 or depthwise (group == C, multiplier 1) as in the reference (:103-149).
