@@ -493,7 +493,7 @@ bool plan_depthwise_planes(const fml_tensor *x, const fml_tensor *w, const fml_t
   // Few planes: fewer to a CTA until every SM has one; its repack and its stores are shared by all of its threads, so a
   // smaller tile is a shorter chain.  (One image, 480-1152 planes of 14 x 14 and 7 x 7: 7-10.5 us a layer with full tiles,
   // 4.4-6.2 so; from 148 full tiles on nothing changes.)
-  while (d.PP > 4 && (d.planes + d.PP - 1) / d.PP < 148) d.PP -= 4;
+  while (d.PP > 4 && (d.planes + d.PP - 1) / d.PP < kSms) d.PP -= 4;
   if (smem_of() > 100 * 1024 || (int64_t)d.PP * d.PH * d.PWn >= 65536) return false;
   *smem = smem_of();
   return true;

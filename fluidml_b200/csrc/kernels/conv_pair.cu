@@ -987,7 +987,7 @@ std::vector<Candidate> conv_pair_candidates(const fml_tensor *x, const fml_tenso
           else if (c.mode == kRun) { c.tiles_w = (c.plane + c.TW - 1) / c.TW; c.tiles_h = 1; c.tiles_img = c.N; }
           else { c.tiles_w = (c.OW + c.TW - 1) / c.TW; c.tiles_h = (c.OH + c.TH - 1) / c.TH; c.tiles_img = c.N; }
           const double ctas = (double)c.tiles_w * c.tiles_h * c.tiles_img * ((c.OC + tn - 1) / tn) * sk;
-          const double slots = 148.0 * occ * (sk == 8 ? 0.86 : sk == 4 ? 0.97 : 1.0);
+          const double slots = (double)kSms * occ * (sk == 8 ? 0.86 : sk == 4 ? 0.97 : 1.0);
           double t_kb = std::max(mt * 6 * std::max(48.0, tn / 2.0) + 40.0, (tn * 128.0 + (double)c.raw_bytes / c.taps) / 45.0);
           // a ring of one stage exposes the load latency, shared out over what the SM has in flight
           t_kb = std::max(t_kb, 1800.0 / (c.stages_b * c.group));
@@ -996,7 +996,7 @@ std::vector<Candidate> conv_pair_candidates(const fml_tensor *x, const fml_tenso
           const double shared = c.icb_per_split * std::max(c.taps * t_kb, t_split) + mt * 128.0 * tn * 4.0 / 40.0;
           const double own = 4500.0 + t_split + (mt == 2 ? tn / 32 : (tn + 63) / 64) * 300.0 +
                              (sk > 1 ? 2500.0 + mt * 128.0 * tn * 4.0 / 13.0 * (sk - 1) / sk : 0.0);
-          const double resident = std::min((double)occ, std::ceil(ctas / 148.0));
+          const double resident = std::min((double)occ, std::ceil(ctas / kSms));
           const double t = std::ceil(ctas / slots) * std::max(resident * shared, shared + own);
           // no more CTAs on an SM than its 512 TMEM columns serve at once
           smem = std::max(smem, kSmemSm / (512 / cols + 1) + 1024);

@@ -230,7 +230,7 @@ bool plan_pointwise(int64_t n, int64_t hw, int64_t oc, int64_t ic, bool scaled, 
       const size_t smem = std::max(2 * (size_t)chunk * (kPwOC + px) * 4 + (scaled ? (size_t)k * 4 : 0), (size_t)8 * 4096);
       if (smem > 110 * 1024) continue;
       const double per = (double)kPwOC * px * (double)k / 128.0 / 1900.0 * 1.25;  // one CTA alone on an SM
-      const double waves = (double)ctas / 148.0;
+      const double waves = (double)ctas / kSms;
       const double t = 2.2 + (wk > 1 ? 0.3 : 0.0) + (split > 1 ? 1.0 : 0.0) + 0.25 * (double)((k + chunk - 1) / chunk) + per * std::max(1.0, waves);
       if (t < best_us) { best_us = t; *best = {wk, split, (int)k, chunk, smem}; }
     }

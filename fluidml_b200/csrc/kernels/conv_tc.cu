@@ -604,7 +604,7 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
     // lose (FLUIDML_CONV_WIDE_TILES=1 takes those too, =0 none).
     static const int wide = [] { const char *e = getenv("FLUIDML_CONV_WIDE_TILES"); return e ? atoi(e) : 2; }();
     const int64_t px_tiles = (int64_t)((a.OW + a.TW - 1) / a.TW) * ((a.OH + a.TH - 1) / a.TH) * a.N;
-    if (wide && a.OC > 128 && a.n_icb * a.taps <= (wide == 2 ? 1 : 8) && (wide == 1 || px_tiles > 148)) {
+    if (wide && a.OC > 128 && a.n_icb * a.taps <= (wide == 2 ? 1 : 8) && (wide == 1 || px_tiles > kSms)) {
       int best = 128, best_cost = ((a.OC + 127) / 128) * (128 + 128);
       for (int tn = 160; tn <= 256; tn += 32) {
         const int cost = ((a.OC + tn - 1) / tn) * (128 + tn);
@@ -637,7 +637,7 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
     // at 112 x 112: 160 -> 203).  FLUIDML_CONV_RING=deep keeps the deep rings.
     static const bool deep = [] { const char *e = getenv("FLUIDML_CONV_RING"); return e && e[0] == 'd'; }();
     const int64_t ctas = (int64_t)((a.OW + a.TW - 1) / a.TW) * ((a.OH + a.TH - 1) / a.TH) * a.N * ((a.OC + a.tile_n - 1) / a.tile_n);
-    if (!deep && ctas > 148 && a.tile_n <= 128) {
+    if (!deep && ctas > kSms && a.tile_n <= 128) {
       stages = std::min(stages, 2);
       a.raw_stages = a.taps == 1 ? std::min(a.raw_stages, 3) : 1;
     }
@@ -653,7 +653,7 @@ int launch_conv_tc(const fml_tensor *x, const fml_tensor *w, const fml_tensor *b
     static const int forced = [] { const char *e = getenv("FLUIDML_CONV_SPLIT_K"); return e ? atoi(e) : -1; }();
     const int64_t tiles = (int64_t)a.tiles_w * a.tiles_h * a.N * ((a.OC + a.tile_n - 1) / a.tile_n);
     int sk = 1;
-    while (sk < 8 && tiles * (sk * 2) <= 148 && a.n_icb >= sk * 2 && a.n_icb * a.taps >= sk * 2 * 4) sk *= 2;
+    while (sk < 8 && tiles * (sk * 2) <= kSms && a.n_icb >= sk * 2 && a.n_icb * a.taps >= sk * 2 * 4) sk *= 2;
     if (forced == 0) sk = 1;
     else if (forced > 0) { sk = 1; while (sk < 8 && sk * 2 <= forced && a.n_icb >= sk * 2) sk *= 2; }
     a.split_k = sk;

@@ -704,11 +704,11 @@ bool plan_gemm_pair(const GemmProblem &p, const GemmExtras &x, const fml_gemm_pa
         size_t smem;
         if (!pair_stages(tn, per, two != 0, &sa, &sb, &smem)) continue;
         const int64_t ctas = tiles_m * ((p.N + tn - 1) / tn) * batch * sk;
-        const int slots = (two ? 296 : 148) * (sk == 8 ? 0.87 : sk == 4 ? 0.97 : 1.0);
+        const int slots = (two ? 2 : 1) * kSms * (sk == 8 ? 0.87 : sk == 4 ? 0.97 : 1.0);
         const double waves = (double)((ctas + slots - 1) / slots);
         const double t_kb = (double)(kPairA + tn * kPairB) / 80e3;
         const double t_fixed = 3.0 + (double)kBM * tn / sk * 4.0 / 20e3 + (sk > 1 ? 0.6 : 0.0);
-        const double t = waves * (t_fixed + per * t_kb * (two && ctas > 148 ? 2.0 : 1.0));
+        const double t = waves * (t_fixed + per * t_kb * (two && ctas > kSms ? 2.0 : 1.0));
         if (t < best) {
           best = t;
           found = true;

@@ -498,7 +498,7 @@ bool plan_gemm_tc(const GemmProblem &p, const fml_gemm_params &gp, TcPlan &plan)
   // a fixed set-up + epilogue cost.  Explicit tile_n / split_k requests bypass the search.
   const int tn_opts[] = {32, 48, 64, 96, 128, 192, 256};
   const int sk_opts[] = {1, 2, 4, 8};
-  const int sk_cap[] = {148, 148, 144, 128};  // CTAs that can be resident for each cluster size
+  const int sk_cap[] = {kSms, kSms, 144, 128};  // CTAs that can be resident for each cluster size
   double best = 1e30;
   int best_tn = 0, best_sk = 0;
   for (int tn : tn_opts) {
@@ -512,7 +512,7 @@ bool plan_gemm_tc(const GemmProblem &p, const fml_gemm_params &gp, TcPlan &plan)
       if (smem_for(tn, 1, plan.three_pass, plan.a_tmem) > kSmemBudget + 8192) continue;
       const int64_t tiles = tiles_m * ((p.N + tn - 1) / tn) * batch;
       const int64_t ctas = tiles * sk;
-      const int cap = sk <= 1 ? 148 : sk <= 2 ? sk_cap[1] : sk <= 4 ? sk_cap[2] : sk_cap[3];
+      const int cap = sk <= 1 ? kSms : sk <= 2 ? sk_cap[1] : sk <= 4 ? sk_cap[2] : sk_cap[3];
       const double waves = (double)((ctas + cap - 1) / cap);
       const int per = (kb_total + sk - 1) / sk;
       const double kb_bytes = kABytes + tn * 128.0;

@@ -411,11 +411,11 @@ extern "C" int fml_layernorm(const fml_tensor *in, const fml_tensor *residual,
   if (rows_vec_ok(a, out->data, in->data, rp) && res_vec && gs == 1 && bs == 1 &&
       aligned16(scale->data) && aligned16(bias->data)) {
     const int64_t per_lane = (a.len / 4 + 31) / 32;
-    const int threads = a.rows.total <= 148 ? 32 : a.rows.total <= 296 ? 64 : kLnThreads;
+    const int threads = a.rows.total <= kSms ? 32 : a.rows.total <= 2 * kSms ? 64 : kLnThreads;
     const unsigned ctas = (unsigned)((a.rows.total * 32 + threads - 1) / threads);
 #define LN_GO(NV, EARLY, MB) \
   FML_LAUNCH((layernorm_rows_vec<NV, EARLY, MB>), ctas, threads, 0, s, a, (float *)out->data, (const float *)in->data, rp, (const float *)scale->data, (const float *)bias->data, eps)
-    const auto one_wave = [&](int per_sm) { return a.rows.total <= 148ll * per_sm * (kLnThreads / 32); };
+    const auto one_wave = [&](int per_sm) { return a.rows.total <= (int64_t)kSms * per_sm * (kLnThreads / 32); };
     if (per_lane <= 6 && one_wave(5)) {
       if (per_lane <= 1) LN_GO(1, true, 5);
       else if (per_lane <= 2) LN_GO(2, true, 5);

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kSeThreads) squeeze_excite_gate_kernel(const S
   // shared-memory map (every CTA of the cluster uses the same offsets: peers address `own` and `hid_own`)
   float *w1_s = se_smem;                                                   // [hid_per_rank][C]     (stage_w)
   float *w2_s = w1_s + (a.stage_w ? (size_t)a.hid_per_rank * a.C : 0);     // [per_rank][Cr]        (stage_w)
-  float *own = w2_s + (a.stage_w ? (size_t)a.per_rank * (a.Cr | 1) : 0);  // (an odd pitch: a thread has a row in the last phase)         // [per_rank] means of this CTA's channels
+  float *own = w2_s + (a.stage_w ? (size_t)a.per_rank * (a.Cr | 1) : 0);  // [per_rank] means of this CTA's channels (W2 has an odd pitch: a thread has a row of it in the last phase)
   float *hid_own = own + a.per_rank;                                       // [images][hid_per_rank] this CTA's hidden units
   float *mean_s = hid_own + a.hid_per_rank * a.images;                     // [images][C]
   float *hid_s = mean_s + a.C * a.images;                                  // [images][Cr]
@@ -385,7 +385,7 @@ static int gate_impl(const fml_tensor *x, int64_t plane, const fml_tensor *w1, c
   // other (672 channels, where all clusters fit: 5.4 us with one image, 6.7 with two, 10.1 with four).
   auto waves = [&] {
     const int64_t per_sm = std::min<int64_t>(2048 / kSeThreads, (int64_t)(228 * 1024 / (smem_of() + 1024)));
-    return (double)((a.N + a.images - 1) / a.images) * ranks / (148.0 * (double)std::max<int64_t>(1, per_sm));
+    return (double)((a.N + a.images - 1) / a.images) * ranks / ((double)kSms * (double)std::max<int64_t>(1, per_sm));
   };
   while (plane && a.images < 4 && waves() > 1.0) {
     a.images *= 2;
