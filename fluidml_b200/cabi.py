@@ -60,6 +60,7 @@ class ConvParams(ctypes.Structure):
                 ("pointwise_fma", ctypes.c_int32), ("plane_sums", ctypes.c_void_p), ("max_pool", ctypes.c_int32)]
 
 
+ABI_VERSION = 2  # FML_ABI_VERSION of the structures above
 _lib = None
 
 
@@ -70,6 +71,9 @@ def lib():
             raise ImportError(f"{_LIB_PATH} is missing: run `python -m fluidml_b200.build` "
                               "(there is no fallback implementation)")
         _lib = ctypes.CDLL(_LIB_PATH)
+        if not hasattr(_lib, "fml_abi_version") or _lib.fml_abi_version() != ABI_VERSION:
+            _lib = None
+            raise ImportError(f"{_LIB_PATH} is of another version than its bindings: run `python -m fluidml_b200.build`")
         _lib.fml_last_error.restype = ctypes.c_char_p
     return _lib
 

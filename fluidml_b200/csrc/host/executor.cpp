@@ -42,6 +42,7 @@ class ExecutorImpl : public Executor {
 public:
   ExecutorImpl(std::string &&name, size_t epoch, LayoutMode layout, MemoryPlanKind plan)
       : name_(std::move(name)), epoch_(epoch ? epoch : 1), layout_(layout), plan_(plan) {
+    if (fml_abi_version() != FML_ABI_VERSION) throw Error("the kernel library is of another version than this one");
     SetOption("device", EnvOr("FLUIDML_DEVICE", "0"));
     SetOption("gemm_precision", EnvOr("FLUIDML_GEMM_PRECISION", "auto"));
     SetOption("fusion", EnvOr("FLUIDML_FUSION", "1"));

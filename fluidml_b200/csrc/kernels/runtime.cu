@@ -76,6 +76,8 @@ int fml_mem_info(size_t *free_bytes, size_t *total_bytes) {
   return FML_OK;
 }
 
+int fml_abi_version(void) { return FML_ABI_VERSION; }
+
 int fml_set_device(int device) {
   FML_CUDA(cudaSetDevice(device));
   return FML_OK;

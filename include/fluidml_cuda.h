@@ -32,6 +32,12 @@ extern "C" {
 
 #define FML_MAX_RANK 8
 
+/* The parameter structures grow at their ends from one version to the next.  Before its first call a caller compares
+ * fml_abi_version() with the FML_ABI_VERSION it was compiled with and goes no further where they differ: the library would
+ * read, or a fml_*_default_params write, past the end of a shorter structure.  (1: without that function.) */
+#define FML_ABI_VERSION 2
+int fml_abi_version(void);
+
 typedef enum fml_status {
   FML_OK = 0,
   FML_BAD_ARG = 1,        /* null pointer, rank/shape mismatch, axis out of range        */
