@@ -1,6 +1,6 @@
 """Tiles of the packed-weight GEMM that leave by bulk tensor stores: ragged edges in both dims, results inside wider
-buffers (nothing outside may be touched), batches, every activation.  8e-6 of the largest magnitude, as for every
-product of that kernel; the activations' slopes are at most 1.2."""
+buffers (nothing outside may be touched), batches, every activation.  8e-6 of the largest magnitude, as in that
+kernel's own tests (test_joined_products_gpu.py says where it comes from); the activations' slopes are at most 1.2."""
 import numpy as np
 import pytest
 

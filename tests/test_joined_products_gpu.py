@@ -1,8 +1,10 @@
 """Products joined into one launch: several projections side by side (rotation of the first columns, activation of the
 last) and two left-hand sides, against fp64 and against the parts run one by one; and the rewrites that make them.
 
-Tolerance 2e-5 of the largest magnitude, as for every product of the packed-weight kernel (operands of 22 bits,
-fp32 accumulation in chunks); a rotation or a GELU of it adds two roundings.
+Tolerance, of the largest magnitude.  On the packed-weight kernel 8e-6, as in its own tests (operands of 22 bits), and for more
+than 600 products what cutting the accumulator to 24 bits comes to: three times per sixteen products, 2^-24 of it on average.
+2e-5 where the parts run on the 3xTF32 kernel (operands of 21 to 22 truncated bits, eight products at a time), as in its tests.
+A rotation or a GELU adds two roundings.
 """
 import math
 
@@ -14,12 +16,13 @@ from fluidml_b200.cabi import DeviceTensor as DT
 from fluidml_b200.executor import Executor
 from fluidml_b200.onnx_lite import FLOAT
 
-TOL = 2e-5
+PAIRS, TF32 = 8e-6, 2e-5
+pairs = lambda k: max(PAIRS, 3 * k / 16 * 2.0 ** -24 + 2.0 ** -21)
 erf = np.vectorize(math.erf)
 
 
-def close(got, ref):
-    return np.abs(got.astype(np.float64) - ref).max() <= TOL * np.abs(ref).max()
+def close(got, ref, tol=PAIRS):
+    return np.abs(got.astype(np.float64) - ref).max() <= tol * np.abs(ref).max()
 
 
 def params(b, packed, **kw):
@@ -52,7 +55,7 @@ def test_two_left_hand_sides(m, k1, k2, n, tile, split):
         cabi.gemm(DT.from_numpy(a1), db, c, DT.from_numpy(bias), DT.from_numpy(res), p)
         cabi.check_device()
         rows = np.abs(ref).max(1, keepdims=True)  # each row by its own magnitude
-        assert (np.abs(c.numpy() - ref) <= TOL * np.maximum(rows, 1.0)).all()
+        assert (np.abs(c.numpy() - ref) <= (pairs(k1 + k2) if packed else TF32) * np.maximum(rows, 1.0)).all()
 
 
 @pytest.mark.gpu
@@ -80,7 +83,7 @@ def test_projections_side_by_side(batch, length, heads, size, rot, tile, split):
                          rot_cols=2 * h, rot_len=length, rot_cos=dc.c().data, rot_sin=ds.c().data)
         cabi.gemm(DT.from_numpy(a), db, c, DT.from_numpy(bias), None, p)
         cabi.check_device()
-        assert close(c.numpy(), ref)
+        assert close(c.numpy(), ref, PAIRS if packed else TF32)
 
 
 def refused(a, b, c, **kw):
