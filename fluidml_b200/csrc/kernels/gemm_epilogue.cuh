@@ -11,25 +11,24 @@ namespace fml {
 // cheap uniform predicates inside one short loop: every CTA runs each phase of this kernel
 // once, so the cost of a phase is largely the instruction fetch of its (cold) code, and a
 // compact, straight-line epilogue matters more than a branch-free one.
-// erf by Abramowitz & Stegun 7.1.26 with the fast exponential and reciprocal: absolute error about
-// 6e-7 in fp32 arithmetic (the formula's 1.5e-7 plus the cancellation in 1 - p t exp(-x^2) near 0;
-// tests/test_erf_formula_cpu.py restates it on the host), below 1e-6 with ex2.approx's rounding,
-// i.e. a GELU value off by at most 5e-7 |v| -- far below the 3xTF32 product it is applied to.
-// The exact erff is ~45 dependent instructions per element; with one epilogue warp per scheduler
-// that was 35 us of a 134 us FFN launch at 2048 rows (4096 columns each).
-// The reciprocal and the exponential in their flushing forms: the reciprocal's argument is at least 1 and an exponential
-// below 2^-126 vanishes beside 1, so the values are those of __fdividef and __expf without the instructions that look after
-// denormals (1024 x 768 x 3072 in tiles of 192 with GELU 22.3 -> 20.8 us).
+// erf by Abramowitz & Stegun 7.1.26: erf(x) = 1 - P(t) exp(-x^2) with t = 1 / (1 + 0.3275911 x), x >= 0, the formula itself
+// within 1.5e-7.  With y = sqrt(log2 e) x both pieces come from one product: exp(-x^2) = 2^(-y^2), for PTX's ex2.approx (2^-22
+// of the result; it flushes what is below 2^-126, where x is beyond 9 and erf is 1), and t = 1 / (1 + (0.3275911 / sqrt(log2 e)) y)
+// for its rcp.approx (1 ulp; the argument is at least 1).  In fp32 arithmetic the absolute error is about 6e-7, most of it
+// the cancellation in 1 - P exp(-x^2) near 0 (tests/test_erf_formula_cpu.py restates it on the host and
+// tests/test_gelu_epilogue_gpu.py holds the kernels to it), i.e. a GELU value off by at most 5e-7 |v| -- far below the
+// product it is applied to.
+// The exact erff is ~45 dependent instructions per element; with one epilogue warp per scheduler that was 35 us of a
+// 134 us FFN launch at 2048 rows (4096 columns each).
 __device__ __forceinline__ float erf_fast(float x) {
-  const float ax = fabsf(x);
-  float t, g;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.3275911f, ax, 1.0f)));
+  const float y = fabsf(x) * 1.2011224087864498f;  // sqrt(log2 e)
+  float t;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.27273748f, y, 1.0f)));
   float p = fmaf(1.061405429f, t, -1.453152027f);
   p = fmaf(p, t, 1.421413741f);
   p = fmaf(p, t, -0.284496736f);
   p = fmaf(p, t, 0.254829592f);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(-ax * ax * 1.4426950408889634f));
-  return copysignf(fmaf(-p * t, g, 1.0f), x);
+  return copysignf(fmaf(-p * t, ex2_approx(-y * y), 1.0f), x);
 }
 
 template <int ACT>
