@@ -86,6 +86,29 @@ def test_projections_side_by_side(batch, length, heads, size, rot, tile, split):
         assert close(c.numpy(), ref, PAIRS if packed else TF32)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("split", [3, 5, 6, 7])
+def test_rotation_with_splits_that_are_no_power_of_two(split):
+    """Their epilogue goes element by element and does not rotate: the rotation is a launch of its own."""
+    rng = np.random.default_rng(split)
+    length, heads, size, rot, k = 64, 2, 32, 16, 256
+    m, n = 2 * length, 3 * heads * size
+    a, b, bias = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (k, n), (n,)))
+    ang = rng.standard_normal((length, rot))
+    cos, sin = np.cos(ang).astype(np.float32), np.sin(ang).astype(np.float32)
+    ref = a.astype(np.float64) @ b + bias
+    qk = ref[:, :2 * heads * size].reshape(2, length, 2 * heads, size)
+    x = qk[..., :rot].copy()
+    qk[..., :rot] = x * cos[None, :, None] + np.concatenate([-x[..., rot // 2:], x[..., :rot // 2]], -1) * sin[None, :, None]
+    ref[:, :2 * heads * size] = qk.reshape(m, -1)
+    db, c, dc, ds = DT.from_numpy(b), DT((m, n), np.float32), DT.from_numpy(cos), DT.from_numpy(sin)
+    p, blob = params(db, True, tile=64, split=split, rot=rot, rot_head=size, rot_cols=2 * heads * size, rot_len=length,
+                     rot_cos=dc.c().data, rot_sin=ds.c().data)
+    cabi.gemm(DT.from_numpy(a), db, c, DT.from_numpy(bias), None, p)
+    cabi.check_device()
+    assert close(c.numpy(), ref)
+
+
 def refused(a, b, c, **kw):
     p = cabi.gemm_params(act=kw.pop("act", cabi.ACT_NONE))
     for k, v in kw.items():
