@@ -136,7 +136,7 @@ template <int ACT, int NT, bool COL_SCALE, bool PROJ = false> struct TileEpilogu
       const int64_t r_step = (int64_t)rows_pass * p.res_sm;
       const float *bp = bias ? bias + (m_base + r) * p.bias_sm + (p.bias_sn ? n : 0) : nullptr;
       const int64_t b_step = (int64_t)rows_pass * p.bias_sm;
-      const bool act_here = !PROJ || n >= x.act_from;
+      const int act_at = PROJ ? x.act_from - (int)n : 0;  // the first of these four columns that has the activation
       // The rotary embedding pairs feature d with d +- rot / 2: the thread rot / 8 quads away in the same row, which is
       // in this warp because rot / 4 quads are an aligned power of two.
       const int feature = PROJ && x.rot && n < x.rot_cols ? (int)n % x.rot_head : 1 << 30;
@@ -170,9 +170,9 @@ template <int ACT, int NT, bool COL_SCALE, bool PROJ = false> struct TileEpilogu
               v[j] = __fadd_rn(__fmul_rn(v[j], co[j]), __fmul_rn(sgn * other, si[j]));
             }
           }
-          if (act_here) {
+          if (act_at < 4) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = act_op<ACT>(e, v[j]);
+            for (int j = 0; j < 4; ++j) v[j] = j >= act_at ? act_op<ACT>(e, v[j]) : v[j];
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) v[j] += rv[j];

@@ -109,6 +109,26 @@ def test_rotation_with_splits_that_are_no_power_of_two(split):
     assert close(c.numpy(), ref)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("act_from", [1, 50, 63, 95])
+@pytest.mark.parametrize("tile,split,residual", [(32, 1, False), (48, 1, False), (64, 2, False), (96, 1, True)])
+def test_activation_from_any_column(act_from, tile, split, residual):
+    """Column groups of four that the activation begins inside, in either ending of the kernel."""
+    rng = np.random.default_rng(act_from + tile)
+    m, n, k = 129, 96, 128
+    a, b, bias, res = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (k, n), (n,), (m, n)))
+    ref = a.astype(np.float64) @ b + bias
+    f = ref[:, act_from:]
+    ref[:, act_from:] = f * (erf(f / np.sqrt(2.0)) + 1) * 0.5
+    if residual:
+        ref += res
+    db, c = DT.from_numpy(b), DT((m, n), np.float32)
+    p, blob = params(db, True, act=cabi.ACT_GELU_ERF, tile=tile, split=split, act_from=act_from)
+    cabi.gemm(DT.from_numpy(a), db, c, DT.from_numpy(bias), DT.from_numpy(res) if residual else None, p)
+    cabi.check_device()
+    assert close(c.numpy(), ref)
+
+
 def refused(a, b, c, **kw):
     p = cabi.gemm_params(act=kw.pop("act", cabi.ACT_NONE))
     for k, v in kw.items():
