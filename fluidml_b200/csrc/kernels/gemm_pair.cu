@@ -500,6 +500,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       atomicOr(a.status, kStatusTimeout);
       *abort_flag = 1;
     }
+    tc_fence_after();  // the accumulator's loads stay behind the wait for the MMAs of the last attempt, in either ending
     if (BULK) {
       // behind the boxes, in what a staged tile's padding would take
       float *cols = reinterpret_cast<float *>(smem + (size_t)BN * kBM * 4);
@@ -510,7 +511,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else {
     // Accumulator row -> staging row; the rings are free (every load has been consumed).  The two
     // sets take alternate groups of 32 columns.
-    tc_fence_after();
     float *dst = staging + (size_t)row * pitch;
     for (int c0 = set * 32; c0 < BN; c0 += 64) {
       float v[32];

@@ -69,3 +69,21 @@ def test_rows_that_are_done_twice():
     cabi.check_device()
     ref = a.astype(np.float64) @ b
     assert (np.abs(c.numpy() - ref) <= 8e-6 * np.abs(ref).max(1, keepdims=True)).all()
+
+
+@pytest.mark.parametrize("m,k,tile", [(128, 1024, 256), (300, 64, 32), (2500, 320, 96)])
+def test_whole_tiles_done_twice(m, k, tile):
+    """Every row outgrows its first block's scale: what is stored waits for the second attempt's products, one k block or many."""
+    rng = np.random.default_rng(m)
+    a, b, bias = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (k, 512), (512,)))
+    a[:, 33:] *= 2e5
+    db = DT.from_numpy(b)
+    blob = cabi.gemm_pack(db)
+    c = DT((m, 512), np.float32)
+    p = cabi.gemm_params(act=cabi.ACT_RELU, tile_n=tile, split_k=1)
+    p.b_constant, p.b_packed = 1, blob.ptr
+    cabi.gemm(DT.from_numpy(a), db, c, DT.from_numpy(bias), None, p)
+    cabi.check_device()
+    ref = np.maximum(a.astype(np.float64) @ b + bias, 0)
+    tol = max(8e-6, 3 * k / 16 * 2.0 ** -24 + 2.0 ** -21)  # (longer k: as test_joined_products_gpu.py)
+    assert (np.abs(c.numpy() - ref) <= tol * np.abs(ref).max(1, keepdims=True)).all()
