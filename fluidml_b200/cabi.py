@@ -57,10 +57,11 @@ class ConvParams(ctypes.Structure):
                 ("dilations", ctypes.c_int64 * 2), ("group", ctypes.c_int64),
                 ("act", ctypes.c_int32), ("precision", ctypes.c_int32), ("w_packed", ctypes.c_void_p),
                 ("tile_n", ctypes.c_int32), ("strips", ctypes.c_int32), ("split_k", ctypes.c_int32), ("ctas_per_sm", ctypes.c_int32),
-                ("pointwise_fma", ctypes.c_int32), ("plane_sums", ctypes.c_void_p), ("max_pool", ctypes.c_int32)]
+                ("pointwise_fma", ctypes.c_int32), ("plane_sums", ctypes.c_void_p), ("max_pool", ctypes.c_int32),
+                ("w_constant", ctypes.c_int32)]
 
 
-ABI_VERSION = 2  # FML_ABI_VERSION of the structures above
+ABI_VERSION = 3  # FML_ABI_VERSION of the structures above
 _lib = None
 
 

@@ -911,6 +911,7 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
     p.act = n.act;
     p.precision = options.gemm_precision;
     p.max_pool = n.pooled ? 1 : 0;
+    p.w_constant = 1;
     const char *name = n.kind == Kind::ConvWithPadding ? "ConvWithPaddingKernel" : "ConvWithoutPaddingKernel";
     return std::make_unique<ConvKernel>(name, C(0), n.has_bias, n.has_bias ? C(1) : fml_tensor{}, n.has_in_scale, n.has_residual, p, options.autotune);
   }

@@ -5,7 +5,7 @@
 // SM in five's FMA units -- and the tensor-core kernel spends 8 to 11 us on it (patch, split into pairs, tensor memory,
 // staged epilogue, split-K over a cluster).  Here a CTA owns 32 output channels x PX pixels; both operands are read as
 // they lie (x [IC][pixels], w [IC][OC]: a row of each per input channel), every row of its k range is on its way at once
-// by asynchronous copies, the weights' before the preceding kernel has finished, and a lane multiplies 8 channels x 4
+// by asynchronous copies, constant weights' before the preceding kernel has finished, and a lane multiplies 8 channels x 4
 // pixels in f32x2 pairs (3 shared-memory reads of 16 bytes for 16 instructions).  The eight warps take different pixels,
 // or share the pixels and take WK slices of k, added in slice order through shared memory; a cluster of S CTAs splits k
 // further where the tiles alone leave most SMs idle (7 x 7 maps), its partial tiles added in rank order.
@@ -31,7 +31,7 @@ struct PwArgs {
   float *y;
   int OC, IC, HW, tiles_px, k_per_cta, k_chunk;
   int64_t x_sn, x_sc, y_sn, y_sc, w_sc, scale_sn, scale_sc, bias_stride;
-  int act;
+  int act, w_constant;
 };
 
 __device__ __forceinline__ void cp16_or_zero(unsigned dst, const float *src, bool live) {
@@ -100,8 +100,9 @@ __global__ void __launch_bounds__(kPwThreads, 2) conv_pointwise_kernel(const PwA
 
   const int chunks = (nk + kc - 1) / kc;
   pdl_launch_dependents();
-  if (chunks > 0) load_w(0, 0);  // constants: before the wait
+  if (chunks > 0 && a.w_constant) load_w(0, 0);
   pdl_wait();
+  if (chunks > 0 && !a.w_constant) load_w(0, 0);
   if (chunks > 0) load_x(0, 0);
   commit();
   if (a.scale)
@@ -277,6 +278,7 @@ int launch_pointwise_fma(const fml_tensor *x, const fml_tensor *w, const fml_ten
   a.OC = (int)w->shape[0]; a.IC = (int)w->shape[1]; a.HW = (int)HW;
   a.x_sn = x->stride[0]; a.x_sc = x->stride[1]; a.y_sn = y->stride[0]; a.y_sc = y->stride[1]; a.w_sc = w->stride[1];
   a.act = p->act;
+  a.w_constant = p->w_constant;
   a.k_per_cta = plan.k_per_cta; a.k_chunk = plan.k_chunk;
   const int px = 32 * (8 / plan.wk);
   a.tiles_px = (int)((HW + px - 1) / px);

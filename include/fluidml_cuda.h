@@ -35,7 +35,7 @@ extern "C" {
 /* The parameter structures grow at their ends from one version to the next.  Before its first call a caller compares
  * fml_abi_version() with the FML_ABI_VERSION it was compiled with and goes no further where they differ: the library would
  * read, or a fml_*_default_params write, past the end of a shorter structure.  (1: without that function.) */
-#define FML_ABI_VERSION 2
+#define FML_ABI_VERSION 3
 int fml_abi_version(void);
 
 typedef enum fml_status {
@@ -188,7 +188,8 @@ int fml_sum_of_products(int n, const fml_tensor *const *a, const fml_tensor *con
  *   gate[n, c, 0, 0] = act2(b2[c] + sum_j w2[c, j] * act1(b1[j] + sum_k w1[j, k] * mean(x[n, k, :, :])))
  * x [N, C, H, W] (any strides; dense planes are the fast case), w1 [Cr, C(, 1, 1)], w2 [C, Cr(, 1, 1)],
  * b1 / b2 may be NULL, act1 / act2 from fml_activation (none, relu, tanh, sigmoid, silu).  At most
- * 4096 channels and 512 hidden units (FML_UNSUPPORTED beyond). */
+ * 4096 channels and 512 hidden units (FML_UNSUPPORTED beyond).  Weights and biases are constants: the
+ * kernel reads them before the launch in front of it has finished. */
 int fml_squeeze_excite_gate(const fml_tensor *x, const fml_tensor *w1, const fml_tensor *b1,
                             const fml_tensor *w2, const fml_tensor *b2, int act1, int act2,
                             const fml_tensor *gate, void *stream);
@@ -445,6 +446,9 @@ typedef struct fml_conv_params {
    * leaves the chip.  With packed weights, FML_ACT_RELU, more than one tap, no scale and no residual, where
    * fml_conv_uses_packed says so for these parameters; FML_UNSUPPORTED otherwise. */
   int32_t max_pool;
+  /* Non-zero: w holds weights that no earlier launch on the stream writes.  Kernels may then fetch them before the
+   * preceding kernel has finished. */
+  int32_t w_constant;
 } fml_conv_params;
 
 /* Partial sums per output plane that fml_conv leaves in plane_sums for this layer, 0 when its kernel leaves none.  Pure

@@ -126,3 +126,26 @@ def test_small_images_through_the_executor(image):
     Executor.make_dp_greedy("t").compile(model.to_bytes()).invoke({**x, **out})
     for k, ref in orc.run_model(model, x, acc64=True).items():
         assert np.abs(out[k] - ref).max() <= 1e-4 * np.abs(ref).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("constant", [0, 1])
+def test_weights_of_an_earlier_launch(constant):
+    """Weights that the launch in front writes are read when it has finished; constant ones may be on their way before."""
+    rng = np.random.default_rng(5)
+    oc, ic, hw = 256, 2048, 4
+    x, bias = rng.standard_normal((1, ic, hw, hw)).astype(np.float32), rng.standard_normal(oc).astype(np.float32)
+    weights = [rng.standard_normal((ic, oc)).astype(np.float32) for _ in range(2)]
+    dx, db, dy = DT.from_numpy(x), DT.from_numpy(bias), DT((1, oc, hw, hw), np.float32)
+    sources = [DT.from_numpy(np.ascontiguousarray(w.T)) for w in weights]  # (a transposing copy)
+    dw = DT.from_numpy(weights[0])
+    w4 = dw.view((oc, ic, 1, 1), [1, oc, 1, 1], 0)
+    p = params(cabi.ACT_NONE, 0, 0)
+    p.w_constant = constant
+    for i in range(8):
+        w = weights[i % 2 if not constant else 0]
+        if not constant:
+            cabi.copy_strided(sources[i % 2].view((ic, oc), [1, ic], 0), dw)
+        cabi.check(cabi.lib().fml_conv(_ref(dx), _ref(w4), _ref(db), _ref(dy), ctypes.byref(p), None))
+        cabi.check_device()
+        check(dy.numpy(), x, w.T[:, :, None, None], bias, None, None, cabi.ACT_NONE)
