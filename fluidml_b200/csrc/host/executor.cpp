@@ -199,11 +199,11 @@ private:
     }
   };
 
-  // (j2: the fusion passes that join products and order layers by rows name other nodes and tensors; a file from before them is a miss)
+  // (j3: the fusion passes that share LayerNorms, join products and order layers by rows name other nodes and tensors; a file from before them is a miss)
   std::string PlanCachePath() const {
     if (options_.plan_cache.empty() || model_hash_ == 0) return std::string();
     char buf[160];
-    snprintf(buf, sizeof(buf), "/%016llx-%s-%s-p%d-f%d-c%d-a%d-t%d-r%d-j2.plan", (unsigned long long)model_hash_,
+    snprintf(buf, sizeof(buf), "/%016llx-%s-%s-p%d-f%d-c%d-a%d-t%d-r%d-j3.plan", (unsigned long long)model_hash_,
              layout_ == LayoutMode::kDP ? "dp" : "plain", plan_ == MemoryPlanKind::kGreedy ? "greedy" : "linear",
              options_.gemm_precision, options_.fusion ? 1 : 0, options_.dp_constant_cost ? 1 : 0, (int)options_.alignment,
              options_.autotune ? 1 : 0, options_.resident ? 1 : 0);

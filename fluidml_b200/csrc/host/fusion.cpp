@@ -723,9 +723,48 @@ bool FuseRotaryIntoGemm(Rewriter &rw, const NodePtr &rot) {
   return true;
 }
 
+// Gains that LayerNorms of one tensor may share: powers of two near the geometric mean of theirs, feature by feature.  What is
+// left of a norm's own, the factor of its products' weights, must not lie more than 12 times below its root mean square
+// anywhere: else false.
+//
+// Why not 1: a row enters the products with one scale, and what lies far below the row's largest keeps an absolute error
+// only.  Trained norms hold down the features that grow by orders of magnitude; without their gains such a feature sets the
+// scale of all others.  Relative error (2-norm, operands split as the kernel splits them, exact sums, 64 x 1024 x 64) of
+// separate norms / a shared one without gains / with these, two features of the row 10^4 times the others: 7e-8 / 1.8e-6 /
+// 8e-8 with both gains 2^-10 there; 10^6 times, both 2^-17: 8e-8 / 1.8e-4 / 8e-8.  Where one norm holds down what the other
+// lets through, half of the difference (in bits) stays: 10^6 times, 2^-4 against 1 (a factor 4): 6e-8 / 6e-7 / 1.5e-7; 2^-8
+// (16): 6e-8 / 9e-6 / 6e-7.
+bool SharedGains(const std::vector<NodePtr> &norms, int64_t K, std::vector<float> *shared, std::vector<std::vector<uint8_t>> *own) {
+  auto gain = [&](const NodePtr &n, int64_t k) { return reinterpret_cast<const float *>(n->consts[0]->constant->Bytes().data())[k]; };
+  shared->resize((size_t)K);
+  for (int64_t k = 0; k < K; ++k) {
+    double bits = 0.0;
+    for (const NodePtr &n : norms) {
+      const float g = std::fabs(gain(n, k));
+      if (!(g >= 0x1p-60f && g <= 0x1p60f)) return false;
+      bits += std::log2((double)g);
+    }
+    (*shared)[k] = std::ldexp(1.0f, (int)std::lround(bits / (double)norms.size()));
+  }
+  own->clear();
+  for (const NodePtr &n : norms) {
+    std::vector<uint8_t> left((size_t)K * 4);
+    float *l = reinterpret_cast<float *>(left.data());
+    double least = 1e300, squares = 0.0;
+    for (int64_t k = 0; k < K; ++k) {
+      l[k] = gain(n, k) / (*shared)[k];  // (exact)
+      least = std::min(least, (double)std::fabs(l[k]));
+      squares += (double)l[k] * (double)l[k];
+    }
+    if (least * 12.0 < std::sqrt(squares / (double)K)) return false;
+    own->push_back(std::move(left));
+  }
+  return true;
+}
+
 // ---- LayerNorms of one tensor that feed products only (the two halves of a parallel-residual block): scale and
-// shift move into the products, (x^ g + b) W + c = x^ (g W) + (b W + c), worked out in 64 bits, and one LayerNorm
-// without them serves all.  Its readers are then siblings and merge.
+// shift move into the products, (x^ g + b) W + c = (x^ s) (g / s W) + (b W + c), worked out in 64 bits, and one LayerNorm with
+// the gains s and no shift serves all.  Its readers are then siblings and merge.
 bool FoldSharedLayerNorms(Rewriter &rw) {
   for (const NodePtr &first : rw.f.nodes) {
     if (first->kind != Kind::LayerNormalizationConstantScaleBias || first->inputs.size() != 1) continue;
@@ -749,9 +788,12 @@ bool FoldSharedLayerNorms(Rewriter &rw) {
     }
     if (norms.size() < 2) continue;
     const int64_t K = shape[last];
-    std::vector<uint8_t> ones((size_t)K * 4), zeros((size_t)K * 4);
-    for (int64_t k = 0; k < K; ++k) reinterpret_cast<float *>(ones.data())[k] = 1.0f;
-    for (const NodePtr &n : norms) {
+    std::vector<float> shared;
+    std::vector<std::vector<uint8_t>> own;
+    if (!SharedGains(norms, K, &shared, &own)) continue;
+    for (size_t i = 0; i < norms.size(); ++i) {
+      const NodePtr &n = norms[i];
+      const auto factors = std::make_shared<Tensor>(n->consts[0]->meta, std::move(own[i]));
       const float *b = reinterpret_cast<const float *>(n->consts[1]->constant->Bytes().data());
       for (const NodePtr &r : rw.consumers[n->output.get()]) {
         const int64_t N = r->consts[0]->meta.GetShape()[1];
@@ -764,7 +806,7 @@ bool FoldSharedLayerNorms(Rewriter &rw) {
         for (int64_t k = 0; k < K; ++k)
           for (int64_t j = 0; j < N; ++j) shift[j] += (double)b[k] * (double)w[k * N + j];
         for (int64_t j = 0; j < N; ++j) co[j] = (float)shift[j];
-        r->consts[0] = MakeConstant(rw.f, r->name + "_normed.w", {K, N}, {{r->consts[0]->constant, 0, 0, n->consts[0]->constant}});
+        r->consts[0] = MakeConstant(rw.f, r->name + "_normed.w", {K, N}, {{r->consts[0]->constant, 0, 0, factors}});
         const RegionPtr nc = MakeConstant(rw.f, r->name + "_normed.b", {N}, std::move(cb));
         if (r->has_bias) r->consts[1] = nc;
         else r->consts.insert(r->consts.begin() + 1, nc);
@@ -773,8 +815,10 @@ bool FoldSharedLayerNorms(Rewriter &rw) {
       }
       if (n != norms[0]) rw.Kill(n);
     }
-    norms[0]->consts = {MakeConstant(rw.f, norms[0]->name + "_plain.g", {K}, std::move(ones)),
-                        MakeConstant(rw.f, norms[0]->name + "_plain.b", {K}, std::move(zeros))};
+    std::vector<uint8_t> gains((size_t)K * 4), zeros((size_t)K * 4);
+    memcpy(gains.data(), shared.data(), gains.size());
+    norms[0]->consts = {MakeConstant(rw.f, norms[0]->name + "_shared.g", {K}, std::move(gains)),
+                        MakeConstant(rw.f, norms[0]->name + "_shared.b", {K}, std::move(zeros))};
     rw.Commit();
     return true;
   }
@@ -803,25 +847,25 @@ void JoinWeights(flow::Flow &f, const NodePtr &into, const NodePtr &top, const N
 // meet weights like the others': what it costs, it costs a part of the sum that is small.  A small A2 against a large
 // column of W2 (or A1, W1) is not: with halves that contribute alike, the joined product's relative error (2-norm, operands
 // split as the kernel splits them, exact sums) against the separate ones' is 7.7e-8 / 7.7e-8 at weights 4 times apart,
-// 8.9e-8 / 7.6e-8 at 16, 2.0e-7 at 64, 1.2e-5 at 4096, 3e-3 at 2^20.  So the largest weights of every column have to be
-// within a factor of 4; blocks of which that does not hold stay two launches.
+// 8.9e-8 / 7.6e-8 at 16, 2.0e-7 at 64, 1.2e-5 at 4096, 3e-3 at 2^20.  An element's absolute error goes into a column by the
+// column's root mean square, so these have to be within a factor of 4, column by column; blocks of which that does not
+// hold stay two launches.  (The columns' scales do no harm: what is below them keeps 2^-39 of the largest.)
 bool AlikeByColumns(const RegionPtr &a, const RegionPtr &b) {
   const int64_t N = a->meta.GetShape()[1];
-  std::vector<float> most[2];
+  std::vector<double> mean[2];
   for (int i = 0; i < 2; ++i) {
     const RegionPtr &w = i ? b : a;
-    most[i].assign((size_t)N, 0.0f);
+    const int64_t K = w->meta.GetShape()[0];
+    mean[i].assign((size_t)N, 0.0);
     std::vector<float> v((size_t)N);
-    for (int64_t k = 0; k < w->meta.GetShape()[0]; ++k) {
+    for (int64_t k = 0; k < K; ++k) {
       w->constant->WriteRow(k, v.data());
-      for (int64_t j = 0; j < N; ++j) {
-        const float m = std::fabs(v[j]);
-        most[i][j] = m > most[i][j] ? m : most[i][j];
-      }
+      for (int64_t j = 0; j < N; ++j) mean[i][j] += (double)v[j] * (double)v[j];
     }
+    for (int64_t j = 0; j < N; ++j) mean[i][j] /= (double)K;
   }
-  for (int64_t j = 0; j < N; ++j)
-    if (!(most[0][j] <= 4.0f * most[1][j] && most[1][j] <= 4.0f * most[0][j])) return false;
+  for (int64_t j = 0; j < N; ++j)  // (squares)
+    if (!(mean[0][j] <= 16.0 * mean[1][j] && mean[1][j] <= 16.0 * mean[0][j])) return false;
   return true;
 }
 

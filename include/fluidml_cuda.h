@@ -357,7 +357,7 @@ typedef struct fml_gemm_params {
    * dim).  No activation, divisor, alpha or beta.  What the packed path does not take in one launch runs as
    * two or more products (act_from, a2) or as a product and a rotation in place.  With packed B a row of [A | A2] has
    * one power-of-two scale and a column of B another, as with any A: halves whose weights differ in magnitude
-   * (the largest of a column by more than 4) are more exact as two products. */
+   * (a column's root mean square by more than 4) are more exact as two products. */
   fml_tensor a2;
 } fml_gemm_params;
 

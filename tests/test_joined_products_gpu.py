@@ -276,3 +276,48 @@ def test_halves_that_differ_in_magnitude(apart, top):
     Executor.make_dp_greedy("t").compile(model.to_bytes()).invoke({**feeds, **out})
     steps = 3 * (256 + 512) // 16
     assert (np.abs(out["y"] - ref) <= (2.0 ** -21 + (steps + 2) * 2.0 ** -23) * size).all()
+
+
+def two_norms(grow, gains, rows=64, k=128, n=64):
+    """ln1(x) W1 and ln2(x) W2 where two features of x, of opposite sign, are `grow` times the others and the norms' gains there as given."""
+    rng = np.random.default_rng(3)
+    f32 = lambda *s: rng.standard_normal(s).astype(np.float32)
+    x = np.round(f32(rows, k) * 8)  # (whole numbers below 2^24: their sum, hence the mean, is exact)
+    x[:, 5] = np.float32(grow) * (1 + np.minimum(np.abs(x[:, 5]), 8))
+    x[:, 6] = -x[:, 5]
+    g = models.GraphBuilder("norms")
+    xin, ref, wide = g.input("x", FLOAT, x.shape), [], x.astype(np.float64)
+    normed = (wide - wide.mean(1, keepdims=True)) / np.sqrt(wide.var(1, keepdims=True) + 1e-5)
+    for i in (1, 2):
+        scale = np.exp(f32(k) * 0.3).astype(np.float32)
+        scale[5:7] = gains[i - 1]
+        w, shift = f32(k, n), f32(k)
+        h = g.layernorm(xin, g.const(f"g{i}", scale), g.const(f"b{i}", np.float32(1e-6) * shift), -1, 1e-5)
+        g.add(g.const(f"c{i}", np.float32(1e-5) * shift[:n]), g.matmul(h, g.const(f"w{i}", w)), out=f"y{i}")
+        g.output(f"y{i}")
+        ref.append((normed * scale + 1e-6 * shift.astype(np.float64)) @ w + 1e-5 * shift[:n].astype(np.float64))
+    return g.finish(), {"x": x}, ref
+
+
+def norms(model):
+    return [n["kind"] for n in Executor.make_plain_greedy("t").plan(model.to_bytes())["sequence"]].count("LayerNormalizationConstantScaleBias")
+
+
+def test_norms_are_shared_where_their_gains_are_alike():
+    for gains in ((1, 1), (2.0 ** -17, 2.0 ** -17), (0.25, 1), (-1, 1), (2.0 ** -10, 2.0 ** -13)):
+        assert norms(two_norms(1, gains)[0]) == 1
+    for gains in ((2.0 ** -17, 1), (0, 1), (1, 2.0 ** -9)):
+        assert norms(two_norms(1, gains)[0]) == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gains", [(1, 1), (2.0 ** -17, 2.0 ** -17), (2.0 ** -17, 1), (2.0 ** -16, 2.0 ** -18)])
+@pytest.mark.parametrize("grow", [1.0, 2.0 ** 14, 2.0 ** 20])
+def test_norms_that_hold_features_down(grow, gains):
+    """Each output by its own 2-norm: x - mean (the grown features cancel in it), its factor 1 / deviation and the gain round
+    three times, the operands' halves twice more, 2^-22 together at most; 24 accumulator steps cut 2^-24 each on average."""
+    model, feeds, ref = two_norms(grow, gains)
+    out = {f"y{i}": np.zeros(r.shape, np.float32) for i, r in zip((1, 2), ref)}
+    Executor.make_dp_greedy("t").compile(model.to_bytes()).invoke({**feeds, **out})
+    for i, r in zip((1, 2), ref):
+        assert np.linalg.norm(out[f"y{i}"] - r) <= (2.0 ** -22 + 24 * 2.0 ** -24) * np.linalg.norm(r)
