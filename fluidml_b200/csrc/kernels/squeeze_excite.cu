@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kSeThreads) squeeze_excite_gate_kernel(const S
     for (int c = threadIdx.x; c < a.C * ims; c += kSeThreads) {  // images lie side by side
       float t = 0.0f;
 #pragma unroll 4
-      for (int q = 0; q < a.sum_parts; ++q) t += sn[c * a.sum_parts + q];
+      for (int q = 0; q < a.sum_parts; ++q) t += sn[(int64_t)c * a.sum_parts + q];
       mean_s[c] = t / (float)HW;
     }
   }
