@@ -12,7 +12,7 @@ namespace fml {
 // once, so the cost of a phase is largely the instruction fetch of its (cold) code, and a
 // compact, straight-line epilogue matters more than a branch-free one.
 // erf by Abramowitz & Stegun 7.1.26: erf(x) = 1 - P(t) exp(-x^2) with t = 1 / (1 + 0.3275911 x), x >= 0, the formula itself
-// within 1.5e-7.  With y = sqrt(log2 e) x both pieces come from one product: exp(-x^2) = 2^(-y^2), for PTX's ex2.approx (2^-22
+// within 1.5e-7.  Both pieces come from y = sqrt(log2 e) x, which is what is passed: exp(-x^2) = 2^(-y^2), for PTX's ex2.approx (2^-22
 // of the result; it flushes what is below 2^-126, where x is beyond 9 and erf is 1), and t = 1 / (1 + (0.3275911 / sqrt(log2 e)) y)
 // for its rcp.approx (1 ulp; the argument is at least 1).  In fp32 arithmetic the absolute error is about 6e-7, most of it
 // the cancellation in 1 - P exp(-x^2) near 0 (tests/test_erf_formula_cpu.py restates it on the host and
@@ -20,20 +20,21 @@ namespace fml {
 // product it is applied to.
 // The exact erff is ~45 dependent instructions per element; with one epilogue warp per scheduler that was 35 us of a
 // 134 us FFN launch at 2048 rows (4096 columns each).
-__device__ __forceinline__ float erf_fast(float x) {
-  const float y = fabsf(x) * 1.2011224087864498f;  // sqrt(log2 e)
+constexpr float kSqrtLog2e = 1.2011224087864498f;
+__device__ __forceinline__ float erf_fast(float x_scaled) {
+  const float y = fabsf(x_scaled);
   float t;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.27273748f, y, 1.0f)));
   float p = fmaf(1.061405429f, t, -1.453152027f);
   p = fmaf(p, t, 1.421413741f);
   p = fmaf(p, t, -0.284496736f);
   p = fmaf(p, t, 0.254829592f);
-  return copysignf(fmaf(-p * t, ex2_approx(-y * y), 1.0f), x);
+  return copysignf(fmaf(-p * t, ex2_approx(-y * y), 1.0f), x_scaled);
 }
 
 template <int ACT>
 __device__ __forceinline__ float act_op(const GemmEpilogue &e, float v) {
-  if (ACT == FML_ACT_GELU_ERF) return v * (erf_fast(v * __frcp_rn(e.c0)) + e.c1) * e.c2;  // (the reciprocal is loop-invariant)
+  if (ACT == FML_ACT_GELU_ERF) return v * (erf_fast(v * (kSqrtLog2e * __frcp_rn(e.c0))) + e.c1) * e.c2;  // (the factor is loop-invariant)
   if (ACT == FML_ACT_RELU) return fmaxf(v, 0.0f);
   if (ACT == FML_ACT_TANH) return tanhf(v);
   if (ACT == FML_ACT_SIGMOID) return 1.0f / (1.0f + expf(-v));
