@@ -650,7 +650,8 @@ bool pair_rotates(const GemmProblem &p, const GemmExtras &x, const PairPlan &pla
   if (!pow2 || x.rot < 8 || x.rot > 128 || x.rot_head % x.rot || plan.tile_n % x.rot) return false;
   if (!aligned16(x.rot_cos) || !aligned16(x.rot_sin)) return false;
   // tiles of rotated columns take the epilogue's 16-byte path (TileEpilogue::Where), which a split of 3, 5, 6 or 7 does not
-  if ((plan.split_k & (plan.split_k - 1)) != 0) return false;
+  // -- nor an activation from inside a group of four columns
+  if ((plan.split_k & (plan.split_k - 1)) != 0 || x.act_from % 4 != 0) return false;
   if ((x.rot_cols + plan.tile_n - 1) / plan.tile_n * (int64_t)plan.tile_n > p.N) return false;
   if (p.c_sn != 1 || p.c_sm % 4 || p.c_b0 % 4 || p.c_b1 % 4 || !aligned16(p.c) || p.res) return false;
   return !p.bias || (p.bias_sn == 1 && p.bias_sm % 4 == 0 && p.bias_b0 % 4 == 0 && p.bias_b1 % 4 == 0 && aligned16(p.bias));
