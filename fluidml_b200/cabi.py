@@ -49,7 +49,8 @@ class GemmParams(ctypes.Structure):
                 ("tile_n", ctypes.c_int32), ("b_constant", ctypes.c_int32), ("l2_prefetch", ctypes.c_void_p),
                 ("l2_prefetch_bytes", ctypes.c_uint64), ("b_packed", ctypes.c_void_p), ("ctas_per_sm", ctypes.c_int32),
                 ("act_from", ctypes.c_int32), ("rot", ctypes.c_int32), ("rot_head", ctypes.c_int32), ("rot_cols", ctypes.c_int32),
-                ("rot_len", ctypes.c_int32), ("rot_cos", ctypes.c_void_p), ("rot_sin", ctypes.c_void_p), ("a2", Tensor)]
+                ("rot_len", ctypes.c_int32), ("rot_cos", ctypes.c_void_p), ("rot_sin", ctypes.c_void_p), ("a2", Tensor),
+                ("summed", ctypes.c_int32)]
 
 
 class ConvParams(ctypes.Structure):
@@ -61,7 +62,7 @@ class ConvParams(ctypes.Structure):
                 ("w_constant", ctypes.c_int32)]
 
 
-ABI_VERSION = 3  # FML_ABI_VERSION of the structures above
+ABI_VERSION = 4  # FML_ABI_VERSION of the structures above
 _lib = None
 
 

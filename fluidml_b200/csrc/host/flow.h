@@ -94,6 +94,7 @@ struct Node {
   // columns followed by those of inputs[1].
   int64_t act_from = 0, rot = 0, rot_head = 0, rot_cols = 0, rot_len = 1;
   bool two_a = false;
+  bool summed = false;      // ... which stands for the sum of two products
   int64_t span = 0;  // FusedMulAddChain: a span convolution of that many taps, pads[0] rows of padding in front
   bool b_is_const = false;  // FusedGemm: B is a captured constant (consts[0]) rather than inputs[1]
   // Scratch bytes the REFERENCE kernel of this kind needs (one float per row for Softmax and

@@ -870,7 +870,7 @@ bool AlikeByColumns(const RegionPtr &a, const RegionPtr &b) {
 }
 
 // ---- A1 W1 + (A2 W2 + x) -> [A1 | A2] [W1; W2] + x: one launch, one reduction and one pass over the result for both
-// halves of a parallel-residual block, where their weights are of one magnitude.
+// halves of a parallel-residual block, where their weights are of one magnitude and the rows few enough (fml_gemm_joins_sums).
 bool JoinSummedProducts(Rewriter &rw, const NodePtr &mm) {
   if (!IsJoinable(mm) || mm->act != 0 || mm->rot || !mm->has_residual || mm->inputs.size() != 2) return false;
   const RegionPtr r = mm->inputs[1];
@@ -882,13 +882,14 @@ bool JoinSummedProducts(Rewriter &rw, const NodePtr &mm) {
   const bool swap = mm->consts[0]->meta.GetShape()[0] % 32 != 0;  // k blocks must not straddle the seam
   const NodePtr &top = swap ? g : mm, &bottom = swap ? mm : g;
   if (top->consts[0]->meta.GetShape()[0] % 32 != 0) return false;
-  if (!AlikeByColumns(top->consts[0], bottom->consts[0])) return false;
+  const int64_t N = top->consts[0]->meta.GetShape()[1];
+  if (!fml_gemm_joins_sums((int64_t)mm->output->meta.GetElementsNum() / N, N) || !AlikeByColumns(top->consts[0], bottom->consts[0])) return false;
   std::vector<RegionPtr> inputs = {top->inputs[0], bottom->inputs[0]};
   if (g->has_residual) inputs.push_back(g->inputs[1]);
   JoinWeights(rw.f, mm, top, bottom);
   mm->inputs = inputs;
   mm->has_residual = g->has_residual;
-  mm->two_a = true;
+  mm->two_a = mm->summed = true;
   rw.Kill(g);
   return true;
 }

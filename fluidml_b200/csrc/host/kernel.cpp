@@ -887,6 +887,7 @@ std::unique_ptr<Kernel> SelectKernel(const flow::Node &n, const ConstResolver &r
     if (n.has_mask) { c.has_bias = true; c.bias_is_input = true; }  // a variable addend (attention mask)
     c.has_residual = n.has_residual;
     c.two_a = n.two_a;
+    c.params.summed = n.summed ? 1 : 0;
     c.params.act_from = (int32_t)n.act_from;
     if (n.rot) {
       if (!utils::IsDefaultLayout(n.consts.at(k)->layout) || !utils::IsDefaultLayout(n.consts.at(k + 1)->layout)) throw Error("rotary tables must be row-major");

@@ -225,7 +225,7 @@ static int resolve(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c
     GemmProblem p2;
     const int st = analyse_gemm(a2, &b2, c, bias, res, p2);
     if (st != FML_OK) return st;
-    x.a2 = p2.a; x.a2_sm = p2.a_sm; x.a2_b0 = p2.a_b0; x.a2_b1 = p2.a_b1; x.k1 = k1;
+    x.a2 = p2.a; x.a2_sm = p2.a_sm; x.a2_b0 = p2.a_b0; x.a2_b1 = p2.a_b1; x.k1 = k1; x.summed = gp->summed != 0;
     whole = *a;
     whole.shape[a->rank - 1] = k1 + k2;
     a = &whole;
@@ -359,9 +359,9 @@ extern "C" int fml_gemm(const fml_tensor *a, const fml_tensor *b, const fml_tens
 static std::string tuning_key(int device, const GemmProblem &p, const Choice &ch, const fml_gemm_params &gp, bool bias, bool residual) {
   const bool pair = ch.path == Path::kPair;
   char key[256];
-  snprintf(key, sizeof(key), "%d|%lld,%lld,%lld,%lld,%lld|%d%d%d|%d,%d,%d,%d|%lld,%lld|%d,%d,%lld", device, (long long)p.M, (long long)p.N, (long long)p.K,
+  snprintf(key, sizeof(key), "%d|%lld,%lld,%lld,%lld,%lld|%d%d%d|%d,%d,%d,%d|%lld,%lld|%d,%d,%lld,%d", device, (long long)p.M, (long long)p.N, (long long)p.K,
            (long long)p.nb0, (long long)p.nb1, pair, pair ? 0 : ch.tc.b_mn_major, pair ? 1 : ch.tc.three_pass, gp.act, bias, residual,
-           gp.divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn, ch.x.act_from, ch.x.rot ? ch.x.rot_cols : 0, (long long)ch.x.k1);
+           gp.divisor != 1.0f, (long long)p.c_sm, (long long)p.c_sn, ch.x.act_from, ch.x.rot ? ch.x.rot_cols : 0, (long long)ch.x.k1, ch.x.summed);
   return key;
 }
 
@@ -421,6 +421,7 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
   float best = 1e30f;
   Tiles best_tiles = pair ? Tiles{ch.pair.tile_n, ch.pair.split_k, ch.pair.ctas_per_sm} : Tiles{ch.tc.tile_n, ch.tc.split_k, 0};
   std::vector<Tiles> seen;
+  const bool exact = pair && pair_exact(p, ch.x, ch.pair.split_k, ch.pair.two_accs);  // (the plan without tuning is, if any is)
   for (int tn : tn_opts)
     for (int sk : sk_opts)
       for (int ctas = 1; ctas <= (pair ? 2 : 1); ++ctas) {
@@ -430,6 +431,7 @@ extern "C" int fml_gemm_autotune(const fml_tensor *a, const fml_tensor *b, const
         q.ctas_per_sm = ctas;
         Choice cand;
         if (pair ? !plan_gemm_pair(p, ch.x, q, cand.pair) : !plan_gemm_tc(p, q, cand.tc)) continue;
+        if (pair && exact && !pair_exact(p, ch.x, cand.pair.split_k, cand.pair.two_accs)) continue;
         const Tiles id = pair ? Tiles{cand.pair.tile_n, cand.pair.split_k, cand.pair.ctas_per_sm}
                               : Tiles{cand.tc.tile_n, cand.tc.split_k, 0};
         bool dup = false;

@@ -52,6 +52,7 @@ __device__ __forceinline__ float gemm_epilogue(const GemmEpilogue &e, float acc,
 struct GemmExtras {
   const float *a2 = nullptr;  // columns k1 .. K of A, with strides of their own
   int64_t a2_sm = 0, a2_b0 = 0, a2_b1 = 0, k1 = 0;
+  bool summed = false;        // [A | A2] * B stands for two products: no less exact than they are
   int act_from = 0;           // the activation is applied from this column on
   int rot = 0, rot_head = 0, rot_cols = 0, rot_len = 1;  // rotary embedding of columns below rot_cols
   const float *rot_cos = nullptr, *rot_sin = nullptr;    // [rot_len][rot]
@@ -88,11 +89,13 @@ int launch_gemm_tc(const GemmProblem &p, const GemmEpilogue &e, const TcPlan &pl
 // half-precision-pair path with packed weights (gemm_pair.cu) ------------------------------
 struct PairPlan {
   int tile_n, split_k, stages_a, stages_b, ctas_per_sm;
+  bool two_accs;
   size_t smem_bytes;
 };
 size_t pair_packed_bytes(int64_t K, int64_t N);
 int pair_pack(const float *b, int64_t K, int64_t N, int64_t sk, int64_t sn, void *dst, cudaStream_t s);
 bool plan_gemm_pair(const GemmProblem &p, const GemmExtras &x, const fml_gemm_params &gp, PairPlan &plan);
+bool pair_exact(const GemmProblem &p, const GemmExtras &x, int split, bool two_accs);  // false for joined products that are cut more often than apart
 // Whether this plan's epilogue can apply the rotary embedding (else fml_gemm launches it on its own).
 bool pair_rotates(const GemmProblem &p, const GemmExtras &x, const PairPlan &plan);
 int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const GemmExtras &x, const PairPlan &plan, const void *packed, cudaStream_t s);

@@ -57,7 +57,7 @@ struct PairArgs {
   const char *packed;       // B atoms
   const float *col_scale;   // 2^-s of each column
   int n_pad;                // columns in the packed image (multiple of 16)
-  int tile_n, split_k, stages_a, stages_b;
+  int tile_n, split_k, stages_a, stages_b, two_accs;
   int tiles_m, tiles_n, kb_total, kb_per_split;
   int *status;
 };
@@ -142,7 +142,9 @@ __device__ __forceinline__ void store_tile_bulk(const PairArgs &a, const CUtenso
 // values of an attention block and the first product of a feed-forward layer), with the rotary embedding on the
 // first columns and the activation on the last (TileEpilogue).  kTwoA: A's columns come from two tensors, [A | A2] * B:
 // the sum of two products (both halves of a parallel-residual block) or a concatenation's product, one launch
-// and one reduction for both; k blocks do not straddle the seam (k1 is a multiple of 32).
+// and one reduction for both; k blocks do not straddle the seam (k1 is a multiple of 32).  A sum has a second accumulator where
+// tensor memory has room (two_accs): lo * hi + hi * lo there, 2^-11 of the other's size, whose cuts then come once per
+// sixteen k values instead of three times (pair_exact).
 enum { kPlain = 0, kProj = 1, kTwoA = 2 };
 
 // BULK: store_tile_bulk ends the launch.  (Both endings in one kernel cost its main loop 3 % -- registers.)
@@ -179,7 +181,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int kb0 = min(a.kb_total, split * a.kb_per_split);
   const int kb1 = min(a.kb_total, kb0 + a.kb_per_split);
   const int nkb = kb1 - kb0;
-  const uint32_t a_col0 = ((uint32_t)BN + 31u) & ~31u;
+  const uint32_t acc_cols = ((uint32_t)BN + 31u) & ~31u, small = MODE == kTwoA && a.two_accs ? acc_cols : 0u;  // second accumulator
+  const uint32_t a_col0 = acc_cols + small;
   uint32_t tmem_cols = 32;
   while (tmem_cols < a_col0 + 32u * (uint32_t)a.stages_b) tmem_cols <<= 1;
   // the packed run of this tile in k block kb; the last tile of a ragged N stops at the image's edge
@@ -333,9 +336,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           for (int j = 0; j < kPK / 16; ++j) {
             const uint32_t a_hi = ta + (uint32_t)j * 8u, a_lo = a_hi + 16u;
             const uint64_t db = db0 + (uint32_t)j * 2u, dbl = db + (kAtom >> 4);
-            umma_f16_ts(tmem_base, a_lo, db, idesc, (it == 0 && j == 0) ? 0u : 1u);
-            umma_f16_ts(tmem_base, a_hi, dbl, idesc, 1u);
-            umma_f16_ts(tmem_base, a_hi, db, idesc, 1u);
+            umma_f16_ts(tmem_base + small, a_lo, db, idesc, (it == 0 && j == 0) ? 0u : 1u);
+            umma_f16_ts(tmem_base + small, a_hi, dbl, idesc, 1u);
+            umma_f16_ts(tmem_base, a_hi, db, idesc, MODE == kTwoA && small && it == 0 && j == 0 ? 0u : 1u);
           }
           umma_commit(bar_empty_b + 8u * rb.s);  // B stage and TMEM stage reusable
         }
@@ -516,6 +519,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       float v[32];
       if (ok && nkb > 0) {
         tmem_ld32(lane_addr + (uint32_t)c0, v);
+        if (MODE == kTwoA && small) {
+          float w[32];
+          tmem_ld32(lane_addr + small + (uint32_t)c0, w);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] += w[i];
+        }
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = 0.0f;
@@ -603,8 +612,8 @@ constexpr size_t kSmemHalf = kSmemSm / 2 - 1024;  // what lets two CTAs share an
 // the other set's block is still on its way the parity of the phase before it reads as this set's own -- stale
 // values would be converted and the slot given back a second time.  (B's barriers need no such care from two
 // stages on: MMAs end in order, and a set's previous wait covers the phase before.)
-bool pair_stages(int tile_n, int per, bool two_ctas, int *stages_a, int *stages_b, size_t *smem) {
-  const int acc = (tile_n + 31) / 32 * 32;
+bool pair_stages(int tile_n, int per, bool two_ctas, bool two_accs, int *stages_a, int *stages_b, size_t *smem) {
+  const int acc = (tile_n + 31) / 32 * 32 * (two_accs ? 2 : 1);
   const size_t budget = two_ctas ? kSmemHalf : kSmemCta;
   const int tmem = two_ctas ? 256 : 512;
   int best_a = 0, best_b = 0;
@@ -660,12 +669,42 @@ bool pair_rotates(const GemmProblem &p, const GemmExtras &x, const PairPlan &pla
 // Whether finished tiles may leave by bulk stores (store_tile_bulk): boxes of 32 columns, rows of C that begin and end on
 // 16-byte boundaries, and an epilogue of column scale, per-column bias, rotation by 16 features and activation.
 static bool bulk_stores(const GemmProblem &p, const GemmEpilogue &e, const GemmExtras &x, const PairPlan &plan) {
-  if (plan.split_k != 1 || plan.tile_n % 32 || p.res || e.divisor != 1.0f || e.alpha != 1.0f || (p.bias && e.beta != 1.0f)) return false;
+  if (plan.two_accs || plan.split_k != 1 || plan.tile_n % 32 || p.res || e.divisor != 1.0f || e.alpha != 1.0f || (p.bias && e.beta != 1.0f)) return false;
   // (a bulk store clips at 16-byte steps: with 50 columns it would write zeros into two more)
   if (p.N % 4 || p.c_sn != 1 || p.c_sm <= 0 || p.c_sm % 4 || !aligned16(p.c)) return false;
   if (p.c_b0 < 0 || p.c_b0 % 4 || p.c_b1 < 0 || p.c_b1 % 4 || (p.nb0 > 1 && !p.c_b0) || (p.nb1 > 1 && !p.c_b1)) return false;
   if (p.bias && (p.bias_sm != 0 || p.bias_sn != 1)) return false;
   return !x.rot || (x.rot == 16 && x.rot_head % 16 == 0);
+}
+
+// An accumulator is cut to 24 bits at every instruction, once or (one accumulator for all three products) three times per
+// sixteen k values, and that is nearly all of a long product's error.  Joined products fill the SMs with fewer slices of k than
+// they would apart, and a sum has the k range of both.  So a sum only takes splits that cut no more often than its longer
+// half would be cut alone, in the split that fills the SMs with tiles of 256; products side by side as many slices, up to the four
+// that they mostly have apart, as the SMs hold with tiles of 128, two to an SM.
+// Error (relative 2-norm, rows x (1024 + 4096) x 1024, activations non-negative) and time, best tiles, of two launches / one with
+// one accumulator / as chosen here: 77 rows 1.2e-6 21.1 us / 1.7e-6 14.8 / 6.0e-7 14.9; 308 2.2e-6 29.2 / 1.7e-6 20.6 / 1.2e-6 22.5;
+// 1024 2.3e-6 39.5 / 3.4e-6 29.9 / 2.4e-6 38.0; 2048 4.6e-6 62.5 / 7.1e-6 55.3 / 3.4e-6 61.1 (four slices of tiles of 256, which
+// leave no room for a second accumulator).  Side by side: 77 x 1024 x (3072 + 4096) takes tiles of 64 unsplit or of 128 in four
+// slices within 2 %, and a whole model was off by 4.3e-6 with the former, 1.4e-6 with the latter; 512 rows, which fill the
+// SMs unsplit, would pay 20 % of a pass for two slices (4.1e-6 -> 2.7e-6, 3.9e-6 with all products apart).
+static int fill_slices(int64_t tiles) {
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= kSms) s *= 2;
+  return s;
+}
+static int sum_slices(int64_t M, int64_t N, int64_t batch) { return fill_slices((M + kBM - 1) / kBM * ((N + 255) / 256) * batch); }
+bool pair_exact(const GemmProblem &p, const GemmExtras &x, int split, bool two_accs) {
+  const int64_t batch = p.nb0 * p.nb1, kb = k_blocks(p.K), per = (kb + split - 1) / split;
+  if (x.summed) {
+    const int64_t longer = k_blocks(std::max(x.k1, p.K - x.k1)), s = sum_slices(p.M, p.N, batch);
+    return per * (two_accs ? 1 : 3) <= (longer + s - 1) / s * 3;
+  }
+  if (x.act_from) {
+    const int64_t tiles = (p.M + kBM - 1) / kBM * ((p.N + 127) / 128) * batch, s = std::min(4, fill_slices((tiles + 1) / 2));  // (two CTAs to an SM)
+    return per <= (kb + s - 1) / s;
+  }
+  return true;
 }
 
 bool plan_gemm_pair(const GemmProblem &p, const GemmExtras &x, const fml_gemm_params &gp, PairPlan &plan) {
@@ -704,18 +743,20 @@ bool plan_gemm_pair(const GemmProblem &p, const GemmExtras &x, const fml_gemm_pa
         if (gp.tile_n && gp.ctas_per_sm && gp.ctas_per_sm != two + 1) continue;
         int sa, sb;
         size_t smem;
-        if (!pair_stages(tn, per, two != 0, &sa, &sb, &smem)) continue;
+        const bool accs = x.summed && pair_stages(tn, per, two != 0, true, &sa, &sb, &smem);
+        if (!accs && !pair_stages(tn, per, two != 0, false, &sa, &sb, &smem)) continue;
         const int64_t ctas = tiles_m * ((p.N + tn - 1) / tn) * batch * sk;
         const int slots = (two ? 2 : 1) * kSms * (sk == 8 ? 0.87 : sk == 4 ? 0.97 : 1.0);
         const double waves = (double)((ctas + slots - 1) / slots);
         const double t_kb = (double)(kPairA + tn * kPairB) / 80e3;
         const double t_fixed = 3.0 + (double)kBM * tn / sk * 4.0 / 20e3 + (sk > 1 ? 0.6 : 0.0);
-        const double t = waves * (t_fixed + per * t_kb * (two && ctas > kSms ? 2.0 : 1.0));
+        const double inexact = gp.split_k || pair_exact(p, x, sk, accs) ? 0.0 : 1e9;  // only where there is nothing else
+        const double t = waves * (t_fixed + per * t_kb * (two && ctas > kSms ? 2.0 : 1.0)) + inexact;
         if (t < best) {
           best = t;
           found = true;
           plan.tile_n = tn; plan.split_k = sk; plan.stages_a = sa; plan.stages_b = sb;
-          plan.smem_bytes = smem; plan.ctas_per_sm = two + 1;
+          plan.smem_bytes = smem; plan.ctas_per_sm = two + 1; plan.two_accs = accs;
         }
       }
       if (gp.split_k) break;
@@ -736,6 +777,7 @@ int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const GemmExtr
   a.col_scale = reinterpret_cast<const float *>(a.packed + atoms_bytes(p.K, p.N));
   a.n_pad = n_padded(p.N);
   a.tile_n = plan.tile_n; a.split_k = plan.split_k; a.stages_a = plan.stages_a; a.stages_b = plan.stages_b;
+  a.two_accs = plan.two_accs;
   a.tiles_m = (int)((p.M + kBM - 1) / kBM);
   a.tiles_n = (int)((p.N + plan.tile_n - 1) / plan.tile_n);
   a.kb_total = k_blocks(p.K);
@@ -793,3 +835,7 @@ int launch_gemm_pair(const GemmProblem &p, const GemmEpilogue &e, const GemmExtr
 }
 
 }  // namespace fml
+
+// Declared in fluidml_cuda.h: while the longer product would be split at all (sum_slices).  With more tiles two launches lose
+// nothing and an exact sum does: 4000 x (1024 + 4096) x 1024 116 us, 107 as two.
+extern "C" int fml_gemm_joins_sums(int64_t rows, int64_t n) { return rows >= 1 && n >= 1 && fml::sum_slices(rows, n, 1) > 1 ? 1 : 0; }

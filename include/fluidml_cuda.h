@@ -35,7 +35,7 @@ extern "C" {
 /* The parameter structures grow at their ends from one version to the next.  Before its first call a caller compares
  * fml_abi_version() with the FML_ABI_VERSION it was compiled with and goes no further where they differ: the library would
  * read, or a fml_*_default_params write, past the end of a shorter structure.  (1: without that function.) */
-#define FML_ABI_VERSION 3
+#define FML_ABI_VERSION 4
 int fml_abi_version(void);
 
 typedef enum fml_status {
@@ -359,6 +359,9 @@ typedef struct fml_gemm_params {
    * one power-of-two scale and a column of B another, as with any A: halves whose weights differ in magnitude
    * (a column's root mean square by more than 4) are more exact as two products. */
   fml_tensor a2;
+  /* With a2 and packed B: the call stands for the sum of two products, A * B's upper rows + A2 * B's lower ones, and the tiles
+   * that the library chooses make it no less exact than those (fml_gemm_joins_sums: where that is also faster). */
+  int32_t summed;
 } fml_gemm_params;
 
 /* Packs a constant right-hand side [K, N] (any strides) for fml_gemm_params::b_packed: about 4 bytes
@@ -419,6 +422,9 @@ int fml_gemm_uses_tensor_cores(const fml_tensor *a, const fml_tensor *b, const f
  * of k, and whether a constant B is better stored that way in the first place.  Pure host computation. */
 int fml_gemm_uses_columns(const fml_tensor *a, const fml_tensor *b, const fml_tensor *c, const fml_gemm_params *p, int *uses);
 int fml_gemm_prefers_k_major(int64_t rows, int64_t n, int64_t k);
+/* Whether a sum of two products of `rows` rows and `n` columns is worth one launch (fml_gemm_params::summed).  Pure host
+ * computation. */
+int fml_gemm_joins_sums(int64_t rows, int64_t n);
 
 /* ---------------------------------------------------------------- convolution, pooling
  * ConvWithoutPaddingKernel / ConvWithPaddingKernel (conv.cpp:27-280): NCHW x OIHW, 1-D or

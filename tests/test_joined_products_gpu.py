@@ -321,3 +321,79 @@ def test_norms_that_hold_features_down(grow, gains):
     Executor.make_dp_greedy("t").compile(model.to_bytes()).invoke({**feeds, **out})
     for i, r in zip((1, 2), ref):
         assert np.linalg.norm(out[f"y{i}"] - r) <= (2.0 ** -22 + 24 * 2.0 ** -24) * np.linalg.norm(r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [32, 77, 129, 300])
+@pytest.mark.parametrize("k1,k2", [(32, 32), (64, 20), (512, 2048)])
+@pytest.mark.parametrize("n,tile,split", [(16, 0, 0), (96, 32, 1), (260, 256, 1), (200, 192, 2), (768, 128, 8), (128, 64, 3)])
+def test_sums_of_two_products(m, k1, k2, n, tile, split):
+    """With a second accumulator (tiles up to 192) and without; small and large second parts, rows done twice.  Tolerance of
+    two left-hand sides."""
+    rng = np.random.default_rng(m + k1 + n)
+    a1, a2 = rng.standard_normal((m, k1)).astype(np.float32), rng.standard_normal((m, k2)).astype(np.float32)
+    a2[:: 3] *= 1e-3
+    a2[1:: 4] *= 3e4
+    b, bias, res = (rng.standard_normal(s).astype(np.float32) for s in ((k1 + k2, n), (n,), (m, n)))
+    db, c = DT.from_numpy(b), DT((m, n), np.float32)
+    for residual in (True, False):
+        ref = np.concatenate([a1, a2], 1).astype(np.float64) @ b + bias + (res if residual else 0)
+        p, blob = params(db, True, tile=tile, split=split)
+        d2 = DT.from_numpy(a2)
+        p.a2, p.summed = d2.c(), 1
+        cabi.gemm(DT.from_numpy(a1), db, c, DT.from_numpy(bias), DT.from_numpy(res) if residual else None, p)
+        cabi.check_device()
+        rows = np.abs(ref).max(1, keepdims=True)
+        assert (np.abs(c.numpy() - ref) <= pairs(k1 + k2) * np.maximum(rows, 1.0)).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [40, 300, 1024, 2048])
+def test_a_sum_is_no_less_exact_than_two_products(m):
+    """Activations of one sign, whose sums are cut the most.  Each side with the tiles that tuning finds; two of them may be
+    split differently from run to run, a factor of two in the error at most."""
+    rng = np.random.default_rng(m)
+    k1, k2, n = 512, 2048, 512
+    a1, a2 = rng.standard_normal((m, k1)).astype(np.float32), np.abs(rng.standard_normal((m, k2))).astype(np.float32)
+    b = (rng.standard_normal((k1 + k2, n)) * 0.02).astype(np.float32)
+    ref = np.concatenate([a1, a2], 1).astype(np.float64) @ b
+    d1, d2, db = DT.from_numpy(a1), DT.from_numpy(a2), DT.from_numpy(b)
+
+    def product(a, w, residual=None, **kw):
+        c = DT((m, n), np.float32)
+        p, blob = params(w, True, **kw)
+        cabi.gemm(a, w, c, None, residual, cabi.gemm_autotune(a, w, c, p, None, residual))
+        cabi.check_device()
+        return c
+
+    error = lambda c: np.linalg.norm(c.numpy() - ref) / np.linalg.norm(ref)
+    two = product(d2, DT.from_numpy(b[k1:].copy()), product(d1, DT.from_numpy(b[:k1].copy())))
+    assert error(product(d1, db, a2=d2.c(), summed=1)) <= 2 * error(two)
+
+
+def test_sums_are_joined_while_their_tiles_are_few():
+    few, many = [two_halves(1, 0, rows=r, n=128)[0] for r in (64, 128 * 80)]
+    assert products(few) == 1 and products(many) == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,k", [(40, 1024), (200, 512), (77, 768)])
+def test_projections_side_by_side_are_no_less_exact(m, k):
+    """Rows of one sign, tuned tiles on both sides: as test_a_sum_is_no_less_exact_than_two_products."""
+    rng = np.random.default_rng(m)
+    n1, n2 = 3 * k, 4 * k
+    a, b = np.abs(rng.standard_normal((m, k))).astype(np.float32), (rng.standard_normal((k, n1 + n2)) * 0.02).astype(np.float32)
+    ref = a.astype(np.float64) @ b
+    ref[:, n1:] = ref[:, n1:] * (erf(ref[:, n1:] / np.sqrt(2.0)) + 1) * 0.5
+    da = DT.from_numpy(a)
+
+    def product(w, **kw):
+        dw, c = DT.from_numpy(np.ascontiguousarray(w)), DT((m, w.shape[1]), np.float32)
+        p, blob = params(dw, True, **kw)
+        cabi.gemm(da, dw, c, None, None, cabi.gemm_autotune(da, dw, c, p))
+        cabi.check_device()
+        return c.numpy()
+
+    error = lambda y: np.linalg.norm(y[:, :n1] - ref[:, :n1]) / np.linalg.norm(ref[:, :n1])
+    apart = product(b[:, :n1])
+    assert error(product(b, act=cabi.ACT_GELU_ERF, act_from=n1)) <= 2 * error(apart)
