@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kThreads) attention_flash_kernel(AttnArgs a) {
 //   - 87 KB of shared memory for head size 64 (the partial contexts lie over K) and at most 128 registers: two
 //     CTAs per SM overlap each other's phases where there are many (8 x 6 heads of 128: 384 CTAs).
 // Captured graphs of one call after another, attention_kernel / attention_flash_kernel -> this one, us: 12 heads of
-// 128 x 128 8.4 -> 7.3 (inside a BERT-base pass 10.4 -> 7.2), 36 of 77 9.8 -> 7.0, 48 of 128 22.6 -> 12.6, 16 of 77
+// 128 x 128 8.4 -> 7.3 (inside a BERT-base pass 10.3 -> 8.4), 36 of 77 9.8 -> 7.0, 48 of 128 22.6 -> 12.6, 16 of 77
 // causal 10.5 -> 5.9, 12 of 256 30.2 -> 14.2, 8 of 300 38.7 -> 17.7, 64 of 128 x 32 16.7 -> 10.4, 2 of 16 5.3 -> 3.6.
 // Left of a 7 us launch: 1.4 us to the first scores, 2.0 scores, 1.2 softmax, 1.1 context, 0.6 sum and store.
 constexpr int kRowsKeys = 128;              // keys per chunk
